@@ -6,20 +6,22 @@
 // mini-batches are in flight and one team's barrier latency is covered by the others' memory traffic.
 //
 // Per hop, for the current node list (the seeds of the hop), in the fused kernel:
-//   A  count     k_s = min(deg, fanout) per seed from the degrees cached when the node joined the list (coalesced),
-//                one partial sum per CTA
-//   B  sample    block-CSR offsets by a two-level scan; each seed is served by a group of 8/16/32 lanes that choose
+//   B  sample    block-CSR offsets by a scan over the edge counts of the hop's node tiles, which were added up when the
+//                nodes joined the list; each seed is served by a group of 8/16/32 lanes that choose
 //                the picks (Philox4x32-10; Floyd's algorithm for a k-subset, run by the group in registers), read the
 //                picked sources and insert them into the open-addressing table (64-bit slots {key, value}, atomicCAS
 //                to claim, atomicMin of the edge number to find the first occurrence).  A thread that claims a slot or
 //                lowers its edge number marks its edge "possibly first" and moves one unit of the per-CTA count of
 //                first occurrences from the displaced edge's CTA to its own, so no counting pass is needed
 //   D  rank      scan over the possibly-first edges that still hold their slot -> local id, publish it in the slot,
-//                append the node (and its adjacency offset and degree, for the next hop) to the list
+//                append the node (its slot, and for the next hop its adjacency offset, its degree and min(degree, next
+//                fanout) in its tile's edge count) to the list
 //   E  relabel   replace the slot position kept in the remaining edge entries by the local id
+// Two barriers per hop: after B and after D.  E needs none behind it: it reads slots that hold their final id, and the
+// next hop's inserts touch only empty and pending ones.
 // With FGL_MAP_ARRIVAL_ORDER the claiming thread takes the next id from a warp-aggregated counter in phase B and
-// phase D is skipped.  The drop-in kernels (fgl_sample: phases A + B without a table; fgl_map: explicit edges) keep
-// a counting pass (C) between B and D.
+// phase D is skipped.  The drop-in kernels (fgl_sample: a counting pass A over the seeds, then B without a table;
+// fgl_map: explicit edges) keep a counting pass (C) between B and D.
 //
 // Replaces sample_node_cuda (sample.cu:102-203), transfer_edge_id_cuda (id_map.cu:386-493) and the
 // hashtable of id_map.cu:26-255 / cuda_hashtable.cuh.
@@ -68,6 +70,8 @@ struct KParams {
     int32_t* blk_src[FGL_MAX_HOPS];
     int64_t blk_src_stride[FGL_MAX_HOPS];
     int32_t* out_dst;  // MODE_SAMPLE: global seed id per edge (may be NULL)
+    int32_t* blk_dst[FGL_MAX_HOPS];  // MODE_FUSED, one mini-batch: local destination id per edge (may be NULL)
+    int32_t tile_shift[FGL_MAX_HOPS];  // MODE_FUSED: a hop's node tile has 2^shift nodes
     // MODE_MAP: explicit edges
     int32_t* map_src;
     int32_t* map_dst;
@@ -77,11 +81,14 @@ struct KParams {
     int64_t table_slots;  // per team, power of two
     int32_t table_shift;  // 32 - log2(table_slots)
     unsigned long long* barriers;  // one per team, 16 words apart
-    int32_t* team_sums;            // [n_teams][team_size]: per-CTA edge counts of the hop
-    int32_t* team_cnt;             // [n_teams][team_size]: per-CTA counts of first occurrences (fused kernel)
+    int32_t* team_sums;            // drop-in kernels: per-CTA counts
+    int32_t* tile_sums;            // [n_teams][3][kMaxTiles]: edge counts of the node tiles (hops rotate through three)
+    int32_t* team_cnt;             // [n_teams][3][team_size]: per-CTA counts of first occurrences (likewise)
     long long* node_start;         // [n_teams][deg_stride]: adjacency offset of every node that can still be a seed
     int32_t* node_deg;             // [n_teams][deg_stride]: and its degree
     int64_t deg_stride;
+    int32_t* node_slot;            // [n_teams][slot_stride]: table slot of every node (to empty the table again)
+    int64_t slot_stride;
     int32_t* status;               // [0] first error, [1] abort flag
 };
 
@@ -241,16 +248,21 @@ struct Hop {
     int32_t* counts;       // this mini-batch's counts row
     int32_t* blk_indptr;   // may be NULL (MODE_SAMPLE without CSR output)
     int32_t* blk_src;      // edge array: global ids (MODE_SAMPLE) or local ids / pending entries
-    int32_t* out_dst;      // MODE_SAMPLE only
+    int32_t* out_dst;      // destination of every edge: global seed id (MODE_SAMPLE), local id (fused); may be NULL
     long long* node_start; // fused: adjacency offset and degree of the nodes that can still become seeds
     int32_t* node_deg;
     int64_t deg_cap;
+    int32_t* node_slot;    // fused: table slot of every node
+    int32_t* sums;         // fused: edge counts of this hop's node tiles ...
+    int32_t* next_sums;    // ... and of the next hop's, which this hop's new nodes are added to
+    int tile_shift, next_shift, next_fanout;
     int hop, fanout, n_seeds;
     bool last_hop;
     uint64_t ctr;
 };
 
-constexpr int kMaxTeam = 512;  // CTAs per team (a cooperative grid of 512-thread CTAs has at most a few hundred)
+constexpr int kMaxTiles = 4096;  // node tiles per hop; a thread of a 512-thread CTA scans eight of their counts
+constexpr int kMinTileShift = 3;
 
 struct Smem {
     int scan[40];
@@ -259,7 +271,9 @@ struct Smem {
     long long start[kThreads];
     int deg[kThreads];
     int off[kThreads];
-    int prefix[kMaxTeam + 1];  // fused: first edge of every CTA of the team (the owner of an edge number)
+    int prefix[kMaxTiles + 1];  // fused: first edge of every node tile (offsets, and the owner of an edge number)
+    int tiles_per;              // fused: tiles per CTA of the team
+    int n_tiles;
 };
 
 // Fused kernel, first-occurrence order: an edge entry is a local id (>= 0) or, while the id is pending,
@@ -288,34 +302,42 @@ __device__ __forceinline__ void load_adj(const KParams& p, int v, long long& sta
     deg = d < 0 ? 0 : (d > 0x7fffffffLL ? 0x7fffffff : (int)d);
 }
 
-// The CTA of the team whose edge range holds edge number e (sm.prefix is the exclusive scan of the CTAs' edge counts).
-__device__ __forceinline__ int edge_owner(const Smem& sm, int team_size, int e) {
-    int lo = 0, hi = team_size;  // invariant: prefix[lo] <= e < prefix[hi]
+// The CTA of the team whose edge range holds edge number e (sm.prefix is the exclusive scan of the tiles' edge counts).
+__device__ __forceinline__ int edge_owner(const Smem& sm, int e) {
+    int lo = 0, hi = sm.n_tiles;  // invariant: prefix[lo] <= e < prefix[hi]
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (sm.prefix[mid] <= e) lo = mid; else hi = mid;
     }
-    return lo;
+    return lo / sm.tiles_per;
+}
+
+// A node that joins the list with local id `local`: what the next hop and the final clearing of the table need of it.
+template <typename PtrT>
+__device__ __forceinline__ void note_node(const KParams& p, const Hop& h, int local, int g, uint32_t pos) {
+    __stcg(h.node_slot + local, (int)pos);
+    if (!h.last_hop && (int64_t)local < h.deg_cap) {
+        long long start;
+        int deg;
+        load_adj<PtrT>(p, g, start, deg);
+        __stcg(h.node_start + local, start);
+        __stcg(h.node_deg + local, deg);
+        atomicAdd(h.next_sums + (local >> h.next_shift), min(deg, h.next_fanout));
+    }
 }
 
 // Second half of an insert in arrival-order mode: the claiming thread takes the next local id and publishes it.
 template <typename PtrT>
-__device__ __forceinline__ int arrival_assign(const KParams& p, const Hop& h, const Table& tab, int g, int r) {
+__device__ __forceinline__ int arrival_assign(const KParams& p, const Hop& h, const Table& tab, int32_t* team_cnt, int g, int r) {
     cg::coalesced_group grp = cg::coalesced_threads();  // one atomicAdd per group of claiming lanes
     int base = 0;
-    if (grp.thread_rank() == 0) base = atomicAdd(h.counts + h.hop + 1, (int)grp.size());
+    if (grp.thread_rank() == 0) base = h.n_seeds + atomicAdd(team_cnt, (int)grp.size());
     base = grp.shfl(base, 0);
     const int local = base + (int)grp.thread_rank();
     const uint32_t pos = (uint32_t)~r;
     if ((int64_t)local < h.nodes_cap) {
         h.nodes[local] = g;
-        if (h.node_deg && !h.last_hop && (int64_t)local < h.deg_cap) {
-            long long start;
-            int deg;
-            load_adj<PtrT>(p, g, start, deg);
-            __stcg(h.node_start + local, start);
-            __stcg(h.node_deg + local, deg);
-        }
+        note_node<PtrT>(p, h, local, g, pos);
         atomicExch(tab.slots + pos, ((unsigned long long)(uint32_t)g << 32) | (uint32_t)local);
         return local;
     }
@@ -324,14 +346,14 @@ __device__ __forceinline__ int arrival_assign(const KParams& p, const Hop& h, co
     return 0;
 }
 
-// One sampled edge of the wide-fanout path: picked source `g` of seed `v`, edge number e within the hop.
+// One sampled edge of the wide-fanout path: picked source `g` of destination `v`, edge number e within the hop.
 // first_cnt counts the edges of this thread that may be first occurrences (fused, first-occurrence order).
 template <typename PtrT, int MODE, bool ARRIVAL>
-__device__ __forceinline__ void emit_edge(const KParams& p, const Hop& h, const Table& tab, const Smem& sm, int team_size,
+__device__ __forceinline__ void emit_edge(const KParams& p, const Hop& h, const Table& tab, const Smem& sm,
                                           int32_t* team_cnt, int v, int g, int e, int& first_cnt) {
+    if (h.out_dst) h.out_dst[e] = v;
     if (MODE == MODE_SAMPLE) {
         h.blk_src[e] = g;
-        if (h.out_dst) h.out_dst[e] = v;
         return;
     }
     if (g < 0 || (int64_t)g >= p.n_nodes) {
@@ -342,7 +364,7 @@ __device__ __forceinline__ void emit_edge(const KParams& p, const Hop& h, const 
     if (ARRIVAL) {
         bool created;
         int r = table_insert<true>(tab, (uint32_t)g, (uint32_t)e, p.status, created);
-        if (created) r = arrival_assign<PtrT>(p, h, tab, g, r);
+        if (created) r = arrival_assign<PtrT>(p, h, tab, team_cnt, g, r);
         h.blk_src[e] = r;
     } else {
         bool created;
@@ -351,7 +373,7 @@ __device__ __forceinline__ void emit_edge(const KParams& p, const Hop& h, const 
         if (r < 0 && (created || displaced >= 0)) {
             r = ~((~r) | kTentative);
             ++first_cnt;
-            if (displaced >= 0) atomicAdd(team_cnt + edge_owner(sm, team_size, displaced), -1);
+            if (displaced >= 0) atomicAdd(team_cnt + edge_owner(sm, displaced), -1);
         }
         h.blk_src[e] = r;
     }
@@ -370,7 +392,7 @@ constexpr int kSeedsPerIter = FGL_SM_KS;
 constexpr int kGroupPathMaxFanout = 32;
 
 template <typename PtrT, int MODE, bool ARRIVAL, int G>
-__device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& h, const Table& tab, Smem& sm, int team_size,
+__device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& h, const Table& tab, Smem& sm,
                                                    int32_t* team_cnt, int tile0, int tile_n, int& first_cnt) {
     const bool replace = (p.flags & FGL_SAMPLE_REPLACE) != 0;
     const int fanout = h.fanout;
@@ -426,14 +448,15 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
 #pragma unroll
         for (int q = 0; q < KS; ++q)
             if (has[q]) g[q] = ld_adjacency(p.indices + start[q] + (long long)pk[q]);
+        if (h.out_dst) {
+#pragma unroll
+            for (int q = 0; q < KS; ++q)
+                if (has[q]) h.out_dst[off[q] + gl] = v[q];
+        }
         if (MODE == MODE_SAMPLE) {
 #pragma unroll
-            for (int q = 0; q < KS; ++q) {
-                if (has[q]) {
-                    h.blk_src[off[q] + gl] = g[q];
-                    if (h.out_dst) h.out_dst[off[q] + gl] = v[q];
-                }
-            }
+            for (int q = 0; q < KS; ++q)
+                if (has[q]) h.blk_src[off[q] + gl] = g[q];
         } else {
         // stage 2: first probe of every source
         uint32_t pos[KS];
@@ -484,11 +507,11 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
                 r = table_insert_track(tab, key, (uint32_t)e, (pos[q] + 1) & tab.mask, p.status, created, displaced);
             }
             if (ARRIVAL) {
-                if (created) r = arrival_assign<PtrT>(p, h, tab, g[q], r);
+                if (created) r = arrival_assign<PtrT>(p, h, tab, team_cnt, g[q], r);
             } else if (r < 0 && (created || displaced >= 0)) {
                 r = ~((~r) | kTentative);
                 ++first_cnt;
-                if (displaced >= 0) atomicAdd(team_cnt + edge_owner(sm, team_size, displaced), -1);
+                if (displaced >= 0) atomicAdd(team_cnt + edge_owner(sm, displaced), -1);
             }
             h.blk_src[e] = r;
         }
@@ -498,7 +521,7 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
 
 // Any fanout up to FGL_MAX_FANOUT: one warp per seed, picks in shared memory.
 template <typename PtrT, int MODE, bool ARRIVAL>
-__device__ __forceinline__ void sample_tile_wide(const KParams& p, const Hop& h, const Table& tab, Smem& sm, int team_size,
+__device__ __forceinline__ void sample_tile_wide(const KParams& p, const Hop& h, const Table& tab, Smem& sm,
                                                  int32_t* team_cnt, uint32_t* picks_all, int tile0, int tile_n, int& first_cnt) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool replace = (p.flags & FGL_SAMPLE_REPLACE) != 0;
@@ -509,11 +532,11 @@ __device__ __forceinline__ void sample_tile_wide(const KParams& p, const Hop& h,
         const long long start = sm.start[j];
         if (deg <= fanout) {
             for (int i = lane; i < deg; i += 32)
-                emit_edge<PtrT, MODE, ARRIVAL>(p, h, tab, sm, team_size, team_cnt, v, p.indices[start + i], off + i, first_cnt);
+                emit_edge<PtrT, MODE, ARRIVAL>(p, h, tab, sm, team_cnt, v, p.indices[start + i], off + i, first_cnt);
         } else if (replace) {
             for (int i = lane; i < fanout; i += 32) {
                 const uint32_t r = philox_draw(p.rng_seed, h.ctr, (uint32_t)(tile0 + j), (uint32_t)i);
-                emit_edge<PtrT, MODE, ARRIVAL>(p, h, tab, sm, team_size, team_cnt, v,
+                emit_edge<PtrT, MODE, ARRIVAL>(p, h, tab, sm, team_cnt, v,
                                                ld_adjacency(p.indices + start + (long long)__umulhi(r, (uint32_t)deg)), off + i, first_cnt);
             }
         } else {
@@ -532,7 +555,7 @@ __device__ __forceinline__ void sample_tile_wide(const KParams& p, const Hop& h,
                 __syncwarp();
             }
             for (int i = lane; i < fanout; i += 32)
-                emit_edge<PtrT, MODE, ARRIVAL>(p, h, tab, sm, team_size, team_cnt, v, ld_adjacency(p.indices + start + (long long)picks[i]), off + i,
+                emit_edge<PtrT, MODE, ARRIVAL>(p, h, tab, sm, team_cnt, v, ld_adjacency(p.indices + start + (long long)picks[i]), off + i,
                                                first_cnt);
         }
         __syncwarp();
@@ -564,17 +587,15 @@ __device__ __forceinline__ void phase_count_seeds(const KParams& p, const Hop& h
     if (threadIdx.x == 0) __stcg(team_sums + t.rank, total);
 }
 
-// Phase A of the fused kernel: the same sum from the degrees cached when the nodes joined the list (coalesced);
-// also resets this CTA's count of first occurrences.
-__device__ __forceinline__ void phase_count_cached(const Hop& h, const Team& t, Smem& sm, int32_t* team_sums, int32_t* team_cnt) {
-    int s0, s1;
-    chunk_of(h.n_seeds, t.rank, t.size, s0, s1);
-    int acc = 0;
-    for (int s = s0 + (int)threadIdx.x; s < s1; s += kThreads) acc += min(__ldcg(h.node_deg + s), h.fanout);
-    const int total = block_sum(acc, sm.scan);
-    if (threadIdx.x == 0) {
-        __stcg(team_sums + t.rank, total);
-        __stcg(team_cnt + t.rank, 0);
+// The nodes that are in the list already are destinations of the next hop too: their edges, by tile (eight nodes or
+// more, so eight lanes meet in one addition).
+__device__ __forceinline__ void phase_count_old(const Hop& h, const Team& t) {
+    for (int s0 = t.rank * kThreads; s0 < h.n_seeds; s0 += t.size * kThreads) {
+        const int s = s0 + (int)threadIdx.x;
+        int k = s < h.n_seeds ? min(__ldcg(h.node_deg + s), h.next_fanout) : 0;
+#pragma unroll
+        for (int o = 1; o < (1 << kMinTileShift); o <<= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+        if ((s & ((1 << kMinTileShift) - 1)) == 0 && k > 0) atomicAdd(h.next_sums + (s >> h.next_shift), k);
     }
 }
 
@@ -595,21 +616,40 @@ template <typename PtrT, int MODE, bool ARRIVAL>
 __device__ __forceinline__ void phase_sample(const KParams& p, const Hop& h, const Table& tab, const Team& t,
                                              Smem& sm, uint32_t* picks, const int32_t* team_sums, int32_t* team_cnt, int& e0,
                                              int& e1, int& e_total) {
-    int before, total;
+    int before, total, s0, s1;
     if (MODE == MODE_FUSED) {
-        // the edge ranges of all CTAs of the team (an edge number's owner is looked up when it is displaced)
-        const int x = (int)threadIdx.x < t.size ? __ldcg(team_sums + threadIdx.x) : 0;
-        const int excl = block_excl_scan(x, sm.scan, total);
-        if ((int)threadIdx.x < t.size) sm.prefix[threadIdx.x] = excl;
-        if (threadIdx.x == 0) sm.prefix[t.size] = total;
+        // first edge of every node tile of the hop; the CTAs own runs of tiles
+        constexpr int kPer = kMaxTiles / kThreads;
+        const int n_tiles = (h.n_seeds + (1 << h.tile_shift) - 1) >> h.tile_shift;
+        const int q0 = (int)threadIdx.x * kPer;
+        int c[kPer], mine = 0;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            c[q] = q0 + q < n_tiles ? __ldcg(h.sums + q0 + q) : 0;
+            mine += c[q];
+        }
+        int excl = block_excl_scan(mine, sm.scan, total);
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            if (q0 + q < n_tiles) sm.prefix[q0 + q] = excl;
+            excl += c[q];
+        }
+        const int per = (n_tiles + t.size - 1) / t.size;
+        if (threadIdx.x == 0) {
+            sm.prefix[n_tiles] = total;
+            sm.n_tiles = n_tiles;
+            sm.tiles_per = max(per, 1);
+        }
         __syncthreads();
-        before = sm.prefix[t.rank];
+        const int t0 = min(n_tiles, t.rank * per);
+        before = sm.prefix[t0];
+        s0 = min(h.n_seeds, t0 << h.tile_shift);
+        s1 = min(h.n_seeds, min(n_tiles, t0 + per) << h.tile_shift);
     } else {
         team_prefix(team_sums, t, sm, before, total);
+        chunk_of(h.n_seeds, t.rank, t.size, s0, s1);
     }
     e_total = total;
-    int s0, s1;
-    chunk_of(h.n_seeds, t.rank, t.size, s0, s1);
     if (t.rank == 0 && threadIdx.x == 0) {
         h.counts[8 + h.hop] = total;
         if (h.blk_indptr) h.blk_indptr[h.n_seeds] = total;
@@ -631,7 +671,8 @@ __device__ __forceinline__ void phase_sample(const KParams& p, const Hop& h, con
                 load_adj<PtrT>(p, v, start, deg);
             }
             k = min(deg, h.fanout);
-            sm.v[threadIdx.x] = v;
+            // what goes into out_dst: the seed itself, or its local id (of two equal seeds, the later one's)
+            sm.v[threadIdx.x] = (MODE == MODE_FUSED && h.out_dst) ? (h.hop == 0 && k > 0 ? table_lookup(tab, (uint32_t)v, p.status) : s) : v;
             sm.start[threadIdx.x] = start;
             sm.deg[threadIdx.x] = deg;
         }
@@ -644,13 +685,13 @@ __device__ __forceinline__ void phase_sample(const KParams& p, const Hop& h, con
         __syncthreads();
         const int tile_n = min(kThreads, s1 - tile0);
         if (h.fanout <= 8)
-            sample_tile_groups<PtrT, MODE, ARRIVAL, 8>(p, h, tab, sm, t.size, team_cnt, tile0, tile_n, first_cnt);
+            sample_tile_groups<PtrT, MODE, ARRIVAL, 8>(p, h, tab, sm, team_cnt, tile0, tile_n, first_cnt);
         else if (h.fanout <= 16)
-            sample_tile_groups<PtrT, MODE, ARRIVAL, 16>(p, h, tab, sm, t.size, team_cnt, tile0, tile_n, first_cnt);
+            sample_tile_groups<PtrT, MODE, ARRIVAL, 16>(p, h, tab, sm, team_cnt, tile0, tile_n, first_cnt);
         else if (h.fanout <= kGroupPathMaxFanout)
-            sample_tile_groups<PtrT, MODE, ARRIVAL, 32>(p, h, tab, sm, t.size, team_cnt, tile0, tile_n, first_cnt);
+            sample_tile_groups<PtrT, MODE, ARRIVAL, 32>(p, h, tab, sm, team_cnt, tile0, tile_n, first_cnt);
         else
-            sample_tile_wide<PtrT, MODE, ARRIVAL>(p, h, tab, sm, t.size, team_cnt, picks, tile0, tile_n, first_cnt);
+            sample_tile_wide<PtrT, MODE, ARRIVAL>(p, h, tab, sm, team_cnt, picks, tile0, tile_n, first_cnt);
         running += tile_total;
         __syncthreads();
     }
@@ -715,13 +756,7 @@ __device__ __forceinline__ int phase_rank_tracked(const KParams& p, const Hop& h
                     h.nodes[local] = (int)key;
                     tab.slots[pos] = ((unsigned long long)key << 32) | (uint32_t)local;
                     edges[eb + q] = local;
-                    if (!h.last_hop && (int64_t)local < h.deg_cap) {
-                        long long start;
-                        int deg;
-                        load_adj<PtrT>(p, (int)key, start, deg);
-                        __stcg(h.node_start + local, start);
-                        __stcg(h.node_deg + local, deg);
-                    }
+                    note_node<PtrT>(p, h, local, (int)key, pos);
                 } else {
                     set_status(p.status, FGL_ERR_CAPACITY);
                     tab.slots[pos] = ((unsigned long long)key << 32);
@@ -865,12 +900,15 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
     t.epoch = 0;
     t.bar = p.barriers + (size_t)team_id * 16;
     t.status = p.status;
-    int32_t* team_sums = p.team_sums + (size_t)team_id * p.team_size;
-    int32_t* team_cnt = p.team_cnt + (size_t)team_id * p.team_size;
+    int32_t* tile_sums = MODE == MODE_FUSED ? p.tile_sums + (size_t)team_id * 3 * kMaxTiles : nullptr;
+    int32_t* team_cnt = MODE == MODE_FUSED ? p.team_cnt + (size_t)team_id * 3 * p.team_size : nullptr;
     Table tab;
     tab.slots = p.table + (size_t)team_id * (size_t)p.table_slots;
     tab.mask = (uint32_t)(p.table_slots - 1);
     tab.shift = p.table_shift;
+    // The tile sums and the first-occurrence counts of a hop live in one of three buffers, used in turn over all hops of
+    // all mini-batches: while a hop's phase B reads (and its new nodes add to the next one), the third is zeroed.
+    int turn = 0;
 
     for (int b = team_id; b < p.n_batches; b += p.n_teams) {
         Hop h;
@@ -880,37 +918,39 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
         h.out_dst = p.out_dst;
         h.node_start = nullptr;
         h.node_deg = nullptr;
+        h.node_slot = nullptr;
+        h.sums = h.next_sums = nullptr;
         h.deg_cap = 0;
         int n0 = p.seed_counts ? __ldg(p.seed_counts + b) : p.n_seeds_host;
         n0 = max(0, min(n0, (int)min((int64_t)0x7fffffff, p.seed_stride)));
         const int32_t* seeds = p.seeds + (size_t)b * p.seed_stride;
 
         if (MODE == MODE_FUSED) {
-            // The team's table is empty here: the host cleared it once and every mini-batch clears it again at its
+            // The team's table is empty here: the host cleared it once and every mini-batch empties it again at its
             // end.  Insert the seeds with local id = position; cache their adjacency offsets and degrees.
             h.node_start = p.node_start + (size_t)team_id * p.deg_stride;
             h.node_deg = p.node_deg + (size_t)team_id * p.deg_stride;
+            h.node_slot = p.node_slot + (size_t)team_id * p.slot_stride;
             h.deg_cap = p.deg_stride;
             if (t.rank == 0 && threadIdx.x < FGL_COUNTS_STRIDE) h.counts[threadIdx.x] = threadIdx.x == 0 ? n0 : 0;
-            int s0, s1;
-            chunk_of(n0, t.rank, t.size, s0, s1);
-            for (int s = s0 + (int)threadIdx.x; s < s1; s += kThreads) {
+            int32_t* sums = tile_sums + turn * kMaxTiles;
+            for (int s = t.rank * kThreads + (int)threadIdx.x; s < n0; s += t.size * kThreads) {
                 const int v = seeds[s];
                 h.nodes[s] = v;
                 long long start = 0;
-                int deg = 0;
+                int deg = 0, pos = 0;
                 if (v < 0 || (int64_t)v >= p.n_nodes) {
                     set_status(p.status, FGL_ERR_BOUNDS);
                 } else {
-                    table_insert_seed(tab, (uint32_t)v, (uint32_t)s, p.status);
+                    pos = max(0, table_insert_seed(tab, (uint32_t)v, (uint32_t)s, p.status));
                     load_adj<PtrT>(p, v, start, deg);
                 }
                 __stcg(h.node_start + s, start);
                 __stcg(h.node_deg + s, deg);
+                __stcg(h.node_slot + s, pos);
+                if (deg > 0) atomicAdd(sums + (s >> p.tile_shift[0]), min(deg, p.fanout[0]));
             }
-            // the same CTA (the same thread, even) reads these entries back in phases A and B of the first hop, so no
-            // barrier is needed before them; the barrier after phase A orders the seed inserts before the first
-            // source insert
+            if (!team_barrier(t, &sm.flag)) return;
         } else {
             h.nodes = const_cast<int32_t*>(seeds);  // MODE_SAMPLE reads the seeds in place
         }
@@ -925,36 +965,52 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
             h.blk_indptr = p.blk_indptr[hop] ? p.blk_indptr[hop] + (size_t)b * p.blk_indptr_stride[hop] : nullptr;
             h.blk_src = p.blk_src[hop] + (size_t)b * p.blk_src_stride[hop];
 
-            if (MODE == MODE_FUSED)
-                phase_count_cached(h, t, sm, team_sums, team_cnt);
-            else
-                phase_count_seeds<PtrT>(p, h, t, sm, team_sums);
-            if (MODE == MODE_FUSED && ARRIVAL && t.rank == 0 && threadIdx.x == 0) h.counts[hop + 1] = n_cur;
-            if (!team_barrier(t, &sm.flag)) return;
+            int32_t* cnt = nullptr;
+            if (MODE == MODE_FUSED) {
+                const int next = turn == 2 ? 0 : turn + 1, spare = next == 2 ? 0 : next + 1;
+                h.out_dst = p.blk_dst[hop];
+                h.sums = tile_sums + turn * kMaxTiles;
+                h.next_sums = tile_sums + next * kMaxTiles;
+                h.tile_shift = p.tile_shift[hop];
+                h.next_shift = h.last_hop ? 0 : p.tile_shift[hop + 1];
+                h.next_fanout = h.last_hop ? 0 : p.fanout[hop + 1];
+                cnt = team_cnt + turn * p.team_size;
+                int32_t* zero = tile_sums + spare * kMaxTiles;
+                for (int i = t.rank * kThreads + (int)threadIdx.x; i < kMaxTiles; i += t.size * kThreads) __stcg(zero + i, 0);
+                if (threadIdx.x == 0) __stcg(team_cnt + spare * p.team_size + t.rank, 0);
+                turn = next;
+            } else {
+                phase_count_seeds<PtrT>(p, h, t, sm, p.team_sums);
+                if (!team_barrier(t, &sm.flag)) return;
+            }
 
+            if (MODE == MODE_FUSED && !h.last_hop) phase_count_old(h, t);
             int e0, e1, e_total;
-            phase_sample<PtrT, MODE, ARRIVAL>(p, h, tab, t, sm, picks, team_sums, team_cnt, e0, e1, e_total);
+            phase_sample<PtrT, MODE, ARRIVAL>(p, h, tab, t, sm, picks, p.team_sums, cnt, e0, e1, e_total);
             if (MODE == MODE_SAMPLE) break;
             if (!team_barrier(t, &sm.flag)) return;
 
             if (!ARRIVAL) {
-                n_cur = phase_rank_tracked<PtrT>(p, h, tab, h.blk_src, e0, e1, n_cur, t, sm, team_cnt);
+                n_cur = phase_rank_tracked<PtrT>(p, h, tab, h.blk_src, e0, e1, n_cur, t, sm, cnt);
                 n_cur = (int)min((int64_t)n_cur, h.nodes_cap);
                 if (t.rank == 0 && threadIdx.x == 0) h.counts[hop + 1] = n_cur;
                 if (!team_barrier(t, &sm.flag)) return;
                 phase_relabel_tracked(tab, h.blk_src, e0, e1);
             } else {
-                n_cur = (int)min((int64_t)__ldcg(h.counts + hop + 1), h.nodes_cap);
+                n_cur = (int)min((int64_t)n_cur + __ldcg(cnt), h.nodes_cap);
+                if (t.rank == 0 && threadIdx.x == 0) h.counts[hop + 1] = n_cur;
                 phase_relabel(tab, h.blk_src, e0, e1);
             }
-            // the next hop's phase A only reads the degrees cached before the last barrier; its barrier keeps the
-            // next inserts behind every CTA's relabel reads
         }
         if (MODE == MODE_SAMPLE) break;
-        // Once every CTA has finished reading the table, clear it for the next mini-batch: a coalesced sweep of the
-        // team's (L2-resident) slots.
+        // Once every CTA has finished reading the table, empty it for the next mini-batch: the nodes' slots one by one
+        // while they are few beside the table (a scattered 8-byte store each), else a coalesced sweep over all slots
+        // (a 16-byte store per two).
         if (!team_barrier(t, &sm.flag)) return;
-        {
+        if ((int64_t)n_cur * 4 < p.table_slots) {
+            for (int i = t.rank * kThreads + (int)threadIdx.x; i < n_cur; i += t.size * kThreads)
+                tab.slots[(uint32_t)__ldcg(h.node_slot + i)] = kEmpty;
+        } else {
             const int64_t vecs = p.table_slots / 2;  // two slots per 128-bit store
             uint4* base = reinterpret_cast<uint4*>(tab.slots);
             const uint4 ones = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
@@ -1049,6 +1105,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) map_kernel(const __grid_co
 // ----------------------------------------------------------------------------------------------
 // host side
 // ----------------------------------------------------------------------------------------------
+constexpr int64_t kMaxTableBytes = 512LL << 20;
+
 static int64_t pow2_at_least(int64_t n) {
     int64_t p = 1024;
     while (p < n) p <<= 1;
@@ -1087,26 +1145,46 @@ static int launch_coop(Workspace* ws, K kernel, int grid, size_t dyn_smem, KPara
     return FGL_OK;
 }
 
-// scratch layout: [barriers: n_teams * 16 u64][team_sums: grid i32][team_cnt: grid i32][counts: 16 i32]
-//                 [node_start: n_teams * deg_stride i64][node_deg: n_teams * deg_stride i32]
+// scratch layout of the drop-in kernels: [barrier: 16 u64][team_sums: grid i32][counts: 16 i32]
+// of the fused kernel: [barriers: n_teams * 16 u64][tile_sums: n_teams * 3 * kMaxTiles i32][team_cnt: 3 * grid i32]
+//                      [node_start: n_teams * deg_stride i64][node_deg: n_teams * deg_stride i32]
+//                      [node_slot: n_teams * slot_stride i32]
 // Only the part before node_start is zeroed per call.
-static int64_t sums_bytes(int grid) { return (((int64_t)grid * 4 + 127) / 128) * 128; }
+static int64_t sums_bytes(int64_t words) { return ((words * 4 + 127) / 128) * 128; }
 
-static int64_t scratch_head(int n_teams, int grid) { return (int64_t)n_teams * 128 + 2 * sums_bytes(grid) + 128; }
+static int64_t scratch_head(int grid) { return 128 + sums_bytes(grid) + 128; }
 
-static int64_t scratch_need(int n_teams, int grid, int64_t deg_stride = 0) {
-    return scratch_head(n_teams, grid) + (int64_t)n_teams * deg_stride * 12;
-}
-
-static void place_scratch(Workspace* ws, KParams& kp, int n_teams, int grid, int64_t deg_stride, int32_t** call_counts) {
+static void place_scratch(Workspace* ws, KParams& kp, int grid, int32_t** call_counts) {
     char* base = ws->scratch;
     kp.barriers = (unsigned long long*)base;
-    kp.team_sums = (int32_t*)(base + (size_t)n_teams * 128);
-    kp.team_cnt = (int32_t*)(base + (size_t)n_teams * 128 + sums_bytes(grid));
-    if (call_counts) *call_counts = (int32_t*)(base + scratch_head(n_teams, grid) - 128);
-    kp.node_start = (long long*)(base + scratch_head(n_teams, grid));
-    kp.node_deg = (int32_t*)(base + scratch_head(n_teams, grid) + (size_t)n_teams * deg_stride * 8);
+    kp.team_sums = (int32_t*)(base + 128);
+    *call_counts = (int32_t*)(base + scratch_head(grid) - 128);
+    kp.status = ws->status;
+}
+
+static int64_t fused_head(int n_teams, int grid) {
+    return (int64_t)n_teams * 128 + (int64_t)n_teams * 3 * kMaxTiles * 4 + sums_bytes(3 * (int64_t)grid);
+}
+
+static int64_t fused_need(int n_teams, int grid, int64_t deg_stride, int64_t slot_stride) {
+    return fused_head(n_teams, grid) + (int64_t)n_teams * (deg_stride * 12 + slot_stride * 4);
+}
+
+static void place_fused(Workspace* ws, KParams& kp, int n_teams, int grid, int64_t deg_stride, int64_t slot_stride) {
+    char* base = ws->scratch;
+    kp.barriers = (unsigned long long*)base;
+    base += (size_t)n_teams * 128;
+    kp.tile_sums = (int32_t*)base;
+    base += (size_t)n_teams * 3 * kMaxTiles * 4;
+    kp.team_cnt = (int32_t*)base;
+    base = ws->scratch + fused_head(n_teams, grid);
+    kp.node_start = (long long*)base;
+    base += (size_t)n_teams * deg_stride * 8;
+    kp.node_deg = (int32_t*)base;
+    base += (size_t)n_teams * deg_stride * 4;
+    kp.node_slot = (int32_t*)base;
     kp.deg_stride = deg_stride;
+    kp.slot_stride = slot_stride;
     kp.status = ws->status;
 }
 
@@ -1166,12 +1244,12 @@ int fgl_sample(fgl_ws* ws, const void* indptr, int indptr_is_64, const int32_t* 
     const int lanes = fanout <= 8 ? 8 : (fanout <= 16 ? 16 : 32);
     const int64_t seeds_per_cta = kThreads / lanes;
     int grid = (int)std::max<int64_t>(1, std::min<int64_t>(max_grid, (n_seeds + seeds_per_cta - 1) / seeds_per_cta));
-    rc = ws_ensure(ws, 0, scratch_need(1, grid));
+    rc = ws_ensure(ws, 0, scratch_head(grid));
     if (rc != FGL_OK) return rc;
     KParams kp;
     std::memset(&kp, 0, sizeof(kp));
     int32_t* call_counts = nullptr;
-    place_scratch(ws, kp, 1, grid, 0, &call_counts);
+    place_scratch(ws, kp, grid, &call_counts);
     kp.indptr = indptr;
     kp.indices = indices;
     kp.n_nodes = n_nodes;
@@ -1196,7 +1274,7 @@ int fgl_sample(fgl_ws* ws, const void* indptr, int indptr_is_64, const int32_t* 
     kp.table = nullptr;
     kp.table_slots = 1024;
     kp.table_shift = 22;
-    FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)scratch_head(1, grid), st));
+    FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)scratch_head(grid), st));
     rc = launch_sample_map<MODE_SAMPLE>(ws, kp, indptr_is_64 != 0, false, grid, dyn, st);
     if (rc != FGL_OK) return rc;
     if (n_edges_host) {
@@ -1232,12 +1310,12 @@ int fgl_map(fgl_ws* ws, int32_t* src, int32_t* dst, const int32_t* seeds, int32_
     const int64_t max_keys = (int64_t)n_seeds + n_edges;
     const int64_t slots = pow2_at_least(max_keys + max_keys / 2 + 1);
     if (slots > (1LL << 31)) return FGL_ERR_CAPACITY;
-    rc = ws_ensure(ws, slots, scratch_need(1, grid));
+    rc = ws_ensure(ws, slots, scratch_head(grid));
     if (rc != FGL_OK) return rc;
     KParams kp;
     std::memset(&kp, 0, sizeof(kp));
     int32_t* call_counts = nullptr;
-    place_scratch(ws, kp, 1, grid, 0, &call_counts);
+    place_scratch(ws, kp, grid, &call_counts);
     kp.n_nodes = 0x7fffffff;
     kp.flags = flags;
     kp.n_teams = 1;
@@ -1253,7 +1331,7 @@ int fgl_map(fgl_ws* ws, int32_t* src, int32_t* dst, const int32_t* seeds, int32_
     kp.table = ws->table;
     kp.table_slots = slots;
     kp.table_shift = 32 - log2_of(slots);
-    FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)scratch_head(1, grid), st));
+    FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)scratch_head(grid), st));
     FGL_CUDA_OK(ws, cudaMemsetAsync(ws->table, 0xFF, sizeof(unsigned long long) * (size_t)slots, st));
     ws->table_dirty = true;  // this call leaves its keys in the table
     rc = arrival ? launch_coop(ws, map_kernel<true>, grid, 0, &kp, st) : launch_coop(ws, map_kernel<false>, grid, 0, &kp, st);
@@ -1302,17 +1380,23 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
     int max_grid = 0;
     rc = occupancy_sample_map<MODE_FUSED>(ws, is64, arrival, dyn, &max_grid);
     if (rc != FGL_OK) return rc;
-    int n_teams = a->n_teams > 0 ? a->n_teams : 4;
-    n_teams = std::max(1, std::min(std::min(n_teams, (int)a->n_batches), max_grid));
-    const int team_size = max_grid / n_teams;
-    const int grid = team_size * n_teams;
     // one table per team: sized for the worst case, or by the caller's hint (a smaller table stays in L2;
     // if it fills up the launch reports FGL_ERR_PROBE and the caller retries without a hint)
     int64_t slots = pow2_at_least(cap[a->n_hops] + cap[a->n_hops] / 2 + 1);
     if (a->table_slots_hint > 0) slots = std::min(slots, pow2_at_least(a->table_slots_hint));
     if (slots > (1LL << 29)) return FGL_ERR_CAPACITY;   // pending edge entries keep a slot number in 29 bits
-    if (team_size > kMaxTeam) return FGL_ERR_INVALID;
-    rc = ws_ensure(ws, slots * n_teams, scratch_need(n_teams, grid, deg_stride));
+    // A team per mini-batch of the window, up to 16: the small hops and the barriers of one mini-batch are covered by
+    // the others' traffic.  Beyond four teams the tables together stay below kMaxTableBytes.
+    int n_teams = a->n_teams;
+    if (n_teams <= 0) n_teams = (int)std::max<int64_t>(4, std::min<int64_t>(16, kMaxTableBytes / (slots * 8)));
+    n_teams = std::max(1, std::min(std::min(n_teams, (int)a->n_batches), max_grid));
+    // CTAs per team: two edges per thread at the widest hop's worst case is all a small mini-batch can use
+    int64_t widest = cap[0];
+    for (int h = 0; h < a->n_hops; ++h) widest = std::max(widest, cap[h] * a->fanout[h]);
+    const int team_size = (int)std::max<int64_t>(1, std::min<int64_t>(max_grid / n_teams, (widest + 2 * kThreads - 1) / (2 * kThreads)));
+    const int grid = team_size * n_teams;
+    const int64_t slot_stride = (cap[a->n_hops] + 31) / 32 * 32;
+    rc = ws_ensure(ws, slots * n_teams, fused_need(n_teams, grid, deg_stride, slot_stride));
     if (rc != FGL_OK) return rc;
     if (ws->table_dirty) {
         FGL_CUDA_OK(ws, cudaMemsetAsync(ws->table, 0xFF, sizeof(unsigned long long) * (size_t)ws->table_slots, st));
@@ -1320,7 +1404,7 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
     }
     KParams kp;
     std::memset(&kp, 0, sizeof(kp));
-    place_scratch(ws, kp, n_teams, grid, deg_stride, nullptr);
+    place_fused(ws, kp, n_teams, grid, deg_stride, slot_stride);
     kp.indptr = a->indptr;
     kp.indices = a->indices;
     kp.n_nodes = a->n_nodes;
@@ -1328,6 +1412,8 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
     kp.n_hops = a->n_hops;
     for (int h = 0; h < a->n_hops; ++h) {
         kp.fanout[h] = a->fanout[h];
+        kp.tile_shift[h] = kMinTileShift;
+        while ((cap[h] >> kp.tile_shift[h]) >= kMaxTiles) ++kp.tile_shift[h];
         kp.blk_indptr[h] = a->block_indptr[h];
         kp.blk_indptr_stride[h] = a->block_indptr_stride[h];
         kp.blk_src[h] = a->block_src[h];
@@ -1347,7 +1433,7 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
     kp.table = ws->table;
     kp.table_slots = slots;
     kp.table_shift = 32 - log2_of(slots);
-    FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)scratch_head(n_teams, grid), st));
+    FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)fused_head(n_teams, grid), st));
     return launch_sample_map<MODE_FUSED>(ws, kp, is64, arrival, grid, dyn, st);
 }
 
