@@ -14,8 +14,8 @@
 //                lowers its edge number marks its edge "possibly first" and moves one unit of the per-CTA count of
 //                first occurrences from the displaced edge's CTA to its own, so no counting pass is needed
 //   D  rank      scan over the possibly-first edges that still hold their slot -> local id, publish it in the slot,
-//                append the node (its slot, and for the next hop its adjacency offset, its degree and min(degree, next
-//                fanout) in its tile's edge count) to the list
+//                append the node (and for the next hop its adjacency offset, its degree and min(degree, next fanout)
+//                in its tile's edge count) to the list
 //   E  relabel   replace the slot position kept in the remaining edge entries by the local id
 // Two barriers per hop: after B and after D.  E needs none behind it: it reads slots that hold their final id, and the
 // next hop's inserts touch only empty and pending ones.
@@ -78,8 +78,9 @@ struct KParams {
     int64_t map_edges;
     // workspace
     unsigned long long* table;
-    int64_t table_slots;  // per team, power of two
-    int32_t table_shift;  // 32 - log2(table_slots)
+    int64_t table_slots;  // drop-in map: slots, a power of two
+    int32_t table_shift;  // 32 - log2(buckets)
+    int32_t table_log2_first, table_log2_max;  // fused: smallest and largest table of a team (see hop_table)
     unsigned long long* barriers;  // one per team, 16 words apart
     int32_t* team_sums;            // drop-in kernels: per-CTA counts
     int32_t* tile_sums;            // [n_teams][3][kMaxTiles]: edge counts of the node tiles (hops rotate through three)
@@ -87,25 +88,70 @@ struct KParams {
     long long* node_start;         // [n_teams][deg_stride]: adjacency offset of every node that can still be a seed
     int32_t* node_deg;             // [n_teams][deg_stride]: and its degree
     int64_t deg_stride;
-    int32_t* node_slot;            // [n_teams][slot_stride]: table slot of every node (to empty the table again)
-    int64_t slot_stride;
     int32_t* status;               // [0] first error, [1] abort flag
 };
 
 // ----------------------------------------------------------------------------------------------
 // hashtable: 64-bit slots, key in the high word; low word = local id (bit 31 clear) or, while the
-// key's id is not assigned yet, kPending | (smallest edge number that carries the key)
+// key's id is not assigned yet, kPending | (smallest edge number that carries the key).
+// Four slots make a bucket, one 32-byte sector: a key goes to the first free slot of its bucket (then of the next
+// ones), and a probe reads a bucket at once, so that a second round trip to the L2 is left to the one key in twenty
+// whose bucket is full and not to every neighbour of an occupied slot.
 // ----------------------------------------------------------------------------------------------
+constexpr int kBucket = 4;
+
 struct Table {
     unsigned long long* slots;
-    uint32_t mask;
-    int shift;
+    uint32_t mask;  // buckets - 1
+    int shift;      // 32 - log2(buckets)
 };
 
-__device__ __forceinline__ uint32_t hash_pos(const Table& t, uint32_t key) { return (key * 0x9E3779B1u) >> t.shift; }
+__device__ __forceinline__ uint32_t hash_bucket(const Table& t, uint32_t key) { return (key * 0x9E3779B1u) >> t.shift; }
 
-__device__ __forceinline__ unsigned long long ld_slot(const unsigned long long* p) {
-    return *(const volatile unsigned long long*)p;
+// Read in the L2, where the claims and the ids appear (an old value is as good: a claim or a minimum returns the new one).
+__device__ __forceinline__ unsigned long long ld_slot(const unsigned long long* p) { return __ldcg(p); }
+
+__device__ __forceinline__ void ld_bucket(const Table& t, uint32_t bucket, unsigned long long (&s)[kBucket]) {
+    const unsigned long long* p = t.slots + (size_t)bucket * kBucket;
+    asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(s[0]), "=l"(s[1]) : "l"(p));
+    asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(s[2]), "=l"(s[3]) : "l"(p + 2));
+}
+
+// The same under a predicate, and a predicated claim: without a branch the loads and claims of several keys stay together.
+__device__ __forceinline__ void ld_bucket_if(bool on, const Table& t, uint32_t bucket, unsigned long long (&s)[kBucket]) {
+    const unsigned long long* p = t.slots + (size_t)bucket * kBucket;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
+        "mov.u64 %0, -1;\n\tmov.u64 %1, -1;\n\tmov.u64 %2, -1;\n\tmov.u64 %3, -1;\n\t"
+        "@q ld.global.cg.v2.u64 {%0, %1}, [%4];\n\t@q ld.global.cg.v2.u64 {%2, %3}, [%4 + 16];\n\t}"
+        : "=&l"(s[0]), "=&l"(s[1]), "=&l"(s[2]), "=&l"(s[3])
+        : "l"(p), "r"((int)on));
+}
+
+__device__ __forceinline__ unsigned long long claim_if(bool on, unsigned long long* slot, unsigned long long mine,
+                                                       unsigned long long otherwise) {
+    unsigned long long old;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %4, 0;\n\tmov.u64 %0, %3;\n\t"
+        "@q atom.global.cas.b64 %0, [%1], -1, %2;\n\t}"
+        : "=&l"(old)
+        : "l"(slot), "l"(mine), "l"(otherwise), "r"((int)on)
+        : "memory");
+    return old;
+}
+
+// First slot of a bucket that holds the key or is free (kBucket: neither), and what it holds.
+__device__ __forceinline__ int match_bucket(const unsigned long long (&s)[kBucket], uint32_t key, unsigned long long& cur) {
+    int at = kBucket;
+    cur = kEmpty;
+#pragma unroll
+    for (int i = kBucket - 1; i >= 0; --i) {
+        if (s[i] == kEmpty || (uint32_t)(s[i] >> 32) == key) {
+            at = i;
+            cur = s[i];
+        }
+    }
+    return at;
 }
 
 // A picked neighbour id is read once and never again: a hub's list has thousands of entries and a pick touches one
@@ -120,11 +166,11 @@ __device__ __forceinline__ int ld_adjacency(const int32_t* p) {
     return v;
 }
 
-// A probe sequence gives up after kProbeLimit slots (or the whole table, if smaller): at the load factors the
-// tables are sized for (<= 2/3) clusters are a few slots long, so only a table that is too small for its
+// A probe sequence gives up after kProbeLimit buckets (or the whole table, if smaller): at the load factors the
+// tables are sized for a key is a bucket or two away from its own, so only a table that is too small for its
 // mini-batch gets there.  The failure is recorded and the launch is told to stop at its next team barrier, so an
 // undersized table costs milliseconds, not a scan of the table per key.
-constexpr uint32_t kProbeLimit = 1u << 13;
+constexpr uint32_t kProbeLimit = 1u << 11;
 
 __device__ __forceinline__ uint32_t probe_limit(const Table& t) { return t.mask < kProbeLimit ? t.mask : kProbeLimit; }
 
@@ -133,60 +179,37 @@ __device__ __forceinline__ void probe_failed(int32_t* status) {
     atomicExch(status + 1, 1);
 }
 
-// Seed i gets local id i; of two equal seeds the later position wins, as a sequential run of
-// id_map.cu:259-287 leaves it.
-// Returns the slot position, or -1 when the table is full.
-__device__ __forceinline__ int table_insert_seed(const Table& t, uint32_t key, uint32_t local, int32_t* status) {
-    const unsigned long long mine = ((unsigned long long)key << 32) | local;
-    uint32_t pos = hash_pos(t, key);
-    for (uint32_t probe = 0; probe <= probe_limit(t); ++probe) {
-        unsigned long long cur = ld_slot(t.slots + pos);
-        if (cur == kEmpty) {
-            cur = atomicCAS(t.slots + pos, kEmpty, mine);
-            if (cur == kEmpty) return (int)pos;
+// Slot of a key: the one that holds it (cur = its content), or a free one that this call claimed with `mine` (cur =
+// kEmpty), or -1 when the probes ran out.
+__device__ __forceinline__ int table_find_or_claim(const Table& t, uint32_t key, unsigned long long mine, unsigned long long& cur,
+                                                   int32_t* status) {
+    uint32_t bucket = hash_bucket(t, key);
+    for (uint32_t probe = 0; probe <= probe_limit(t);) {
+        unsigned long long s[kBucket];
+        ld_bucket(t, bucket, s);
+        const int i = match_bucket(s, key, cur);
+        if (i < kBucket) {
+            const int pos = (int)(bucket * kBucket) + i;
+            if (cur == kEmpty) {
+                cur = atomicCAS(t.slots + pos, kEmpty, mine);
+                if (cur != kEmpty && (uint32_t)(cur >> 32) != key) continue;  // another key took the slot: look again
+            }
+            return pos;
         }
-        if ((uint32_t)(cur >> 32) == key) {
-            atomicMax(t.slots + pos, mine);
-            return (int)pos;
-        }
-        pos = (pos + 1) & t.mask;
+        bucket = (bucket + 1) & t.mask;
+        ++probe;
     }
     probe_failed(status);
     return -1;
 }
 
-// Returns the local id (>= 0) if the key already has one, else ~pos of its slot (< 0).  created is set
-// for the thread whose atomicCAS claimed the slot.
-template <bool ARRIVAL>
-__device__ __forceinline__ int table_insert_from(const Table& t, uint32_t key, uint32_t edge, uint32_t pos,
-                                                 int32_t* status, bool& created) {
-    created = false;
-    const unsigned long long mine = ((unsigned long long)key << 32) | (ARRIVAL ? kPending : (kPending | edge));
-    for (uint32_t probe = 0; probe <= probe_limit(t); ++probe) {
-        unsigned long long cur = ld_slot(t.slots + pos);
-        if (cur == kEmpty) {
-            cur = atomicCAS(t.slots + pos, kEmpty, mine);
-            if (cur == kEmpty) {
-                created = true;
-                return ~(int)pos;
-            }
-        }
-        if ((uint32_t)(cur >> 32) == key) {
-            const uint32_t lo = (uint32_t)cur;
-            if (!(lo & kPending)) return (int)lo;
-            if (!ARRIVAL && lo > (kPending | edge)) atomicMin(t.slots + pos, mine);
-            return ~(int)pos;
-        }
-        pos = (pos + 1) & t.mask;
-    }
-    probe_failed(status);
-    return 0;
-}
-
-template <bool ARRIVAL>
-__device__ __forceinline__ int table_insert(const Table& t, uint32_t key, uint32_t edge, int32_t* status,
-                                            bool& created) {
-    return table_insert_from<ARRIVAL>(t, key, edge, hash_pos(t, key), status, created);
+// Seed i gets local id i; of two equal seeds the later position wins, as a sequential run of
+// id_map.cu:259-287 leaves it.
+__device__ __forceinline__ void table_insert_seed(const Table& t, uint32_t key, uint32_t local, int32_t* status) {
+    const unsigned long long mine = ((unsigned long long)key << 32) | local;
+    unsigned long long cur;
+    const int pos = table_find_or_claim(t, key, mine, cur, status);
+    if (pos >= 0 && cur != kEmpty) atomicMax(t.slots + pos, mine);
 }
 
 // Lowers the edge number kept in a pending slot to `edge` if that is smaller.  Returns the edge number that lost
@@ -198,42 +221,34 @@ __device__ __forceinline__ int table_lower_edge(const Table& t, uint32_t pos, ui
     return ((old_lo & kPending) && old_lo > (kPending | edge)) ? (int)(old_lo & ~kPending) : -1;
 }
 
-// table_insert_from for the fused kernel's first-occurrence order: also reports the edge this insert displaced as the
-// key's first occurrence (-1: none).  created or displaced >= 0 means "edge may be the key's first occurrence".
-__device__ __forceinline__ int table_insert_track(const Table& t, uint32_t key, uint32_t edge, uint32_t pos,
-                                                  int32_t* status, bool& created, int& displaced) {
-    created = false;
+// Inserts edge number `edge` of source `key`.  Returns the local id (>= 0) if the key already has one, else ~pos of its
+// slot (< 0).  created is set for the thread that claimed the slot; displaced is the edge that this one displaced as the
+// key's first occurrence (-1: none; never in arrival order).  created or displaced >= 0 means "edge may be the key's
+// first occurrence".
+template <bool ARRIVAL>
+__device__ __forceinline__ int table_insert(const Table& t, uint32_t key, uint32_t edge, int32_t* status, bool& created,
+                                            int& displaced) {
     displaced = -1;
-    const unsigned long long mine = ((unsigned long long)key << 32) | (kPending | edge);
-    for (uint32_t probe = 0; probe <= probe_limit(t); ++probe) {
-        unsigned long long cur = ld_slot(t.slots + pos);
-        if (cur == kEmpty) {
-            cur = atomicCAS(t.slots + pos, kEmpty, mine);
-            if (cur == kEmpty) {
-                created = true;
-                return ~(int)pos;
-            }
-        }
-        if ((uint32_t)(cur >> 32) == key) {
-            const uint32_t lo = (uint32_t)cur;
-            if (!(lo & kPending)) return (int)lo;
-            if (lo > (kPending | edge)) displaced = table_lower_edge(t, pos, key, edge);
-            return ~(int)pos;
-        }
-        pos = (pos + 1) & t.mask;
-    }
-    probe_failed(status);
-    return 0;
+    unsigned long long cur;
+    const int pos = table_find_or_claim(t, key, ((unsigned long long)key << 32) | (ARRIVAL ? kPending : (kPending | edge)), cur, status);
+    created = pos >= 0 && cur == kEmpty;
+    if (pos < 0) return 0;
+    const uint32_t lo = (uint32_t)cur;
+    if (!created && !(lo & kPending)) return (int)lo;
+    if (!ARRIVAL && !created && lo > (kPending | edge)) displaced = table_lower_edge(t, (uint32_t)pos, key, edge);
+    return ~pos;
 }
 
 // Value of a key that must be present (a seed); missing keys report FGL_ERR_BOUNDS and map to 0.
 __device__ __forceinline__ int table_lookup(const Table& t, uint32_t key, int32_t* status) {
-    uint32_t pos = hash_pos(t, key);
+    uint32_t bucket = hash_bucket(t, key);
     for (uint32_t probe = 0; probe <= probe_limit(t); ++probe) {
-        const unsigned long long cur = ld_slot(t.slots + pos);
-        if (cur == kEmpty) break;
-        if ((uint32_t)(cur >> 32) == key) return (int)((uint32_t)cur & ~kPending);
-        pos = (pos + 1) & t.mask;
+        unsigned long long s[kBucket], cur;
+        ld_bucket(t, bucket, s);
+        const int i = match_bucket(s, key, cur);
+        if (i < kBucket && cur == kEmpty) break;
+        if (i < kBucket) return (int)((uint32_t)cur & ~kPending);
+        bucket = (bucket + 1) & t.mask;
     }
     set_status(status, FGL_ERR_BOUNDS);
     return 0;
@@ -252,7 +267,6 @@ struct Hop {
     long long* node_start; // fused: adjacency offset and degree of the nodes that can still become seeds
     int32_t* node_deg;
     int64_t deg_cap;
-    int32_t* node_slot;    // fused: table slot of every node
     int32_t* sums;         // fused: edge counts of this hop's node tiles ...
     int32_t* next_sums;    // ... and of the next hop's, which this hop's new nodes are added to
     int tile_shift, next_shift, next_fanout;
@@ -263,6 +277,7 @@ struct Hop {
 
 constexpr int kMaxTiles = 4096;  // node tiles per hop; a thread of a 512-thread CTA scans eight of their counts
 constexpr int kMinTileShift = 3;
+constexpr int kMaxTeam = 512;    // CTAs per team (a cooperative grid of 512-thread CTAs has at most a few hundred)
 
 struct Smem {
     int scan[40];
@@ -272,8 +287,10 @@ struct Smem {
     int deg[kThreads];
     int off[kThreads];
     int prefix[kMaxTiles + 1];  // fused: first edge of every node tile (offsets, and the owner of an edge number)
-    int tiles_per;              // fused: tiles per CTA of the team
-    int n_tiles;
+    int first_tile[kMaxTeam + 1];  // fused: first node tile of every CTA of the team ...
+    int first_edge[kMaxTeam + 1];  // ... and its first edge
+    int moved[kMaxTeam];        // fused: first occurrences that this CTA's edges took from every CTA of the team
+    float owner_scale;          // fused: CTAs per edge
 };
 
 // Fused kernel, first-occurrence order: an edge entry is a local id (>= 0) or, while the id is pending,
@@ -302,20 +319,32 @@ __device__ __forceinline__ void load_adj(const KParams& p, int v, long long& sta
     deg = d < 0 ? 0 : (d > 0x7fffffffLL ? 0x7fffffff : (int)d);
 }
 
-// The CTA of the team whose edge range holds edge number e (sm.prefix is the exclusive scan of the tiles' edge counts).
-__device__ __forceinline__ int edge_owner(const Smem& sm, int e) {
-    int lo = 0, hi = sm.n_tiles;  // invariant: prefix[lo] <= e < prefix[hi]
-    while (hi - lo > 1) {
+// The CTAs of a team share a hop's node tiles by work, not by number: the nodes at the front of the list are the
+// mini-batch's own seeds and their picks, the ones behind them were reached through an edge and have more edges
+// themselves (with equal numbers of nodes the last CTA took 1.6 times as long as the first).  A tile's position is the
+// edges and nodes before it; CTA r owns the tiles at positions from r / size of the total on.
+__device__ __forceinline__ int first_tile_of(const Smem& sm, int n_tiles, int shift, int rank, int size) {
+    const long long work = sm.prefix[n_tiles] + ((long long)n_tiles << shift);
+    int lo = 0, hi = n_tiles;
+    while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (sm.prefix[mid] <= e) lo = mid; else hi = mid;
+        if ((sm.prefix[mid] + ((long long)mid << shift)) * size >= rank * work) hi = mid; else lo = mid + 1;
     }
-    return lo / sm.tiles_per;
+    return lo;
 }
 
-// A node that joins the list with local id `local`: what the next hop and the final clearing of the table need of it.
+// The CTA of the team whose edge range holds edge number e: the ranges are of nearly equal size, so a guess is at most a
+// step or two away.
+__device__ __forceinline__ int edge_owner(const Smem& sm, int size, int e) {
+    int r = min(size - 1, (int)((float)e * sm.owner_scale));
+    while (e < sm.first_edge[r]) --r;
+    while (e >= sm.first_edge[r + 1]) ++r;
+    return r;
+}
+
+// A node that joins the list with local id `local`: what the next hop needs of it.
 template <typename PtrT>
-__device__ __forceinline__ void note_node(const KParams& p, const Hop& h, int local, int g, uint32_t pos) {
-    __stcg(h.node_slot + local, (int)pos);
+__device__ __forceinline__ void note_node(const KParams& p, const Hop& h, int local, int g) {
     if (!h.last_hop && (int64_t)local < h.deg_cap) {
         long long start;
         int deg;
@@ -337,7 +366,7 @@ __device__ __forceinline__ int arrival_assign(const KParams& p, const Hop& h, co
     const uint32_t pos = (uint32_t)~r;
     if ((int64_t)local < h.nodes_cap) {
         h.nodes[local] = g;
-        note_node<PtrT>(p, h, local, g, pos);
+        note_node<PtrT>(p, h, local, g);
         atomicExch(tab.slots + pos, ((unsigned long long)(uint32_t)g << 32) | (uint32_t)local);
         return local;
     }
@@ -349,7 +378,7 @@ __device__ __forceinline__ int arrival_assign(const KParams& p, const Hop& h, co
 // One sampled edge of the wide-fanout path: picked source `g` of destination `v`, edge number e within the hop.
 // first_cnt counts the edges of this thread that may be first occurrences (fused, first-occurrence order).
 template <typename PtrT, int MODE, bool ARRIVAL>
-__device__ __forceinline__ void emit_edge(const KParams& p, const Hop& h, const Table& tab, const Smem& sm,
+__device__ __forceinline__ void emit_edge(const KParams& p, const Hop& h, const Table& tab, Smem& sm,
                                           int32_t* team_cnt, int v, int g, int e, int& first_cnt) {
     if (h.out_dst) h.out_dst[e] = v;
     if (MODE == MODE_SAMPLE) {
@@ -361,32 +390,45 @@ __device__ __forceinline__ void emit_edge(const KParams& p, const Hop& h, const 
         h.blk_src[e] = 0;
         return;
     }
+    bool created;
+    int displaced;
+    int r = table_insert<ARRIVAL>(tab, (uint32_t)g, (uint32_t)e, p.status, created, displaced);
     if (ARRIVAL) {
-        bool created;
-        int r = table_insert<true>(tab, (uint32_t)g, (uint32_t)e, p.status, created);
         if (created) r = arrival_assign<PtrT>(p, h, tab, team_cnt, g, r);
-        h.blk_src[e] = r;
-    } else {
-        bool created;
-        int displaced;
-        int r = table_insert_track(tab, (uint32_t)g, (uint32_t)e, hash_pos(tab, (uint32_t)g), p.status, created, displaced);
-        if (r < 0 && (created || displaced >= 0)) {
-            r = ~((~r) | kTentative);
-            ++first_cnt;
-            if (displaced >= 0) atomicAdd(team_cnt + edge_owner(sm, displaced), -1);
-        }
-        h.blk_src[e] = r;
+    } else if (r < 0 && (created || displaced >= 0)) {
+        r = ~((~r) | kTentative);
+        ++first_cnt;
+        if (displaced >= 0) atomicSub(&sm.moved[edge_owner(sm, p.team_size, displaced)], 1);
     }
+    h.blk_src[e] = r;
 }
 
 // Fanouts up to 32: a group of G lanes per seed, one lane per pick; a group works on kSeedsPerIter seeds at a time.
-// Stage 0, picks: every lane draws its own Philox word; for a k-subset (Floyd's algorithm: slot i draws t in
-// [0, deg-k+i] and takes deg-k+i instead if an earlier slot already holds t) the group walks the slots in order, lane i
-// settling slot i after a ballot over the earlier lanes -- the picks never leave the registers.  Stages 1-4 issue the
-// dependent loads of the group's seeds stage by stage -- picked sources, first table probes, claims -- so that
-// kSeedsPerIter independent round trips are in flight per lane instead of one chain after the other.
+// Picks: a Philox block holds the words of four consecutive pick slots, so lane 4b + q of a group computes block b of the
+// group's q-th seed and a 4 x 4 transposition inside the quads hands every lane its words.  A k-subset is Floyd's
+// algorithm (slot i draws t in [0, deg-k+i] and takes deg-k+i instead if an earlier slot already holds t) for all slots
+// at once: slot i is replaced if an earlier slot drew the same t -- whoever holds it by then -- or if t is the
+// replacement deg-k+j of an earlier slot j that was replaced itself; the second rule is iterated on ballots until nothing
+// changes, nearly always once.  (Walking the slots one after the other and drawing a block per lane were half of the
+// phase's instructions.)
+// The dependent loads of the group's seeds -- picked sources, buckets, claims -- are issued seed by seed before the
+// first is used, so that kSeedsPerIter round trips are in flight per lane; a key whose bucket is full goes round again
+// together with the others' retries.
+// Element (i, j) of the 4 x 4 words of a quad of lanes (lane i holds row i) goes to (j, i).
+__device__ __forceinline__ void quad_transpose(uint4& w) {
+    const bool odd = threadIdx.x & 1, high = threadIdx.x & 2;
+    uint32_t t = __shfl_xor_sync(0xffffffffu, odd ? w.x : w.y, 1);
+    if (odd) w.x = t; else w.y = t;
+    t = __shfl_xor_sync(0xffffffffu, odd ? w.z : w.w, 1);
+    if (odd) w.z = t; else w.w = t;
+    t = __shfl_xor_sync(0xffffffffu, high ? w.x : w.z, 2);
+    if (high) w.x = t; else w.z = t;
+    t = __shfl_xor_sync(0xffffffffu, high ? w.y : w.w, 2);
+    if (high) w.y = t; else w.w = t;
+}
+
 #ifndef FGL_SM_KS
-#define FGL_SM_KS 4
+#define FGL_SM_KS 2
 #endif
 constexpr int kSeedsPerIter = FGL_SM_KS;
 constexpr int kGroupPathMaxFanout = 32;
@@ -400,13 +442,11 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
     constexpr int KS = kSeedsPerIter;
     const int gid = threadIdx.x / G, gl = threadIdx.x % G;
     const int gbase = (threadIdx.x & 31) & ~(G - 1);  // first lane of the group within its warp
-    const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << G) - 1u);
     for (int it = 0; it * kGroups * KS < tile_n; ++it) {
         int v[KS], off[KS], g[KS], deg[KS];
         long long start[KS];
-        bool has[KS], hub[KS];
-        uint32_t pk[KS], draw[KS];
-        // stage 0: the picks
+        bool has[KS];
+        uint32_t pk[KS];
         bool any_hub = false;
 #pragma unroll
         for (int q = 0; q < KS; ++q) {
@@ -423,24 +463,36 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
                 start[q] = sm.start[j];
             }
             has[q] = gl < min(deg[q], fanout);
-            hub[q] = deg[q] > fanout;
             pk[q] = (uint32_t)gl;
-            draw[q] = 0;
-            if (hub[q] && gl < fanout) {
-                draw[q] = philox_draw(p.rng_seed, h.ctr, (uint32_t)(tile0 + (it * KS + q) * kGroups + gid), (uint32_t)gl);
-                if (replace) pk[q] = __umulhi(draw[q], (uint32_t)deg[q]);
-            }
-            any_hub |= hub[q];
+            any_hub |= deg[q] > fanout;
         }
-        if (!replace && __any_sync(0xffffffffu, any_hub)) {  // warp-uniform
-            for (int i = 0; i < fanout; ++i) {
+        // the picks of the rows that have more edges than the fanout
+        if (__any_sync(0xffffffffu, any_hub)) {  // warp-uniform
+            uint4 w = make_uint4(0, 0, 0, 0);
+            const int wq = gl & 3;
+            if (wq < KS) w = philox_block(p.rng_seed, h.ctr, (uint32_t)(tile0 + (it * KS + wq) * kGroups + gid), (uint32_t)(gl >> 2));
+            quad_transpose(w);
+            const uint32_t draw[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                for (int q = 0; q < KS; ++q) {
-                    const uint32_t ri = __shfl_sync(0xffffffffu, draw[q], gbase + i);
-                    const uint32_t jj = (uint32_t)(deg[q] - fanout + i);
-                    const uint32_t tt = __umulhi(ri, jj + 1u);
-                    const unsigned same = __ballot_sync(0xffffffffu, hub[q] && gl < i && pk[q] == tt);
-                    if (hub[q] && gl == i) pk[q] = ((same >> gbase) & gmask) ? jj : tt;
+            for (int q = 0; q < KS; ++q) {
+                const bool pick = deg[q] > fanout && gl < fanout;
+                if (replace) {
+                    if (pick) pk[q] = __umulhi(draw[q], (uint32_t)deg[q]);
+                } else {
+                    const int floor_q = deg[q] - fanout;
+                    const uint32_t jj = (uint32_t)(floor_q + gl);
+                    const uint32_t tt = __umulhi(draw[q], jj + 1u);
+                    const unsigned same = __match_any_sync(0xffffffffu, pick ? tt : (0x80000000u | (unsigned)gl));
+                    const unsigned earlier = (1u << gl) - 1u;
+                    unsigned replaced = __ballot_sync(0xffffffffu, pick && ((same >> gbase) & earlier)) >> gbase;
+                    const int ref = (int)tt - floor_q;  // the slot whose replacement t is
+                    const bool may = pick && ref >= 0 && ref < gl;
+                    for (;;) {
+                        const unsigned more = __ballot_sync(0xffffffffu, may && !((replaced >> gl) & 1u) && ((replaced >> ref) & 1u));
+                        if (!more) break;
+                        replaced |= more >> gbase;
+                    }
+                    if (pick) pk[q] = ((replaced >> gl) & 1u) ? jj : tt;
                 }
             }
         }
@@ -458,9 +510,10 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
             for (int q = 0; q < KS; ++q)
                 if (has[q]) h.blk_src[off[q] + gl] = g[q];
         } else {
-        // stage 2: first probe of every source
-        uint32_t pos[KS];
-        unsigned long long cur[KS], seen[KS];
+        // stage 2: find or claim the slots.  open: sources that are still looking for theirs
+        uint32_t bucket[KS];
+        int r[KS];
+        unsigned open = 0;
 #pragma unroll
         for (int q = 0; q < KS; ++q) {
             if (has[q] && (g[q] < 0 || (int64_t)g[q] >= p.n_nodes)) {
@@ -468,52 +521,67 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
                 h.blk_src[off[q] + gl] = 0;
                 has[q] = false;
             }
-            pos[q] = hash_pos(tab, (uint32_t)g[q]);
-            cur[q] = has[q] ? ld_slot(tab.slots + pos[q]) : 0ULL;
+            bucket[q] = hash_bucket(tab, (uint32_t)g[q]);
+            r[q] = 0;
+            if (has[q]) open |= 1u << q;
         }
-        // stage 3: claim the slots that looked empty
+        unsigned created = 0, lower = 0;
+#pragma unroll 1
+        for (uint32_t probe = 0; open != 0; ++probe) {
+            if (probe > probe_limit(tab) + 64u) {  // the odd round more: a claim that lost its slot looks again
+                probe_failed(p.status);
+                break;
+            }
+            unsigned long long cur[KS];
+            int at[KS];
+            {
+                unsigned long long s[KS][kBucket];
 #pragma unroll
-        for (int q = 0; q < KS; ++q) {
-            seen[q] = cur[q];
-            if (has[q] && cur[q] == kEmpty) {
+                for (int q = 0; q < KS; ++q) ld_bucket_if(open >> q & 1u, tab, bucket[q], s[q]);
+#pragma unroll
+                for (int q = 0; q < KS; ++q) at[q] = match_bucket(s[q], (uint32_t)g[q], cur[q]);
+            }
+            unsigned claimed = 0;
+#pragma unroll
+            for (int q = 0; q < KS; ++q) {
+                const bool claim = (open >> q & 1u) && at[q] < kBucket && cur[q] == kEmpty;
                 const uint32_t e = (uint32_t)(off[q] + gl);
-                seen[q] = atomicCAS(tab.slots + pos[q], kEmpty,
-                                    ((unsigned long long)(uint32_t)g[q] << 32) | (ARRIVAL ? kPending : (kPending | e)));
+                cur[q] = claim_if(claim, tab.slots + bucket[q] * kBucket + at[q],
+                                  ((unsigned long long)(uint32_t)g[q] << 32) | (ARRIVAL ? kPending : (kPending | e)), cur[q]);
+                if (claim) claimed |= 1u << q;
+            }
+#pragma unroll
+            for (int q = 0; q < KS; ++q) {
+                const bool full = at[q] == kBucket;
+                const bool mine = (claimed >> q & 1u) && cur[q] == kEmpty;
+                const bool hit = (open >> q & 1u) && !full && (mine || (uint32_t)(cur[q] >> 32) == (uint32_t)g[q]);
+                const uint32_t lo = (uint32_t)cur[q];
+                const bool pending = mine || (lo & kPending);
+                if (hit) r[q] = pending ? ~((int)(bucket[q] * kBucket) + at[q]) : (int)lo;
+                if (hit && mine) created |= 1u << q;
+                if (!ARRIVAL && hit && pending && !mine && lo > (kPending | (uint32_t)(off[q] + gl))) lower |= 1u << q;
+                if (hit) open &= ~(1u << q);
+                if (full) bucket[q] = (bucket[q] + 1) & tab.mask;
             }
         }
-        // stage 4: settle every edge; collisions continue probing one by one
+        // stage 3: settle every edge
+        int displaced[KS];
+        if (!ARRIVAL) {
+#pragma unroll
+            for (int q = 0; q < KS; ++q)
+                displaced[q] = (lower >> q & 1u) ? table_lower_edge(tab, (uint32_t)~r[q], (uint32_t)g[q], (uint32_t)(off[q] + gl)) : -1;
+        }
 #pragma unroll
         for (int q = 0; q < KS; ++q) {
             if (!has[q]) continue;
-            const uint32_t key = (uint32_t)g[q];
-            const int e = off[q] + gl;
-            bool created = false;
-            int displaced = -1;
-            int r;
-            if (cur[q] == kEmpty && seen[q] == kEmpty) {
-                created = true;
-                r = ~(int)pos[q];
-            } else if ((uint32_t)(seen[q] >> 32) == key) {
-                const uint32_t lo = (uint32_t)seen[q];
-                if (!(lo & kPending)) {
-                    r = (int)lo;
-                } else {
-                    if (!ARRIVAL && lo > (kPending | (uint32_t)e)) displaced = table_lower_edge(tab, pos[q], key, (uint32_t)e);
-                    r = ~(int)pos[q];
-                }
-            } else if (ARRIVAL) {
-                r = table_insert_from<true>(tab, key, (uint32_t)e, (pos[q] + 1) & tab.mask, p.status, created);
-            } else {
-                r = table_insert_track(tab, key, (uint32_t)e, (pos[q] + 1) & tab.mask, p.status, created, displaced);
-            }
             if (ARRIVAL) {
-                if (created) r = arrival_assign<PtrT>(p, h, tab, team_cnt, g[q], r);
-            } else if (r < 0 && (created || displaced >= 0)) {
-                r = ~((~r) | kTentative);
+                if (created >> q & 1u) r[q] = arrival_assign<PtrT>(p, h, tab, team_cnt, g[q], r[q]);
+            } else if ((created >> q & 1u) || displaced[q] >= 0) {
+                r[q] = ~((~r[q]) | kTentative);
                 ++first_cnt;
-                if (displaced >= 0) atomicAdd(team_cnt + edge_owner(sm, displaced), -1);
+                if (displaced[q] >= 0) atomicSub(&sm.moved[edge_owner(sm, p.team_size, displaced[q])], 1);
             }
-            h.blk_src[e] = r;
+            h.blk_src[off[q] + gl] = r[q];
         }
         }  // MODE != MODE_SAMPLE
     }
@@ -611,11 +679,30 @@ __device__ __forceinline__ void team_prefix(const int32_t* team_sums, const Team
     total = block_sum(b, sm.scan);
 }
 
-// Phase B: offsets, picks, source reads, table inserts.  Returns the CTA's first edge and edge count.
+// The fused kernel's table of 2^log2 slots: it lies at slot 2^log2 of the team's region, so the tables of a mini-batch do
+// not overlap.  A mini-batch starts with a small one and moves to a larger one when a hop could fill it -- once the hop's
+// edge count is known, not for the worst case: the random accesses of all teams have to stay in the L2, where a slot
+// costs the 128-byte line that it lies in.  (With worst-case tables, 16 MB for each of eight teams at the benchmark's
+// sizes, the inserts of the last hop took longer than the adjacency reads.)
+__device__ __forceinline__ Table hop_table(const KParams& p, int team_id, int log2) {
+    Table tab;
+    tab.slots = p.table + ((size_t)team_id << (p.table_log2_max + 1)) + ((size_t)1 << log2);
+    tab.mask = (1u << (log2 - 2)) - 1u;
+    tab.shift = 34 - log2;
+    return tab;
+}
+
+// Room for every node in the list and a new one for every edge, at a load of at most 0.8 (in practice a third of it).
+__device__ __forceinline__ int table_log2_for(const KParams& p, int log2, long long keys) {
+    while (log2 < p.table_log2_max && (4LL << log2) < 5 * keys) ++log2;
+    return log2;
+}
+
+// Phase B: offsets, picks, source reads, table inserts.  Returns the CTA's first edge and edge count; false: aborted.
 template <typename PtrT, int MODE, bool ARRIVAL>
-__device__ __forceinline__ void phase_sample(const KParams& p, const Hop& h, const Table& tab, const Team& t,
-                                             Smem& sm, uint32_t* picks, const int32_t* team_sums, int32_t* team_cnt, int& e0,
-                                             int& e1, int& e_total) {
+__device__ __forceinline__ bool phase_sample(const KParams& p, const Hop& h, Table& tab, int& log2, unsigned& used, int team_id,
+                                             Team& t, Smem& sm, uint32_t* picks, const int32_t* team_sums, int32_t* team_cnt,
+                                             int& e0, int& e1) {
     int before, total, s0, s1;
     if (MODE == MODE_FUSED) {
         // first edge of every node tile of the hop; the CTAs own runs of tiles
@@ -634,22 +721,38 @@ __device__ __forceinline__ void phase_sample(const KParams& p, const Hop& h, con
             if (q0 + q < n_tiles) sm.prefix[q0 + q] = excl;
             excl += c[q];
         }
-        const int per = (n_tiles + t.size - 1) / t.size;
         if (threadIdx.x == 0) {
             sm.prefix[n_tiles] = total;
-            sm.n_tiles = n_tiles;
-            sm.tiles_per = max(per, 1);
+            sm.owner_scale = (float)t.size / (float)max(total, 1);
         }
         __syncthreads();
-        const int t0 = min(n_tiles, t.rank * per);
-        before = sm.prefix[t0];
-        s0 = min(h.n_seeds, t0 << h.tile_shift);
-        s1 = min(h.n_seeds, min(n_tiles, t0 + per) << h.tile_shift);
+        for (int i = threadIdx.x; i <= t.size; i += kThreads) {
+            const int tile = i == t.size ? n_tiles : first_tile_of(sm, n_tiles, h.tile_shift, i, t.size);
+            sm.first_tile[i] = tile;
+            sm.first_edge[i] = sm.prefix[tile];
+            if (i < t.size) sm.moved[i] = 0;
+        }
+        __syncthreads();
+        before = sm.first_edge[t.rank];
+        s0 = min(h.n_seeds, sm.first_tile[t.rank] << h.tile_shift);
+        s1 = min(h.n_seeds, sm.first_tile[t.rank + 1] << h.tile_shift);
     } else {
         team_prefix(team_sums, t, sm, before, total);
         chunk_of(h.n_seeds, t.rank, t.size, s0, s1);
     }
-    e_total = total;
+    if (MODE == MODE_FUSED) {
+        const int want = table_log2_for(p, log2, (long long)h.n_seeds + total);
+        if (want > log2) {  // the same for every CTA of the team
+            log2 = want;
+            used |= 1u << log2;
+            tab = hop_table(p, team_id, log2);
+            for (int s = t.rank * kThreads + (int)threadIdx.x; s < h.n_seeds; s += t.size * kThreads) {
+                const int v = __ldcg(h.nodes + s);
+                if (v >= 0 && (int64_t)v < p.n_nodes) table_insert_seed(tab, (uint32_t)v, (uint32_t)s, p.status);
+            }
+            if (!team_barrier(t, &sm.flag)) return false;
+        }
+    }
     if (t.rank == 0 && threadIdx.x == 0) {
         h.counts[8 + h.hop] = total;
         if (h.blk_indptr) h.blk_indptr[h.n_seeds] = total;
@@ -697,9 +800,15 @@ __device__ __forceinline__ void phase_sample(const KParams& p, const Hop& h, con
     }
     e1 = running;
     if (MODE == MODE_FUSED && !ARRIVAL) {
+        // The counts of first occurrences that moved between CTAs meet here, in one addition per pair of CTAs: added edge
+        // by edge, the few dozen counters of a team are a handful of L2 lines that tens of thousands of atomics wait for.
         const int mine = block_sum(first_cnt, sm.scan);
-        if (threadIdx.x == 0 && mine != 0) atomicAdd(team_cnt + t.rank, mine);
+        if (threadIdx.x == 0) sm.moved[t.rank] += mine;
+        __syncthreads();
+        for (int i = threadIdx.x; i < t.size; i += kThreads)
+            if (sm.moved[i] != 0) atomicAdd(team_cnt + i, sm.moved[i]);
     }
+    return true;
 }
 
 // ---- fused kernel, first-occurrence order ------------------------------------------------------------------------------
@@ -756,7 +865,7 @@ __device__ __forceinline__ int phase_rank_tracked(const KParams& p, const Hop& h
                     h.nodes[local] = (int)key;
                     tab.slots[pos] = ((unsigned long long)key << 32) | (uint32_t)local;
                     edges[eb + q] = local;
-                    note_node<PtrT>(p, h, local, (int)key, pos);
+                    note_node<PtrT>(p, h, local, (int)key);
                 } else {
                     set_status(p.status, FGL_ERR_CAPACITY);
                     tab.slots[pos] = ((unsigned long long)key << 32);
@@ -902,10 +1011,6 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
     t.status = p.status;
     int32_t* tile_sums = MODE == MODE_FUSED ? p.tile_sums + (size_t)team_id * 3 * kMaxTiles : nullptr;
     int32_t* team_cnt = MODE == MODE_FUSED ? p.team_cnt + (size_t)team_id * 3 * p.team_size : nullptr;
-    Table tab;
-    tab.slots = p.table + (size_t)team_id * (size_t)p.table_slots;
-    tab.mask = (uint32_t)(p.table_slots - 1);
-    tab.shift = p.table_shift;
     // The tile sums and the first-occurrence counts of a hop live in one of three buffers, used in turn over all hops of
     // all mini-batches: while a hop's phase B reads (and its new nodes add to the next one), the third is zeroed.
     int turn = 0;
@@ -918,19 +1023,21 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
         h.out_dst = p.out_dst;
         h.node_start = nullptr;
         h.node_deg = nullptr;
-        h.node_slot = nullptr;
         h.sums = h.next_sums = nullptr;
         h.deg_cap = 0;
         int n0 = p.seed_counts ? __ldg(p.seed_counts + b) : p.n_seeds_host;
         n0 = max(0, min(n0, (int)min((int64_t)0x7fffffff, p.seed_stride)));
         const int32_t* seeds = p.seeds + (size_t)b * p.seed_stride;
 
+        int log2 = p.table_log2_first;
+        unsigned used = 1u << log2;
+        Table tab{};
         if (MODE == MODE_FUSED) {
-            // The team's table is empty here: the host cleared it once and every mini-batch empties it again at its
+            tab = hop_table(p, team_id, log2);
+            // The team's tables are empty here: the host cleared them once and every mini-batch empties them again at its
             // end.  Insert the seeds with local id = position; cache their adjacency offsets and degrees.
             h.node_start = p.node_start + (size_t)team_id * p.deg_stride;
             h.node_deg = p.node_deg + (size_t)team_id * p.deg_stride;
-            h.node_slot = p.node_slot + (size_t)team_id * p.slot_stride;
             h.deg_cap = p.deg_stride;
             if (t.rank == 0 && threadIdx.x < FGL_COUNTS_STRIDE) h.counts[threadIdx.x] = threadIdx.x == 0 ? n0 : 0;
             int32_t* sums = tile_sums + turn * kMaxTiles;
@@ -938,16 +1045,15 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
                 const int v = seeds[s];
                 h.nodes[s] = v;
                 long long start = 0;
-                int deg = 0, pos = 0;
+                int deg = 0;
                 if (v < 0 || (int64_t)v >= p.n_nodes) {
                     set_status(p.status, FGL_ERR_BOUNDS);
                 } else {
-                    pos = max(0, table_insert_seed(tab, (uint32_t)v, (uint32_t)s, p.status));
+                    table_insert_seed(tab, (uint32_t)v, (uint32_t)s, p.status);
                     load_adj<PtrT>(p, v, start, deg);
                 }
                 __stcg(h.node_start + s, start);
                 __stcg(h.node_deg + s, deg);
-                __stcg(h.node_slot + s, pos);
                 if (deg > 0) atomicAdd(sums + (s >> p.tile_shift[0]), min(deg, p.fanout[0]));
             }
             if (!team_barrier(t, &sm.flag)) return;
@@ -985,8 +1091,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
             }
 
             if (MODE == MODE_FUSED && !h.last_hop) phase_count_old(h, t);
-            int e0, e1, e_total;
-            phase_sample<PtrT, MODE, ARRIVAL>(p, h, tab, t, sm, picks, p.team_sums, cnt, e0, e1, e_total);
+            int e0, e1;
+            if (!phase_sample<PtrT, MODE, ARRIVAL>(p, h, tab, log2, used, team_id, t, sm, picks, p.team_sums, cnt, e0, e1)) return;
             if (MODE == MODE_SAMPLE) break;
             if (!team_barrier(t, &sm.flag)) return;
 
@@ -1003,18 +1109,14 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
             }
         }
         if (MODE == MODE_SAMPLE) break;
-        // Once every CTA has finished reading the table, empty it for the next mini-batch: the nodes' slots one by one
-        // while they are few beside the table (a scattered 8-byte store each), else a coalesced sweep over all slots
-        // (a 16-byte store per two).
+        // Once every CTA has finished reading the tables, empty them for the next mini-batch: a coalesced sweep of the
+        // team's (L2-resident) slots, a 16-byte store per two.
         if (!team_barrier(t, &sm.flag)) return;
-        if ((int64_t)n_cur * 4 < p.table_slots) {
-            for (int i = t.rank * kThreads + (int)threadIdx.x; i < n_cur; i += t.size * kThreads)
-                tab.slots[(uint32_t)__ldcg(h.node_slot + i)] = kEmpty;
-        } else {
-            const int64_t vecs = p.table_slots / 2;  // two slots per 128-bit store
-            uint4* base = reinterpret_cast<uint4*>(tab.slots);
+        for (unsigned m = used; m; m &= m - 1) {
+            const int k = __ffs(m) - 1;
+            uint4* base = reinterpret_cast<uint4*>(hop_table(p, team_id, k).slots);
             const uint4 ones = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-            for (int64_t i = (int64_t)t.rank * kThreads + threadIdx.x; i < vecs; i += (int64_t)t.size * kThreads) base[i] = ones;
+            for (int i = t.rank * kThreads + (int)threadIdx.x; i < (1 << (k - 1)); i += t.size * kThreads) base[i] = ones;
         }
         if (b + p.n_teams < p.n_batches) {
             if (!team_barrier(t, &sm.flag)) return;
@@ -1035,7 +1137,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) map_kernel(const __grid_co
     int32_t* team_sums = p.team_sums;
     Table tab;
     tab.slots = p.table;
-    tab.mask = (uint32_t)(p.table_slots - 1);
+    tab.mask = (uint32_t)(p.table_slots / kBucket - 1);
     tab.shift = p.table_shift;
     const int n_seeds = p.n_seeds_host;
     const int n_edges = (int)p.map_edges;
@@ -1065,7 +1167,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) map_kernel(const __grid_co
         } else {
             // same table as the fused kernel; n_nodes is not known here
             bool created;
-            int r = table_insert<ARRIVAL>(tab, (uint32_t)g, (uint32_t)e, p.status, created);
+            int displaced;
+            int r = table_insert<ARRIVAL>(tab, (uint32_t)g, (uint32_t)e, p.status, created, displaced);
             if (ARRIVAL && created) {
                 cg::coalesced_group grp = cg::coalesced_threads();
                 int base = 0;
@@ -1105,7 +1208,9 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) map_kernel(const __grid_co
 // ----------------------------------------------------------------------------------------------
 // host side
 // ----------------------------------------------------------------------------------------------
-constexpr int64_t kMaxTableBytes = 512LL << 20;
+constexpr int64_t kMaxTableBytes = 1LL << 30;
+
+constexpr int64_t kSmallTable = 1 << 16;
 
 static int64_t pow2_at_least(int64_t n) {
     int64_t p = 1024;
@@ -1148,7 +1253,6 @@ static int launch_coop(Workspace* ws, K kernel, int grid, size_t dyn_smem, KPara
 // scratch layout of the drop-in kernels: [barrier: 16 u64][team_sums: grid i32][counts: 16 i32]
 // of the fused kernel: [barriers: n_teams * 16 u64][tile_sums: n_teams * 3 * kMaxTiles i32][team_cnt: 3 * grid i32]
 //                      [node_start: n_teams * deg_stride i64][node_deg: n_teams * deg_stride i32]
-//                      [node_slot: n_teams * slot_stride i32]
 // Only the part before node_start is zeroed per call.
 static int64_t sums_bytes(int64_t words) { return ((words * 4 + 127) / 128) * 128; }
 
@@ -1166,11 +1270,11 @@ static int64_t fused_head(int n_teams, int grid) {
     return (int64_t)n_teams * 128 + (int64_t)n_teams * 3 * kMaxTiles * 4 + sums_bytes(3 * (int64_t)grid);
 }
 
-static int64_t fused_need(int n_teams, int grid, int64_t deg_stride, int64_t slot_stride) {
-    return fused_head(n_teams, grid) + (int64_t)n_teams * (deg_stride * 12 + slot_stride * 4);
+static int64_t fused_need(int n_teams, int grid, int64_t deg_stride) {
+    return fused_head(n_teams, grid) + (int64_t)n_teams * deg_stride * 12;
 }
 
-static void place_fused(Workspace* ws, KParams& kp, int n_teams, int grid, int64_t deg_stride, int64_t slot_stride) {
+static void place_fused(Workspace* ws, KParams& kp, int n_teams, int grid, int64_t deg_stride) {
     char* base = ws->scratch;
     kp.barriers = (unsigned long long*)base;
     base += (size_t)n_teams * 128;
@@ -1181,10 +1285,7 @@ static void place_fused(Workspace* ws, KParams& kp, int n_teams, int grid, int64
     kp.node_start = (long long*)base;
     base += (size_t)n_teams * deg_stride * 8;
     kp.node_deg = (int32_t*)base;
-    base += (size_t)n_teams * deg_stride * 4;
-    kp.node_slot = (int32_t*)base;
     kp.deg_stride = deg_stride;
-    kp.slot_stride = slot_stride;
     kp.status = ws->status;
 }
 
@@ -1273,7 +1374,7 @@ int fgl_sample(fgl_ws* ws, const void* indptr, int indptr_is_64, const int32_t* 
     kp.out_dst = out_dst;
     kp.table = nullptr;
     kp.table_slots = 1024;
-    kp.table_shift = 22;
+    kp.table_shift = 24;
     FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)scratch_head(grid), st));
     rc = launch_sample_map<MODE_SAMPLE>(ws, kp, indptr_is_64 != 0, false, grid, dyn, st);
     if (rc != FGL_OK) return rc;
@@ -1330,7 +1431,7 @@ int fgl_map(fgl_ws* ws, int32_t* src, int32_t* dst, const int32_t* seeds, int32_
     kp.map_edges = n_edges;
     kp.table = ws->table;
     kp.table_slots = slots;
-    kp.table_shift = 32 - log2_of(slots);
+    kp.table_shift = 32 - log2_of(slots / kBucket);
     FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)scratch_head(grid), st));
     FGL_CUDA_OK(ws, cudaMemsetAsync(ws->table, 0xFF, sizeof(unsigned long long) * (size_t)slots, st));
     ws->table_dirty = true;  // this call leaves its keys in the table
@@ -1380,23 +1481,23 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
     int max_grid = 0;
     rc = occupancy_sample_map<MODE_FUSED>(ws, is64, arrival, dyn, &max_grid);
     if (rc != FGL_OK) return rc;
-    // one table per team: sized for the worst case, or by the caller's hint (a smaller table stays in L2;
-    // if it fills up the launch reports FGL_ERR_PROBE and the caller retries without a hint)
+    // The largest table of a team: sized for the worst case, or by the caller's hint (if it fills up the launch reports
+    // FGL_ERR_PROBE and the caller retries without a hint).  All tables of a team together take twice that.
     int64_t slots = pow2_at_least(cap[a->n_hops] + cap[a->n_hops] / 2 + 1);
     if (a->table_slots_hint > 0) slots = std::min(slots, pow2_at_least(a->table_slots_hint));
     if (slots > (1LL << 29)) return FGL_ERR_CAPACITY;   // pending edge entries keep a slot number in 29 bits
     // A team per mini-batch of the window, up to 16: the small hops and the barriers of one mini-batch are covered by
     // the others' traffic.  Beyond four teams the tables together stay below kMaxTableBytes.
     int n_teams = a->n_teams;
-    if (n_teams <= 0) n_teams = (int)std::max<int64_t>(4, std::min<int64_t>(16, kMaxTableBytes / (slots * 8)));
+    if (n_teams <= 0) n_teams = (int)std::max<int64_t>(4, std::min<int64_t>(16, kMaxTableBytes / (slots * 16)));
     n_teams = std::max(1, std::min(std::min(n_teams, (int)a->n_batches), max_grid));
     // CTAs per team: two edges per thread at the widest hop's worst case is all a small mini-batch can use
     int64_t widest = cap[0];
     for (int h = 0; h < a->n_hops; ++h) widest = std::max(widest, cap[h] * a->fanout[h]);
     const int team_size = (int)std::max<int64_t>(1, std::min<int64_t>(max_grid / n_teams, (widest + 2 * kThreads - 1) / (2 * kThreads)));
+    if (team_size > kMaxTeam) return FGL_ERR_INVALID;
     const int grid = team_size * n_teams;
-    const int64_t slot_stride = (cap[a->n_hops] + 31) / 32 * 32;
-    rc = ws_ensure(ws, slots * n_teams, fused_need(n_teams, grid, deg_stride, slot_stride));
+    rc = ws_ensure(ws, 2 * slots * n_teams, fused_need(n_teams, grid, deg_stride));
     if (rc != FGL_OK) return rc;
     if (ws->table_dirty) {
         FGL_CUDA_OK(ws, cudaMemsetAsync(ws->table, 0xFF, sizeof(unsigned long long) * (size_t)ws->table_slots, st));
@@ -1404,7 +1505,7 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
     }
     KParams kp;
     std::memset(&kp, 0, sizeof(kp));
-    place_fused(ws, kp, n_teams, grid, deg_stride, slot_stride);
+    place_fused(ws, kp, n_teams, grid, deg_stride);
     kp.indptr = a->indptr;
     kp.indices = a->indices;
     kp.n_nodes = a->n_nodes;
@@ -1431,8 +1532,9 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
     kp.nodes_stride = a->nodes_stride;
     kp.counts = a->counts;
     kp.table = ws->table;
-    kp.table_slots = slots;
-    kp.table_shift = 32 - log2_of(slots);
+    // the first table covers the first hop's worst case, and every small mini-batch as a whole
+    kp.table_log2_max = log2_of(slots);
+    kp.table_log2_first = log2_of(std::min(slots, std::max(kSmallTable, pow2_at_least(cap[1] + cap[1] / 4))));
     FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)fused_head(n_teams, grid), st));
     return launch_sample_map<MODE_FUSED>(ws, kp, is64, arrival, grid, dyn, st);
 }
