@@ -83,6 +83,8 @@ struct AggParams {
     int64_t indptr_stride, src_stride, row_map_stride;
     int32_t n_batches;
     const int64_t* out_row_off;  // [n_batches + 1]: first output row of batch b, then the total
+    const int32_t* counts;       // or: rows of batch b at counts[b * counts_stride]
+    int64_t counts_stride;
     // optional: the real number of destination rows, read on the device (n_dst is then the padded row count
     // the launch is sized for; forward rows beyond the real count are zero-filled)
     const int32_t* n_dst_dev;
@@ -131,6 +133,26 @@ __device__ __forceinline__ const float* x_row(const AggParams& p, int64_t r) {
     return p.shards[s] + (r - s * p.rows_per_shard) * p.ldx;
 }
 
+constexpr int kAggMaxWindow = 512;  // mini-batches per window launch (their row offsets are staged in shared memory)
+
+// First output row of every mini-batch of the window, into shared memory.
+__device__ __forceinline__ void window_offsets(const AggParams& p, long long* s_off) {
+    if (p.counts == nullptr) {
+        for (int i = threadIdx.x; i <= p.n_batches; i += blockDim.x) s_off[i] = __ldg(p.out_row_off + i);
+    } else if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        long long before = 0;
+        for (int b0 = 0; b0 < p.n_batches; b0 += 32) {
+            const int n = b0 + lane < p.n_batches ? max(__ldg(p.counts + (int64_t)(b0 + lane) * p.counts_stride), 0) : 0;
+            const int incl = warp_incl_scan(n, lane);
+            if (b0 + lane < p.n_batches) s_off[b0 + lane] = before + incl - n;
+            before += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) s_off[p.n_batches] = before;
+    }
+    __syncthreads();
+}
+
 // Forward: out[d,:] = scale_d * sum_e w_e * x[row(src[e]),:]
 // NACC vector accumulators per lane cover 32 * NACC * VEC floats per pass; UNR neighbours' loads are in
 // flight before their FMAs.  In window mode (out_row_off != NULL) the rows of all mini-batches form one
@@ -144,8 +166,6 @@ __device__ __forceinline__ const float* x_row(const AggParams& p, int64_t r) {
 // entries of row i+1, the source ids of row i+2 and the offsets of row i+3 are in flight, and every loaded value is
 // first touched one iteration after it was requested.  The row's own input row (the "self" copy) is requested
 // together with the first batch of neighbour rows, not before it.
-constexpr int kAggMaxWindow = 512;  // mini-batches per window launch (their row offsets are staged in shared memory)
-
 template <int VEC, int MODE, bool HAS_MAP, int NACC, int UNR>
 __global__ void __launch_bounds__(kAggThreads, FGL_AGG_MIN_CTAS) agg_fwd_kernel(const AggParams p) {
     using V = Vec<VEC>;
@@ -155,11 +175,8 @@ __global__ void __launch_bounds__(kAggThreads, FGL_AGG_MIN_CTAS) agg_fwd_kernel(
     const int warp_global = blockIdx.x * kAggWarps + (threadIdx.x >> 5);
     const int n_warps = gridDim.x * kAggWarps;
     const int chunks = p.dim / VEC;  // dim % VEC == 0 by dispatch
-    const bool window = p.out_row_off != nullptr;
-    if (window) {
-        for (int i = threadIdx.x; i <= p.n_batches; i += blockDim.x) s_off[i] = __ldg(p.out_row_off + i);
-        __syncthreads();
-    }
+    const bool window = p.n_batches > 0;
+    if (window) window_offsets(p, s_off);
     const int64_t padded = window ? s_off[p.n_batches] : (int64_t)p.n_dst;
     const int64_t total = p.n_dst_dev ? min((int64_t)max(__ldg(p.n_dst_dev), 0), padded) : padded;
     // padding rows of a launch sized for more rows than the block has: zero them
@@ -430,11 +447,8 @@ __global__ void __launch_bounds__(kAggStagedMaxWarps * 32, 1) agg_fwd_staged_ker
     const int n_warps = gridDim.x * cta_warps;
     const int chunks = p.dim / 4;  // <= 32
     const unsigned slot_bytes = (unsigned)chunks * 16u;
-    const bool window = p.out_row_off != nullptr;
-    if (window) {
-        for (int i = threadIdx.x; i <= p.n_batches; i += blockDim.x) s_off[i] = __ldg(p.out_row_off + i);
-        __syncthreads();
-    }
+    const bool window = p.n_batches > 0;
+    if (window) window_offsets(p, s_off);
     const int64_t padded = window ? s_off[p.n_batches] : (int64_t)p.n_dst;
     const int64_t total = p.n_dst_dev ? min((int64_t)max(__ldg(p.n_dst_dev), 0), padded) : padded;
     const bool lane_on = lane < chunks;
@@ -799,7 +813,7 @@ static void launch_fwd_staged(const AggParams& p, cudaStream_t st) {
     const int64_t per_warp = (int64_t)kAggSlots * (p.dim / 4) * 16;
     const int warps = (int)std::max<int64_t>(1, std::min<int64_t>(kAggStagedMaxWarps, ((int64_t)smem_optin - 8 * 1024) / per_warp));
     const size_t dyn = (size_t)warps * per_warp;
-    const int64_t rows = p.out_row_off ? 0x7fffffff : p.n_dst;  // window launches fill the GPU
+    const int64_t rows = p.n_batches > 0 ? 0x7fffffff : p.n_dst;  // window launches fill the GPU
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sms, (rows + warps - 1) / warps));
     if (p.row_map) {
         cudaFuncSetAttribute(agg_fwd_staged_kernel<MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
@@ -930,9 +944,9 @@ int fgl_agg_fwd_sharded(fgl_ws* ws, int32_t mode, const int32_t* indptr, const i
                           (cudaStream_t)stream);
 }
 
-int fgl_agg_fwd_window(fgl_ws* ws, int32_t mode, int32_t n_batches, const int32_t* indptr, int64_t indptr_stride,
+static int agg_fwd_window(fgl_ws* ws, int32_t mode, int32_t n_batches, const int32_t* indptr, int64_t indptr_stride,
                        const int32_t* src, int64_t src_stride, const int32_t* row_map, int64_t row_map_stride,
-                       const int64_t* out_row_off, int64_t total_rows, const float* x, const float* const* shards,
+                       const int64_t* out_row_off, const int32_t* counts, int64_t counts_stride, int64_t total_rows, const float* x, const float* const* shards,
                        int64_t rows_per_shard, int64_t n_rows, int64_t ldx, int32_t dim, int32_t flags, float* out,
                        int64_t ldo, float* self_out, int64_t ld_self, void* stream) {
     if ((mode != FGL_AGG_SUM && mode != FGL_AGG_MEAN) || n_batches < 0 || n_batches > kAggMaxWindow || total_rows < 0 ||
@@ -940,7 +954,7 @@ int fgl_agg_fwd_window(fgl_ws* ws, int32_t mode, int32_t n_batches, const int32_
         dim < 1 || ldx < dim || ldo < dim || (self_out && ld_self < dim) || n_rows < 0)
         return FGL_ERR_INVALID;
     if (n_batches == 0 || total_rows == 0) return FGL_OK;
-    if (!indptr || !src || !out_row_off || (!x && !shards) || (shards && rows_per_shard < 1) || !out || n_rows < 1)
+    if (!indptr || !src || (!out_row_off && !counts) || (!x && !shards) || (shards && rows_per_shard < 1) || !out || n_rows < 1)
         return FGL_ERR_INVALID;
     AggParams p{};
     p.indptr = indptr;
@@ -964,11 +978,29 @@ int fgl_agg_fwd_window(fgl_ws* ws, int32_t mode, int32_t n_batches, const int32_
     p.row_map_stride = row_map_stride;
     p.n_batches = n_batches;
     p.out_row_off = out_row_off;
+    p.counts = counts;
+    p.counts_stride = counts_stride;
     const int vec = pick_vec(dim, shards ? nullptr : x, ldx, out, ldo, self_out, self_out ? ld_self : 4);
     timing_begin(ws, (cudaStream_t)stream);
     const int rc = launch_fwd_any(mode, p, dim3(agg_grid_x((int)total_rows, 1), 1), vec, (cudaStream_t)stream);
     timing_end(ws, (cudaStream_t)stream);
     return rc;
+}
+
+int fgl_agg_fwd_window(fgl_ws* ws, int32_t mode, int32_t n_batches, const int32_t* indptr, int64_t indptr_stride,
+                       const int32_t* src, int64_t src_stride, const int32_t* row_map, int64_t row_map_stride,
+                       const int64_t* out_row_off, int64_t total_rows, const float* x, const float* const* shards,
+                       int64_t rows_per_shard, int64_t n_rows, int64_t ldx, int32_t dim, int32_t flags, float* out,
+                       int64_t ldo, float* self_out, int64_t ld_self, void* stream) {
+    return agg_fwd_window(ws, mode, n_batches, indptr, indptr_stride, src, src_stride, row_map, row_map_stride, out_row_off, nullptr, 0, total_rows, x, shards, rows_per_shard, n_rows, ldx, dim, flags, out, ldo, self_out, ld_self, stream);
+}
+
+int fgl_agg_fwd_window_counts(fgl_ws* ws, int32_t mode, int32_t n_batches, const int32_t* indptr, int64_t indptr_stride,
+                       const int32_t* src, int64_t src_stride, const int32_t* row_map, int64_t row_map_stride,
+                       const int32_t* counts, int64_t counts_stride, int64_t total_rows, const float* x, const float* const* shards,
+                       int64_t rows_per_shard, int64_t n_rows, int64_t ldx, int32_t dim, int32_t flags, float* out,
+                       int64_t ldo, float* self_out, int64_t ld_self, void* stream) {
+    return agg_fwd_window(ws, mode, n_batches, indptr, indptr_stride, src, src_stride, row_map, row_map_stride, nullptr, counts, counts_stride, total_rows, x, shards, rows_per_shard, n_rows, ldx, dim, flags, out, ldo, self_out, ld_self, stream);
 }
 
 int fgl_agg_edge_fwd(fgl_ws* ws, const int32_t* indptr, const int32_t* src, const float* edge_w, int32_t n_heads,

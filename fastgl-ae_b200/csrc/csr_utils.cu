@@ -2,6 +2,7 @@
 // utilis.cu:17-79).  The fused sampler emits the block CSR itself; these stay for callers that build
 // it from a COO edge list the way GraphConv.py:93-96 does.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 #include "common.cuh"
@@ -18,6 +19,56 @@ __global__ void __launch_bounds__(256) cal_deg_kernel(const int32_t* __restrict_
         const int32_t v = ids[i];
         if (v >= 0 && v < n_nodes) atomicAdd(deg + v, 1);  // utilis.cu:55-57
     }
+}
+
+// The same histogram by one CTA in shared memory, for blocks that a mini-batch's inner layers have: no zero-fill launch in
+// front of it, and the launches of such calls are what they cost.
+constexpr int kSmallDegNodes = 12 * 1024;   // 48 KB of counters
+constexpr int64_t kSmallDegIds = 32 * 1024;
+
+__global__ void __launch_bounds__(1024) cal_deg_small_kernel(const int32_t* __restrict__ ids, int n_ids, int32_t* __restrict__ deg,
+                                                             int32_t n_nodes) {
+    __shared__ int32_t cnt[kSmallDegNodes];
+    for (int i = threadIdx.x; i < n_nodes; i += 1024) cnt[i] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_ids; i += 4 * 1024) {
+        int32_t v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = i + q * 1024 < n_ids ? ids[i + q * 1024] : -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (v[q] >= 0 && v[q] < n_nodes) atomicAdd(cnt + v[q], 1);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_nodes; i += 1024) deg[i] = cnt[i];
+}
+
+// Scan by one CTA, sixteen entries per thread and pass: up to kSmallScan entries a second level (its barrier, its scratch to
+// be zeroed, a cooperative launch) takes longer than the scan.
+constexpr int64_t kSmallScan = 32 * 1024;
+
+__global__ void __launch_bounds__(1024) exclusive_sum_small_kernel(const int32_t* __restrict__ in, int n, int32_t* __restrict__ out) {
+    __shared__ int s_scan[40];
+    constexpr int kPer = 16;
+    int running = 0;
+    for (int tile = 0; tile < n; tile += 1024 * kPer) {
+        const int base = tile + (int)threadIdx.x * kPer;
+        int v[kPer], sum = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            v[k] = base + k < n ? in[base + k] : 0;
+            sum += v[k];
+        }
+        int total;
+        int excl = running + block_excl_scan(sum, s_scan, total);
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if (base + k < n) out[base + k] = excl;
+            excl += v[k];
+        }
+        running += total;
+    }
+    if (threadIdx.x == 0) out[n] = running;
 }
 
 // Two-level scan in one cooperative launch: per-CTA totals, team barrier, per-CTA rescan with its base.
@@ -218,6 +269,10 @@ extern "C" {
 int fgl_cal_deg(const int32_t* ids, int64_t n_ids, int32_t* deg, int32_t n_nodes, void* stream) {
     if (n_ids < 0 || n_nodes < 0 || (n_ids > 0 && !ids) || (n_nodes > 0 && !deg)) return FGL_ERR_INVALID;
     cudaStream_t st = (cudaStream_t)stream;
+    if (n_nodes > 0 && n_nodes <= kSmallDegNodes && n_ids <= kSmallDegIds) {
+        cal_deg_small_kernel<<<1, 1024, 0, st>>>(ids, (int)n_ids, deg, n_nodes);
+        return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
+    }
     if (n_nodes > 0 && cudaMemsetAsync(deg, 0, sizeof(int32_t) * (size_t)n_nodes, st) != cudaSuccess) return FGL_ERR_CUDA;
     if (n_ids == 0 || n_nodes == 0) return FGL_OK;
     const int grid = (int)std::min<int64_t>((n_ids + 255) / 256, 148 * 16);
@@ -297,8 +352,17 @@ int fgl_exclusive_sum(fgl_ws* ws, const int32_t* in, int64_t n, int32_t* out, vo
     std::lock_guard<std::mutex> lock(ws->mu);
     DeviceGuard guard(ws->device);
     cudaStream_t st = (cudaStream_t)stream;
-    int per_sm = 0;
-    FGL_CUDA_OK(ws, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, exclusive_sum_kernel, kScanThreads, 0));
+    if (n <= kSmallScan) {
+        exclusive_sum_small_kernel<<<1, 1024, 0, st>>>(in, (int)n, out);
+        FGL_CUDA_OK(ws, cudaGetLastError());
+        return FGL_OK;
+    }
+    static std::atomic<int> cached{0};   // the same on every device of this architecture
+    int per_sm = cached.load(std::memory_order_relaxed);
+    if (per_sm == 0) {
+        FGL_CUDA_OK(ws, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, exclusive_sum_kernel, kScanThreads, 0));
+        cached.store(per_sm, std::memory_order_relaxed);
+    }
     const int64_t tiles = (n + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems);
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * ws->sm_count, tiles));
     const int64_t need = 128 + (int64_t)grid * 4;

@@ -28,6 +28,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 #include "common.cuh"
@@ -89,6 +90,8 @@ struct KParams {
     int32_t* node_deg;             // [n_teams][deg_stride]: and its degree
     int64_t deg_stride;
     int32_t* status;               // [0] first error, [1] abort flag
+    int32_t* counts_host;          // pinned host copies (may be NULL)
+    int32_t* status_host;
 };
 
 // ----------------------------------------------------------------------------------------------
@@ -996,13 +999,19 @@ __device__ __forceinline__ void phase_relabel(const Table& tab, int32_t* edges, 
 // ----------------------------------------------------------------------------------------------
 // kernels
 // ----------------------------------------------------------------------------------------------
+// The launch reports an error to the host itself (see fgl_fused_extra); true where the caller returns.
+__device__ __forceinline__ bool given_up(const KParams& p, bool ok) {
+    if (!ok && p.status_host && threadIdx.x == 0) *(volatile int32_t*)p.status_host = *(volatile int32_t*)p.status;
+    return !ok;
+}
+
 template <typename PtrT, int MODE, bool ARRIVAL>
 __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __grid_constant__ KParams p) {
     __shared__ Smem sm;
     extern __shared__ uint32_t picks[];
     const int team_id = blockIdx.x / p.team_size;
     if (team_id >= p.n_teams) return;
-    if (*(volatile int32_t*)(p.status + 1) != 0) return;  // an earlier launch gave up: wait for fgl_ws_check
+    if (given_up(p, *(volatile int32_t*)(p.status + 1) == 0)) return;  // an earlier launch gave up: wait for fgl_ws_check
     Team t;
     t.rank = blockIdx.x % p.team_size;
     t.size = p.team_size;
@@ -1056,7 +1065,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
                 __stcg(h.node_deg + s, deg);
                 if (deg > 0) atomicAdd(sums + (s >> p.tile_shift[0]), min(deg, p.fanout[0]));
             }
-            if (!team_barrier(t, &sm.flag)) return;
+            if (given_up(p, team_barrier(t, &sm.flag))) return;
         } else {
             h.nodes = const_cast<int32_t*>(seeds);  // MODE_SAMPLE reads the seeds in place
         }
@@ -1087,20 +1096,20 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
                 turn = next;
             } else {
                 phase_count_seeds<PtrT>(p, h, t, sm, p.team_sums);
-                if (!team_barrier(t, &sm.flag)) return;
+                if (given_up(p, team_barrier(t, &sm.flag))) return;
             }
 
             if (MODE == MODE_FUSED && !h.last_hop) phase_count_old(h, t);
             int e0, e1;
-            if (!phase_sample<PtrT, MODE, ARRIVAL>(p, h, tab, log2, used, team_id, t, sm, picks, p.team_sums, cnt, e0, e1)) return;
+            if (given_up(p, phase_sample<PtrT, MODE, ARRIVAL>(p, h, tab, log2, used, team_id, t, sm, picks, p.team_sums, cnt, e0, e1))) return;
             if (MODE == MODE_SAMPLE) break;
-            if (!team_barrier(t, &sm.flag)) return;
+            if (given_up(p, team_barrier(t, &sm.flag))) return;
 
             if (!ARRIVAL) {
                 n_cur = phase_rank_tracked<PtrT>(p, h, tab, h.blk_src, e0, e1, n_cur, t, sm, cnt);
                 n_cur = (int)min((int64_t)n_cur, h.nodes_cap);
                 if (t.rank == 0 && threadIdx.x == 0) h.counts[hop + 1] = n_cur;
-                if (!team_barrier(t, &sm.flag)) return;
+                if (given_up(p, team_barrier(t, &sm.flag))) return;
                 phase_relabel_tracked(tab, h.blk_src, e0, e1);
             } else {
                 n_cur = (int)min((int64_t)n_cur + __ldcg(cnt), h.nodes_cap);
@@ -1109,9 +1118,18 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
             }
         }
         if (MODE == MODE_SAMPLE) break;
+        if (p.counts_host && t.rank == 0 && threadIdx.x < 32) {  // the counts row is this warp's own
+            __syncwarp();
+            if (threadIdx.x < FGL_COUNTS_STRIDE)
+                p.counts_host[(size_t)b * FGL_COUNTS_STRIDE + threadIdx.x] = *(volatile int32_t*)(h.counts + threadIdx.x);
+        }
         // Once every CTA has finished reading the tables, empty them for the next mini-batch: a coalesced sweep of the
         // team's (L2-resident) slots, a 16-byte store per two.
-        if (!team_barrier(t, &sm.flag)) return;
+        if (given_up(p, team_barrier(t, &sm.flag))) return;
+        if (p.status_host && t.rank == 0 && threadIdx.x == 0) {
+            const int32_t code = *(volatile int32_t*)p.status;
+            if (code != FGL_OK) *(volatile int32_t*)p.status_host = code;
+        }
         for (unsigned m = used; m; m &= m - 1) {
             const int k = __ffs(m) - 1;
             uint4* base = reinterpret_cast<uint4*>(hop_table(p, team_id, k).slots);
@@ -1119,7 +1137,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
             for (int i = t.rank * kThreads + (int)threadIdx.x; i < (1 << (k - 1)); i += t.size * kThreads) base[i] = ones;
         }
         if (b + p.n_teams < p.n_batches) {
-            if (!team_barrier(t, &sm.flag)) return;
+            if (given_up(p, team_barrier(t, &sm.flag))) return;
         }
     }
 }
@@ -1224,12 +1242,18 @@ static int log2_of(int64_t pow2) {
     return l;
 }
 
-template <typename K>
-static int max_coresident(Workspace* ws, K kernel, size_t dyn_smem, int* out) {
+template <auto kernel>
+static int max_coresident(Workspace* ws, size_t dyn_smem, int* out) {
     if (dyn_smem > 48 * 1024)
         FGL_CUDA_OK(ws, cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem));
-    int per_sm = 0;
-    FGL_CUDA_OK(ws, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, dyn_smem));
+    // the answer does not change, and asking costs more than a launch (one static per kernel; the dynamic shared memory
+    // is zero except for wide fanouts)
+    static std::atomic<int> cached{0};
+    int per_sm = dyn_smem == 0 ? cached.load(std::memory_order_relaxed) : 0;
+    if (per_sm == 0) {
+        FGL_CUDA_OK(ws, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, dyn_smem));
+        if (dyn_smem == 0) cached.store(per_sm, std::memory_order_relaxed);
+    }
     if (per_sm < 1) {
         ws->last_error = "kernel does not fit on an SM";
         return FGL_ERR_CUDA;
@@ -1299,7 +1323,7 @@ static int launch_sample_map(Workspace* ws, KParams& kp, bool is64, bool arrival
 
 template <int MODE>
 static int occupancy_sample_map(Workspace* ws, bool is64, bool arrival, size_t dyn, int* out) {
-#define FGL_OCC(PT, AR) max_coresident(ws, sample_map_kernel<PT, MODE, AR>, dyn, out)
+#define FGL_OCC(PT, AR) max_coresident<sample_map_kernel<PT, MODE, AR>>(ws, dyn, out)
     if (is64) return arrival ? FGL_OCC(int64_t, true) : FGL_OCC(int64_t, false);
     return arrival ? FGL_OCC(int32_t, true) : FGL_OCC(int32_t, false);
 #undef FGL_OCC
@@ -1403,7 +1427,7 @@ int fgl_map(fgl_ws* ws, int32_t* src, int32_t* dst, const int32_t* seeds, int32_
     cudaStream_t st = (cudaStream_t)stream;
     const bool arrival = (flags & FGL_MAP_ARRIVAL_ORDER) != 0;
     int max_grid = 0;
-    int rc = arrival ? max_coresident(ws, map_kernel<true>, 0, &max_grid) : max_coresident(ws, map_kernel<false>, 0, &max_grid);
+    int rc = arrival ? max_coresident<map_kernel<true>>(ws, 0, &max_grid) : max_coresident<map_kernel<false>>(ws, 0, &max_grid);
     if (rc != FGL_OK) return rc;
     const int64_t work = std::max<int64_t>(n_edges, n_seeds);
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(max_grid, (work + 2 * kThreads - 1) / (2 * kThreads)));
@@ -1453,8 +1477,13 @@ int fgl_map(fgl_ws* ws, int32_t* src, int32_t* dst, const int32_t* seeds, int32_
 }
 
 int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
+    if (!a || !a->seed_counts) return FGL_ERR_INVALID;
+    return fgl_sample_map_fused_extra(ws, a, nullptr, stream);
+}
+
+int fgl_sample_map_fused_extra(fgl_ws* ws, const fgl_fused_args* a, const fgl_fused_extra* extra, void* stream) {
     if (!ws || !a || !a->indptr || !a->indices || a->n_nodes <= 0 || a->n_batches < 0 || a->n_hops < 1 ||
-        a->n_hops > FGL_MAX_HOPS || !a->seeds || !a->seed_counts || !a->nodes || !a->counts || a->seed_stride < 0)
+        a->n_hops > FGL_MAX_HOPS || !a->seeds || !a->nodes || !a->counts || a->seed_stride < 0)
         return FGL_ERR_INVALID;
     if (a->n_batches == 0) return FGL_OK;
     int64_t cap[FGL_MAX_HOPS + 1];
@@ -1469,6 +1498,8 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
             return FGL_ERR_INVALID;
     }
     if (a->nodes_stride < cap[a->n_hops]) return FGL_ERR_INVALID;
+    for (int h = 0; extra && h < a->n_hops; ++h)
+        if (extra->block_dst[h] && a->n_batches != 1) return FGL_ERR_INVALID;
     for (int h = 0; h < a->n_hops; ++h)   // the relabelling passes read and write the edge entries four at a time
         if (((uintptr_t)a->block_src[h] & 15) != 0 || a->block_src_stride[h] % 4 != 0) return FGL_ERR_INVALID;
     const int64_t deg_stride = (cap[a->n_hops - 1] + 31) / 32 * 32;   // nodes that can still become seeds
@@ -1528,9 +1559,15 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* a, void* stream) {
     kp.seeds = a->seeds;
     kp.seed_stride = a->seed_stride;
     kp.seed_counts = a->seed_counts;
+    kp.n_seeds_host = (int32_t)a->seed_stride;  // without counts every mini-batch is full
     kp.nodes = a->nodes;
     kp.nodes_stride = a->nodes_stride;
     kp.counts = a->counts;
+    if (extra) {
+        kp.counts_host = extra->counts_host;
+        kp.status_host = extra->status_host;
+        for (int h = 0; h < a->n_hops; ++h) kp.blk_dst[h] = extra->block_dst[h];
+    }
     kp.table = ws->table;
     // the first table covers the first hop's worst case, and every small mini-batch as a whole
     kp.table_log2_max = log2_of(slots);

@@ -1,0 +1,601 @@
+// The host path of the ``fastgl`` operators: argument checks, output allocation and the call into the C ABI, in one
+// native call per operator.  Spelled in Python (ctypes), a call spent 10 to 20 us on the host for kernels of 2 to 5 us,
+// and a layer is a dozen of them; here it is 2 to 4 us, most of it the launch.
+//
+// The kernels stay behind the C ABI: this module resolves the entry points from the library it is given (init) and holds
+// no device code.  Every failed check and every status is a RuntimeError.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <array>
+#include <mutex>
+#include <string>
+#include <vector>
+
+#include "fastgl_b200.h"
+
+namespace py = pybind11;
+
+namespace {
+
+// ---------------------------------------------------------------------------------------------------------------------
+// the library
+// ---------------------------------------------------------------------------------------------------------------------
+void* g_lib = nullptr;
+
+#define FGL_ENTRIES(X)                                                                                                  \
+    X(fgl_status_str) X(fgl_last_error) X(fgl_ws_create) X(fgl_ws_check) X(fgl_sample) X(fgl_map) X(fgl_fused_capacity) \
+    X(fgl_sample_map_fused_extra) X(fgl_cal_deg) X(fgl_exclusive_sum) X(fgl_stage_segments) X(fgl_agg_fwd)              \
+    X(fgl_agg_fwd_window_counts) X(fgl_agg_edge_fwd) X(fgl_agg_edge_bwd) X(fgl_agg_edge_wgrad) X(fgl_agg_bwd)            \
+    X(fgl_agg_bwd_self) X(fgl_block_transpose) X(fgl_agg_bwd_gather) X(fgl_gather_rows) X(fgl_ws_time_next_launch)
+
+struct Api {
+#define FGL_FIELD(name) decltype(&::name) name = nullptr;
+    FGL_ENTRIES(FGL_FIELD)
+#undef FGL_FIELD
+} api;
+
+void init(const std::string& path) {
+    g_lib = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+    TORCH_CHECK(g_lib, "cannot load ", path, ": ", dlerror());
+#define FGL_LOAD(name)                                                       \
+    api.name = reinterpret_cast<decltype(&::name)>(dlsym(g_lib, #name));     \
+    TORCH_CHECK(api.name, path, " lacks the symbol " #name);
+    FGL_ENTRIES(FGL_LOAD)
+#undef FGL_LOAD
+}
+
+std::mutex g_ws_lock;
+std::array<fgl_ws*, 64> g_ws{};
+
+fgl_ws* workspace(int device) {
+    TORCH_CHECK(device >= 0 && device < (int)g_ws.size(), "device index ", device, " out of range");
+    std::lock_guard<std::mutex> lock(g_ws_lock);
+    if (!g_ws[device]) {
+        const int rc = api.fgl_ws_create(device, &g_ws[device]);
+        TORCH_CHECK(rc == FGL_OK, "fgl_ws_create(device=", device, ") failed: ", api.fgl_status_str(rc));
+    }
+    return g_ws[device];
+}
+
+void check(int rc, const char* what, fgl_ws* ws = nullptr) {
+    if (rc == FGL_OK) return;
+    const char* msg = ws ? api.fgl_last_error(ws) : "";
+    TORCH_CHECK(false, what, " failed: ", api.fgl_status_str(rc), msg && *msg ? std::string(" (") + msg + ")" : std::string());
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// arguments
+// ---------------------------------------------------------------------------------------------------------------------
+// CHECK_INPUT of the reference: CUDA and contiguous (aggregate_acc.cpp:4-6)
+const at::Tensor& tensor(const py::handle& o, const char* name) {
+    TORCH_CHECK(THPVariable_Check(o.ptr()), name, " must be a torch.Tensor");
+    return THPVariable_Unpack(o.ptr());
+}
+
+const at::Tensor& input(const py::handle& o, const char* name) {
+    const at::Tensor& t = tensor(o, name);
+    TORCH_CHECK(t.is_cuda(), name, " must be a CUDA tensor");
+    TORCH_CHECK(t.is_contiguous(), name, " must be contiguous");
+    return t;
+}
+
+const at::Tensor& i32(const py::handle& o, const char* name) {
+    const at::Tensor& t = input(o, name);
+    TORCH_CHECK(t.scalar_type() == at::kInt, name, " must be int32 (got ", t.scalar_type(), ")");
+    return t;
+}
+
+const at::Tensor& f32(const py::handle& o, const char* name) {
+    const at::Tensor& t = input(o, name);
+    TORCH_CHECK(t.scalar_type() == at::kFloat, name, " must be float32 (got ", t.scalar_type(), ")");
+    return t;
+}
+
+const at::Tensor& matrix(const py::handle& o, const char* name) {
+    const at::Tensor& t = f32(o, name);
+    TORCH_CHECK(t.dim() == 2, name, " must be 2-D");
+    return t;
+}
+
+// A float32 CUDA matrix whose rows are contiguous (a column slice of a wider buffer is fine).
+const at::Tensor& rows_f32(const py::handle& o, const char* name) {
+    const at::Tensor& t = tensor(o, name);
+    TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.dim() == 2 && t.stride(1) == 1, name,
+                " must be a float32 CUDA matrix with unit column stride");
+    return t;
+}
+
+template <typename T>
+T* ptr(const at::Tensor& t) {
+    return t.defined() && t.numel() > 0 ? static_cast<T*>(t.data_ptr()) : nullptr;
+}
+
+at::Tensor optional_i32(const py::handle& o, const char* name) { return o.is_none() ? at::Tensor() : i32(o, name); }
+
+struct Call {  // the device of a call, made current, with its stream and workspace
+    c10::cuda::CUDAGuard guard;
+    int device;
+    fgl_ws* ws;
+    c10::cuda::CUDAStream stream;
+    explicit Call(const at::Tensor& t)
+        : guard(t.device()), device(t.device().index()), ws(workspace(device)), stream(c10::cuda::getCurrentCUDAStream(device)) {}
+    void* st() const { return stream.stream(); }
+};
+
+// ---------------------------------------------------------------------------------------------------------------------
+// sampling and mapping
+// ---------------------------------------------------------------------------------------------------------------------
+bool is_64(const at::Tensor& edge_ptr) {
+    TORCH_CHECK(edge_ptr.scalar_type() == at::kInt || edge_ptr.scalar_type() == at::kLong, "edge_ptr must be int32 or int64");
+    return edge_ptr.scalar_type() == at::kLong;
+}
+
+py::tuple sample_node_csr(py::handle src_o, py::handle ptr_o, py::handle seeds_o, int64_t fanout, int flags, uint64_t rng_seed,
+                          uint64_t rng_ctr, bool want_dst) {
+    const at::Tensor &src = i32(src_o, "src_edges"), &edge_ptr = input(ptr_o, "edge_ptr"), &seeds = i32(seeds_o, "seed_nodes");
+    const bool wide = is_64(edge_ptr);
+    const int64_t S = seeds.numel();
+    TORCH_CHECK(fanout >= 1 && fanout <= FGL_MAX_FANOUT && S * fanout <= 0x7fffffffLL, "sample_node failed: ",
+                api.fgl_status_str(FGL_ERR_INVALID));
+    Call c(seeds);
+    auto opt = seeds.options();
+    at::Tensor out_src = at::empty({std::max<int64_t>(1, S * fanout)}, opt);
+    at::Tensor out_dst = want_dst ? at::empty({std::max<int64_t>(1, S * fanout)}, opt) : at::Tensor();
+    at::Tensor out_ptr = at::empty({S + 1}, opt);
+    int64_t n_edges = 0;
+    int rc;
+    {
+        py::gil_scoped_release nogil;
+        rc = api.fgl_sample(c.ws, ptr<void>(edge_ptr), wide, ptr<int32_t>(src), edge_ptr.numel() - 1, ptr<int32_t>(seeds), (int32_t)S,
+                            (int32_t)fanout, flags, rng_seed, rng_ctr, ptr<int32_t>(out_ptr), ptr<int32_t>(out_src),
+                            ptr<int32_t>(out_dst), &n_edges, c.st());
+    }
+    check(rc, "sample_node", c.ws);
+    return py::make_tuple(out_src.slice(0, 0, n_edges), want_dst ? py::cast(out_dst.slice(0, 0, n_edges)) : py::none(), out_ptr, n_edges);
+}
+
+at::Tensor transfer_edge_id(py::handle src_o, py::handle dst_o, py::handle seeds_o, int64_t dst_nodes, int64_t unique_num,
+                            int64_t n_edges, int flags) {
+    const at::Tensor &src = i32(src_o, "src_edges"), &dst = i32(dst_o, "dst_edges"), &seeds = i32(seeds_o, "dst_edges_unique");
+    const int64_t S = std::min<int64_t>(dst_nodes, seeds.numel());
+    TORCH_CHECK(n_edges <= src.numel() && n_edges <= dst.numel(), "edge_nums exceeds the edge arrays");
+    const int64_t cap = S + std::max<int64_t>(0, std::min<int64_t>(unique_num, n_edges));
+    Call c(src);
+    at::Tensor unique = at::empty({std::max<int64_t>(1, cap)}, src.options());
+    int64_t n_unique = 0;
+    int rc;
+    {
+        py::gil_scoped_release nogil;
+        rc = api.fgl_map(c.ws, ptr<int32_t>(src), ptr<int32_t>(dst), ptr<int32_t>(seeds), (int32_t)S, n_edges, ptr<int32_t>(unique), cap,
+                         flags, &n_unique, c.st());
+    }
+    check(rc, "transfer_edge_id", c.ws);
+    return unique.slice(0, 0, n_unique);
+}
+
+struct FusedShape {
+    int hops;
+    int32_t fanout[FGL_MAX_HOPS];
+    int64_t cap[FGL_MAX_HOPS + 1];
+};
+
+bool fused_shape(FusedShape& f, int64_t n_nodes, int64_t max_seeds, const std::vector<int64_t>& fanouts) {
+    f.hops = (int)fanouts.size();
+    if (f.hops < 1 || f.hops > FGL_MAX_HOPS || max_seeds > 0x7fffffffLL) return false;
+    for (int h = 0; h < f.hops; ++h) {
+        if (fanouts[h] < 1 || fanouts[h] > FGL_MAX_FANOUT) return false;
+        f.fanout[h] = (int32_t)fanouts[h];
+    }
+    return api.fgl_fused_capacity(n_nodes, (int32_t)max_seeds, f.hops, f.fanout, f.cap) == FGL_OK;
+}
+
+void fused_graph(fgl_fused_args& a, const at::Tensor& edge_ptr, const at::Tensor& src, const FusedShape& f) {
+    a.indptr = ptr<void>(edge_ptr);
+    a.indices = ptr<int32_t>(src);
+    a.n_nodes = edge_ptr.numel() - 1;
+    a.indptr_is_64 = is_64(edge_ptr);
+    a.n_hops = f.hops;
+    for (int h = 0; h < f.hops; ++h) a.fanout[h] = f.fanout[h];
+}
+
+// One launch for a window of mini-batches, into the buffers of a FusedBatch; counts_host / status_host: its pinned copies.
+void sample_map_fused(py::handle ptr_o, py::handle src_o, py::handle seeds_o, py::handle seed_counts_o, const std::vector<int64_t>& fanouts,
+                      int flags, uint64_t rng_seed, uint64_t rng_ctr, int n_teams, int64_t table_slots, const at::Tensor& nodes,
+                      const at::Tensor& counts, const std::vector<at::Tensor>& indptr, const std::vector<at::Tensor>& block_src,
+                      py::handle counts_host, py::handle status_host) {
+    const at::Tensor &src = i32(src_o, "src_edges"), &edge_ptr = input(ptr_o, "edge_ptr"), &seeds = i32(seeds_o, "seeds"),
+                     &seed_counts = i32(seed_counts_o, "seed_counts");
+    FusedShape f;
+    TORCH_CHECK(fused_shape(f, edge_ptr.numel() - 1, seeds.size(1), fanouts), "sample_map_fused failed: ", api.fgl_status_str(FGL_ERR_INVALID));
+    Call c(seeds);
+    fgl_fused_args a{};
+    fused_graph(a, edge_ptr, src, f);
+    a.n_batches = (int32_t)seeds.size(0);
+    for (int h = 0; h < f.hops; ++h) {
+        a.block_indptr[h] = ptr<int32_t>(indptr[h]);
+        a.block_indptr_stride[h] = indptr[h].stride(0);
+        a.block_src[h] = ptr<int32_t>(block_src[h]);
+        a.block_src_stride[h] = block_src[h].stride(0);
+    }
+    a.flags = flags;
+    a.n_teams = n_teams;
+    a.table_slots_hint = table_slots;
+    a.rng_seed = rng_seed;
+    a.rng_ctr = rng_ctr;
+    a.seeds = ptr<int32_t>(seeds);
+    a.seed_stride = seeds.stride(0);
+    a.seed_counts = ptr<int32_t>(seed_counts);
+    a.nodes = ptr<int32_t>(nodes);
+    a.nodes_stride = nodes.stride(0);
+    a.counts = ptr<int32_t>(counts);
+    fgl_fused_extra x{};
+    if (!counts_host.is_none()) {
+        x.counts_host = static_cast<int32_t*>(tensor(counts_host, "counts_host").data_ptr());
+        x.status_host = static_cast<int32_t*>(tensor(status_host, "status_host").data_ptr());
+        *x.status_host = 0;
+    }
+    check(api.fgl_sample_map_fused_extra(c.ws, &a, &x, c.st()), "sample_map_fused", c.ws);
+}
+
+// Pinned words the blocking calls of a thread are answered in (one per thread: two threads may wait at once).
+int32_t* answer_words() {
+    static thread_local at::Tensor words;
+    if (!words.defined()) words = at::empty({2 * FGL_COUNTS_STRIDE}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    return static_cast<int32_t*>(words.data_ptr());
+}
+
+// Above this size of the worst case, results are copied out of it into tensors of their own size: what a caller keeps then
+// holds the memory it needs.  Below, the copy costs more than the memory.
+constexpr int64_t kKeepArena = 1 << 18;       // int32 words
+constexpr int64_t kMaxArena = 1LL << 29;      // beyond 2 GB of worst case the caller walks the hops one by one
+
+// All hops of one mini-batch in one launch: (input nodes, [(indptr, src, dst, n_src, n_dst)] input layer first), or None when
+// the worst case is too large for that.  ``fanouts`` in sampling order.
+py::object sample_blocks(py::handle src_o, py::handle ptr_o, py::handle seeds_o, const std::vector<int64_t>& fanouts, int flags,
+                         uint64_t rng_seed, uint64_t rng_ctr) {
+    const at::Tensor &src = i32(src_o, "src_edges"), &edge_ptr = input(ptr_o, "edge_ptr"), &seeds = i32(seeds_o, "seed_nodes");
+    FusedShape f;
+    const int64_t S = seeds.numel();
+    if (S == 0 || !fused_shape(f, edge_ptr.numel() - 1, S, fanouts)) return py::none();
+    auto up = [](int64_t n) { return (n + 31) / 32 * 32; };
+    const int64_t head = 2 * 32;  // the seed count, then the counts row
+    int64_t total = head + up(f.cap[f.hops]);
+    for (int h = 0; h < f.hops; ++h) total += up(f.cap[h] + 1) + 2 * up(f.cap[h] * f.fanout[h]);
+    if (total > kMaxArena) return py::none();
+    Call c(seeds);
+    at::Tensor arena = at::empty({total}, seeds.options());
+    int32_t* base = static_cast<int32_t*>(arena.data_ptr());
+    fgl_fused_args a{};
+    fused_graph(a, edge_ptr, src, f);
+    fgl_fused_extra x{};
+    int32_t* words = answer_words();
+    x.counts_host = words;
+    x.status_host = words + FGL_COUNTS_STRIDE;
+    *x.status_host = 0;
+    int64_t at_word = head, ptr_at[FGL_MAX_HOPS], src_at[FGL_MAX_HOPS], dst_at[FGL_MAX_HOPS];
+    const int64_t nodes_at = at_word;
+    at_word += up(f.cap[f.hops]);
+    for (int h = 0; h < f.hops; ++h) {
+        ptr_at[h] = at_word;
+        src_at[h] = ptr_at[h] + up(f.cap[h] + 1);
+        dst_at[h] = src_at[h] + up(f.cap[h] * f.fanout[h]);
+        at_word = dst_at[h] + up(f.cap[h] * f.fanout[h]);
+        a.block_indptr[h] = base + ptr_at[h];
+        a.block_indptr_stride[h] = up(f.cap[h] + 1);
+        a.block_src[h] = base + src_at[h];
+        a.block_src_stride[h] = up(f.cap[h] * f.fanout[h]);
+        x.block_dst[h] = base + dst_at[h];
+    }
+    a.n_batches = 1;
+    a.flags = flags;
+    a.rng_seed = rng_seed;
+    a.rng_ctr = rng_ctr;
+    a.seeds = ptr<int32_t>(seeds);
+    a.seed_stride = S;
+    a.seed_counts = nullptr;  // every seed
+    a.nodes = base + nodes_at;
+    a.nodes_stride = up(f.cap[f.hops]);
+    a.counts = base + 32;
+    int rc;
+    {
+        py::gil_scoped_release nogil;
+        rc = api.fgl_sample_map_fused_extra(c.ws, &a, &x, c.st());
+        if (rc == FGL_OK) {
+            c.stream.synchronize();
+            if (*x.status_host != FGL_OK) rc = api.fgl_ws_check(c.ws, c.st());
+        }
+    }
+    check(rc, "sample_blocks", c.ws);
+    const int32_t* n = words;
+    if (total > kKeepArena) {
+        int64_t exact = up(n[f.hops]);
+        for (int h = 0; h < f.hops; ++h) exact += up(n[h] + 1) + 2 * up(n[8 + h]);
+        at::Tensor own = at::empty({exact}, seeds.options());
+        int32_t* to = static_cast<int32_t*>(own.data_ptr());
+        std::vector<fgl_segment> seg;
+        at_word = 0;
+        auto move = [&](int64_t from, int64_t words_n) {
+            seg.push_back({to + at_word, base + from, words_n * 4});
+            const int64_t where = at_word;
+            at_word += up(words_n);
+            return where;
+        };
+        const int64_t new_nodes = move(nodes_at, n[f.hops]);
+        TORCH_INTERNAL_ASSERT(new_nodes == 0);
+        for (int h = 0; h < f.hops; ++h) {
+            ptr_at[h] = move(ptr_at[h], n[h] + 1);
+            src_at[h] = move(src_at[h], n[8 + h]);
+            dst_at[h] = move(dst_at[h], n[8 + h]);
+        }
+        for (size_t i = 0; i < seg.size(); i += FGL_MAX_SEGMENTS)
+            check(api.fgl_stage_segments(seg.data() + i, (int32_t)std::min<size_t>(FGL_MAX_SEGMENTS, seg.size() - i), nullptr, nullptr, 0,
+                                         c.st()), "sample_blocks");
+        arena = own;
+    }
+    py::list blocks;
+    for (int h = f.hops - 1; h >= 0; --h)
+        blocks.append(py::make_tuple(arena.slice(0, ptr_at[h], ptr_at[h] + n[h] + 1), arena.slice(0, src_at[h], src_at[h] + n[8 + h]),
+                                     arena.slice(0, dst_at[h], dst_at[h] + n[8 + h]), n[h + 1], n[h]));
+    const int64_t first = total > kKeepArena ? 0 : nodes_at;
+    return py::make_tuple(arena.slice(0, first, first + n[f.hops]), blocks);
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// block CSR
+// ---------------------------------------------------------------------------------------------------------------------
+at::Tensor cal_deg(py::handle edges_o, int64_t n) {
+    const at::Tensor& edges = i32(edges_o, "edges");
+    Call c(edges);
+    at::Tensor deg = at::empty({n}, edges.options());
+    check(api.fgl_cal_deg(ptr<int32_t>(edges), edges.numel(), ptr<int32_t>(deg), (int32_t)n, c.st()), "cal_deg");
+    return deg;
+}
+
+at::Tensor exclusive_sum(py::handle degs_o) {
+    const at::Tensor& degs = i32(degs_o, "in_degs");
+    Call c(degs);
+    at::Tensor out = at::empty({degs.numel() + 1}, degs.options());
+    check(api.fgl_exclusive_sum(c.ws, ptr<int32_t>(degs), degs.numel(), ptr<int32_t>(out), c.st()), "exclusive_sum", c.ws);
+    return out;
+}
+
+void stage_segments(const std::vector<std::pair<py::object, py::object>>& copies, py::handle words_dst, const std::vector<int64_t>& words) {
+    TORCH_CHECK(copies.size() <= FGL_MAX_SEGMENTS && words.size() <= FGL_MAX_SEGMENTS, "at most 8 copies and 8 words per call");
+    fgl_segment seg[FGL_MAX_SEGMENTS];
+    int32_t values[FGL_MAX_SEGMENTS];
+    const at::Tensor* on = nullptr;
+    for (size_t i = 0; i < copies.size(); ++i) {
+        const at::Tensor &dst = tensor(copies[i].first, "dst"), &src = tensor(copies[i].second, "src");
+        TORCH_CHECK(dst.element_size() == 4 && src.element_size() == 4 && dst.is_cuda() && src.is_cuda(),
+                    "stage_segments copies 4-byte CUDA tensors");
+        TORCH_CHECK(dst.numel() >= src.numel() && src.is_contiguous() && dst.is_contiguous(),
+                    "stage_segments needs contiguous tensors and a destination at least as large as the source");
+        seg[i] = {dst.data_ptr(), src.data_ptr(), src.numel() * 4};
+        on = &dst;
+    }
+    int32_t* to = nullptr;
+    if (!words_dst.is_none()) {
+        const at::Tensor& w = i32(words_dst, "words_dst");
+        to = ptr<int32_t>(w);
+        on = &w;
+    }
+    for (size_t i = 0; i < words.size(); ++i) values[i] = (int32_t)words[i];
+    TORCH_CHECK(on, "stage_segments needs a destination");
+    Call c(*on);
+    check(api.fgl_stage_segments(seg, (int32_t)copies.size(), to, values, (int32_t)words.size(), c.st()), "stage_segments");
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// aggregation
+// ---------------------------------------------------------------------------------------------------------------------
+at::Tensor agg_fwd(int mode, const at::Tensor& edge_ptr, const at::Tensor& src, const at::Tensor& x, int64_t n_dst, const at::Tensor& src_deg,
+                   const at::Tensor& dst_deg, bool passthrough, const at::Tensor& row_map, const at::Tensor& out_given,
+                   const at::Tensor& n_dst_dev) {
+    TORCH_CHECK(edge_ptr.numel() >= n_dst + 1, "edge_ptr is shorter than dst_nodes + 1");
+    if (mode == FGL_AGG_SYMNORM) {
+        const int64_t n_src = row_map.defined() ? row_map.numel() : x.size(0);
+        TORCH_CHECK(src_deg.defined() && dst_deg.defined() && dst_deg.numel() >= n_dst && src_deg.numel() >= n_src,
+                    "sym-norm needs src_norm_degs[n_src] and dst_norm_degs[n_dst]");
+    }
+    Call c(x);
+    at::Tensor out = out_given.defined() ? out_given : at::empty({n_dst, x.size(1)}, x.options());
+    check(api.fgl_agg_fwd(c.ws, mode, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), ptr<int32_t>(src_deg), ptr<int32_t>(dst_deg),
+                          ptr<int32_t>(row_map), row_map.defined() ? row_map.numel() : 0, ptr<float>(x), x.size(0), x.stride(0),
+                          (int32_t)x.size(1), (int32_t)n_dst, passthrough ? FGL_AGG_ZERO_DEG_PASSTHROUGH : 0, ptr<float>(out),
+                          out.stride(0), ptr<int32_t>(n_dst_dev), c.st()), "aggregate");
+    return out;
+}
+
+at::Tensor aggregate(int mode, py::handle ptr_o, py::handle src_o, py::handle x_o, int64_t n_dst, py::handle src_deg, py::handle dst_deg,
+                     bool passthrough, py::handle row_map, py::handle out, py::handle n_dst_dev) {
+    return agg_fwd(mode, i32(ptr_o, "edge_ptr"), i32(src_o, "src_edges"), matrix(x_o, "input_feat"), n_dst,
+                   optional_i32(src_deg, "src_norm_degs"), optional_i32(dst_deg, "dst_norm_degs"), passthrough,
+                   optional_i32(row_map, "row_map"), out.is_none() ? at::Tensor() : rows_f32(out, "out"),
+                   n_dst_dev.is_none() ? at::Tensor() : tensor(n_dst_dev, "n_dst_dev"));
+}
+
+struct Transposed {
+    at::Tensor t_indptr, t_dst, hubs;
+};
+
+at::Tensor agg_bwd(int mode, const at::Tensor& edge_ptr, const at::Tensor& src, const at::Tensor& dy, int64_t n_src, const at::Tensor& src_deg,
+                   const at::Tensor& dst_deg, const at::Tensor& n_dst_dev, const at::Tensor& d_self, const at::Tensor& out_given,
+                   const Transposed* tb) {
+    const int64_t n_dst = dy.size(0), dim = dy.size(1);
+    TORCH_CHECK(mode != FGL_AGG_SYMNORM || (src_deg.defined() && dst_deg.defined() && src_deg.numel() >= n_src && dst_deg.numel() >= n_dst),
+                "sym-norm needs src_norm_degs[src_nodes] and dst_norm_degs[n_dst]");
+    TORCH_CHECK(edge_ptr.numel() >= n_dst + 1, "edge_ptr is shorter than n_dst + 1");
+    TORCH_CHECK(!out_given.defined() || (out_given.size(0) >= n_src && out_given.size(1) == dim), "out must be float32[src_nodes, dim]");
+    TORCH_CHECK(!d_self.defined() || (d_self.size(0) == n_dst && d_self.size(1) == dim), "d_self must be float32[n_dst, dim]");
+    Call c(dy);
+    at::Tensor dx = out_given.defined() ? out_given : at::empty({n_src, dim}, dy.options());
+    int rc;
+    if (tb)
+        rc = api.fgl_agg_bwd_gather(c.ws, mode, ptr<int32_t>(edge_ptr), ptr<int32_t>(tb->t_indptr), ptr<int32_t>(tb->t_dst),
+                                    ptr<int32_t>(tb->hubs), ptr<int32_t>(src_deg), ptr<int32_t>(dst_deg), ptr<float>(dy), dy.stride(0),
+                                    ptr<float>(d_self), d_self.defined() ? d_self.stride(0) : dim, (int32_t)dim, (int32_t)n_dst,
+                                    (int32_t)n_src, ptr<float>(dx), dx.stride(0), ptr<int32_t>(n_dst_dev), c.st());
+    else if (d_self.defined())
+        rc = api.fgl_agg_bwd_self(c.ws, mode, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), ptr<int32_t>(src_deg), ptr<int32_t>(dst_deg),
+                                  ptr<float>(dy), dy.stride(0), ptr<float>(d_self), d_self.stride(0), (int32_t)dim, (int32_t)n_dst,
+                                  (int32_t)n_src, ptr<float>(dx), dx.stride(0), ptr<int32_t>(n_dst_dev), c.st());
+    else
+        rc = api.fgl_agg_bwd(c.ws, mode, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), ptr<int32_t>(src_deg), ptr<int32_t>(dst_deg),
+                             ptr<float>(dy), dy.stride(0), (int32_t)dim, (int32_t)n_dst, (int32_t)n_src, ptr<float>(dx), dx.stride(0),
+                             ptr<int32_t>(n_dst_dev), c.st());
+    check(rc, tb ? "aggregate_backward (gather)" : "aggregate_backward", tb ? c.ws : nullptr);
+    return dx;
+}
+
+at::Tensor aggregate_backward(int mode, py::handle ptr_o, py::handle src_o, py::handle dy_o, int64_t n_src, py::handle src_deg,
+                              py::handle dst_deg, py::handle n_dst_dev, py::handle d_self, py::handle out, py::handle t_indptr,
+                              py::handle t_dst, py::handle hubs) {
+    Transposed tb;
+    const bool gather = !t_indptr.is_none();
+    if (gather) tb = {tensor(t_indptr, "t_indptr"), tensor(t_dst, "t_dst"), tensor(hubs, "hubs")};
+    return agg_bwd(mode, i32(ptr_o, "edge_ptr"), i32(src_o, "src_edges"), rows_f32(dy_o, "d_input"), n_src,
+                   optional_i32(src_deg, "src_norm_degs"), optional_i32(dst_deg, "dst_norm_degs"),
+                   n_dst_dev.is_none() ? at::Tensor() : tensor(n_dst_dev, "n_dst_dev"),
+                   d_self.is_none() ? at::Tensor() : rows_f32(d_self, "d_self"), out.is_none() ? at::Tensor() : rows_f32(out, "out"),
+                   gather ? &tb : nullptr);
+}
+
+void transpose_block(py::handle ptr_o, py::handle src_o, int64_t n_dst, int64_t n_src, py::handle n_dst_dev, const at::Tensor& t_indptr,
+                     const at::Tensor& t_dst, int64_t edge_cap, const at::Tensor& hubs, const at::Tensor& work) {
+    const at::Tensor &edge_ptr = i32(ptr_o, "edge_ptr"), &src = i32(src_o, "src_edges");
+    Call c(edge_ptr);
+    check(api.fgl_block_transpose(c.ws, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), (int32_t)n_dst, (int32_t)n_src, ptr<int32_t>(t_indptr),
+                                  ptr<int32_t>(t_dst), edge_cap, ptr<int32_t>(hubs), ptr<int32_t>(work),
+                                  n_dst_dev.is_none() ? nullptr : ptr<int32_t>(tensor(n_dst_dev, "n_dst_dev")), c.st()),
+          "transpose_block", c.ws);
+}
+
+// One layer of a window from the counts on the device; n_dst: the batches' destination counts as the host read them.
+// start / end: addresses of CUDA events to record around the launch, or 0.
+void aggregate_window(int mode, const at::Tensor& counts, int64_t hop, int64_t total, const at::Tensor& indptr, const at::Tensor& src,
+                      py::handle nodes_o, py::handle x_o, py::handle out_o, py::handle self_o, uint64_t start, uint64_t end) {
+    const at::Tensor &x = rows_f32(x_o, "input_feat"), &out = rows_f32(out_o, "out");
+    const at::Tensor self = self_o.is_none() ? at::Tensor() : rows_f32(self_o, "self_out");
+    const at::Tensor nodes = nodes_o.is_none() ? at::Tensor() : tensor(nodes_o, "nodes");
+    TORCH_CHECK(out.size(0) >= total && (!self.defined() || self.size(0) >= total), "out is too small for the window's destination rows");
+    Call c(x);
+    if (start) check(api.fgl_ws_time_next_launch(c.ws, (void*)start, (void*)end), "time_next_launch");
+    check(api.fgl_agg_fwd_window_counts(c.ws, mode, (int32_t)counts.size(0), ptr<int32_t>(indptr), indptr.stride(0), ptr<int32_t>(src),
+                                        src.stride(0), ptr<int32_t>(nodes), nodes.defined() ? nodes.stride(0) : 0,
+                                        ptr<int32_t>(counts) + hop, counts.stride(0), total, ptr<float>(x), nullptr, 0, x.size(0),
+                                        x.stride(0), (int32_t)x.size(1), 0, ptr<float>(out), out.stride(0), ptr<float>(self),
+                                        self.defined() ? self.stride(0) : x.size(1), c.st()),
+          "aggregate_window");
+}
+
+at::Tensor gather_rows(py::handle table_o, py::handle ids_o, py::handle out_o) {
+    const at::Tensor &x = rows_f32(table_o, "input_feat"), &ids = i32(ids_o, "ids");
+    Call c(x);
+    at::Tensor out = out_o.is_none() ? at::empty({ids.numel(), x.size(1)}, x.options()) : rows_f32(out_o, "out");
+    check(api.fgl_gather_rows(c.ws, ptr<float>(x), nullptr, 0, x.size(0), x.stride(0), (int32_t)x.size(1), ptr<int32_t>(ids), ids.numel(),
+                              ptr<float>(out), out.stride(0), c.st()), "gather_rows");
+    return out;
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// the reference's layer operators
+// ---------------------------------------------------------------------------------------------------------------------
+std::vector<at::Tensor> forward_gcn(py::handle ptr_o, py::handle src_o, py::handle src_deg, py::handle dst_deg, py::handle x_o, py::handle w_o,
+                                    int64_t n_dst) {
+    const at::Tensor &w = f32(w_o, "weight"), &x = f32(x_o, "input_feat");
+    return {agg_fwd(FGL_AGG_SYMNORM, i32(ptr_o, "edge_ptr"), i32(src_o, "src_edges"), at::mm(x, w), n_dst, i32(src_deg, "src_norm_degs"),
+                    i32(dst_deg, "dst_norm_degs"), true, at::Tensor(), at::Tensor(), at::Tensor())};
+}
+
+std::vector<at::Tensor> backward_gcn(py::handle ptr_o, py::handle src_o, py::handle src_deg, py::handle dst_deg, py::handle dy_o,
+                                     py::handle w_o, py::handle x_o) {
+    const at::Tensor &w = f32(w_o, "weight"), &x = f32(x_o, "input_feat");
+    const at::Tensor d = agg_bwd(FGL_AGG_SYMNORM, i32(ptr_o, "edge_ptr"), i32(src_o, "src_edges"), rows_f32(dy_o, "d_input"), x.size(0),
+                                 i32(dst_deg, "src_norm_degs"), i32(src_deg, "dst_norm_degs"), at::Tensor(), at::Tensor(), at::Tensor(), nullptr);
+    return {at::mm(d, w.t()), at::mm(x.t(), d)};
+}
+
+std::vector<at::Tensor> forward_gin(py::handle ptr_o, py::handle src_o, py::handle x_o, py::handle w_o, int64_t n_dst) {
+    const at::Tensor& w = f32(w_o, "weight");
+    at::Tensor tmp = agg_fwd(FGL_AGG_SUM, i32(ptr_o, "edge_ptr"), i32(src_o, "src_edges"), matrix(x_o, "input_feat"), n_dst, at::Tensor(),
+                             at::Tensor(), true, at::Tensor(), at::Tensor(), at::Tensor());
+    return {at::mm(tmp, w), tmp};
+}
+
+std::vector<at::Tensor> backward_gin(py::handle ptr_o, py::handle src_o, py::handle dy_o, py::handle w_o, py::handle x_o, int64_t n_src) {
+    const at::Tensor &w = f32(w_o, "weight"), &x = f32(x_o, "input_feat"), &dy = f32(dy_o, "d_input");
+    const at::Tensor d_tmp = at::mm(dy, w.t());
+    at::Tensor d_w = at::mm(x.t(), dy);
+    return {agg_bwd(FGL_AGG_SUM, i32(ptr_o, "edge_ptr"), i32(src_o, "src_edges"), d_tmp, n_src, at::Tensor(), at::Tensor(), at::Tensor(),
+                    at::Tensor(), at::Tensor(), nullptr), d_w};
+}
+
+std::vector<at::Tensor> forward_gat(py::handle ptr_o, py::handle w_o, py::handle src_o, py::handle x_o, int64_t n_dst, int64_t heads) {
+    const at::Tensor &edge_ptr = i32(ptr_o, "edge_ptr"), &src = i32(src_o, "src_edges"), &w = f32(w_o, "edge_data"),
+                     &x = f32(x_o, "input_feat");
+    TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && w.size(1) == heads && x.size(1) % heads == 0 && w.size(0) >= src.numel(),
+                "edge_data must be [n_edges, num_heads] and num_heads must divide the feature width");
+    const int64_t dim = x.size(1);
+    Call c(x);
+    at::Tensor out = at::empty({n_dst, dim}, x.options());
+    check(api.fgl_agg_edge_fwd(c.ws, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), ptr<float>(w), (int32_t)heads, ptr<float>(x),
+                               (int32_t)x.size(0), x.stride(0), (int32_t)dim, (int32_t)n_dst, FGL_AGG_ZERO_DEG_PASSTHROUGH, ptr<float>(out),
+                               dim, c.st()), "forward_gat");
+    return {out};
+}
+
+std::vector<at::Tensor> backward_gat(py::handle ptr_o, py::handle w_o, py::handle src_o, py::handle dy_o, int64_t n_src, int64_t heads) {
+    const at::Tensor &edge_ptr = i32(ptr_o, "edge_ptr"), &src = i32(src_o, "src_edges"), &w = f32(w_o, "edge_data"), &dy = f32(dy_o, "d_input");
+    TORCH_CHECK(dy.dim() == 2 && w.dim() == 2 && w.size(1) == heads && dy.size(1) % heads == 0,
+                "edge_data must be [n_edges, num_heads] and num_heads must divide the feature width");
+    const int64_t dim = dy.size(1);
+    Call c(dy);
+    at::Tensor dx = at::empty({n_src, dim}, dy.options());
+    check(api.fgl_agg_edge_bwd(c.ws, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), ptr<float>(w), (int32_t)heads, ptr<float>(dy), dy.stride(0),
+                               (int32_t)dim, (int32_t)dy.size(0), (int32_t)n_src, ptr<float>(dx), dim, c.st()), "backward_gat");
+    return {dx};
+}
+
+at::Tensor edge_weight_grad(py::handle ptr_o, py::handle src_o, py::handle x_o, py::handle dy_o, int64_t heads) {
+    const at::Tensor &edge_ptr = i32(ptr_o, "edge_ptr"), &src = i32(src_o, "src_edges"), &x = matrix(x_o, "input_feat"),
+                     &dy = matrix(dy_o, "d_out");
+    Call c(dy);
+    at::Tensor dw = at::empty({src.numel(), heads}, dy.options());
+    check(api.fgl_agg_edge_wgrad(c.ws, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), (int32_t)heads, ptr<float>(x), (int32_t)x.size(0),
+                                 x.stride(0), ptr<float>(dy), dy.stride(0), (int32_t)dy.size(1), (int32_t)dy.size(0), src.numel(),
+                                 ptr<float>(dw), c.st()), "edge_weight_grad");
+    return dw;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_ops, m) {
+    m.def("init", &init);
+    m.def("workspace", [](int device) { return (uintptr_t)workspace(device); });
+    m.def("sample_node_csr", &sample_node_csr);
+    m.def("transfer_edge_id", &transfer_edge_id);
+    m.def("sample_map_fused", &sample_map_fused);
+    m.def("sample_blocks", &sample_blocks);
+    m.def("cal_deg", &cal_deg);
+    m.def("exclusive_sum", &exclusive_sum);
+    m.def("stage_segments", &stage_segments);
+    m.def("aggregate", &aggregate);
+    m.def("aggregate_backward", &aggregate_backward);
+    m.def("transpose_block", &transpose_block);
+    m.def("aggregate_window", &aggregate_window);
+    m.def("gather_rows", &gather_rows);
+    m.def("forward_gcn", &forward_gcn);
+    m.def("backward_gcn", &backward_gcn);
+    m.def("forward_gin", &forward_gin);
+    m.def("backward_gin", &backward_gin);
+    m.def("forward_gat", &forward_gat);
+    m.def("backward_gat", &backward_gat);
+    m.def("edge_weight_grad", &edge_weight_grad);
+}

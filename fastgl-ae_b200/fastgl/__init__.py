@@ -8,7 +8,8 @@ with the same names, positional arguments, dtypes, return lists and error behavi
     forward_gcn, backward_gcn, forwaed_gin (sic), backward_gin, forward_gat, backward_gat
 
 Each op allocates its outputs with torch and calls the C ABI of ``libfastgl_b200.so``
-(include/fastgl_b200.h) with raw device pointers and torch's current CUDA stream.  The dense weight
+(include/fastgl_b200.h) with raw device pointers and torch's current CUDA stream; the operators that run once or more
+per layer or mini-batch do so in one native call (``_ops``, csrc/torch_ops.cpp), the others through ctypes.  The dense weight
 products stay in torch (cuBLAS), as the reference keeps them in ``torch::mm``.  There is no CPU path:
 importing this module without the built library raises ImportError, and every op raises
 RuntimeError for a tensor that is not CUDA or not contiguous (aggregate_acc.cpp:4-6).
@@ -25,13 +26,13 @@ import threading
 
 import torch
 
-from . import _capi
+from . import _capi, _ops
 from ._capi import (AGG_MEAN, AGG_SUM, AGG_SYMNORM, COUNTS_STRIDE, FLAG_MAP_ARRIVAL_ORDER,
-                    FLAG_SAMPLE_REPLACE, FLAG_ZERO_DEG_PASSTHROUGH, MAX_HOPS, FusedArgs, lib)
+                    FLAG_SAMPLE_REPLACE, FLAG_ZERO_DEG_PASSTHROUGH, MAX_HOPS, lib)
 
 __all__ = [
     "sample_node", "transfer_edge_id", "cal_deg", "exclusive_sum", "forward_gcn", "backward_gcn",
-    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "sample_node_csr", "aggregate", "aggregate_backward", "aggregate_window",
+    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "sample_node_csr", "sample_blocks", "aggregate", "aggregate_backward", "aggregate_window",
     "sample_map_fused", "fused_capacity", "stage_segments", "stage_segments_raw", "gather_rows", "ShardedTable", "set_sampling", "seed", "FusedBatch",
     "exclusive_sum_noalloc", "exclusive_sum_noalloc_status", "check_status", "status_str", "PeerSync", "allreduce_adam_", "window_overlap", "TransposedBlock", "transpose_block", "split_tf32", "split_tf32_raw", "fold_blocks", "probe_access_pattern",
     "AGG_SUM", "AGG_MEAN", "AGG_SYMNORM",
@@ -39,6 +40,8 @@ __all__ = [
 
 # status codes of include/fastgl_b200.h that callers branch on
 ERR_CAPACITY, ERR_PROBE, ERR_BOUNDS, ERR_TIMEOUT = 4, 5, 6, 7
+
+_ops.init(_capi.LIB_PATH)
 
 _state_lock = threading.Lock()
 _workspaces: dict[int, ctypes.c_void_p] = {}
@@ -78,14 +81,9 @@ def _check_rows_f32(t: torch.Tensor, name: str) -> None:
 
 def _ws(device: torch.device) -> ctypes.c_void_p:
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    with _state_lock:
-        ws = _workspaces.get(idx)
-        if ws is None:
-            ws = ctypes.c_void_p()
-            rc = lib().fgl_ws_create(ctypes.c_int(idx), ctypes.byref(ws))
-            if rc != 0:
-                raise RuntimeError(f"fgl_ws_create(device={idx}) failed: {_capi.status_str(rc)}")
-            _workspaces[idx] = ws
+    ws = _workspaces.get(idx)
+    if ws is None:
+        ws = _workspaces[idx] = ctypes.c_void_p(_ops.workspace(idx))
     return ws
 
 
@@ -93,11 +91,17 @@ def _stream(device: torch.device) -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
-def _time_next_launch(dev, timing) -> None:
-    """Have the library record the pair of ``torch.cuda.Event`` directly around its next window-level launch."""
+def _recorded(timing):
+    """Addresses of a pair of ``torch.cuda.Event``."""
     for ev in timing:
         ev.record()         # torch creates the CUDA event at its first record; the library records it again
-    rc = lib().fgl_ws_time_next_launch(_ws(dev), ctypes.c_void_p(timing[0].cuda_event), ctypes.c_void_p(timing[1].cuda_event))
+    return timing[0].cuda_event, timing[1].cuda_event
+
+
+def _time_next_launch(dev, timing) -> None:
+    """Have the library record the pair of ``torch.cuda.Event`` directly around its next window-level launch."""
+    start, end = _recorded(timing)
+    rc = lib().fgl_ws_time_next_launch(_ws(dev), ctypes.c_void_p(start), ctypes.c_void_p(end))
     _raise(rc, "time_next_launch")
 
 
@@ -163,29 +167,10 @@ def _next_ctr() -> int:
 def sample_node_csr(src_edges, edge_ptr, seed_nodes, neighbor_num, replace=None, rng_seed=None, rng_ctr=None,
                     want_dst=True):
     """Sample and also return the block CSR offsets: (src_out, dst_out | None, block_indptr, n_edges)."""
-    _check_i32(src_edges, "src_edges")
-    _check_input(edge_ptr, "edge_ptr")
-    _check_i32(seed_nodes, "seed_nodes")
-    if edge_ptr.dtype not in (torch.int32, torch.int64):
-        raise RuntimeError("edge_ptr must be int32 or int64")
-    dev = seed_nodes.device
-    S = seed_nodes.numel()
-    fanout = int(neighbor_num)
-    out_src = torch.empty(max(1, S * fanout), dtype=torch.int32, device=dev)
-    out_dst = torch.empty(max(1, S * fanout), dtype=torch.int32, device=dev) if want_dst else None
-    out_ptr = torch.empty(S + 1, dtype=torch.int32, device=dev)
     flags = FLAG_SAMPLE_REPLACE if (_config["replace"] if replace is None else replace) else 0
-    n_edges = ctypes.c_int64(0)
-    ws = _ws(dev)
-    rc = lib().fgl_sample(ws, _ptr(edge_ptr), ctypes.c_int(1 if edge_ptr.dtype == torch.int64 else 0), _ptr(src_edges),
-                          ctypes.c_int64(edge_ptr.numel() - 1), _ptr(seed_nodes), ctypes.c_int32(S),
-                          ctypes.c_int32(fanout), ctypes.c_int32(flags),
-                          ctypes.c_uint64(_config["rng_seed"] if rng_seed is None else rng_seed),
-                          ctypes.c_uint64(_next_ctr() if rng_ctr is None else rng_ctr), _ptr(out_ptr), _ptr(out_src),
-                          _ptr(out_dst), ctypes.byref(n_edges), _stream(dev))
-    _raise(rc, "sample_node", ws)
-    E = int(n_edges.value)
-    return out_src[:E], (out_dst[:E] if want_dst else None), out_ptr, E
+    return _ops.sample_node_csr(src_edges, edge_ptr, seed_nodes, int(neighbor_num), flags,
+                                _config["rng_seed"] if rng_seed is None else rng_seed,
+                                _next_ctr() if rng_ctr is None else rng_ctr, bool(want_dst))
 
 
 def sample_node(src_edges, dst_edges, edge_ptr, seed_nodes, dst_nodes, neighbor_num):
@@ -213,24 +198,20 @@ def transfer_edge_id(src_edges, dst_edges, dst_edges_unique, dst_nodes, total_it
     ``[src_edges, dst_edges, unique_nodes]`` where ``unique_nodes`` = the seeds followed by every new
     source once (first-occurrence order unless ``set_sampling(arrival_order=True)``).
     """
-    _check_i32(src_edges, "src_edges")
-    _check_i32(dst_edges, "dst_edges")
-    _check_i32(dst_edges_unique, "dst_edges_unique")
-    dev = src_edges.device
-    S = min(int(dst_nodes), dst_edges_unique.numel())
-    E = int(edge_nums)
-    if E > src_edges.numel() or E > dst_edges.numel():
-        raise RuntimeError("edge_nums exceeds the edge arrays")
-    cap = S + max(0, min(int(unique_num), E))
-    unique = torch.empty(max(1, cap), dtype=torch.int32, device=dev)
-    n_unique = ctypes.c_int64(0)
     flags = FLAG_MAP_ARRIVAL_ORDER if _config["arrival_order"] else 0
-    ws = _ws(dev)
-    rc = lib().fgl_map(ws, _ptr(src_edges), _ptr(dst_edges), _ptr(dst_edges_unique), ctypes.c_int32(S),
-                       ctypes.c_int64(E), _ptr(unique), ctypes.c_int64(cap), ctypes.c_int32(flags),
-                       ctypes.byref(n_unique), _stream(dev))
-    _raise(rc, "transfer_edge_id", ws)
-    return [src_edges, dst_edges, unique[: int(n_unique.value)]]
+    unique = _ops.transfer_edge_id(src_edges, dst_edges, dst_edges_unique, int(dst_nodes), int(unique_num), int(edge_nums), flags)
+    return [src_edges, dst_edges, unique]
+
+
+def sample_blocks(src_edges, edge_ptr, seed_nodes, fanouts, replace=None, rng_seed=None, rng_ctr=None):
+    """Every hop of one mini-batch in one launch and one wait: ``(input_nodes, [(indptr, src, dst, n_src, n_dst), ...])``,
+    input layer first, with the same contents as ``sample_node_csr`` + ``transfer_edge_id`` hop by hop under the counters
+    ``rng_ctr + hop``; ``dst`` are the local destination ids of the edges.  ``fanouts`` in sampling order.  Returns None where
+    the worst case of the whole mini-batch is too large to be allocated at once: the caller then goes hop by hop."""
+    flags = FLAG_SAMPLE_REPLACE if (_config["replace"] if replace is None else replace) else 0
+    flags |= FLAG_MAP_ARRIVAL_ORDER if _config["arrival_order"] else 0
+    return _ops.sample_blocks(src_edges, edge_ptr, seed_nodes, [int(f) for f in fanouts], flags,
+                              _config["rng_seed"] if rng_seed is None else rng_seed, _next_ctr() if rng_ctr is None else rng_ctr)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -238,25 +219,12 @@ def transfer_edge_id(src_edges, dst_edges, dst_edges_unique, dst_nodes, total_it
 # ------------------------------------------------------------------------------------------------
 def cal_deg(edges, nodes_num):
     """aggregate_acc.cpp:522-529 -> cal_deg_cuda (utilis.cu:60-79): histogram of an id array."""
-    _check_i32(edges, "edges")
-    dev = edges.device
-    deg = torch.empty(int(nodes_num), dtype=torch.int32, device=dev)
-    with _on_device(dev):
-        rc = lib().fgl_cal_deg(_ptr(edges), ctypes.c_int64(edges.numel()), _ptr(deg), ctypes.c_int32(int(nodes_num)),
-                               _stream(dev))
-    _raise(rc, "cal_deg")
-    return deg
+    return _ops.cal_deg(edges, int(nodes_num))
 
 
 def exclusive_sum(in_degs):
     """aggregate_acc.cpp:514-520 -> exclusive_sum_cuda (utilis.cu:17-41): int32[n+1] offsets."""
-    _check_i32(in_degs, "in_degs")
-    dev = in_degs.device
-    out = torch.empty(in_degs.numel() + 1, dtype=torch.int32, device=dev)
-    ws = _ws(dev)
-    rc = lib().fgl_exclusive_sum(ws, _ptr(in_degs), ctypes.c_int64(in_degs.numel()), _ptr(out), _stream(dev))
-    _raise(rc, "exclusive_sum", ws)
-    return out
+    return _ops.exclusive_sum(in_degs)
 
 
 def exclusive_sum_noalloc(in_degs, out):
@@ -329,6 +297,8 @@ def _table_args(input_feat):
 
 def gather_rows(table, ids, out=None):
     """``out[i] = table[ids[i]]`` for a dense CUDA matrix or a ``ShardedTable``; ``ids`` int32."""
+    if not isinstance(table, ShardedTable):
+        return _ops.gather_rows(table, ids, out)
     _check_i32(ids, "ids")
     x, shards, rps, n_rows, ld, dim, dev = _table_args(table)
     if out is None:
@@ -352,12 +322,11 @@ def aggregate(mode, edge_ptr, src_edges, input_feat, dst_nodes, src_norm_degs=No
     AGG_SYMNORM); ``row_map`` (int32) turns block-local ids into rows of ``input_feat``.  ``n_dst_dev`` (int32
     CUDA tensor, optional) holds the real row count on the device; ``dst_nodes`` is then the padded count the
     output is sized for (used to replay a captured CUDA graph on blocks of different sizes)."""
+    if not isinstance(input_feat, ShardedTable):
+        return _ops.aggregate(int(mode), edge_ptr, src_edges, input_feat, int(dst_nodes), src_norm_degs, dst_norm_degs,
+                              bool(zero_deg_passthrough), row_map, out, n_dst_dev)
     _check_i32(edge_ptr, "edge_ptr")
     _check_i32(src_edges, "src_edges")
-    if not isinstance(input_feat, ShardedTable):
-        _check_f32(input_feat, "input_feat")
-        if input_feat.dim() != 2:
-            raise RuntimeError("input_feat must be 2-D")
     for t, n in ((src_norm_degs, "src_norm_degs"), (dst_norm_degs, "dst_norm_degs"), (row_map, "row_map")):
         if t is not None:
             _check_i32(t, n)
@@ -366,7 +335,7 @@ def aggregate(mode, edge_ptr, src_edges, input_feat, dst_nodes, src_norm_degs=No
         raise RuntimeError("edge_ptr is shorter than dst_nodes + 1")
     x, shards, rps, n_rows, ld, dim, dev = _table_args(input_feat)
     if mode == AGG_SYMNORM:
-        n_src = row_map.numel() if row_map is not None else (input_feat.size(0) if torch.is_tensor(input_feat) else None)
+        n_src = row_map.numel() if row_map is not None else None
         if (src_norm_degs is None or dst_norm_degs is None or dst_norm_degs.numel() < n_dst
                 or (n_src is not None and src_norm_degs.numel() < n_src)):
             raise RuntimeError("sym-norm needs src_norm_degs[n_src] and dst_norm_degs[n_dst]")
@@ -396,15 +365,18 @@ def aggregate_window(mode, fb, hop, input_feat, out, self_out=None, use_row_map=
     window's global node ids (aggregation straight from the feature table); ``self_out`` also receives each
     destination's own input row.  ``timing``: a pair of ``torch.cuda.Event`` that the library records directly around the
     kernel launch, so that the interval holds the kernel and not the host's way to it."""
+    row_off = [0]
+    for row in fb.counts_list():
+        row_off.append(row_off[-1] + row[hop])
+    if not isinstance(input_feat, ShardedTable) and row_off[-1] > 0:
+        start, end = (0, 0) if timing is None else _recorded(timing)
+        _ops.aggregate_window(int(mode), fb.counts, int(hop), row_off[-1], fb.block_indptr[hop], fb.block_src[hop],
+                              fb.nodes if use_row_map else None, input_feat, out, self_out, start, end)
+        return row_off
     x, shards, rps, n_rows, ld, dim, dev = _table_args(input_feat)
     _check_rows_f32(out, "out")
     if self_out is not None:
         _check_rows_f32(self_out, "self_out")
-    counts = fb.counts_host()
-    n_dst = counts[:, hop].tolist()
-    row_off = [0]
-    for n in n_dst:
-        row_off.append(row_off[-1] + int(n))
     if out.size(0) < row_off[-1] or (self_out is not None and self_out.size(0) < row_off[-1]):
         raise RuntimeError("out is too small for the window's destination rows")
     off_dev = torch.tensor(row_off, dtype=torch.int64).to(dev, non_blocking=True)
@@ -445,19 +417,13 @@ class TransposedBlock:
 def transpose_block(edge_ptr, src_edges, dst_nodes, src_nodes, n_dst_dev=None, out: TransposedBlock | None = None):
     """Transpose a block CSR (destination rows -> per-source lists).  ``src_edges`` holds at least ``edge_ptr[dst_nodes]``
     entries; ``out`` reuses buffers sized for at least ``src_nodes`` sources and ``src_edges.numel()`` edges."""
-    _check_i32(edge_ptr, "edge_ptr")
-    _check_i32(src_edges, "src_edges")
-    dev = edge_ptr.device
     n_src, n_dst = int(src_nodes), int(dst_nodes)
     if out is None:
-        out = TransposedBlock(n_src, src_edges.numel(), dev)
+        _check_i32(edge_ptr, "edge_ptr")
+        out = TransposedBlock(n_src, src_edges.numel(), edge_ptr.device)
     elif out.n_src < n_src or out.edge_cap < src_edges.numel():
         raise RuntimeError("the TransposedBlock is too small for this block")
-    ws = _ws(dev)
-    rc = lib().fgl_block_transpose(ws, _ptr(edge_ptr), _ptr(src_edges), ctypes.c_int32(n_dst), ctypes.c_int32(n_src),
-                                   _ptr(out.t_indptr), _ptr(out.t_dst), ctypes.c_int64(out.edge_cap), _ptr(out.hubs),
-                                   _ptr(out.work), _ptr(n_dst_dev), _stream(dev))
-    _raise(rc, "transpose_block", ws)
+    _ops.transpose_block(edge_ptr, src_edges, n_dst, n_src, n_dst_dev, out.t_indptr, out.t_dst, out.edge_cap, out.hubs, out.work)
     return out
 
 
@@ -468,57 +434,9 @@ def aggregate_backward(mode, edge_ptr, src_edges, d_out, src_nodes, src_norm_deg
     d_x starts from it in its first n_dst rows instead of from zero.  ``d_out`` may be a column slice too;
     ``out`` receives the result when given.  With ``transposed`` (``transpose_block`` of the same block) the result is
     gathered row by row in a fixed order -- bit-reproducible -- instead of scattered with atomic reductions."""
-    _check_i32(edge_ptr, "edge_ptr")
-    _check_i32(src_edges, "src_edges")
-    _check_rows_f32(d_out, "d_input")
-    for t, n in ((src_norm_degs, "src_norm_degs"), (dst_norm_degs, "dst_norm_degs")):
-        if t is not None:
-            _check_i32(t, n)
-    dev = d_out.device
-    n_dst, dim = d_out.size(0), d_out.size(1)
-    if mode == AGG_SYMNORM and (src_norm_degs is None or dst_norm_degs is None or src_norm_degs.numel() < int(src_nodes)
-                                or dst_norm_degs.numel() < n_dst):
-        raise RuntimeError("sym-norm needs src_norm_degs[src_nodes] and dst_norm_degs[n_dst]")
-    if edge_ptr.numel() < n_dst + 1:
-        raise RuntimeError("edge_ptr is shorter than n_dst + 1")
-    if out is None:
-        d_x = torch.empty((int(src_nodes), dim), dtype=torch.float32, device=dev)
-    else:
-        _check_rows_f32(out, "out")
-        if out.size(0) < int(src_nodes) or out.size(1) != dim:
-            raise RuntimeError("out must be float32[src_nodes, dim]")
-        d_x = out
-    if transposed is not None:
-        if d_self is not None:
-            _check_rows_f32(d_self, "d_self")
-            if d_self.size(0) != n_dst or d_self.size(1) != dim:
-                raise RuntimeError("d_self must be float32[n_dst, dim]")
-        ws = _ws(dev)
-        rc = lib().fgl_agg_bwd_gather(ws, ctypes.c_int32(mode), _ptr(edge_ptr), _ptr(transposed.t_indptr), _ptr(transposed.t_dst),
-                                      _ptr(transposed.hubs), _ptr(src_norm_degs), _ptr(dst_norm_degs), _ptr(d_out),
-                                      ctypes.c_int64(d_out.stride(0)), _ptr(d_self),
-                                      ctypes.c_int64(d_self.stride(0) if d_self is not None else dim), ctypes.c_int32(dim),
-                                      ctypes.c_int32(n_dst), ctypes.c_int32(int(src_nodes)), _ptr(d_x),
-                                      ctypes.c_int64(d_x.stride(0)), _ptr(n_dst_dev), _stream(dev))
-        _raise(rc, "aggregate_backward (gather)", ws)
-        return d_x
-    with _on_device(dev):
-        if d_self is None:
-            rc = lib().fgl_agg_bwd(_ws(dev), ctypes.c_int32(mode), _ptr(edge_ptr), _ptr(src_edges), _ptr(src_norm_degs),
-                                   _ptr(dst_norm_degs), _ptr(d_out), ctypes.c_int64(d_out.stride(0)), ctypes.c_int32(dim),
-                                   ctypes.c_int32(n_dst), ctypes.c_int32(int(src_nodes)), _ptr(d_x),
-                                   ctypes.c_int64(d_x.stride(0)), _ptr(n_dst_dev), _stream(dev))
-        else:
-            _check_rows_f32(d_self, "d_self")
-            if d_self.size(0) != n_dst or d_self.size(1) != dim:
-                raise RuntimeError("d_self must be float32[n_dst, dim]")
-            rc = lib().fgl_agg_bwd_self(_ws(dev), ctypes.c_int32(mode), _ptr(edge_ptr), _ptr(src_edges), _ptr(src_norm_degs),
-                                        _ptr(dst_norm_degs), _ptr(d_out), ctypes.c_int64(d_out.stride(0)), _ptr(d_self),
-                                        ctypes.c_int64(d_self.stride(0)), ctypes.c_int32(dim), ctypes.c_int32(n_dst),
-                                        ctypes.c_int32(int(src_nodes)), _ptr(d_x), ctypes.c_int64(d_x.stride(0)),
-                                        _ptr(n_dst_dev), _stream(dev))
-    _raise(rc, "aggregate_backward")
-    return d_x
+    tb = transposed
+    return _ops.aggregate_backward(int(mode), edge_ptr, src_edges, d_out, int(src_nodes), src_norm_degs, dst_norm_degs, n_dst_dev,
+                                   d_self, out, *((None, None, None) if tb is None else (tb.t_indptr, tb.t_dst, tb.hubs)))
 
 
 # ------------------------------------------------------------------------------------------------
@@ -828,22 +746,7 @@ def forward_gat(edge_ptr, edge_data, src_edges, input_feat, neighbor_num, dst_no
     ``edge_data`` float32[E, num_heads] holds one attention coefficient per edge and head; head ``h`` owns the
     columns ``[h * dim / num_heads, (h + 1) * dim / num_heads)`` of ``input_feat``.  Returns ``[out]`` with
     ``out[d] = sum_e edge_data[e, head] * input_feat[src[e]]``; a row without in-edges copies its own input row."""
-    _check_i32(edge_ptr, "edge_ptr")
-    _check_i32(src_edges, "src_edges")
-    _check_f32(edge_data, "edge_data")
-    _check_f32(input_feat, "input_feat")
-    H, dim, n_dst = int(num_heads), input_feat.size(1), int(dst_nodes)
-    if edge_data.dim() != 2 or edge_data.size(1) != H or dim % H != 0 or edge_data.size(0) < src_edges.numel():
-        raise RuntimeError("edge_data must be [n_edges, num_heads] and num_heads must divide the feature width")
-    dev = input_feat.device
-    out = torch.empty((n_dst, dim), dtype=torch.float32, device=dev)
-    with _on_device(dev):
-        rc = lib().fgl_agg_edge_fwd(_ws(dev), _ptr(edge_ptr), _ptr(src_edges), _ptr(edge_data), ctypes.c_int32(H), _ptr(input_feat),
-                                    ctypes.c_int32(input_feat.size(0)), ctypes.c_int64(input_feat.stride(0)),
-                                    ctypes.c_int32(dim), ctypes.c_int32(n_dst),
-                                    ctypes.c_int32(FLAG_ZERO_DEG_PASSTHROUGH), _ptr(out), ctypes.c_int64(dim), _stream(dev))
-    _raise(rc, "forward_gat")
-    return [out]
+    return _ops.forward_gat(edge_ptr, edge_data, src_edges, input_feat, int(dst_nodes), int(num_heads))
 
 
 def backward_gat(edge_ptr, edge_data, src_edges, d_input, src_nodes, num_heads):
@@ -851,40 +754,13 @@ def backward_gat(edge_ptr, edge_data, src_edges, d_input, src_nodes, num_heads):
 
     Returns ``[d_x]`` with ``d_x[src[e]] += edge_data[e, head] * d_input[d]``; like the reference, no gradient
     is produced for ``edge_data`` (GraphConv.py:227)."""
-    _check_i32(edge_ptr, "edge_ptr")
-    _check_i32(src_edges, "src_edges")
-    _check_f32(edge_data, "edge_data")
-    _check_f32(d_input, "d_input")
-    H, dim, n_dst = int(num_heads), d_input.size(1), d_input.size(0)
-    if edge_data.dim() != 2 or edge_data.size(1) != H or dim % H != 0:
-        raise RuntimeError("edge_data must be [n_edges, num_heads] and num_heads must divide the feature width")
-    dev = d_input.device
-    d_x = torch.empty((int(src_nodes), dim), dtype=torch.float32, device=dev)
-    with _on_device(dev):
-        rc = lib().fgl_agg_edge_bwd(_ws(dev), _ptr(edge_ptr), _ptr(src_edges), _ptr(edge_data), ctypes.c_int32(H), _ptr(d_input),
-                                    ctypes.c_int64(d_input.stride(0)), ctypes.c_int32(dim), ctypes.c_int32(n_dst),
-                                    ctypes.c_int32(int(src_nodes)), _ptr(d_x), ctypes.c_int64(dim), _stream(dev))
-    _raise(rc, "backward_gat")
-    return [d_x]
+    return _ops.backward_gat(edge_ptr, edge_data, src_edges, d_input, int(src_nodes), int(num_heads))
 
 
 def edge_weight_grad(edge_ptr, src_edges, input_feat, d_out, num_heads):
     """Gradient of ``forward_gat`` with respect to ``edge_data`` (not computed by the reference):
     ``d_w[e, h] = <d_out[d, head h], input_feat[src[e], head h]>`` for every edge ``e`` of row ``d``."""
-    _check_i32(edge_ptr, "edge_ptr")
-    _check_i32(src_edges, "src_edges")
-    _check_f32(input_feat, "input_feat")
-    _check_f32(d_out, "d_out")
-    H, dim, E = int(num_heads), d_out.size(1), src_edges.numel()
-    dev = d_out.device
-    d_w = torch.empty((E, H), dtype=torch.float32, device=dev)
-    with _on_device(dev):
-        rc = lib().fgl_agg_edge_wgrad(_ws(dev), _ptr(edge_ptr), _ptr(src_edges), ctypes.c_int32(H), _ptr(input_feat),
-                                      ctypes.c_int32(input_feat.size(0)), ctypes.c_int64(input_feat.stride(0)), _ptr(d_out), ctypes.c_int64(d_out.stride(0)),
-                                      ctypes.c_int32(dim), ctypes.c_int32(d_out.size(0)), ctypes.c_int64(E), _ptr(d_w),
-                                      _stream(dev))
-    _raise(rc, "edge_weight_grad")
-    return d_w
+    return _ops.edge_weight_grad(edge_ptr, src_edges, input_feat, d_out, int(num_heads))
 
 
 def forward_gcn(edge_ptr, src_edges, src_norm_degs, dst_norm_degs, input_feat, weight, neighbor_num, dst_nodes):
@@ -892,10 +768,7 @@ def forward_gcn(edge_ptr, src_edges, src_norm_degs, dst_norm_degs, input_feat, w
 
     ``tmp = input_feat @ weight`` then the sym-normalised neighbour sum; a row without in-edges returns
     ``tmp[row]``.  ``neighbor_num`` only sized the reference's shared memory and is not needed here."""
-    _check_f32(weight, "weight")
-    _check_f32(input_feat, "input_feat")
-    tmp = torch.mm(input_feat, weight)
-    return [aggregate(AGG_SYMNORM, edge_ptr, src_edges, tmp, dst_nodes, src_norm_degs, dst_norm_degs)]
+    return _ops.forward_gcn(edge_ptr, src_edges, src_norm_degs, dst_norm_degs, input_feat, weight, int(dst_nodes))
 
 
 def backward_gcn(edge_ptr, src_edges, src_norm_degs, dst_norm_degs, d_input, weight, input_feat):
@@ -904,11 +777,7 @@ def backward_gcn(edge_ptr, src_edges, src_norm_degs, dst_norm_degs, d_input, wei
     The third argument is indexed by the destination row and the fourth by the edge's source -- the
     reference kernel reads them that way (:490,:508) and GraphConv.py:37 passes the degree tensors in
     that (swapped) order.  Returns ``[d_x, d_w]``."""
-    _check_f32(weight, "weight")
-    _check_f32(input_feat, "input_feat")
-    d_out = aggregate_backward(AGG_SYMNORM, edge_ptr, src_edges, d_input, input_feat.size(0),
-                               src_norm_degs=dst_norm_degs, dst_norm_degs=src_norm_degs)
-    return [torch.mm(d_out, weight.t()), torch.mm(input_feat.t(), d_out)]
+    return _ops.backward_gcn(edge_ptr, src_edges, src_norm_degs, dst_norm_degs, d_input, weight, input_feat)
 
 
 def forwaed_gin(edge_ptr, src_edges, input_feat, weight, neighbor_num, dst_nodes):
@@ -916,9 +785,7 @@ def forwaed_gin(edge_ptr, src_edges, input_feat, weight, neighbor_num, dst_nodes
 
     The name keeps the reference's spelling.  Returns ``[tmp @ weight, tmp]`` with ``tmp`` the plain
     neighbour sum (a row without in-edges copies its own input row)."""
-    _check_f32(weight, "weight")
-    tmp = aggregate(AGG_SUM, edge_ptr, src_edges, input_feat, dst_nodes)
-    return [torch.mm(tmp, weight), tmp]
+    return _ops.forward_gin(edge_ptr, src_edges, input_feat, weight, int(dst_nodes))
 
 
 def backward_gin(edge_ptr, src_edges, d_input, weight, input_feat, src_nodes):
@@ -926,12 +793,7 @@ def backward_gin(edge_ptr, src_edges, d_input, weight, input_feat, src_nodes):
 
     ``input_feat`` is the aggregated ``tmp`` saved by the forward pass (GraphConv.py:117).  Returns
     ``[d_x, d_w]``."""
-    _check_f32(weight, "weight")
-    _check_f32(input_feat, "input_feat")
-    _check_f32(d_input, "d_input")
-    d_tmp = torch.mm(d_input, weight.t())
-    d_w = torch.mm(input_feat.t(), d_input)
-    return [aggregate_backward(AGG_SUM, edge_ptr, src_edges, d_tmp, src_nodes), d_w]
+    return _ops.backward_gin(edge_ptr, src_edges, d_input, weight, input_feat, int(src_nodes))
 
 
 # ------------------------------------------------------------------------------------------------
@@ -963,8 +825,10 @@ class FusedBatch:
         self.block_src = block_src
         self._arena = arena
         self._counts_host = None
-        self._counts_pinned = None
-        self._status_pinned = None
+        # pinned copies of the counts and of the workspace's status word, written by the sampling launch itself
+        self._counts_pinned = torch.empty(tuple(counts.shape), dtype=torch.int32, pin_memory=True)
+        self._status_pinned = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        self._event = torch.cuda.Event()
         self._readback = None
         self.device_status = 0   # the workspace's status word as of the last asynchronous read-back (0 = no error)
 
@@ -973,17 +837,10 @@ class FusedBatch:
         return self.nodes.size(0)
 
     def start_readback(self) -> None:
-        """Enqueue the copy of the counts to pinned host memory on the current stream, without waiting: the next
-        ``counts_host()`` waits for that copy only, not for work enqueued after it."""
-        dev = self.counts.device
-        if self._counts_pinned is None:
-            self._counts_pinned = torch.empty(self.counts.shape, dtype=self.counts.dtype).pin_memory()
-            self._status_pinned = torch.zeros(1, dtype=torch.int32).pin_memory()
-        self._counts_pinned.copy_(self.counts, non_blocking=True)
-        ws = _ws(dev)
-        _raise(lib().fgl_ws_status_peek(ws, ctypes.c_void_p(self._status_pinned.data_ptr()), _stream(dev)), "status_peek", ws)
-        self._readback = torch.cuda.Event()
-        self._readback.record(torch.cuda.current_stream(self.counts.device))
+        """Mark the point of the current stream behind the launch that writes the counts to pinned host memory, without
+        waiting: the next ``counts_host()`` waits for that point only, not for work enqueued after it."""
+        self._event.record(torch.cuda.current_stream(self.counts.device))
+        self._readback = self._event
 
     def counts_host(self) -> torch.Tensor:
         if self._counts_host is None:
@@ -1026,10 +883,7 @@ def sample_map_fused(edge_ptr, src_edges, seeds, seed_counts, fanouts, replace=N
     order (the reference walks ``reversed(self.fanouts)``, FusedMapSampler.py:72).  Nothing is copied to
     the host; pass ``out`` (a previous result of the same geometry) to reuse its buffers.  ``timing``: a pair of
     ``torch.cuda.Event`` that the library records directly around the kernel launch (``fgl_ws_time_next_launch``)."""
-    _check_i32(src_edges, "src_edges")
-    _check_input(edge_ptr, "edge_ptr")
     _check_i32(seeds, "seeds")
-    _check_i32(seed_counts, "seed_counts")
     if seeds.dim() != 2 or seed_counts.numel() != seeds.size(0):
         raise RuntimeError("seeds must be [n_batches, seed_stride] with one count per batch")
     if edge_ptr.dtype not in (torch.int32, torch.int64):
@@ -1038,10 +892,9 @@ def sample_map_fused(edge_ptr, src_edges, seeds, seed_counts, fanouts, replace=N
     if not 1 <= L <= MAX_HOPS:
         raise RuntimeError(f"1..{MAX_HOPS} hops supported")
     dev = seeds.device
-    nb, stride = seeds.size(0), seeds.size(1)
-    n_nodes = edge_ptr.numel() - 1
-    cap = fused_capacity(n_nodes, stride, fanouts)
     if out is None:
+        nb, stride = seeds.size(0), seeds.size(1)
+        cap = fused_capacity(edge_ptr.numel() - 1, stride, fanouts)
         sizes = [cap[L], COUNTS_STRIDE] + [cap[h] + 1 for h in range(L)] + [cap[h] * int(fanouts[h]) for h in range(L)]
         # 128-byte aligned rows, except the counts rows whose stride the ABI fixes
         sizes = [s if i == 1 else (s + 31) // 32 * 32 for i, s in enumerate(sizes)]
@@ -1053,38 +906,16 @@ def sample_map_fused(edge_ptr, src_edges, seeds, seed_counts, fanouts, replace=N
         out = FusedBatch(fanouts, views[0], views[1], views[2: 2 + L], views[2 + L: 2 + 2 * L], arena)
     out._counts_host = None
     out._readback = None
-    a = FusedArgs()
-    a.indptr = edge_ptr.data_ptr()
-    a.indices = src_edges.data_ptr()
-    a.n_nodes = n_nodes
-    a.indptr_is_64 = 1 if edge_ptr.dtype == torch.int64 else 0
-    a.n_batches = nb
-    a.n_hops = L
-    for h in range(L):
-        a.fanout[h] = int(fanouts[h])
-        a.block_indptr[h] = out.block_indptr[h].data_ptr()
-        a.block_indptr_stride[h] = out.block_indptr[h].stride(0)
-        a.block_src[h] = out.block_src[h].data_ptr()
-        a.block_src_stride[h] = out.block_src[h].stride(0)
     use_replace = _config["replace"] if replace is None else replace
     use_arrival = _config["arrival_order"] if arrival_order is None else arrival_order
-    a.flags = (FLAG_SAMPLE_REPLACE if use_replace else 0) | (FLAG_MAP_ARRIVAL_ORDER if use_arrival else 0)
-    a.n_teams = int(n_teams)
-    a.table_slots_hint = int(table_slots)
-    a.rng_seed = _config["rng_seed"] if rng_seed is None else rng_seed
-    a.rng_ctr = _next_ctr() if rng_ctr is None else rng_ctr
-    a.seeds = seeds.data_ptr()
-    a.seed_stride = seeds.stride(0)
-    a.seed_counts = seed_counts.data_ptr()
-    a.nodes = out.nodes.data_ptr()
-    a.nodes_stride = out.nodes.stride(0)
-    a.counts = out.counts.data_ptr()
-    ws = _ws(dev)
+    flags = (FLAG_SAMPLE_REPLACE if use_replace else 0) | (FLAG_MAP_ARRIVAL_ORDER if use_arrival else 0)
     if timing is not None:
         with _on_device(dev):
             _time_next_launch(dev, timing)
-    rc = lib().fgl_sample_map_fused(ws, ctypes.byref(a), _stream(dev))
-    _raise(rc, "sample_map_fused", ws)
+    _ops.sample_map_fused(edge_ptr, src_edges, seeds, seed_counts, [int(f) for f in fanouts], flags,
+                          _config["rng_seed"] if rng_seed is None else rng_seed, _next_ctr() if rng_ctr is None else rng_ctr,
+                          int(n_teams), int(table_slots), out.nodes, out.counts, out.block_indptr, out.block_src,
+                          out._counts_pinned, out._status_pinned)
     return out
 
 
@@ -1114,25 +945,7 @@ def stage_segments(copies, words_dst=None, words=()):
     """``copies``: up to 8 ``(dst, src)`` pairs of CUDA tensors (``src.numel()`` elements of a 4-byte dtype are
     copied to the front of ``dst``); ``words`` (up to 8 ints) are written to the int32 tensor ``words_dst``.
     One kernel launch on the current stream."""
-    n = len(copies)
-    if n > _capi.MAX_SEGMENTS or len(words) > _capi.MAX_SEGMENTS:
-        raise RuntimeError("at most 8 copies and 8 words per call")
-    segs = (_capi.Segment * max(1, n))()
-    dev = None
-    for i, (dst, src) in enumerate(copies):
-        if dst.element_size() != 4 or src.element_size() != 4 or not dst.is_cuda or not src.is_cuda:
-            raise RuntimeError("stage_segments copies 4-byte CUDA tensors")
-        if dst.numel() < src.numel() or not src.is_contiguous() or not dst.is_contiguous():
-            raise RuntimeError("stage_segments needs contiguous tensors and a destination at least as large as the source")
-        segs[i].dst, segs[i].src, segs[i].bytes = dst.data_ptr(), src.data_ptr(), src.numel() * 4
-        dev = dst.device
-    if words_dst is not None:
-        _check_i32(words_dst, "words_dst")
-        dev = words_dst.device
-    vals = (ctypes.c_int32 * max(1, len(words)))(*[int(w) for w in words])
-    with _on_device(dev):
-        rc = lib().fgl_stage_segments(segs, ctypes.c_int32(n), _ptr(words_dst), vals, ctypes.c_int32(len(words)), _stream(dev))
-    _raise(rc, "stage_segments")
+    _ops.stage_segments(copies, words_dst, words)
 
 
 def stage_segments_raw(segments, words_dst_ptr, words, device):

@@ -1,9 +1,9 @@
 """The Fused-Map sampler on top of the ``fastgl`` ops.
 
 ``FusedMapSampler.sample_blocks`` keeps the reference's per-hop loop and return value
-(FusedMapSampler.py:63-109): walk ``reversed(fanouts)``, ``fastgl.sample_node`` then
-``fastgl.transfer_edge_id``, the unique nodes of one hop are the seeds of the next, blocks come back
-input-layer first.  ``sample_window`` is the B200 path: every hop of a whole window of mini-batches (the
+(FusedMapSampler.py:63-109): walk ``reversed(fanouts)``, the unique nodes of one hop are the seeds of the next,
+blocks come back input-layer first -- in one launch and one wait (``fastgl.sample_blocks``), or with
+``fastgl.sample_node`` and ``fastgl.transfer_edge_id`` per hop where the worst case of a mini-batch is too large.  ``sample_window`` is the B200 path: every hop of a whole window of mini-batches (the
 batches Match-Reorder looks at together, utilis.py:35-39) in one persistent kernel launch, with a single
 read-back of the per-batch counts.
 """
@@ -37,6 +37,11 @@ class FusedMapSampler:
         blocks = []
         ctr = self.batch_counter * 8
         self.batch_counter += 1
+        at_once = fastgl.sample_blocks(self.edge_src, self.edge_ptr, cur, self.fanouts[::-1], replace=self.replace,
+                                       rng_seed=self.rng_seed, rng_ctr=ctr)
+        if at_once is not None:
+            input_nodes, parts = at_once
+            return input_nodes, output_nodes, [Block(ptr, src, n_src, n_dst, dst) for ptr, src, dst, n_src, n_dst in parts]
         for hop, fanout in enumerate(reversed(self.fanouts)):
             src_g, dst_g, ptr, n_edges = fastgl.sample_node_csr(self.edge_src, self.edge_ptr, cur, fanout,
                                                                 replace=self.replace, rng_seed=self.rng_seed,

@@ -165,6 +165,19 @@ int fgl_fused_capacity(int64_t n_nodes, int32_t max_seeds, int32_t n_hops, const
                        int64_t* cap_nodes /* n_hops + 1 */);
 int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* args, void* stream);
 
+/* The same launch with further outputs, each of which may be NULL; args->seed_counts may be NULL too (every mini-batch has
+ * seed_stride seeds).  block_dst[h] (n_batches == 1 only) receives the
+ * block-local destination id of every edge of hop h (what fgl_map leaves in dst).  counts_host and status_host are
+ * pinned host memory that the kernel itself writes: the counts rows, and the workspace's status word if it is not zero
+ * (the caller zeroes it before the launch).  They hold their values once the launch has completed, so that waiting for
+ * an event behind it is all a read-back takes. */
+typedef struct fgl_fused_extra {
+    int32_t* block_dst[FGL_MAX_HOPS];
+    int32_t* counts_host;
+    int32_t* status_host;
+} fgl_fused_extra;
+int fgl_sample_map_fused_extra(fgl_ws* ws, const fgl_fused_args* args, const fgl_fused_extra* extra, void* stream);
+
 /* Histogram of an id array; replaces cal_deg_cuda (utilis.cu:60-79; binding aggregate_acc.cpp:522-529).
  * deg[0 .. n_nodes) is zeroed and then counts the occurrences of each id. */
 int fgl_cal_deg(const int32_t* ids, int64_t n_ids, int32_t* deg, int32_t n_nodes, void* stream);
@@ -282,6 +295,14 @@ int fgl_gather_rows(fgl_ws* ws, const float* table, const float* const* shards, 
 int fgl_agg_fwd_window(fgl_ws* ws, int32_t mode, int32_t n_batches, const int32_t* indptr, int64_t indptr_stride,
                        const int32_t* src, int64_t src_stride, const int32_t* row_map, int64_t row_map_stride,
                        const int64_t* out_row_off, int64_t total_rows, const float* x, const float* const* shards,
+                       int64_t rows_per_shard, int64_t n_rows, int64_t ldx, int32_t dim, int32_t flags, float* out,
+                       int64_t ldo, float* self_out, int64_t ld_self, void* stream);
+
+/* fgl_agg_fwd_window with the row offsets taken on the device: batch b has counts[b * counts_stride] destination rows
+ * (the hop's column of the counts that fgl_sample_map_fused leaves), and its rows follow those of batch b - 1. */
+int fgl_agg_fwd_window_counts(fgl_ws* ws, int32_t mode, int32_t n_batches, const int32_t* indptr, int64_t indptr_stride,
+                       const int32_t* src, int64_t src_stride, const int32_t* row_map, int64_t row_map_stride,
+                       const int32_t* counts, int64_t counts_stride, int64_t total_rows, const float* x, const float* const* shards,
                        int64_t rows_per_shard, int64_t n_rows, int64_t ldx, int32_t dim, int32_t flags, float* out,
                        int64_t ldo, float* self_out, int64_t ld_self, void* stream);
 
