@@ -273,7 +273,7 @@ struct Hop {
     int32_t* sums;         // fused: edge counts of this hop's node tiles ...
     int32_t* next_sums;    // ... and of the next hop's, which this hop's new nodes are added to
     int tile_shift, next_shift, next_fanout;
-    int hop, fanout, n_seeds;
+    int hop, fanout, n_seeds, n_first;  // n_first: the mini-batch's own seeds, which may hold a node twice
     bool last_hop;
     uint64_t ctr;
 };
@@ -778,7 +778,7 @@ __device__ __forceinline__ bool phase_sample(const KParams& p, const Hop& h, Tab
             }
             k = min(deg, h.fanout);
             // what goes into out_dst: the seed itself, or its local id (of two equal seeds, the later one's)
-            sm.v[threadIdx.x] = (MODE == MODE_FUSED && h.out_dst) ? (h.hop == 0 && k > 0 ? table_lookup(tab, (uint32_t)v, p.status) : s) : v;
+            sm.v[threadIdx.x] = (MODE == MODE_FUSED && h.out_dst) ? (s < h.n_first && k > 0 ? table_lookup(tab, (uint32_t)v, p.status) : s) : v;
             sm.start[threadIdx.x] = start;
             sm.deg[threadIdx.x] = deg;
         }
@@ -1037,6 +1037,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
         int n0 = p.seed_counts ? __ldg(p.seed_counts + b) : p.n_seeds_host;
         n0 = max(0, min(n0, (int)min((int64_t)0x7fffffff, p.seed_stride)));
         const int32_t* seeds = p.seeds + (size_t)b * p.seed_stride;
+        h.n_first = n0;
 
         int log2 = p.table_log2_first;
         unsigned used = 1u << log2;

@@ -33,7 +33,8 @@ void* g_lib = nullptr;
     X(fgl_status_str) X(fgl_last_error) X(fgl_ws_create) X(fgl_ws_check) X(fgl_sample) X(fgl_map) X(fgl_fused_capacity) \
     X(fgl_sample_map_fused_extra) X(fgl_cal_deg) X(fgl_exclusive_sum) X(fgl_stage_segments) X(fgl_agg_fwd)              \
     X(fgl_agg_fwd_window_counts) X(fgl_agg_edge_fwd) X(fgl_agg_edge_bwd) X(fgl_agg_edge_wgrad) X(fgl_agg_bwd)            \
-    X(fgl_agg_bwd_self) X(fgl_block_transpose) X(fgl_agg_bwd_gather) X(fgl_gather_rows) X(fgl_ws_time_next_launch)
+    X(fgl_agg_bwd_self) X(fgl_block_transpose) X(fgl_agg_bwd_gather) X(fgl_gather_rows) X(fgl_ws_time_next_launch)           \
+    X(fgl_gat_fwd) X(fgl_gat_bwd) X(fgl_gat_bwd_partials) X(fgl_softmax_xent) X(fgl_adam_step)
 
 struct Api {
 #define FGL_FIELD(name) decltype(&::name) name = nullptr;
@@ -574,6 +575,78 @@ at::Tensor edge_weight_grad(py::handle ptr_o, py::handle src_o, py::handle x_o, 
     return dw;
 }
 
+// Attention of a GAT layer behind its linear map: (out, alpha, el, er).
+py::tuple gat_attention(py::handle ptr_o, py::handle src_o, py::handle feat_o, py::handle l_o, py::handle r_o, int64_t n_dst, int64_t heads,
+                        double slope) {
+    const at::Tensor &edge_ptr = i32(ptr_o, "edge_ptr"), &src = i32(src_o, "src_edges"), &feat = rows_f32(feat_o, "feat"),
+                     &l = f32(l_o, "attn_l"), &r = f32(r_o, "attn_r");
+    const int64_t dim = feat.size(1);
+    TORCH_CHECK(heads >= 1 && dim % heads == 0 && l.numel() == dim && r.numel() == dim && n_dst <= feat.size(0) && edge_ptr.numel() >= n_dst + 1,
+                "gat_attention: the attention vectors must have the feature width, and the destinations be the first sources");
+    Call c(feat);
+    auto opt = feat.options();
+    at::Tensor out = at::empty({n_dst, dim}, opt), alpha = at::empty({src.numel(), heads}, opt), el = at::empty({feat.size(0), heads}, opt),
+               er = at::empty({n_dst, heads}, opt);
+    check(api.fgl_gat_fwd(c.ws, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), ptr<float>(feat), feat.stride(0), ptr<float>(l), ptr<float>(r),
+                          (int32_t)heads, (int32_t)(dim / heads), (int32_t)n_dst, (int32_t)feat.size(0), (float)slope, ptr<float>(el),
+                          ptr<float>(er), ptr<float>(alpha), ptr<float>(out), dim, c.st()), "gat_attention");
+    return py::make_tuple(out, alpha, el, er);
+}
+
+// (d_feat, d_attn_l, d_attn_r)
+py::tuple gat_attention_backward(py::handle ptr_o, py::handle src_o, py::handle feat_o, py::handle l_o, py::handle r_o, py::handle el,
+                                 py::handle er, py::handle alpha, py::handle dy_o, int64_t heads, double slope) {
+    const at::Tensor &edge_ptr = i32(ptr_o, "edge_ptr"), &src = i32(src_o, "src_edges"), &feat = rows_f32(feat_o, "feat"),
+                     &dy = rows_f32(dy_o, "d_out"), &l = f32(l_o, "attn_l"), &r = f32(r_o, "attn_r");
+    const int64_t dim = feat.size(1), n_dst = dy.size(0), E = src.numel();
+    Call c(feat);
+    auto opt = feat.options();
+    const int rows = api.fgl_gat_bwd_partials(c.ws, (int32_t)heads, (int32_t)(dim / heads), (int32_t)n_dst);
+    at::Tensor scratch = at::empty({(int64_t)rows * 2 * dim + (E + n_dst) * heads}, opt);
+    at::Tensor dfeat = at::empty({feat.size(0), dim}, opt), dattn = at::empty({2, dim}, opt);
+    check(api.fgl_gat_bwd(c.ws, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), ptr<float>(feat), feat.stride(0), ptr<float>(l), ptr<float>(r),
+                          ptr<float>(f32(el, "el")), ptr<float>(f32(er, "er")), ptr<float>(f32(alpha, "alpha")), ptr<float>(dy),
+                          dy.stride(0), (int32_t)heads, (int32_t)(dim / heads), (int32_t)n_dst, (int32_t)feat.size(0), E, (float)slope,
+                          ptr<float>(scratch), ptr<float>(dfeat), ptr<float>(dattn), c.st()), "gat_attention_backward");
+    return py::make_tuple(dfeat, dattn.select(0, 0).view(l.sizes()), dattn.select(0, 1).view(r.sizes()));
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// loss and optimizer
+// ---------------------------------------------------------------------------------------------------------------------
+py::tuple softmax_xent(py::handle logits_o, py::handle labels_o, py::handle ids_o, py::handle n_valid_o, py::handle loss_o, py::handle d_o,
+                       py::handle rows_o) {
+    const at::Tensor &logits = rows_f32(logits_o, "logits"), &labels = input(labels_o, "labels");
+    TORCH_CHECK(labels.scalar_type() == at::kLong, "labels must be int64");
+    const at::Tensor ids = optional_i32(ids_o, "label_ids");
+    const int64_t n = logits.size(0), classes = logits.size(1);
+    Call c(logits);
+    auto opt = logits.options();
+    at::Tensor loss = loss_o.is_none() ? at::empty({1}, opt) : tensor(loss_o, "loss");
+    at::Tensor d = d_o.is_none() ? at::empty({n, classes}, opt) : rows_f32(d_o, "dlogits");
+    at::Tensor rows = rows_o.is_none() ? at::empty({std::max<int64_t>(n, 1)}, opt) : f32(rows_o, "row_loss");
+    TORCH_CHECK(rows.numel() >= n, "row_loss must hold one float per row");
+    const bool on_device = THPVariable_Check(n_valid_o.ptr());
+    const at::Tensor n_dev = on_device ? i32(n_valid_o, "n_valid") : at::Tensor();
+    const int64_t n_host = on_device || n_valid_o.is_none() ? n : n_valid_o.cast<int64_t>();
+    check(api.fgl_softmax_xent(c.ws, ptr<float>(logits), logits.stride(0), ptr<int64_t>(labels), ptr<int32_t>(ids), labels.numel(), (int32_t)n,
+                               (int32_t)classes, ptr<int32_t>(n_dev), (int32_t)n_host, ptr<float>(loss), ptr<float>(d), d.stride(0),
+                               ptr<float>(rows), c.st()), "softmax_xent", c.ws);
+    return py::make_tuple(loss, d);
+}
+
+void adam_step(py::handle p_o, py::handle g_o, py::handle m_o, py::handle v_o, py::handle step_o, double lr, double b1, double b2, double eps,
+               double wd) {
+    const at::Tensor &p = f32(p_o, "param"), &g = f32(g_o, "grad"), &m = f32(m_o, "exp_avg"), &v = f32(v_o, "exp_avg_sq"),
+                     &step = i32(step_o, "step_dev");
+    TORCH_CHECK(g.numel() == p.numel() && m.numel() == p.numel() && v.numel() == p.numel(),
+                "param, grad and the two moment buffers must have the same length");
+    TORCH_CHECK(step.numel() >= 2, "step_dev must hold two int32 words");
+    Call c(p);
+    check(api.fgl_adam_step(ptr<float>(p), ptr<float>(g), ptr<float>(m), ptr<float>(v), p.numel(), (float)lr, (float)b1, (float)b2, (float)eps,
+                            (float)wd, ptr<int32_t>(step), c.st()), "adam_step_");
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_ops, m) {
@@ -598,4 +671,8 @@ PYBIND11_MODULE(_ops, m) {
     m.def("forward_gat", &forward_gat);
     m.def("backward_gat", &backward_gat);
     m.def("edge_weight_grad", &edge_weight_grad);
+    m.def("softmax_xent", &softmax_xent);
+    m.def("adam_step", &adam_step);
+    m.def("gat_attention", &gat_attention);
+    m.def("gat_attention_backward", &gat_attention_backward);
 }

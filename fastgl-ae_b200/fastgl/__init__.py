@@ -32,7 +32,7 @@ from ._capi import (AGG_MEAN, AGG_SUM, AGG_SYMNORM, COUNTS_STRIDE, FLAG_MAP_ARRI
 
 __all__ = [
     "sample_node", "transfer_edge_id", "cal_deg", "exclusive_sum", "forward_gcn", "backward_gcn",
-    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "sample_node_csr", "sample_blocks", "aggregate", "aggregate_backward", "aggregate_window",
+    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "gat_attention", "gat_attention_backward", "sample_node_csr", "sample_blocks", "aggregate", "aggregate_backward", "aggregate_window",
     "sample_map_fused", "fused_capacity", "stage_segments", "stage_segments_raw", "gather_rows", "ShardedTable", "set_sampling", "seed", "FusedBatch",
     "exclusive_sum_noalloc", "exclusive_sum_noalloc_status", "check_status", "status_str", "PeerSync", "allreduce_adam_", "window_overlap", "TransposedBlock", "transpose_block", "split_tf32", "split_tf32_raw", "fold_blocks", "probe_access_pattern",
     "AGG_SUM", "AGG_MEAN", "AGG_SYMNORM",
@@ -508,32 +508,7 @@ def softmax_xent(logits, labels, label_ids=None, n_valid=None, loss=None, dlogit
     """Mean softmax cross-entropy over the first ``n_valid`` rows (an int, an int32 CUDA tensor read on the device, or
     all rows) and its gradient: returns (loss float32[1], dlogits).  ``row_loss`` (float32[n_rows]) is scratch.  Row r's label is ``labels[label_ids[r]]`` when
     ``label_ids`` (int32) is given, else ``labels[r]``; ``labels`` is int64."""
-    _check_rows_f32(logits, "logits")
-    _check_input(labels, "labels")
-    if labels.dtype != torch.int64:
-        raise RuntimeError("labels must be int64")
-    if label_ids is not None:
-        _check_i32(label_ids, "label_ids")
-    dev = logits.device
-    n_rows, n_classes = logits.size(0), logits.size(1)
-    loss = torch.empty(1, dtype=torch.float32, device=dev) if loss is None else loss
-    dlogits = torch.empty((n_rows, n_classes), dtype=torch.float32, device=dev) if dlogits is None else dlogits
-    _check_rows_f32(dlogits, "dlogits")
-    row_loss = torch.empty(max(n_rows, 1), dtype=torch.float32, device=dev) if row_loss is None else row_loss
-    _check_f32(row_loss, "row_loss")
-    if row_loss.numel() < n_rows:
-        raise RuntimeError("row_loss must hold one float per row")
-    n_valid_dev = n_valid if torch.is_tensor(n_valid) else None
-    if n_valid_dev is not None:
-        _check_i32(n_valid_dev, "n_valid")
-    ws = _ws(dev)
-    with _on_device(dev):
-        rc = lib().fgl_softmax_xent(ws, _ptr(logits), ctypes.c_int64(logits.stride(0)), _ptr(labels), _ptr(label_ids),
-                                    ctypes.c_int64(labels.numel()), ctypes.c_int32(n_rows), ctypes.c_int32(n_classes),
-                                    _ptr(n_valid_dev), ctypes.c_int32(n_rows if n_valid is None or n_valid_dev is not None else int(n_valid)),
-                                    _ptr(loss), _ptr(dlogits), ctypes.c_int64(dlogits.stride(0)), _ptr(row_loss), _stream(dev))
-    _raise(rc, "softmax_xent", ws)
-    return loss, dlogits
+    return _ops.softmax_xent(logits, labels, label_ids, n_valid, loss, dlogits, row_loss)
 
 
 def linear_softmax_xent(x, weight, bias, labels, label_ids=None, n_valid=None, loss=None, dlogits=None, row_loss=None,
@@ -584,19 +559,7 @@ def linear_softmax_xent(x, weight, bias, labels, label_ids=None, n_valid=None, l
 def adam_step_(param, grad, exp_avg, exp_avg_sq, step_dev, lr=1e-3, betas=(0.9, 0.999), eps=1e-8, weight_decay=0.0):
     """One Adam step (torch.optim.Adam's arithmetic, L2 weight decay) over flat float32 buffers, in place.
     ``step_dev``: int32[2] CUDA tensor, zero before the first step; the launch itself advances ``step_dev[0]``."""
-    for t, n in ((param, "param"), (grad, "grad"), (exp_avg, "exp_avg"), (exp_avg_sq, "exp_avg_sq")):
-        _check_f32(t, n)
-        if t.numel() != param.numel():
-            raise RuntimeError("param, grad and the two moment buffers must have the same length")
-    _check_i32(step_dev, "step_dev")
-    if step_dev.numel() < 2:
-        raise RuntimeError("step_dev must hold two int32 words")
-    dev = param.device
-    with _on_device(dev):
-        rc = lib().fgl_adam_step(_ptr(param), _ptr(grad), _ptr(exp_avg), _ptr(exp_avg_sq), ctypes.c_int64(param.numel()),
-                                 ctypes.c_float(lr), ctypes.c_float(betas[0]), ctypes.c_float(betas[1]), ctypes.c_float(eps),
-                                 ctypes.c_float(weight_decay), _ptr(step_dev), _stream(dev))
-    _raise(rc, "adam_step_")
+    _ops.adam_step(param, grad, exp_avg, exp_avg_sq, step_dev, lr, betas[0], betas[1], eps, weight_decay)
 
 
 def split_tf32(x, dst=None):
@@ -761,6 +724,20 @@ def edge_weight_grad(edge_ptr, src_edges, input_feat, d_out, num_heads):
     """Gradient of ``forward_gat`` with respect to ``edge_data`` (not computed by the reference):
     ``d_w[e, h] = <d_out[d, head h], input_feat[src[e], head h]>`` for every edge ``e`` of row ``d``."""
     return _ops.edge_weight_grad(edge_ptr, src_edges, input_feat, d_out, int(num_heads))
+
+
+def gat_attention(edge_ptr, src_edges, feat, attn_l, attn_r, dst_nodes, num_heads, negative_slope=0.2):
+    """Attention of a GAT layer behind its linear map (GraphConv.py:262-283) in two launches: scores
+    ``leaky_relu(<feat, attn_l>[src] + <feat, attn_r>[dst])`` per head, softmax over every row's in-edges, weighted sum.
+    ``feat`` float32[n_src, num_heads * width], the destinations first.  Returns ``(out, alpha, el, er)``; the last three
+    are what ``gat_attention_backward`` takes."""
+    return _ops.gat_attention(edge_ptr, src_edges, feat, attn_l, attn_r, int(dst_nodes), int(num_heads), float(negative_slope))
+
+
+def gat_attention_backward(edge_ptr, src_edges, feat, attn_l, attn_r, el, er, alpha, d_out, num_heads, negative_slope=0.2):
+    """Gradients ``(d_feat, d_attn_l, d_attn_r)`` of ``gat_attention``."""
+    return _ops.gat_attention_backward(edge_ptr, src_edges, feat, attn_l, attn_r, el, er, alpha, d_out, int(num_heads),
+                                       float(negative_slope))
 
 
 def forward_gcn(edge_ptr, src_edges, src_norm_degs, dst_norm_degs, input_feat, weight, neighbor_num, dst_nodes):

@@ -209,6 +209,33 @@ def edge_softmax(e: torch.Tensor, dst: torch.Tensor, n_dst: int) -> torch.Tensor
     return ex / denom[idx]
 
 
+class _GATAttention(torch.autograd.Function):
+    """``fastgl.gat_attention`` with its gradients.  With ``attention_grad=False`` the coefficients are constants, as in the
+    reference: only the weighted sum is differentiated."""
+
+    @staticmethod
+    def forward(ctx, edge_ptr, src_edges, n_dst, feat, attn_l, attn_r, num_heads, slope, attention_grad):
+        out, alpha, el, er = fastgl.gat_attention(edge_ptr, src_edges, feat, attn_l, attn_r, n_dst, num_heads, slope)
+        ctx.num_heads, ctx.slope, ctx.attention_grad, ctx.n_src = num_heads, slope, attention_grad, feat.size(0)
+        ctx.save_for_backward(edge_ptr, src_edges, feat, attn_l, attn_r, alpha, el, er)
+        return out
+
+    @staticmethod
+    def backward(ctx, d_out):
+        edge_ptr, src_edges, feat, attn_l, attn_r, alpha, el, er = ctx.saved_tensors
+        d_out = d_out.contiguous()
+        if not ctx.attention_grad:
+            d_feat = fastgl.backward_gat(edge_ptr, alpha, src_edges, d_out, ctx.n_src, ctx.num_heads)[0]
+            return None, None, None, d_feat, None, None, None, None, None
+        d_feat, d_l, d_r = fastgl.gat_attention_backward(edge_ptr, src_edges, feat, attn_l, attn_r, el, er, alpha, d_out,
+                                                         ctx.num_heads, ctx.slope)
+        return None, None, None, d_feat, d_l, d_r, None, None, None
+
+
+# two rows of column sums fit the shared memory of a CTA up to this width (fgl_gat_bwd)
+_GAT_MAX_DIM = 24 * 1024
+
+
 class GATConv(nn.Module):
     """GraphConv.py:231-283: shared linear map, additive attention, edge softmax, weighted multi-head sum."""
 
@@ -229,13 +256,18 @@ class GATConv(nn.Module):
     def forward(self, block, input_feat, neighbor_num):
         n_dst = block.num_dst_nodes()
         feat_src = self.fc(input_feat).view(-1, self.num_heads, self.out_feats)
+        edge_ptr, src_edges = block_csr(block)
+        flat = feat_src.reshape(-1, self.num_heads * self.out_feats)
+        if (flat.is_cuda and flat.dtype == torch.float32 and flat.size(1) <= _GAT_MAX_DIM
+                and not (self.training and self.attn_drop.p > 0)):
+            return _GATAttention.apply(edge_ptr, src_edges, n_dst, flat, self.attn_l, self.attn_r, self.num_heads,
+                                       self.leaky_relu.negative_slope, self.attention_grad)
+        # dropped coefficients: op by op
         el = (feat_src * self.attn_l).sum(dim=-1)
         er = (feat_src[:n_dst] * self.attn_r).sum(dim=-1)
-        edge_ptr, src_edges = block_csr(block)
         dst_edges = block.edges()[1]
         e = self.leaky_relu(el[src_edges.long()] + er[dst_edges.long()])
         edge_data = self.attn_drop(edge_softmax(e, dst_edges, n_dst))
-        flat = feat_src.reshape(-1, self.num_heads * self.out_feats)
         return MA_Function_GAT.apply(edge_ptr, edge_data, src_edges, dst_edges, n_dst, flat, self.num_heads, neighbor_num,
                                      self.attention_grad)
 

@@ -39,17 +39,18 @@ def shard_seeds(train_nids: torch.Tensor, rank: int, world: int, epoch_seed: int
 
 
 class FlatGrads:
-    """All parameter gradients as views of one buffer, so that the data-parallel step is one all-reduce."""
+    """All parameter gradients as views of one buffer, so that the data-parallel step is one all-reduce.  Every parameter
+    starts on a 128-byte line (``offsets``), so that products and vector accesses on it are aligned; the padding stays zero."""
 
     def __init__(self, params):
         self.params = [p for p in params if p.requires_grad]
-        total = sum(p.numel() for p in self.params)
-        total = (total + 3) // 4 * 4      # whole 128-bit vectors: the padding stays zero
-        self.buffer = torch.zeros(total, dtype=self.params[0].dtype, device=self.params[0].device)
-        off = 0
+        self.offsets, total = [], 0
         for p in self.params:
+            self.offsets.append(total)
+            total += (p.numel() + 31) // 32 * 32
+        self.buffer = torch.zeros(total, dtype=self.params[0].dtype, device=self.params[0].device)
+        for p, off in zip(self.params, self.offsets):
             p.grad = self.buffer[off: off + p.numel()].view_as(p)
-            off += p.numel()
 
     def zero(self):
         self.buffer.zero_()
@@ -73,26 +74,50 @@ class FlatAdam:
     def __init__(self, grads: FlatGrads, lr, weight_decay, betas=(0.9, 0.999), eps=1e-8, peers=None):
         self.grads = grads
         self.peers = peers
-        self.lr, self.weight_decay, self.betas, self.eps = lr, weight_decay, betas, eps
+        # one group in torch.optim's form: a caller that changes the learning rate does it there
+        self.param_groups = [dict(params=grads.params, lr=lr, betas=betas, eps=eps, weight_decay=weight_decay)]
         self.flat = torch.zeros_like(grads.buffer)
-        off = 0
         with torch.no_grad():
-            for p in grads.params:
-                view = self.flat[off: off + p.numel()].view_as(p)
+            for p, view in zip(grads.params, self._views(self.flat)):
                 view.copy_(p.data)
                 p.data = view
-                off += p.numel()
         self.exp_avg = torch.zeros_like(self.flat)
         self.exp_avg_sq = torch.zeros_like(self.flat)
         self.step_dev = torch.zeros(3, dtype=torch.int32, device=self.flat.device)
 
+    def _views(self, flat):
+        """The parameters' parts of a flat buffer, in their shapes."""
+        return [flat[off: off + p.numel()].view_as(p) for p, off in zip(self.grads.params, self.grads.offsets)]
+
     def step(self):
+        g = self.param_groups[0]
         if self.peers is not None:
             fastgl.allreduce_adam_(self.peers, self.flat, self.grads.buffer, self.exp_avg, self.exp_avg_sq, self.step_dev,
-                                   lr=self.lr, betas=self.betas, eps=self.eps, weight_decay=self.weight_decay)
+                                   lr=g["lr"], betas=g["betas"], eps=g["eps"], weight_decay=g["weight_decay"])
         else:
-            fastgl.adam_step_(self.flat, self.grads.buffer, self.exp_avg, self.exp_avg_sq, self.step_dev, lr=self.lr,
-                              betas=self.betas, eps=self.eps, weight_decay=self.weight_decay)
+            fastgl.adam_step_(self.flat, self.grads.buffer, self.exp_avg, self.exp_avg_sq, self.step_dev, lr=g["lr"],
+                              betas=g["betas"], eps=g["eps"], weight_decay=g["weight_decay"])
+
+    def zero_grad(self, set_to_none=False):
+        self.grads.zero()
+
+    def state_dict(self):
+        """The state in the form of torch.optim.Adam's."""
+        step = self.step_dev[0].to(torch.float32)
+        state = {i: dict(step=step.clone(), exp_avg=m.clone(), exp_avg_sq=v.clone())
+                 for i, (m, v) in enumerate(zip(self._views(self.exp_avg), self._views(self.exp_avg_sq)))}
+        group = {k: v for k, v in self.param_groups[0].items() if k != "params"}
+        return dict(state=state, param_groups=[dict(group, params=list(range(len(self.grads.params))))])
+
+    def load_state_dict(self, state_dict):
+        self.param_groups[0].update({k: v for k, v in state_dict["param_groups"][0].items() if k in ("lr", "betas", "eps", "weight_decay")})
+        self.zero_state()
+        for i, (m, v) in enumerate(zip(self._views(self.exp_avg), self._views(self.exp_avg_sq))):
+            if i in state_dict["state"]:
+                part = state_dict["state"][i]
+                m.copy_(part["exp_avg"])
+                v.copy_(part["exp_avg_sq"])
+                self.step_dev[0] = int(part["step"])
 
     def zero_state(self):
         self.exp_avg.zero_()
@@ -248,6 +273,9 @@ class Trainer:
         self.oneshot = can_oneshot and grad_sync != "nccl"
         self._peers = None
         self.reset_optimizer()
+        # the loss kernel counts every row; torch's also skips the label -100 and takes class probabilities
+        self._plain_labels = (labels.is_cuda and labels.dtype == torch.int64 and labels.dim() == 1 and labels.is_contiguous()
+                              and labels.numel() > 0 and int(labels.min()) >= 0)
         self.train_nids = train_nids
         self._train_nids_host = train_nids.cpu()
         self._shuffler = ThreadPoolExecutor(max_workers=1)
@@ -296,19 +324,12 @@ class Trainer:
         self.opt.step()
 
     def reset_optimizer(self):
-        if self.sage:
-            self.opt = FlatAdam(self.grads, self.lr, self.weight_decay, peers=self._peer_sync() if self.oneshot else None)
-        else:
-            self.opt = torch.optim.Adam(self.model.parameters(), lr=self.lr, weight_decay=self.weight_decay, fused=True)
+        # torch's fused Adam walks a few large parameters with a handful of CTAs (36 us for 165 k of them) behind 50 us of
+        # host work; the flat one is 5 us
+        self.opt = FlatAdam(self.grads, self.lr, self.weight_decay, peers=self._peer_sync() if self.oneshot else None)
 
     def zero_optimizer_state(self):
-        if isinstance(self.opt, FlatAdam):
-            self.opt.zero_state()
-            return
-        for state in self.opt.state.values():
-            for v in state.values():
-                if torch.is_tensor(v):
-                    v.zero_()
+        self.opt.zero_state()
 
     def _sampler_teams(self) -> int:
         """Teams of the fused sampler: as many mini-batches in flight as the window has (up to 16) once the tables
@@ -436,7 +457,6 @@ class Trainer:
                 return loss
         input_nodes, blocks = self.sampler.window_blocks(fb, b)
         seeds = input_nodes[: blocks[-1].n_dst]
-        y = self.labels[seeds.long()] if labels_of is None else labels_of
         if layer0 is not None:
             buf, row_off = layer0
             logits = self.model(blocks, None, layer0=buf[row_off[b]: row_off[b + 1]])
@@ -450,9 +470,15 @@ class Trainer:
             # the reference's models (GCN / GIN) take the gathered input rows (train_fastgl.py:357,365)
             batch_inputs = fastgl.gather_rows(self.feat, input_nodes)
             logits = self.model(blocks, batch_inputs, neighbor_list=self.fanouts)
-        loss = F.cross_entropy(logits, y)
         self.grads.zero()
-        loss.backward()
+        if labels_of is None and self._plain_labels and logits.dtype == torch.float32 and logits.stride(1) == 1:
+            # loss and gradient of the logits by one kernel, instead of a gather of the labels and eight launches
+            loss, d_logits = fastgl.softmax_xent(logits.detach(), self.labels, label_ids=seeds)
+            loss = loss.view(())
+            torch.autograd.backward(logits, d_logits)
+        else:
+            loss = F.cross_entropy(logits, self.labels[seeds.long()] if labels_of is None else labels_of)
+            loss.backward()
         self._sync_and_step()
         self.sampled_edges += sum(blk.num_edges() for blk in blocks)
         self.last_loss = loss

@@ -254,6 +254,22 @@ int fgl_agg_fwd_sharded(fgl_ws* ws, int32_t mode, const int32_t* indptr, const i
                         const float* const* shards, int64_t rows_per_shard, int64_t n_rows, int64_t ldx, int32_t dim,
                         int32_t n_dst, int32_t flags, float* out, int64_t ldo, const int32_t* n_dst_dev, void* stream);
 
+/* The attention part of a GAT layer (GraphConv.py:262-283 behind the linear map): el = sum_f feat * attn_l per source and
+ * head, er likewise with attn_r for the destinations (the first n_dst sources), alpha = softmax over a row's in-edges of
+ * leaky_relu(el[src] + er[dst]), out[d] = sum_e alpha[e] * feat[src[e]] per head (a row without in-edges copies its own
+ * input row).  feat is float32 [n_src][heads * width]; el, er, alpha ([n_edges][heads]) are outputs that the backward takes
+ * again.  fgl_gat_bwd: gradients of feat (dfeat [n_src][heads * width], contiguous) and of the two attention vectors
+ * (dattn [2][heads * width]) from dy; scratch holds fgl_gat_bwd_partials(...) * 2 * heads * width + (n_edges + n_dst) * heads
+ * floats.  fgl_gat_bwd_partials returns 0 where heads * width is too wide (above 24576). */
+int fgl_gat_fwd(fgl_ws* ws, const int32_t* indptr, const int32_t* src, const float* feat, int64_t ldf, const float* attn_l,
+                const float* attn_r, int32_t heads, int32_t width, int32_t n_dst, int32_t n_src, float slope, float* el, float* er,
+                float* alpha, float* out, int64_t ldo, void* stream);
+int fgl_gat_bwd_partials(fgl_ws* ws, int32_t heads, int32_t width, int32_t n_dst);
+int fgl_gat_bwd(fgl_ws* ws, const int32_t* indptr, const int32_t* src, const float* feat, int64_t ldf, const float* attn_l,
+                const float* attn_r, const float* el, const float* er, const float* alpha, const float* dy, int64_t ldy, int32_t heads,
+                int32_t width, int32_t n_dst, int32_t n_src, int64_t n_edges, float slope, float* scratch, float* dfeat, float* dattn,
+                void* stream);
+
 /* Edge-weighted multi-head aggregation; replaces computation_aware_forward_gat_cuda /
  * computation_aware_backward_gat_cuda (aggregate_acc_kernel.cu:789-979; bindings aggregate_acc.cpp
  * forward_gat / backward_gat).  edge_w is float32 [n_edges][n_heads] (the attention coefficients after the

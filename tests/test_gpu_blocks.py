@@ -75,3 +75,37 @@ def test_cal_deg_at_its_dispatch_sizes(n_nodes, n_ids):
     ids = torch.randint(-3, n_nodes + 3, (n_ids,), dtype=torch.int32, device="cuda")
     inside = ids[(ids >= 0) & (ids < n_nodes)].long()
     assert torch.equal(fastgl.cal_deg(ids, n_nodes).long(), torch.bincount(inside, minlength=n_nodes))
+
+
+@pytest.mark.parametrize("heads,width,n_dst,n_src,fanout", [(1, 10, 1, 1, 1), (8, 32, 700, 3000, 12), (3, 27, 65, 300, 70), (40, 4, 33, 90, 5),
+                                                          (2, 512, 40, 100, 9)])
+@pytest.mark.parametrize("slope", [0.2, 1.0])
+def test_gat_attention_and_its_gradients_match_torch(heads, width, n_dst, n_src, fanout, slope):
+    """float64 torch algebra; a difference is bounded by the rounding of sums of at most fanout * width float32 terms."""
+    import fastgl
+    from fastgl_b200.layers import edge_softmax
+    rng = np.random.default_rng(heads)
+    deg = rng.integers(0, fanout + 1, n_dst)
+    deg[0] = fanout
+    ptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)).cuda()
+    src = torch.from_numpy(rng.integers(0, n_src, int(deg.sum())).astype(np.int32)).cuda()
+    dst = torch.from_numpy(np.repeat(np.arange(n_dst), deg)).cuda()
+    gen = torch.Generator("cuda").manual_seed(1)
+    feat = torch.randn((n_src, heads * width), generator=gen, device="cuda")
+    l, r = (torch.randn((1, heads, width), generator=gen, device="cuda") / width ** 0.5 for _ in range(2))
+    dy = torch.randn((n_dst, heads * width), generator=gen, device="cuda")
+    out, alpha, el, er = fastgl.gat_attention(ptr, src, feat, l, r, n_dst, heads, slope)
+    grads = fastgl.gat_attention_backward(ptr, src, feat, l, r, el, er, alpha, dy, heads, slope)
+    fastgl.check_status()
+    f64, l64, r64 = (t.double().requires_grad_() for t in (feat, l, r))
+    x = f64.view(n_src, heads, width)
+    score = torch.nn.functional.leaky_relu((x * l64).sum(-1)[src.long()] + (x[:n_dst] * r64).sum(-1)[dst], slope)
+    a64 = edge_softmax(score, dst, n_dst)
+    want = torch.zeros((n_dst, heads, width), dtype=torch.float64, device="cuda").index_add_(0, dst, a64.unsqueeze(-1) * x[src.long()])
+    has = torch.from_numpy(deg > 0).cuda()
+    want = want.reshape(n_dst, -1)
+    refs = torch.autograd.grad(want, (f64, l64, r64), dy.double())
+    want = torch.where(has[:, None], want, feat[:n_dst].double())
+    for got, ref in zip((out, *grads), (want, *refs)):
+        assert got.shape == ref.shape
+        assert float((got - ref).abs().max()) <= 1e-5 * max(1.0, float(ref.abs().max())) * max(1.0, (fanout * width) ** 0.5 / 8)
