@@ -43,6 +43,29 @@ __global__ void __launch_bounds__(1024) cal_deg_small_kernel(const int32_t* __re
     for (int i = threadIdx.x; i < n_nodes; i += 1024) deg[i] = cnt[i];
 }
 
+// Degrees of a block's two sides from its CSR: what the sym-norm weights of a layer take, in one pass over the edges.
+__global__ void __launch_bounds__(256) block_degrees_kernel(const int32_t* __restrict__ indptr, const int32_t* __restrict__ src,
+                                                            int n_dst, int n_src, int64_t n_edges, int32_t* __restrict__ dst_deg,
+                                                            int32_t* __restrict__ src_deg) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t i = first; i < n_dst; i += stride) dst_deg[i] = __ldg(indptr + i + 1) - __ldg(indptr + i);
+    for (int64_t e = first; e < n_edges; e += stride) {
+        const int s = __ldg(src + e);
+        if (s >= 0 && s < n_src) atomicAdd(src_deg + s, 1);
+    }
+}
+
+// y = x with the rows of destinations that have no in-edges zeroed.
+__global__ void __launch_bounds__(256) mask_rows_kernel(const int32_t* __restrict__ indptr, int n_dst, int dim, const float* __restrict__ x,
+                                                        int64_t ldx, float* __restrict__ y, int64_t ldy) {
+    const int64_t total = (int64_t)n_dst * dim;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = i / dim;
+        const int c = (int)(i - r * dim);
+        y[r * ldy + c] = __ldg(indptr + r + 1) > __ldg(indptr + r) ? x[r * ldx + c] : 0.f;
+    }
+}
+
 // Scan by one CTA, sixteen entries per thread and pass: up to kSmallScan entries a second level (its barrier, its scratch to
 // be zeroed, a cooperative launch) takes longer than the scan.
 constexpr int64_t kSmallScan = 32 * 1024;
@@ -277,6 +300,26 @@ int fgl_cal_deg(const int32_t* ids, int64_t n_ids, int32_t* deg, int32_t n_nodes
     if (n_ids == 0 || n_nodes == 0) return FGL_OK;
     const int grid = (int)std::min<int64_t>((n_ids + 255) / 256, 148 * 16);
     cal_deg_kernel<<<grid, 256, 0, st>>>(ids, n_ids, deg, n_nodes);
+    return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
+}
+
+int fgl_block_degrees(const int32_t* indptr, const int32_t* src, int32_t n_dst, int32_t n_src, int64_t n_edges, int32_t* dst_deg,
+                      int32_t* src_deg, void* stream) {
+    if (n_dst < 0 || n_src < 0 || n_edges < 0 || (n_dst > 0 && (!indptr || !dst_deg)) || (n_src > 0 && !src_deg) || (n_edges > 0 && !src))
+        return FGL_ERR_INVALID;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (n_src > 0 && cudaMemsetAsync(src_deg, 0, sizeof(int32_t) * (size_t)n_src, st) != cudaSuccess) return FGL_ERR_CUDA;
+    const int64_t items = std::max<int64_t>(n_dst, n_edges);
+    if (items == 0) return FGL_OK;
+    block_degrees_kernel<<<(int)std::min<int64_t>((items + 255) / 256, 148 * 8), 256, 0, st>>>(indptr, src, n_dst, n_src, n_edges, dst_deg, src_deg);
+    return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
+}
+
+int fgl_mask_rows(const int32_t* indptr, int32_t n_dst, int32_t dim, const float* x, int64_t ldx, float* y, int64_t ldy, void* stream) {
+    if (n_dst < 0 || dim < 1 || ldx < dim || ldy < dim || (n_dst > 0 && (!indptr || !x || !y))) return FGL_ERR_INVALID;
+    if (n_dst == 0) return FGL_OK;
+    const int64_t items = (int64_t)n_dst * dim;
+    mask_rows_kernel<<<(int)std::min<int64_t>((items + 255) / 256, 148 * 8), 256, 0, (cudaStream_t)stream>>>(indptr, n_dst, dim, x, ldx, y, ldy);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 

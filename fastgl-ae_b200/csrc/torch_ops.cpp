@@ -34,7 +34,8 @@ void* g_lib = nullptr;
     X(fgl_sample_map_fused_extra) X(fgl_cal_deg) X(fgl_exclusive_sum) X(fgl_stage_segments) X(fgl_agg_fwd)              \
     X(fgl_agg_fwd_window_counts) X(fgl_agg_edge_fwd) X(fgl_agg_edge_bwd) X(fgl_agg_edge_wgrad) X(fgl_agg_bwd)            \
     X(fgl_agg_bwd_self) X(fgl_block_transpose) X(fgl_agg_bwd_gather) X(fgl_gather_rows) X(fgl_ws_time_next_launch)           \
-    X(fgl_gat_fwd) X(fgl_gat_bwd) X(fgl_gat_bwd_partials) X(fgl_softmax_xent) X(fgl_adam_step)
+    X(fgl_gat_fwd) X(fgl_gat_bwd) X(fgl_gat_bwd_partials) X(fgl_softmax_xent) X(fgl_adam_step) \
+    X(fgl_block_degrees) X(fgl_mask_rows)
 
 struct Api {
 #define FGL_FIELD(name) decltype(&::name) name = nullptr;
@@ -647,6 +648,208 @@ void adam_step(py::handle p_o, py::handle g_o, py::handle m_o, py::handle v_o, p
                             (float)wd, ptr<int32_t>(step), c.st()), "adam_step_");
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// one training step of the reference's models, without autograd
+// ---------------------------------------------------------------------------------------------------------------------
+// Forward, loss and backward of GCN / GIN / GAT (layers.py) on one mini-batch of a window, as the launches they are.  Under
+// autograd a two-layer step is some forty operators and graph nodes and 0.6 ms of host time; spelled out it is about
+// twenty launches.  The arithmetic is that of the layers' autograd functions, call by call.
+struct BlockRef {
+    const int32_t *indptr, *src;
+    int32_t n_src, n_dst;
+    int64_t n_edges;
+};
+
+struct StepBatch {
+    std::vector<BlockRef> blocks;  // input layer first
+    const int32_t* nodes;          // global ids of the input layer's sources, seeds first
+};
+
+StepBatch step_batch(const at::Tensor& nodes, const std::vector<at::Tensor>& indptr, const std::vector<at::Tensor>& src, int64_t b,
+                     const std::vector<int64_t>& counts) {
+    StepBatch s;
+    s.nodes = ptr<int32_t>(nodes) + b * nodes.stride(0);
+    for (int h = (int)indptr.size() - 1; h >= 0; --h)
+        s.blocks.push_back({ptr<int32_t>(indptr[h]) + b * indptr[h].stride(0), ptr<int32_t>(src[h]) + b * src[h].stride(0),
+                            (int32_t)counts[h + 1], (int32_t)counts[h], counts[8 + h]});
+    return s;
+}
+
+// out [n_dst][x's width] = aggregation of x over the block; rows of x through `map` (n_map entries) if that is given.
+at::Tensor step_agg(const Call& c, int mode, const BlockRef& b, const at::Tensor& x, const int32_t* map, const int32_t* sdeg, const int32_t* ddeg) {
+    at::Tensor out = at::empty({b.n_dst, x.size(1)}, x.options());
+    check(api.fgl_agg_fwd(c.ws, mode, b.indptr, b.src, sdeg, ddeg, map, map ? b.n_src : 0, ptr<float>(x), x.size(0), x.stride(0),
+                          (int32_t)x.size(1), b.n_dst, FGL_AGG_ZERO_DEG_PASSTHROUGH, ptr<float>(out), out.stride(0), nullptr, c.st()),
+          "aggregate");
+    return out;
+}
+
+at::Tensor step_agg_bwd(const Call& c, int mode, const BlockRef& b, const at::Tensor& dy, const int32_t* sdeg, const int32_t* ddeg) {
+    at::Tensor dx = at::empty({b.n_src, dy.size(1)}, dy.options());
+    check(api.fgl_agg_bwd(c.ws, mode, b.indptr, b.src, sdeg, ddeg, ptr<float>(dy), dy.stride(0), (int32_t)dy.size(1), b.n_dst, b.n_src,
+                          ptr<float>(dx), dx.stride(0), nullptr, c.st()), "aggregate_backward");
+    return dx;
+}
+
+// Inverted dropout between two layers, drawing as torch's does.
+struct Drop {
+    double p;
+    std::vector<at::Tensor> masks;
+    at::Tensor forward(const at::Tensor& h) {
+        if (p == 0.0 || h.numel() == 0) {
+            masks.emplace_back();
+            return h;
+        }
+        auto [out, mask] = at::native_dropout(h, p, true);
+        masks.push_back(mask);
+        return out;
+    }
+    at::Tensor backward(const at::Tensor& d) {
+        at::Tensor mask = masks.back();
+        masks.pop_back();
+        return mask.defined() ? at::native_dropout_backward(d, mask, 1.0 / (1.0 - p)) : d;
+    }
+};
+
+std::pair<at::Tensor, at::Tensor> step_loss(const Call& c, const at::Tensor& logits, const at::Tensor& labels, const StepBatch& s) {
+    const int32_t n = s.blocks.back().n_dst;
+    at::Tensor loss = at::empty({1}, logits.options()), d = at::empty_like(logits), rows = at::empty({std::max(n, 1)}, logits.options());
+    check(api.fgl_softmax_xent(c.ws, ptr<float>(logits), logits.stride(0), ptr<int64_t>(labels), s.nodes, labels.numel(), n,
+                               (int32_t)logits.size(1), nullptr, n, ptr<float>(loss), ptr<float>(d), d.stride(0), ptr<float>(rows), c.st()),
+          "softmax_xent", c.ws);
+    return {loss, d};
+}
+
+// GCN with the input layer's rows read in the feature table through the mini-batch's node ids.  aggregate_first: per layer,
+// whether (A x) W is evaluated instead of A (x W).
+at::Tensor gcn_step(const at::Tensor& table, const at::Tensor& nodes, const std::vector<at::Tensor>& indptr, const std::vector<at::Tensor>& src,
+                    int64_t batch, const std::vector<int64_t>& counts, const std::vector<at::Tensor>& weights,
+                    const std::vector<at::Tensor>& grads, const std::vector<bool>& aggregate_first, double p_drop, const at::Tensor& labels) {
+    Call c(table);
+    const StepBatch s = step_batch(nodes, indptr, src, batch, counts);
+    const int L = (int)s.blocks.size();
+    const auto words = nodes.options();
+    Drop drop{p_drop, {}};
+    std::vector<at::Tensor> kept(L), deg(L);  // per layer: the left operand of the weight gradient; both sides' degrees
+    std::vector<const int32_t*> sdeg(L), ddeg(L);
+    at::Tensor h = table;
+    for (int i = 0; i < L; ++i) {
+        const BlockRef& b = s.blocks[i];
+        if (i > 0) h = drop.forward(h);
+        const int64_t pad = (b.n_dst + 31) / 32 * 32;
+        deg[i] = at::empty({pad + b.n_src}, words);
+        int32_t* d = ptr<int32_t>(deg[i]);
+        ddeg[i] = d;
+        sdeg[i] = d + pad;
+        check(api.fgl_block_degrees(b.indptr, b.src, b.n_dst, b.n_src, b.n_edges, d, d + pad, c.st()), "block_degrees");
+        if (i == 0 || aggregate_first[i]) {
+            kept[i] = step_agg(c, FGL_AGG_SYMNORM, b, h, i == 0 ? s.nodes : nullptr, sdeg[i], ddeg[i]);
+            h = at::mm(kept[i], weights[i]);
+        } else {
+            kept[i] = h;
+            h = step_agg(c, FGL_AGG_SYMNORM, b, at::mm(h, weights[i]), nullptr, sdeg[i], ddeg[i]);
+        }
+    }
+    auto [loss, d] = step_loss(c, h, labels, s);
+    for (int i = L - 1; i >= 0; --i) {
+        const BlockRef& b = s.blocks[i];
+        at::Tensor g = grads[i];
+        if (i == 0 || aggregate_first[i]) {
+            at::Tensor masked = at::empty_like(d);
+            check(api.fgl_mask_rows(b.indptr, b.n_dst, (int32_t)d.size(1), ptr<float>(d), d.stride(0), ptr<float>(masked), masked.stride(0),
+                                    c.st()), "mask_rows");
+            at::mm_out(g, kept[i].t(), masked);
+            if (i > 0) d = step_agg_bwd(c, FGL_AGG_SYMNORM, b, at::mm(masked, weights[i].t()), sdeg[i], ddeg[i]);
+        } else {
+            const at::Tensor dx = step_agg_bwd(c, FGL_AGG_SYMNORM, b, d, sdeg[i], ddeg[i]);
+            at::mm_out(g, kept[i].t(), dx);
+            d = at::mm(dx, weights[i].t());
+        }
+        if (i > 0) d = drop.backward(d);
+    }
+    return loss;
+}
+
+// GIN; the input layer sums the rows of the feature table in place, and its input takes no gradient.
+at::Tensor gin_step(const at::Tensor& table, const at::Tensor& nodes, const std::vector<at::Tensor>& indptr, const std::vector<at::Tensor>& src,
+                    int64_t batch, const std::vector<int64_t>& counts, const std::vector<at::Tensor>& weights,
+                    const std::vector<at::Tensor>& grads, double p_drop, const at::Tensor& labels) {
+    Call c(table);
+    const StepBatch s = step_batch(nodes, indptr, src, batch, counts);
+    const int L = (int)s.blocks.size();
+    Drop drop{p_drop, {}};
+    std::vector<at::Tensor> kept(L);
+    at::Tensor h = table;
+    for (int i = 0; i < L; ++i) {
+        if (i > 0) h = drop.forward(h);
+        kept[i] = step_agg(c, FGL_AGG_SUM, s.blocks[i], h, i == 0 ? s.nodes : nullptr, nullptr, nullptr);
+        h = at::mm(kept[i], weights[i]);
+    }
+    auto [loss, d] = step_loss(c, h, labels, s);
+    for (int i = L - 1; i >= 0; --i) {
+        at::Tensor g = grads[i];
+        at::mm_out(g, kept[i].t(), d);
+        if (i > 0) d = drop.backward(step_agg_bwd(c, FGL_AGG_SUM, s.blocks[i], at::mm(d, weights[i].t()), nullptr, nullptr));
+    }
+    return loss;
+}
+
+// GAT.  params / grads: per layer the linear map's weight [heads * width][in] and the two attention vectors; without
+// attention_grad the latter take no gradient (theirs stays zero).
+at::Tensor gat_step(const at::Tensor& table, const at::Tensor& nodes, const std::vector<at::Tensor>& indptr, const std::vector<at::Tensor>& src,
+                    int64_t batch, const std::vector<int64_t>& counts, const std::vector<at::Tensor>& params,
+                    const std::vector<at::Tensor>& grads, const std::vector<int64_t>& heads, const std::vector<double>& slope,
+                    const std::vector<bool>& attention_grad, const at::Tensor& labels) {
+    Call c(table);
+    const StepBatch s = step_batch(nodes, indptr, src, batch, counts);
+    const int L = (int)s.blocks.size();
+    const auto opt = table.options();
+    std::vector<at::Tensor> x(L), feat(L), alpha(L), el(L), er(L);
+    at::Tensor h = at::empty({s.blocks[0].n_src, table.size(1)}, opt);
+    check(api.fgl_gather_rows(c.ws, ptr<float>(table), nullptr, 0, table.size(0), table.stride(0), (int32_t)table.size(1), s.nodes,
+                              s.blocks[0].n_src, ptr<float>(h), h.stride(0), c.st()), "gather_rows");
+    for (int i = 0; i < L; ++i) {
+        const BlockRef& b = s.blocks[i];
+        const at::Tensor &w = params[3 * i], &l = params[3 * i + 1], &r = params[3 * i + 2];
+        const int64_t dim = w.size(0);
+        x[i] = h;
+        feat[i] = at::mm(h, w.t());
+        h = at::empty({b.n_dst, dim}, opt);
+        alpha[i] = at::empty({b.n_edges, heads[i]}, opt);
+        el[i] = at::empty({b.n_src, heads[i]}, opt);
+        er[i] = at::empty({b.n_dst, heads[i]}, opt);
+        check(api.fgl_gat_fwd(c.ws, b.indptr, b.src, ptr<float>(feat[i]), dim, ptr<float>(l), ptr<float>(r), (int32_t)heads[i],
+                              (int32_t)(dim / heads[i]), b.n_dst, b.n_src, (float)slope[i], ptr<float>(el[i]), ptr<float>(er[i]),
+                              ptr<float>(alpha[i]), ptr<float>(h), dim, c.st()), "gat_attention");
+    }
+    auto [loss, d] = step_loss(c, h, labels, s);
+    for (int i = L - 1; i >= 0; --i) {
+        const BlockRef& b = s.blocks[i];
+        const at::Tensor &w = params[3 * i], &l = params[3 * i + 1], &r = params[3 * i + 2];
+        const int64_t dim = w.size(0);
+        at::Tensor dfeat = at::empty({b.n_src, dim}, opt);
+        if (attention_grad[i]) {
+            const int rows = api.fgl_gat_bwd_partials(c.ws, (int32_t)heads[i], (int32_t)(dim / heads[i]), b.n_dst);
+            at::Tensor scratch = at::empty({(int64_t)rows * 2 * dim + (b.n_edges + b.n_dst) * heads[i]}, opt);
+            at::Tensor dattn = at::empty({2, dim}, opt);
+            check(api.fgl_gat_bwd(c.ws, b.indptr, b.src, ptr<float>(feat[i]), dim, ptr<float>(l), ptr<float>(r), ptr<float>(el[i]),
+                                  ptr<float>(er[i]), ptr<float>(alpha[i]), ptr<float>(d), d.stride(0), (int32_t)heads[i],
+                                  (int32_t)(dim / heads[i]), b.n_dst, b.n_src, b.n_edges, (float)slope[i], ptr<float>(scratch),
+                                  ptr<float>(dfeat), ptr<float>(dattn), c.st()), "gat_attention_backward");
+            fgl_segment seg[2] = {{ptr<float>(grads[3 * i + 1]), ptr<float>(dattn), dim * 4},
+                                  {ptr<float>(grads[3 * i + 2]), ptr<float>(dattn) + dim, dim * 4}};
+            check(api.fgl_stage_segments(seg, 2, nullptr, nullptr, 0, c.st()), "gat_attention_backward");
+        } else {
+            check(api.fgl_agg_edge_bwd(c.ws, b.indptr, b.src, ptr<float>(alpha[i]), (int32_t)heads[i], ptr<float>(d), d.stride(0),
+                                       (int32_t)dim, b.n_dst, b.n_src, ptr<float>(dfeat), dim, c.st()), "backward_gat");
+        }
+        at::Tensor g = grads[3 * i];
+        at::mm_out(g, dfeat.t(), x[i]);
+        if (i > 0) d = at::mm(dfeat, w);
+    }
+    return loss;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_ops, m) {
@@ -672,6 +875,9 @@ PYBIND11_MODULE(_ops, m) {
     m.def("backward_gat", &backward_gat);
     m.def("edge_weight_grad", &edge_weight_grad);
     m.def("softmax_xent", &softmax_xent);
+    m.def("gcn_step", &gcn_step);
+    m.def("gin_step", &gin_step);
+    m.def("gat_step", &gat_step);
     m.def("adam_step", &adam_step);
     m.def("gat_attention", &gat_attention);
     m.def("gat_attention_backward", &gat_attention_backward);

@@ -20,6 +20,7 @@ import torch.nn.functional as F
 import fastgl
 
 from .block import Block
+from . import model_step
 from .layers import GCN
 from .sage_step import SageStepProgram
 from .sampler import FusedMapSampler
@@ -49,8 +50,9 @@ class FlatGrads:
             self.offsets.append(total)
             total += (p.numel() + 31) // 32 * 32
         self.buffer = torch.zeros(total, dtype=self.params[0].dtype, device=self.params[0].device)
-        for p, off in zip(self.params, self.offsets):
-            p.grad = self.buffer[off: off + p.numel()].view_as(p)
+        self.views = [self.buffer[off: off + p.numel()].view_as(p) for p, off in zip(self.params, self.offsets)]
+        for p, view in zip(self.params, self.views):
+            p.grad = view
 
     def zero(self):
         self.buffer.zero_()
@@ -276,6 +278,9 @@ class Trainer:
         # the loss kernel counts every row; torch's also skips the label -100 and takes class probabilities
         self._plain_labels = (labels.is_cuda and labels.dtype == torch.int64 and labels.dim() == 1 and labels.is_contiguous()
                               and labels.numel() > 0 and int(labels.min()) >= 0)
+        # GCN, GIN and GAT as they are in layers.py train without autograd (model_step.py)
+        self.grad_views = {id(p): v for p, v in zip(self.grads.params, self.grads.views)}
+        self._model_step = model_step.plan(self)
         self.train_nids = train_nids
         self._train_nids_host = train_nids.cpu()
         self._shuffler = ThreadPoolExecutor(max_workers=1)
@@ -455,6 +460,14 @@ class Trainer:
                 self.sampled_edges += sum(c[8: 8 + len(self.fanouts)])
                 self.last_loss = loss
                 return loss
+        if self._model_step is not None and labels_of is None and layer0 is None:
+            c = fb.counts_list()[b]
+            loss = self._model_step(fb, b, c)
+            if loss is not None:
+                self._sync_and_step()
+                self.sampled_edges += sum(c[8: 8 + len(self.fanouts)])
+                self.last_loss = loss.view(())
+                return self.last_loss
         input_nodes, blocks = self.sampler.window_blocks(fb, b)
         seeds = input_nodes[: blocks[-1].n_dst]
         if layer0 is not None:

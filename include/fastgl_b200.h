@@ -182,6 +182,15 @@ int fgl_sample_map_fused_extra(fgl_ws* ws, const fgl_fused_args* args, const fgl
  * deg[0 .. n_nodes) is zeroed and then counts the occurrences of each id. */
 int fgl_cal_deg(const int32_t* ids, int64_t n_ids, int32_t* deg, int32_t n_nodes, void* stream);
 
+/* Degrees of a block's two sides from its CSR (GraphConv.py:93,96 without the clamping: an edge's ends have at least one):
+ * dst_deg[d] = row length, src_deg[s] = occurrences of s among the n_edges sources. */
+int fgl_block_degrees(const int32_t* indptr, const int32_t* src, int32_t n_dst, int32_t n_src, int64_t n_edges, int32_t* dst_deg,
+                      int32_t* src_deg, void* stream);
+
+/* y[d, :] = x[d, :] where row d has in-edges, else 0: the reference's backward skips those rows
+ * (aggregate_acc_kernel.cu:498-500). */
+int fgl_mask_rows(const int32_t* indptr, int32_t n_dst, int32_t dim, const float* x, int64_t ldx, float* y, int64_t ldy, void* stream);
+
 /* Stages one mini-batch into fixed buffers: up to FGL_MAX_SEGMENTS device-to-device copies (sizes and
  * addresses multiples of 4 bytes) and up to FGL_MAX_SEGMENTS int32 words written to words_dst, in one kernel
  * launch.  No counterpart in the reference; it feeds the static inputs of a captured CUDA graph (block CSR
