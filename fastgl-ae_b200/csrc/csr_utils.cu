@@ -55,14 +55,19 @@ __global__ void __launch_bounds__(256) block_degrees_kernel(const int32_t* __res
     }
 }
 
-// y = x with the rows of destinations that have no in-edges zeroed.
+// y = x with the rows of destinations that have no in-edges zeroed; a warp per row.
+template <typename T>
 __global__ void __launch_bounds__(256) mask_rows_kernel(const int32_t* __restrict__ indptr, int n_dst, int dim, const float* __restrict__ x,
                                                         int64_t ldx, float* __restrict__ y, int64_t ldy) {
-    const int64_t total = (int64_t)n_dst * dim;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / dim;
-        const int c = (int)(i - r * dim);
-        y[r * ldy + c] = __ldg(indptr + r + 1) > __ldg(indptr + r) ? x[r * ldx + c] : 0.f;
+    constexpr int VEC = sizeof(T) / 4;
+    const int lane = threadIdx.x & 31;
+    for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < n_dst; r += gridDim.x * 8) {
+        const bool has = __ldg(indptr + r + 1) > __ldg(indptr + r);
+        for (int c = lane * VEC; c < dim; c += 32 * VEC) {
+            T v{};
+            if (has) v = __ldg(reinterpret_cast<const T*>(x + r * ldx + c));
+            *reinterpret_cast<T*>(y + r * ldy + c) = v;
+        }
     }
 }
 
@@ -318,8 +323,10 @@ int fgl_block_degrees(const int32_t* indptr, const int32_t* src, int32_t n_dst, 
 int fgl_mask_rows(const int32_t* indptr, int32_t n_dst, int32_t dim, const float* x, int64_t ldx, float* y, int64_t ldy, void* stream) {
     if (n_dst < 0 || dim < 1 || ldx < dim || ldy < dim || (n_dst > 0 && (!indptr || !x || !y))) return FGL_ERR_INVALID;
     if (n_dst == 0) return FGL_OK;
-    const int64_t items = (int64_t)n_dst * dim;
-    mask_rows_kernel<<<(int)std::min<int64_t>((items + 255) / 256, 148 * 8), 256, 0, (cudaStream_t)stream>>>(indptr, n_dst, dim, x, ldx, y, ldy);
+    const int grid = (int)std::min<int64_t>(((int64_t)n_dst + 7) / 8, 148 * 8);
+    const bool vec = dim % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
+    if (vec) mask_rows_kernel<float4><<<grid, 256, 0, (cudaStream_t)stream>>>(indptr, n_dst, dim, x, ldx, y, ldy);
+    else mask_rows_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>(indptr, n_dst, dim, x, ldx, y, ldy);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 

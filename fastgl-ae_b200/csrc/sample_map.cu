@@ -1230,6 +1230,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) map_kernel(const __grid_co
 constexpr int64_t kMaxTableBytes = 1LL << 30;
 
 constexpr int64_t kSmallTable = 1 << 16;
+constexpr int64_t kResidentTables = 48LL << 20;   // bytes
 
 static int64_t pow2_at_least(int64_t n) {
     int64_t p = 1024;
@@ -1570,9 +1571,12 @@ int fgl_sample_map_fused_extra(fgl_ws* ws, const fgl_fused_args* a, const fgl_fu
         for (int h = 0; h < a->n_hops; ++h) kp.blk_dst[h] = extra->block_dst[h];
     }
     kp.table = ws->table;
-    // the first table covers the first hop's worst case, and every small mini-batch as a whole
+    // The first table covers the first hop's worst case, and every small mini-batch as a whole.  Tables that all fit the
+    // L2 together are as large as they get from the start: moving to a larger one re-inserts the nodes.
     kp.table_log2_max = log2_of(slots);
-    kp.table_log2_first = log2_of(std::min(slots, std::max(kSmallTable, pow2_at_least(cap[1] + cap[1] / 4))));
+    kp.table_log2_first = slots * n_teams * 8 <= kResidentTables
+                              ? kp.table_log2_max
+                              : log2_of(std::min(slots, std::max(kSmallTable, pow2_at_least(cap[1] + cap[1] / 4))));
     FGL_CUDA_OK(ws, cudaMemsetAsync(ws->scratch, 0, (size_t)fused_head(n_teams, grid), st));
     return launch_sample_map<MODE_FUSED>(ws, kp, is64, arrival, grid, dyn, st);
 }

@@ -35,7 +35,7 @@ void* g_lib = nullptr;
     X(fgl_agg_fwd_window_counts) X(fgl_agg_edge_fwd) X(fgl_agg_edge_bwd) X(fgl_agg_edge_wgrad) X(fgl_agg_bwd)            \
     X(fgl_agg_bwd_self) X(fgl_block_transpose) X(fgl_agg_bwd_gather) X(fgl_gather_rows) X(fgl_ws_time_next_launch)           \
     X(fgl_gat_fwd) X(fgl_gat_bwd) X(fgl_gat_bwd_partials) X(fgl_softmax_xent) X(fgl_adam_step) \
-    X(fgl_block_degrees) X(fgl_mask_rows)
+    X(fgl_block_degrees) X(fgl_mask_rows) X(fgl_weight_grad) X(fgl_weight_grad_scratch)
 
 struct Api {
 #define FGL_FIELD(name) decltype(&::name) name = nullptr;
@@ -423,6 +423,29 @@ at::Tensor aggregate(int mode, py::handle ptr_o, py::handle src_o, py::handle x_
                    n_dst_dev.is_none() ? at::Tensor() : tensor(n_dst_dev, "n_dst_dev"));
 }
 
+// dw = x^T dy, into `out` if given.  A caller who lets torch multiply in TF32 gets torch's product; so does a contraction that is
+// shorter than the output is wide (nothing to split).
+at::Tensor weight_grad(const Call& c, const at::Tensor& x, const at::Tensor& dy, const at::Tensor& out_given = at::Tensor()) {
+    const int64_t k = x.size(0), m = x.size(1), n = dy.size(1);
+    TORCH_CHECK(dy.size(0) == k, "x and dy must have the same number of rows");
+    at::Tensor out = out_given.defined() ? out_given : at::empty({m, n}, x.options());
+    auto rows = [](const at::Tensor& t) { return t.stride(1) == 1 && t.stride(0) >= t.size(1); };
+    if (!rows(x) || !rows(dy) || !rows(out) || k < std::max(m, n) || k > 0x7fffffffLL || at::globalContext().allowTF32CuBLAS())
+        return at::mm_out(out, x.t(), dy);
+    at::Tensor scratch;
+    const int64_t floats = api.fgl_weight_grad_scratch(c.ws, (int32_t)m, (int32_t)n, (int32_t)k);
+    if (floats > 0) scratch = at::empty({floats}, x.options());
+    check(api.fgl_weight_grad(c.ws, (int32_t)m, (int32_t)n, (int32_t)k, ptr<float>(x), x.stride(0), ptr<float>(dy), dy.stride(0),
+                              ptr<float>(out), out.stride(0), ptr<float>(scratch), c.st()), "weight_grad", c.ws);
+    return out;
+}
+
+at::Tensor weight_grad_op(py::handle x_o, py::handle dy_o, py::handle out_o) {
+    const at::Tensor &x = rows_f32(x_o, "x"), &dy = rows_f32(dy_o, "dy");
+    Call c(x);
+    return weight_grad(c, x, dy, out_o.is_none() ? at::Tensor() : rows_f32(out_o, "out"));
+}
+
 struct Transposed {
     at::Tensor t_indptr, t_dst, hubs;
 };
@@ -521,7 +544,8 @@ std::vector<at::Tensor> backward_gcn(py::handle ptr_o, py::handle src_o, py::han
     const at::Tensor &w = f32(w_o, "weight"), &x = f32(x_o, "input_feat");
     const at::Tensor d = agg_bwd(FGL_AGG_SYMNORM, i32(ptr_o, "edge_ptr"), i32(src_o, "src_edges"), rows_f32(dy_o, "d_input"), x.size(0),
                                  i32(dst_deg, "src_norm_degs"), i32(src_deg, "dst_norm_degs"), at::Tensor(), at::Tensor(), at::Tensor(), nullptr);
-    return {at::mm(d, w.t()), at::mm(x.t(), d)};
+    Call c(x);
+    return {at::mm(d, w.t()), weight_grad(c, x, d)};
 }
 
 std::vector<at::Tensor> forward_gin(py::handle ptr_o, py::handle src_o, py::handle x_o, py::handle w_o, int64_t n_dst) {
@@ -534,7 +558,8 @@ std::vector<at::Tensor> forward_gin(py::handle ptr_o, py::handle src_o, py::hand
 std::vector<at::Tensor> backward_gin(py::handle ptr_o, py::handle src_o, py::handle dy_o, py::handle w_o, py::handle x_o, int64_t n_src) {
     const at::Tensor &w = f32(w_o, "weight"), &x = f32(x_o, "input_feat"), &dy = f32(dy_o, "d_input");
     const at::Tensor d_tmp = at::mm(dy, w.t());
-    at::Tensor d_w = at::mm(x.t(), dy);
+    Call c(x);
+    at::Tensor d_w = weight_grad(c, x, dy);
     return {agg_bwd(FGL_AGG_SUM, i32(ptr_o, "edge_ptr"), i32(src_o, "src_edges"), d_tmp, n_src, at::Tensor(), at::Tensor(), at::Tensor(),
                     at::Tensor(), at::Tensor(), nullptr), d_w};
 }
@@ -758,11 +783,11 @@ at::Tensor gcn_step(const at::Tensor& table, const at::Tensor& nodes, const std:
             at::Tensor masked = at::empty_like(d);
             check(api.fgl_mask_rows(b.indptr, b.n_dst, (int32_t)d.size(1), ptr<float>(d), d.stride(0), ptr<float>(masked), masked.stride(0),
                                     c.st()), "mask_rows");
-            at::mm_out(g, kept[i].t(), masked);
+            weight_grad(c, kept[i], masked, g);
             if (i > 0) d = step_agg_bwd(c, FGL_AGG_SYMNORM, b, at::mm(masked, weights[i].t()), sdeg[i], ddeg[i]);
         } else {
             const at::Tensor dx = step_agg_bwd(c, FGL_AGG_SYMNORM, b, d, sdeg[i], ddeg[i]);
-            at::mm_out(g, kept[i].t(), dx);
+            weight_grad(c, kept[i], dx, g);
             d = at::mm(dx, weights[i].t());
         }
         if (i > 0) d = drop.backward(d);
@@ -788,7 +813,7 @@ at::Tensor gin_step(const at::Tensor& table, const at::Tensor& nodes, const std:
     auto [loss, d] = step_loss(c, h, labels, s);
     for (int i = L - 1; i >= 0; --i) {
         at::Tensor g = grads[i];
-        at::mm_out(g, kept[i].t(), d);
+        weight_grad(c, kept[i], d, g);
         if (i > 0) d = drop.backward(step_agg_bwd(c, FGL_AGG_SUM, s.blocks[i], at::mm(d, weights[i].t()), nullptr, nullptr));
     }
     return loss;
@@ -844,7 +869,7 @@ at::Tensor gat_step(const at::Tensor& table, const at::Tensor& nodes, const std:
                                        (int32_t)dim, b.n_dst, b.n_src, ptr<float>(dfeat), dim, c.st()), "backward_gat");
         }
         at::Tensor g = grads[3 * i];
-        at::mm_out(g, dfeat.t(), x[i]);
+        weight_grad(c, dfeat, x[i], g);
         if (i > 0) d = at::mm(dfeat, w);
     }
     return loss;
@@ -875,6 +900,7 @@ PYBIND11_MODULE(_ops, m) {
     m.def("backward_gat", &backward_gat);
     m.def("edge_weight_grad", &edge_weight_grad);
     m.def("softmax_xent", &softmax_xent);
+    m.def("weight_grad", &weight_grad_op);
     m.def("gcn_step", &gcn_step);
     m.def("gin_step", &gin_step);
     m.def("gat_step", &gat_step);

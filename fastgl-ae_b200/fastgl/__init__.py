@@ -32,7 +32,7 @@ from ._capi import (AGG_MEAN, AGG_SUM, AGG_SYMNORM, COUNTS_STRIDE, FLAG_MAP_ARRI
 
 __all__ = [
     "sample_node", "transfer_edge_id", "cal_deg", "exclusive_sum", "forward_gcn", "backward_gcn",
-    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "gat_attention", "gat_attention_backward", "sample_node_csr", "sample_blocks", "aggregate", "aggregate_backward", "aggregate_window",
+    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "weight_grad", "gat_attention", "gat_attention_backward", "sample_node_csr", "sample_blocks", "aggregate", "aggregate_backward", "aggregate_window",
     "sample_map_fused", "fused_capacity", "stage_segments", "stage_segments_raw", "gather_rows", "ShardedTable", "set_sampling", "seed", "FusedBatch",
     "exclusive_sum_noalloc", "exclusive_sum_noalloc_status", "check_status", "status_str", "PeerSync", "allreduce_adam_", "window_overlap", "TransposedBlock", "transpose_block", "split_tf32", "split_tf32_raw", "fold_blocks", "probe_access_pattern",
     "AGG_SUM", "AGG_MEAN", "AGG_SYMNORM",
@@ -726,6 +726,12 @@ def edge_weight_grad(edge_ptr, src_edges, input_feat, d_out, num_heads):
     return _ops.edge_weight_grad(edge_ptr, src_edges, input_feat, d_out, int(num_heads))
 
 
+def weight_grad(x, dy, out=None):
+    """``x^T dy`` for float32 matrices of many rows (the weight gradient of a dense layer), the contraction split over the
+    GPU in a fixed order.  Rows may be column slices of wider buffers; ``out`` receives the result when given."""
+    return _ops.weight_grad(x, dy, out)
+
+
 def gat_attention(edge_ptr, src_edges, feat, attn_l, attn_r, dst_nodes, num_heads, negative_slope=0.2):
     """Attention of a GAT layer behind its linear map (GraphConv.py:262-283) in two launches: scores
     ``leaky_relu(<feat, attn_l>[src] + <feat, attn_r>[dst])`` per head, softmax over every row's in-edges, weighted sum.
@@ -802,10 +808,12 @@ class FusedBatch:
         self.block_src = block_src
         self._arena = arena
         self._counts_host = None
-        # pinned copies of the counts and of the workspace's status word, written by the sampling launch itself
-        self._counts_pinned = torch.empty(tuple(counts.shape), dtype=torch.int32, pin_memory=True)
-        self._status_pinned = torch.zeros(1, dtype=torch.int32, pin_memory=True)
-        self._event = torch.cuda.Event()
+        # Pinned copies of the counts and of the workspace's status word.  The first read-back makes them and copies; the
+        # launches into these buffers after it write them themselves (_written: the point behind the last such launch).
+        self._counts_pinned = None
+        self._status_pinned = None
+        self._event = None
+        self._written = False
         self._readback = None
         self.device_status = 0   # the workspace's status word as of the last asynchronous read-back (0 = no error)
 
@@ -814,10 +822,24 @@ class FusedBatch:
         return self.nodes.size(0)
 
     def start_readback(self) -> None:
-        """Mark the point of the current stream behind the launch that writes the counts to pinned host memory, without
-        waiting: the next ``counts_host()`` waits for that point only, not for work enqueued after it."""
-        self._event.record(torch.cuda.current_stream(self.counts.device))
+        """Have the counts in pinned host memory, without waiting: the next ``counts_host()`` waits for the launch that
+        writes them (or, the first time, for a copy enqueued here) only, not for work enqueued after it."""
+        if not self._written:
+            if self._counts_pinned is None:
+                self._counts_pinned = torch.empty(tuple(self.counts.shape), dtype=torch.int32, pin_memory=True)
+                self._status_pinned = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+                self._event = torch.cuda.Event()
+            dev = self.counts.device
+            self._counts_pinned.copy_(self.counts, non_blocking=True)
+            ws = _ws(dev)
+            _raise(lib().fgl_ws_status_peek(ws, ctypes.c_void_p(self._status_pinned.data_ptr()), _stream(dev)), "status_peek", ws)
+            self._event.record(torch.cuda.current_stream(dev))
         self._readback = self._event
+
+    def __del__(self):
+        # a launch that still writes the pinned words must not find them in other hands
+        if self._written and self._event is not None and not self._event.query():
+            self._event.synchronize()
 
     def counts_host(self) -> torch.Tensor:
         if self._counts_host is None:
@@ -889,10 +911,14 @@ def sample_map_fused(edge_ptr, src_edges, seeds, seed_counts, fanouts, replace=N
     if timing is not None:
         with _on_device(dev):
             _time_next_launch(dev, timing)
+    # (a captured launch is replayed at times that the host does not see)
+    out._written = out._counts_pinned is not None and not torch.cuda.is_current_stream_capturing()
     _ops.sample_map_fused(edge_ptr, src_edges, seeds, seed_counts, [int(f) for f in fanouts], flags,
                           _config["rng_seed"] if rng_seed is None else rng_seed, _next_ctr() if rng_ctr is None else rng_ctr,
                           int(n_teams), int(table_slots), out.nodes, out.counts, out.block_indptr, out.block_src,
-                          out._counts_pinned, out._status_pinned)
+                          *((out._counts_pinned, out._status_pinned) if out._written else (None, None)))
+    if out._written:
+        out._event.record(torch.cuda.current_stream(dev))
     return out
 
 

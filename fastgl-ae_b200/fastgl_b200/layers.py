@@ -316,9 +316,8 @@ class MeanAggregate(torch.autograd.Function):
 class _TallLinear(torch.autograd.Function):
     """x W + b for a tall x (tens of thousands of rows, a few hundred columns).
 
-    The weight gradient x^T dy has a tiny output and a very long reduction; as one GEMM it runs on a handful
-    of CTAs.  Here the rows are split into S slabs, a batched GEMM produces S partial products on S times as
-    many CTAs, and the partials (and the per-slab column sums for the bias) are folded by a 1 x S GEMM."""
+    The weight gradient x^T dy has a tiny output and a very long reduction, which ``fastgl.weight_grad`` splits over the GPU;
+    the bias gradient is a product with a vector of ones."""
 
     @staticmethod
     def forward(ctx, x, weight, bias):
@@ -330,18 +329,9 @@ class _TallLinear(torch.autograd.Function):
         x, weight = ctx.saved_tensors
         dy = dy.contiguous()
         dx = torch.mm(dy, weight.t()) if ctx.needs_input_grad[0] else None
-        n, k, m = x.size(0), x.size(1), dy.size(1)
-        slabs = next((s for s in (16, 8) if n % s == 0 and n // s >= 512), 0)
-        if slabs and x.is_contiguous():
-            ones = dy.new_ones((1, slabs))
-            part = torch.bmm(x.view(slabs, n // slabs, k).transpose(1, 2), dy.view(slabs, n // slabs, m))
-            dw = torch.mm(ones, part.view(slabs, k * m)).view(k, m)
-            col = torch.bmm(dy.new_ones((slabs, 1, n // slabs)), dy.view(slabs, n // slabs, m))
-            db = torch.mm(ones, col.view(slabs, m)).view(m)
-        else:
-            dw = torch.mm(x.t(), dy)
-            db = torch.mv(dy.t(), dy.new_ones(n))
-        return dx, dw, db
+        own = x.is_cuda and x.dtype == torch.float32 and x.stride(1) == 1
+        dw = fastgl.weight_grad(x, dy) if own else torch.mm(x.t(), dy)
+        return dx, dw, torch.mv(dy.t(), dy.new_ones(dy.size(0)))
 
 
 class SAGEConv(nn.Module):

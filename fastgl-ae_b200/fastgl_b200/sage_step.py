@@ -55,15 +55,6 @@ class SageStepProgram:
         self.dlogits = torch.zeros((self.pad_dst[L - 1], outs[L - 1]), **f32)
         self.loss = torch.zeros(1, **f32)
         self.row_loss = torch.zeros(self.pad_dst[L - 1], **f32)
-        # split-K of the tall weight-gradient products: S slabs of rows, folded by a [1 x S] product.  The output is
-        # only a few 128 x 64 tiles, so S is what fills the 148 SMs.
-        self.slabs, self.part, self.ones = [], [], []
-        for i in range(L):
-            n = self.pad_dst[i]
-            s = next((s for s in (32, 16, 8) if n % s == 0 and n // s >= 256), 0)
-            self.slabs.append(s)
-            self.part.append(torch.zeros((s, 2 * ins[i], outs[i]), **f32) if s else None)
-            self.ones.append(torch.ones((1, s), **f32) if s else None)
         if matmul not in ("fp32", "3xtf32"):
             raise ValueError("matmul must be 'fp32' or '3xtf32'")
         # The weight-gradient products feed nothing but the optimizer, so they run on a second stream beside the chain
@@ -196,9 +187,8 @@ class SageStepProgram:
 
     def _weight_grad(self, i: int, dz=None) -> None:
         x, gw = self.cat[i], self.layers[i].weight.grad
-        s = self.slabs[i]
-        n, k, m = x.size(0), x.size(1), gw.size(1)
         if self.split:
+            s, n, k, m = self.slabs[i], x.size(0), x.size(1), gw.size(1)
             # [X_hi | X_lo]^T [dZ_hi | dZ_lo]: four k x m blocks (the lo-lo block is below float32's rounding; adding it
             # costs nothing), folded together with the split-K slabs by one reduction -- not by a product with ones,
             # which would round the partial sums to TF32
@@ -211,8 +201,4 @@ class SageStepProgram:
                 torch.mm(x2.t(), g2, out=part)
             fastgl.fold_blocks(part, 2, 2, k, m, mp, gw)
             return
-        if s:
-            torch.bmm(x.view(s, n // s, k).transpose(1, 2), dz.view(s, n // s, m), out=self.part[i])
-            torch.mm(self.ones[i], self.part[i].view(s, k * m), out=gw.view(1, k * m))
-        else:
-            torch.mm(x.t(), dz, out=gw)
+        fastgl.weight_grad(x, dz, out=gw)

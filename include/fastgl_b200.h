@@ -191,6 +191,13 @@ int fgl_block_degrees(const int32_t* indptr, const int32_t* src, int32_t n_dst, 
  * (aggregate_acc_kernel.cu:498-500). */
 int fgl_mask_rows(const int32_t* indptr, int32_t n_dst, int32_t dim, const float* x, int64_t ldx, float* y, int64_t ldy, void* stream);
 
+/* Weight gradient of a dense layer, dw [m][n] = x^T dy over k rows, in float32 on the FMA units (torch::mm in the reference,
+ * aggregate_acc_kernel.cu:462-463,528-529).  x is [k][m], dy [k][n], row-major with leading dimensions.  scratch holds
+ * fgl_weight_grad_scratch(...) floats (0: may be NULL).  The order of the additions depends on the sizes alone. */
+int64_t fgl_weight_grad_scratch(fgl_ws* ws, int32_t m, int32_t n, int32_t k);
+int fgl_weight_grad(fgl_ws* ws, int32_t m, int32_t n, int32_t k, const float* x, int64_t ldx, const float* dy, int64_t ldy, float* dw,
+                    int64_t ldw, float* scratch, void* stream);
+
 /* Stages one mini-batch into fixed buffers: up to FGL_MAX_SEGMENTS device-to-device copies (sizes and
  * addresses multiples of 4 bytes) and up to FGL_MAX_SEGMENTS int32 words written to words_dst, in one kernel
  * launch.  No counterpart in the reference; it feeds the static inputs of a captured CUDA graph (block CSR

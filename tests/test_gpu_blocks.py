@@ -109,3 +109,19 @@ def test_gat_attention_and_its_gradients_match_torch(heads, width, n_dst, n_src,
     for got, ref in zip((out, *grads), (want, *refs)):
         assert got.shape == ref.shape
         assert float((got - ref).abs().max()) <= 1e-5 * max(1.0, float(ref.abs().max())) * max(1.0, (fanout * width) ** 0.5 / 8)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (1, 1, 70), (5, 3, 64), (64, 32, 65), (65, 33, 1024), (100, 64, 20011), (602, 256, 3001), (256, 41, 1024),
+                                   (13, 200, 4097)])
+def test_weight_grad_matches_float64(m, n, k):
+    """A running sum of k products of unit normals stays within 4 sqrt(k), and its k roundings of 2^-24 of that add up like
+    sqrt(k): 2^-22 k (plus the products' own roundings, which count where k is small)."""
+    import fastgl
+    gen = torch.Generator("cuda").manual_seed(m)
+    wide = torch.randn((k, m + 3), generator=gen, device="cuda")
+    for x in (wide[:, :m], wide[:, 1: m + 1], wide[:, :m].contiguous()):
+        dy = torch.randn((k, n), generator=gen, device="cuda")
+        want = x.double().t() @ dy.double()
+        got = fastgl.weight_grad(x, dy)
+        assert float((got - want).abs().max()) <= 2.0 ** -22 * (k + 16)
+        assert torch.equal(got, fastgl.weight_grad(x, dy))
