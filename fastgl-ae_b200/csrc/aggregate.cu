@@ -16,6 +16,7 @@
 // read-modify-write per neighbour) and K9 / K11 (:468-517, :555-596: scalar atomics, the GCN one built from
 // two atomicExch in a retry loop).
 #include <algorithm>
+#include <atomic>
 
 #include <cooperative_groups.h>
 
@@ -831,10 +832,21 @@ static void launch_fwd_nacc(const AggParams& p, dim3 grid, cudaStream_t st) {
         launch_fwd_staged<MODE == FGL_AGG_EDGE ? FGL_AGG_SUM : MODE>(p, st);
     } else if (chunks <= 32)
         launch_fwd<VEC, MODE, 1, FGL_AGG_UNR1>(p, grid, st);
-    else if (chunks <= 64)
-        launch_fwd<VEC, MODE, 2, 4>(p, grid, st);
+    else if (VEC == 4) {
+        if (chunks <= 64) launch_fwd<VEC, MODE, 2, 4>(p, grid, st);
+        else launch_fwd<VEC, MODE, 4, 2>(p, grid, st);
+    // Rows that are only 8- or 4-byte aligned: a load brings half or a quarter of the bytes, so twice or four times as many
+    // are kept in flight (602 floats: 16 -> 40 KB per SM), and a row of up to 320 vectors is one pass.
+    } else if (chunks <= 64)
+        launch_fwd<VEC, MODE, 2, 8>(p, grid, st);
+    else if (chunks <= 128)
+        launch_fwd<VEC, MODE, 4, VEC == 2 ? 4 : 8>(p, grid, st);
+    else if (chunks <= 160)
+        launch_fwd<VEC, MODE, 5, VEC == 2 ? 3 : 6>(p, grid, st);
+    else if (chunks <= 320)
+        launch_fwd<VEC, MODE, 10, VEC == 2 ? 2 : 3>(p, grid, st);
     else
-        launch_fwd<VEC, MODE, 4, 2>(p, grid, st);
+        launch_fwd<VEC, MODE, 8, VEC == 2 ? 2 : 4>(p, grid, st);
 }
 
 template <int VEC>
@@ -1193,7 +1205,7 @@ int fgl_agg_bwd_self(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int3
 // The scatter above adds every edge's contribution with a vector reduction: its speed is the L2's reduction rate
 // and the order of the additions -- hence the last bits of the result -- changes from run to run.  Here the block is
 // transposed once (per-source lists of destination rows: histogram, scan, fill) and every gradient row dx[s] is
-// then produced by exactly one warp (sources with at most 32 in-block out-edges) or one CTA (hubs), which adds the
+// then produced by exactly one warp (sources with at most kHubThreshold in-block out-edges) or one CTA per tile (hubs), which adds the
 // rows dy[d] of its list in ascending order of d.  The order is a property of the block, not of the schedule, so two
 // runs give the same bits; dx[s] is written once, with the self term folded in, so it needs no initialisation.
 // Replaces K9 / K11 (aggregate_acc_kernel.cu:468-517, :555-596) like agg_bwd_kernel does.
@@ -1203,7 +1215,7 @@ struct GatherParams {
     const int32_t* indptr;    // block CSR over destinations (mean weights)
     const int32_t* t_indptr;  // transposed: per source, [n_src + 1]
     const int32_t* t_dst;     // destination rows, grouped by source (order within a group: arbitrary)
-    const int32_t* hubs;      // [0] number of sources with more than 32 entries, then their ids
+    const int32_t* hubs;      // [0] number of sources with more than kHubThreshold entries, then their ids
     const int32_t* src_deg;
     const int32_t* dst_deg;
     const float* dy;
@@ -1212,10 +1224,10 @@ struct GatherParams {
     int64_t ldy, ld_self, ldx;
     int32_t dim, n_dst, n_src;
     const int32_t* n_dst_dev;
-    int32_t hub_ctas;  // agg_bwd_gather_kernel: the first hub_ctas CTAs take the hubs of 33 .. kHubSplitMin entries
+    int32_t hub_ctas;  // agg_bwd_gather_kernel: so many CTAs take the hubs
 };
 
-constexpr int kHubThreshold = 32;
+constexpr int kHubThreshold = 128;  // sources with more entries than a warp sorts in its registers
 
 template <int MODE>
 __device__ __forceinline__ float gather_weight(const GatherParams& p, int d) {
@@ -1224,38 +1236,137 @@ __device__ __forceinline__ float gather_weight(const GatherParams& p, int d) {
     return 1.0f;
 }
 
-// Histogram of the sources (pass 0) and placement of every edge's destination row behind its source's cursor (pass 1).
-__global__ void __launch_bounds__(256) transpose_edges_kernel(const int32_t* __restrict__ indptr, const int32_t* __restrict__ src,
-                                                              int n_dst, int n_src, const int32_t* __restrict__ n_dst_dev,
-                                                              int32_t* __restrict__ cnt, const int32_t* __restrict__ t_indptr,
-                                                              int32_t* __restrict__ cursor, int32_t* __restrict__ t_dst,
-                                                              int64_t t_cap, int32_t* __restrict__ status, int pass) {
-    const int lane = threadIdx.x & 31;
-    const int warp_global = blockIdx.x * 8 + (threadIdx.x >> 5), n_warps = gridDim.x * 8;
-    if (n_dst_dev) n_dst = min(max(__ldg(n_dst_dev), 0), n_dst);
-    for (int d = warp_global; d < n_dst; d += n_warps) {
-        const int a = __ldg(indptr + d), b = __ldg(indptr + d + 1);
-        for (int e = a + lane; e < b; e += 32) {
-            const int s = __ldg(src + e);
-            if (s < 0 || s >= n_src) {
-                if (status) set_status(status, FGL_ERR_BOUNDS);
-                continue;
-            }
-            if (pass == 0) {
-                atomicAdd(cnt + s, 1);
-            } else {
-                const int64_t at = (int64_t)__ldg(t_indptr + s) + atomicAdd(cursor + s, 1);
-                if (at < t_cap) t_dst[at] = d;
-                else if (status) set_status(status, FGL_ERR_CAPACITY);
-            }
+// The whole transposition in one cooperative launch: sixteen lanes per destination row count their edges' sources and keep
+// (source, rank, destination) in registers over the scan of the counts (two levels, over the CTAs' runs of sources) until they
+// place them.  Edges beyond what the registers hold (rows past the first kKeep of a group of lanes, or entries past the
+// sixteenth of a row) are counted apart and placed behind the others of their source with a second round of atomics.
+// As seven launches -- zeroing, histogram, scan, placement, hubs -- it was 36 us on the device and 20 us on the host for a
+// block of 374 k edges.
+constexpr int kTransposeThreads = 512;
+constexpr int kTransposeMaxCtas = kWsTeamMax;
+constexpr int kKeep = 4;
+
+struct TransposeParams {
+    const int32_t* indptr;
+    const int32_t* src;
+    int32_t n_dst, n_src;
+    const int32_t* n_dst_dev;
+    int32_t* t_indptr;
+    int32_t* t_dst;
+    int64_t t_cap;
+    int32_t* hubs;
+    int32_t* counts;            // 2 * n_src words: kept edges, then the others
+    unsigned long long* bar;    // barrier counter; the next word: what it was at when the last launch ended, read by all
+                                // before the first barrier and raised behind the last
+    int32_t* partial;           // one word per CTA
+    int32_t* status;
+};
+
+__global__ void __launch_bounds__(kTransposeThreads) transpose_block_kernel(const TransposeParams p) {
+    __shared__ int s_scan[40];
+    Team t;
+    t.rank = blockIdx.x;
+    t.size = gridDim.x;
+    t.epoch = 0;
+    t.bar = p.bar;
+    t.base = *(volatile unsigned long long*)(p.bar + 1);
+    t.status = p.status;
+    const int n_dst = p.n_dst_dev ? min(max(__ldg(p.n_dst_dev), 0), p.n_dst) : p.n_dst;
+    const int tid = blockIdx.x * kTransposeThreads + (int)threadIdx.x, n_threads = gridDim.x * kTransposeThreads;
+    int32_t* const more = p.counts + p.n_src;
+    for (int64_t i = tid; i < 2 * (int64_t)p.n_src; i += n_threads) __stcg(p.counts + i, 0);
+    if (tid == 0) p.hubs[0] = 0;
+    const int lane = threadIdx.x & 15, group = tid >> 4, groups = n_threads >> 4;
+    int a[kKeep], b[kKeep], src[kKeep], rank[kKeep];
+#pragma unroll
+    for (int q = 0; q < kKeep; ++q) {
+        const int64_t d = group + (int64_t)q * groups;
+        a[q] = d < n_dst ? __ldg(p.indptr + d) : 0;
+        b[q] = d < n_dst ? __ldg(p.indptr + d + 1) : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kKeep; ++q) src[q] = a[q] + lane < b[q] ? __ldg(p.src + a[q] + lane) : -2;
+    if (!team_barrier(t)) return;
+
+    auto count_more = [&](int from, int to) {
+        for (int e = from + lane; e < to; e += 16) {
+            const int s = __ldg(p.src + e);
+            if (s >= 0 && s < p.n_src) atomicAdd(more + s, 1);
+            else if (p.status) set_status(p.status, FGL_ERR_BOUNDS);
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < kKeep; ++q) {
+        rank[q] = 0;
+        if (src[q] >= 0 && src[q] < p.n_src) {
+            rank[q] = atomicAdd(p.counts + src[q], 1);
+        } else {
+            if (src[q] != -2 && p.status) set_status(p.status, FGL_ERR_BOUNDS);
+            src[q] = -2;
         }
     }
-}
+#pragma unroll
+    for (int q = 0; q < kKeep; ++q) count_more(a[q] + 16, b[q]);
+    for (int64_t d = group + (int64_t)kKeep * groups; d < n_dst; d += groups) count_more(__ldg(p.indptr + d), __ldg(p.indptr + d + 1));
+    if (!team_barrier(t)) return;
 
-// The list of hubs: sources with more than kHubThreshold entries.  hubs[0] was zeroed by the host.
-__global__ void __launch_bounds__(256) list_hubs_kernel(const int32_t* __restrict__ t_indptr, int n_src, int32_t* __restrict__ hubs) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_src; s += gridDim.x * blockDim.x)
-        if (__ldg(t_indptr + s + 1) - __ldg(t_indptr + s) > kHubThreshold) hubs[1 + atomicAdd(hubs, 1)] = s;
+    // every CTA scans a run of sources
+    constexpr int kPer = 4;
+    const int per = ((p.n_src + t.size - 1) / t.size + kPer - 1) / kPer * kPer;
+    const int lo = min((int64_t)p.n_src, (int64_t)t.rank * per), hi = min(p.n_src, lo + per);
+    int acc = 0;
+    for (int i = lo + (int)threadIdx.x; i < hi; i += kTransposeThreads) acc += __ldcg(p.counts + i) + __ldcg(more + i);
+    const int mine = block_sum(acc, s_scan);
+    if (threadIdx.x == 0) __stcg(p.partial + t.rank, mine);
+    if (!team_barrier(t)) return;
+
+    int before = 0, total = 0;
+    for (int q = threadIdx.x; q < t.size; q += kTransposeThreads) {
+        const int x = __ldcg(p.partial + q);
+        total += x;
+        if (q < t.rank) before += x;
+    }
+    int running = block_sum(before, s_scan);
+    total = block_sum(total, s_scan);
+    if (tid == 0) p.t_indptr[p.n_src] = total;
+    for (int tile = lo; tile < hi; tile += kPer * kTransposeThreads) {
+        const int base = tile + (int)threadIdx.x * kPer;
+        int v[kPer], sum = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            v[k] = base + k < hi ? __ldcg(p.counts + base + k) + __ldcg(more + base + k) : 0;
+            sum += v[k];
+        }
+        int tile_total;
+        int excl = running + block_excl_scan(sum, s_scan, tile_total);
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if (base + k < hi) __stcg(p.t_indptr + base + k, excl);
+            if (v[k] > kHubThreshold) p.hubs[1 + atomicAdd(p.hubs, 1)] = base + k;
+            excl += v[k];
+        }
+        running += tile_total;
+    }
+    if (!team_barrier(t)) return;
+
+    auto place = [&](int64_t at, int d) {
+        if (at < p.t_cap) p.t_dst[at] = d;
+        else if (p.status) set_status(p.status, FGL_ERR_CAPACITY);
+    };
+    auto place_more = [&](int from, int to, int d) {
+        for (int e = from + lane; e < to; e += 16) {
+            const int s = __ldg(p.src + e);
+            if (s >= 0 && s < p.n_src)
+                place((int64_t)__ldcg(p.t_indptr + s) + __ldcg(p.counts + s) + atomicSub(more + s, 1) - 1, d);
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < kKeep; ++q)
+        if (src[q] != -2) place((int64_t)__ldcg(p.t_indptr + src[q]) + rank[q], group + q * groups);
+#pragma unroll
+    for (int q = 0; q < kKeep; ++q) place_more(a[q] + 16, b[q], group + q * groups);
+    for (int64_t d = group + (int64_t)kKeep * groups; d < n_dst; d += groups) place_more(__ldg(p.indptr + d), __ldg(p.indptr + d + 1), (int)d);
+    if (tid == 0) p.bar[1] = t.base + (t.size > 1 ? (unsigned long long)t.epoch * t.size : 0ULL);
 }
 
 // acc += sum over j < deg of w_j * dy[d_j, columns c0 ..], lane j holding (d_j, w_j); U rows' loads in flight.
@@ -1301,377 +1412,376 @@ __device__ __forceinline__ int warp_sort_ascending(int v, int lane) {
     return v;
 }
 
-// A warp per source row with at most 32 entries: sort the destination rows, add them in that order.  Most sources of a
-// sampled block have one or two entries: those skip the sorting network (one entry) and request only as many rows as
-// they have (the unrolled batch of eight would otherwise load a single row eight times).  Software-pipelining the id
-// chain over the warp's sources, as the forward kernel does, was measured and bought nothing here: with 64 warps per
-// SM the chain is hidden already, and the launch is bound by the rows it reads and the full output row it writes per
-// source.
+// Up to 32 * R keys of a warp (lane l holds the keys r * 32 + l), sorted ascending.
+template <int R>
+__device__ __forceinline__ void warp_sort_regs(int (&v)[R], int lane) {
+#pragma unroll
+    for (int k = 2; k <= 32 * R; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j >= 32) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int o = r ^ (j / 32);
+                    if (o > r) {
+                        const bool up = ((r * 32) & k) == 0;
+                        const int x = v[r], y = v[o];
+                        v[r] = up ? min(x, y) : max(x, y);
+                        v[o] = up ? max(x, y) : min(x, y);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int other = __shfl_xor_sync(0xffffffffu, v[r], j);
+                    const bool up = ((r * 32 + lane) & k) == 0, lower = (lane & j) == 0;
+                    v[r] = (lower == up) ? min(v[r], other) : max(v[r], other);
+                }
+            }
+        }
+    }
+}
+
+// One source row: the sorted list of `deg` <= 32 * R destination rows, lane l holding entries r * 32 + l.
+template <int VEC, int MODE, int NACC, int R>
+__device__ __forceinline__ void gather_one_source(const GatherParams& p, int s, int a, int deg, int chunks, int n_dst, int lane) {
+    using V = Vec<VEC>;
+    using T = typename V::T;
+    constexpr int UNR = NACC == 1 ? 8 : (NACC == 2 ? 4 : 2);
+    int d[R];
+    float w[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) d[r] = r * 32 + lane < deg ? __ldg(p.t_dst + a + r * 32 + lane) : 0x7fffffff;
+    warp_sort_regs<R>(d, lane);
+#pragma unroll
+    for (int r = 0; r < R; ++r) w[r] = r * 32 + lane < deg ? gather_weight<MODE>(p, d[r]) : 0.0f;
+    const float ws = MODE == FGL_AGG_SYMNORM ? 1.0f / sqrtf((float)__ldg(p.src_deg + s)) : 1.0f;
+    const bool self = p.dy_self != nullptr && s < n_dst;
+    const T* self_row = reinterpret_cast<const T*>(p.dy_self + (self ? (int64_t)s * p.ld_self : 0));
+    T* out = reinterpret_cast<T*>(p.dx + (int64_t)s * p.ldx);
+    for (int c0 = 0; c0 < chunks; c0 += 32 * NACC) {
+        T acc[NACC];
+#pragma unroll
+        for (int k = 0; k < NACC; ++k) acc[k] = V::zero();
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (deg > r * 32) gather_add_rows<VEC, NACC, UNR>(p, d[r], w[r], min(32, deg - r * 32), c0, chunks, lane, acc);
+#pragma unroll
+        for (int k = 0; k < NACC; ++k) {
+            const int c = c0 + k * 32 + lane;
+            if (c < chunks) {
+                T v = (MODE == FGL_AGG_SYMNORM) ? V::scale(acc[k], ws) : acc[k];
+                if (self) V::fma(v, 1.0f, __ldg(self_row + c));
+                out[c] = v;
+            }
+        }
+    }
+}
+
+// Sources with at most kHubThreshold entries: a warp takes eight at a time, a quarter of the ids' range apart from one
+// another (popular sources have neighbouring numbers).  Most sources of a sampled block have one to four entries: their offsets,
+// lists and weights are read by the eight quads at once, sorted in the quads, and then G sources' rows at a time are in flight
+// -- one at a time, the chain offset -> list -> weight -> row of every source stood in the way of the next one's.
+// Sources with more entries follow one by one, their lists sorted in the warp's registers.
 template <int VEC, int MODE, int NACC>
 __device__ __forceinline__ void gather_small_sources(const GatherParams& p, int block, int n_blocks) {
     using V = Vec<VEC>;
     using T = typename V::T;
-    constexpr int UNR = NACC == 1 ? 8 : (NACC == 2 ? 4 : 2);
-    const int lane = threadIdx.x & 31;
+    constexpr int G = NACC == 1 ? 4 : (NACC == 2 ? 2 : 1);
+    const int lane = threadIdx.x & 31, quad = lane >> 2, j = lane & 3;
     const int warp_global = block * 8 + (threadIdx.x >> 5), n_warps = n_blocks * 8;
     const int chunks = p.dim / VEC;
     const int n_dst = p.n_dst_dev ? min(max(__ldg(p.n_dst_dev), 0), p.n_dst) : p.n_dst;
-    for (int s = warp_global; s < p.n_src; s += n_warps) {
-        const int a = __ldg(p.t_indptr + s), deg = __ldg(p.t_indptr + s + 1) - a;
-        if (deg > kHubThreshold) continue;  // a hub CTA owns this row
-        int d = lane < deg ? __ldg(p.t_dst + a + lane) : 0x7fffffff;
-        if (deg > 1) d = warp_sort_ascending(d, lane);
-        const float w = lane < deg ? gather_weight<MODE>(p, d) : 0.0f;
-        const float ws = (MODE == FGL_AGG_SYMNORM && deg > 0) ? 1.0f / sqrtf((float)__ldg(p.src_deg + s)) : 1.0f;
-        const bool self = p.dy_self != nullptr && s < n_dst;
-        const T* self_row = reinterpret_cast<const T*>(p.dy_self + (self ? (int64_t)s * p.ld_self : 0));
-        T* out = reinterpret_cast<T*>(p.dx + (int64_t)s * p.ldx);
-        for (int c0 = 0; c0 < chunks; c0 += 32 * NACC) {
-            T acc[NACC];
-#pragma unroll
-            for (int k = 0; k < NACC; ++k) acc[k] = V::zero();
-            if (deg <= 1)
-                gather_add_rows<VEC, NACC, 1>(p, d, w, deg, c0, chunks, lane, acc);
-            else if (deg <= 2 || UNR <= 2)
-                gather_add_rows<VEC, NACC, 2>(p, d, w, deg, c0, chunks, lane, acc);
-            else if (deg <= 4 || UNR <= 4)
-                gather_add_rows<VEC, NACC, 4>(p, d, w, deg, c0, chunks, lane, acc);
-            else
-                gather_add_rows<VEC, NACC, 8>(p, d, w, deg, c0, chunks, lane, acc);
-#pragma unroll
-            for (int k = 0; k < NACC; ++k) {
-                const int c = c0 + k * 32 + lane;
-                if (c < chunks) {
-                    T r = (MODE == FGL_AGG_SYMNORM) ? V::scale(acc[k], ws) : acc[k];
-                    if (self) V::fma(r, 1.0f, __ldg(self_row + c));
-                    out[c] = r;
-                }
-            }
+    const int eighth = (p.n_src + 7) / 8;
+    for (int u = warp_global; u < eighth; u += n_warps) {
+        const int s = quad * eighth + u;
+        int a = 0, deg = 0;
+        if (s < p.n_src) {
+            a = __ldg(p.t_indptr + s);
+            deg = __ldg(p.t_indptr + s + 1) - a;
         }
-    }
-}
-
-// Hubs of at most kHubSortMax entries.  The hub's destination rows are sorted in shared memory (bitonic network over the
-// list padded to a power of two), warp k then adds the rows of the k-th eighth of the sorted list in order and the eight
-// partial sums are folded in a fixed order: the result does not depend on the order in which the transposition's
-// atomics filled the list.  16 KB of list per CTA, so several hubs are in flight per SM.
-//   CLUSTER = false: a CTA per hub of up to kHubSplitMin entries.
-//   CLUSTER = true:  a thread-block cluster of eight CTAs per hub of kHubSplitMin + 1 .. kHubSortMax entries.  CTA r
-//                    keeps the entries whose destination lies in the r-th eighth of the destination range (a fixed
-//                    partition, whatever the order of the list), sorts and adds them as above, and rank 0 folds the
-//                    eight CTA sums in rank order, reading them through distributed shared memory.  A hub of 4000
-//                    entries is then 8 x 8 warps deep instead of 8.
-constexpr int kHubSortMax = 4096;
-constexpr int kHubSplitMin = 512;
-constexpr int kHubCluster = 8;
-
-template <int VEC, int MODE, int NACC, bool CLUSTER>
-__device__ __forceinline__ void gather_hubs_sorted(const GatherParams& p, int block, int n_blocks) {
-    namespace cg = cooperative_groups;
-    using V = Vec<VEC>;
-    using T = typename V::T;
-    extern __shared__ __align__(16) unsigned char hub_smem[];
-    __shared__ int s_count;
-    int* list = reinterpret_cast<int*>(hub_smem);                          // kHubSortMax entries
-    T* part = reinterpret_cast<T*>(hub_smem + kHubSortMax * sizeof(int));  // [8][NACC][32]
-    T* cta_sum = part + 8 * NACC * 32;                                     // [NACC][32], CLUSTER only
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int chunks = p.dim / VEC;
-    const int n_dst = p.n_dst_dev ? min(max(__ldg(p.n_dst_dev), 0), p.n_dst) : p.n_dst;
-    const int n_hubs = min(__ldg(p.hubs), p.n_src);
-    const int rank = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
-    const int unit = CLUSTER ? block / kHubCluster : block;
-    const int n_units = CLUSTER ? n_blocks / kHubCluster : n_blocks;
-    const int seg = (n_dst + kHubCluster - 1) / kHubCluster;  // destination rows per cluster rank
-    constexpr int UNR = NACC == 1 ? 8 : (NACC == 2 ? 4 : 2);
-    // This unit (CTA or cluster) looks after the hubs h = unit (mod n_units).  Which of them are of its size class is
-    // found 256 at a time, a thread per hub, and compacted in index order -- every CTA of a cluster arrives at the same
-    // list -- instead of one dependent pair of loads per hub in turn; longer lists are counted by agg_bwd_hub_kernel.
-    __shared__ int s_sel[256];
-    __shared__ int s_wcnt[8];
-    for (int base = 0; base < n_hubs; base += 256 * n_units) {
-        const int h_t = base + (int)threadIdx.x * n_units + unit;
-        bool ok = false;
-        if (h_t < n_hubs) {
-            const int s_t = __ldg(p.hubs + 1 + h_t);
-            const int deg_t = __ldg(p.t_indptr + s_t + 1) - __ldg(p.t_indptr + s_t);
-            ok = CLUSTER ? (deg_t > kHubSplitMin && deg_t <= kHubSortMax) : (deg_t <= kHubSplitMin);
+        int d = j < deg ? __ldg(p.t_dst + a + j) : 0x7fffffff;
+        if (deg > 4) d = 0x7fffffff;
+        {  // sorted within the quad
+            int o = __shfl_xor_sync(0xffffffffu, d, 1);
+            d = ((j & 1) == ((j >> 1) & 1)) ? min(d, o) : max(d, o);
+            o = __shfl_xor_sync(0xffffffffu, d, 2);
+            d = (j & 2) ? max(d, o) : min(d, o);
+            o = __shfl_xor_sync(0xffffffffu, d, 1);
+            d = (j & 1) ? max(d, o) : min(d, o);
         }
-        const unsigned bal = __ballot_sync(0xffffffffu, ok);
-        if (lane == 0) s_wcnt[warp] = __popc(bal);
-        __syncthreads();
-        int sel_before = 0, n_sel = 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            if (q < warp) sel_before += s_wcnt[q];
-            n_sel += s_wcnt[q];
-        }
-        if (ok) s_sel[sel_before + __popc(bal & ((1u << lane) - 1u))] = h_t;
-        __syncthreads();
-        for (int q_sel = 0; q_sel < n_sel; ++q_sel) {
-            const int s = __ldg(p.hubs + 1 + s_sel[q_sel]);
-            const int a = __ldg(p.t_indptr + s), deg = __ldg(p.t_indptr + s + 1) - a;
-            int m = deg;
-            if (CLUSTER) {
-                if (threadIdx.x == 0) s_count = 0;
-                __syncthreads();
-                for (int i = threadIdx.x; i < deg; i += 256) {
-                    const int d = __ldg(p.t_dst + a + i);
-                    if (d >= rank * seg && d < (rank + 1) * seg) list[atomicAdd(&s_count, 1)] = d;
-                }
-                __syncthreads();
-                m = s_count;
-            } else {
-                for (int i = threadIdx.x; i < deg; i += 256) list[i] = __ldg(p.t_dst + a + i);
-            }
-            int n2 = 64;
-            while (n2 < m) n2 <<= 1;
-            for (int i = m + (int)threadIdx.x; i < n2; i += 256) list[i] = 0x7fffffff;
-            __syncthreads();
-            for (int k = 2; k <= n2; k <<= 1) {
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    for (int i = threadIdx.x; i < n2; i += 256) {
-                        const int l = i ^ j;
-                        if (l > i) {
-                            const int x = list[i], y = list[l];
-                            if ((x > y) == ((i & k) == 0)) {
-                                list[i] = y;
-                                list[l] = x;
-                            }
-                        }
-                    }
-                    __syncthreads();
-                }
-            }
-            const float ws = (MODE == FGL_AGG_SYMNORM) ? 1.0f / sqrtf((float)__ldg(p.src_deg + s)) : 1.0f;
-            const bool self = p.dy_self != nullptr && s < n_dst;
-            const int per = (m + 7) / 8;
-            const int lo = warp * per, hi = min(lo + per, m);
+        const bool on = j < deg && deg <= 4;
+        const float w = on ? gather_weight<MODE>(p, d) : 0.0f;
+        const float ws = (MODE == FGL_AGG_SYMNORM && deg > 0 && deg <= 4) ? 1.0f / sqrtf((float)__ldg(p.src_deg + s)) : 1.0f;
+        const unsigned few = __ballot_sync(0xffffffffu, s < p.n_src && deg <= 4);   // bit 4 * i: source i is settled here
+        const unsigned many = __ballot_sync(0xffffffffu, deg > 4 && deg <= kHubThreshold);
+        const unsigned entry = __ballot_sync(0xffffffffu, on);
+#pragma unroll 1
+        for (int i0 = 0; i0 < 8; i0 += G) {
+            if (((few >> (4 * i0)) & (G == 4 ? 0xffffu : (G == 2 ? 0xffu : 0xfu))) == 0) continue;
             for (int c0 = 0; c0 < chunks; c0 += 32 * NACC) {
-                T acc[NACC];
+                T acc[G][NACC];
 #pragma unroll
-                for (int k = 0; k < NACC; ++k) acc[k] = V::zero();
-                for (int j0 = lo; j0 < hi; j0 += UNR) {
-                    T v[UNR][NACC];
-                    float wj[UNR];
+                for (int g = 0; g < G; ++g)
 #pragma unroll
-                    for (int u = 0; u < UNR; ++u) {
-                        const int dj = list[min(j0 + u, hi - 1)];
-                        wj[u] = gather_weight<MODE>(p, dj);
-                        const T* row = reinterpret_cast<const T*>(p.dy + (int64_t)dj * p.ldy);
+                    for (int k = 0; k < NACC; ++k) {
+                        acc[g][k] = V::zero();
+                    }
+#pragma unroll 1
+                for (int e = 0; e < 4; ++e) {
+                    unsigned any = 0;
+#pragma unroll
+                    for (int g = 0; g < G; ++g) any |= (entry >> (4 * (i0 + g) + e)) & 1u;
+                    if (!any) break;  // warp-uniform; the entries of a source fill its quad from the front
+                    T v[G][NACC];
+                    float we[G];
+#pragma unroll
+                    for (int g = 0; g < G; ++g) {
+                        const int from = 4 * (i0 + g) + e;
+                        const bool has = (entry >> from) & 1u;
+                        const int de = __shfl_sync(0xffffffffu, d, from);
+                        we[g] = __shfl_sync(0xffffffffu, w, from);
+                        const T* row = reinterpret_cast<const T*>(p.dy + (int64_t)(has ? de : 0) * p.ldy);
 #pragma unroll
                         for (int k = 0; k < NACC; ++k) {
                             const int c = c0 + k * 32 + lane;
-                            v[u][k] = c < chunks ? __ldg(row + c) : V::zero();
+                            v[g][k] = has && c < chunks ? __ldg(row + c) : V::zero();
                         }
                     }
 #pragma unroll
-                    for (int u = 0; u < UNR; ++u)
-                        if (j0 + u < hi) {
+                    for (int g = 0; g < G; ++g)
 #pragma unroll
-                            for (int k = 0; k < NACC; ++k) V::fma(acc[k], wj[u], v[u][k]);
-                        }
+                        for (int k = 0; k < NACC; ++k) V::fma(acc[g][k], we[g], v[g][k]);
                 }
 #pragma unroll
-                for (int k = 0; k < NACC; ++k) part[(warp * NACC + k) * 32 + lane] = acc[k];
-                __syncthreads();
-                T total[NACC];
-                if (warp == 0) {  // the CTA's sum: the eight warps' partial sums in warp order
-#pragma unroll
-                    for (int k = 0; k < NACC; ++k) {
-                        total[k] = V::zero();
-                        for (int q = 0; q < 8; ++q) V::fma(total[k], 1.0f, part[(q * NACC + k) * 32 + lane]);
-                        if (CLUSTER) cta_sum[k * 32 + lane] = total[k];
-                    }
-                }
-                if (CLUSTER) {
-                    cg::this_cluster().sync();  // every CTA's sum is in its shared memory
-                    if (rank == 0 && warp == 0) {
-#pragma unroll
-                        for (int k = 0; k < NACC; ++k) {
-                            for (int q = 1; q < kHubCluster; ++q)
-                                V::fma(total[k], 1.0f, cg::this_cluster().map_shared_rank(cta_sum, q)[k * 32 + lane]);
-                        }
-                    }
-                }
-                if (rank == 0 && warp == 0) {
-                    T* out = reinterpret_cast<T*>(p.dx + (int64_t)s * p.ldx);
+                for (int g = 0; g < G; ++g) {
+                    if (!((few >> (4 * (i0 + g))) & 1u)) continue;
+                    const int sg = (i0 + g) * eighth + u;
+                    const float wg = MODE == FGL_AGG_SYMNORM ? __shfl_sync(0xffffffffu, ws, 4 * (i0 + g)) : 1.0f;
+                    const bool self = p.dy_self != nullptr && sg < n_dst;
+                    const T* self_row = reinterpret_cast<const T*>(p.dy_self + (self ? (int64_t)sg * p.ld_self : 0));
+                    T* out = reinterpret_cast<T*>(p.dx + (int64_t)sg * p.ldx);
 #pragma unroll
                     for (int k = 0; k < NACC; ++k) {
                         const int c = c0 + k * 32 + lane;
                         if (c < chunks) {
-                            T r = (MODE == FGL_AGG_SYMNORM) ? V::scale(total[k], ws) : total[k];
-                            if (self) V::fma(r, 1.0f, __ldg(reinterpret_cast<const T*>(p.dy_self + (int64_t)s * p.ld_self) + c));
+                            T r = (MODE == FGL_AGG_SYMNORM) ? V::scale(acc[g][k], wg) : acc[g][k];
+                            if (self) V::fma(r, 1.0f, __ldg(self_row + c));
                             out[c] = r;
                         }
                     }
                 }
-                if (CLUSTER) cg::this_cluster().sync();  // rank 0 has read the sums: they may be overwritten
-                __syncthreads();
             }
         }
-        __syncthreads();  // the selection is consumed: the next 256 candidates may overwrite it
+        for (unsigned m = many & 0x11111111u; m; m &= m - 1) {  // warp-uniform
+            const int from = __ffs(m) - 1;
+            const int sm = (from >> 2) * eighth + u, am = __shfl_sync(0xffffffffu, a, from), dm = __shfl_sync(0xffffffffu, deg, from);
+            if (dm <= 32) gather_one_source<VEC, MODE, NACC, 1>(p, sm, am, dm, chunks, n_dst, lane);
+            else if (dm <= 64) gather_one_source<VEC, MODE, NACC, 2>(p, sm, am, dm, chunks, n_dst, lane);
+            else gather_one_source<VEC, MODE, NACC, 4>(p, sm, am, dm, chunks, n_dst, lane);
+        }
     }
 }
 
-// One launch for the sources of up to kHubSplitMin entries: the first hub_ctas CTAs (they run longest, so they start
-// first) each take hubs of 33 .. kHubSplitMin entries, the others take the small sources a warp at a time.
-template <int VEC, int MODE, int NACC>
-__global__ void __launch_bounds__(256) agg_bwd_gather_kernel(const GatherParams p) {
-    if ((int)blockIdx.x < p.hub_ctas)
-        gather_hubs_sorted<VEC, MODE, NACC, false>(p, (int)blockIdx.x, p.hub_ctas);
-    else
-        gather_small_sources<VEC, MODE, NACC>(p, (int)blockIdx.x - p.hub_ctas, (int)gridDim.x - p.hub_ctas);
+// Hubs, a tile of 32 vectors of the row at a time.  The list is sorted (bitonic network in shared memory, over the list padded to
+// a power of two), warp k of the CTA adds the k-th eighth of it and the eight partial sums are folded in warp order, so the result
+// does not depend on the order in which the transposition's atomics filled the list.
+//   CLUSTER = false: a CTA per hub of up to kHubSplitMin entries and tile.
+//   CLUSTER = true:  a cluster of eight CTAs per longer hub and tile, for the longest list of a block is what a launch waits for
+//                    (4800 entries: 200 us in one CTA).  CTA r keeps the entries whose destination lies in the r-th eighth of the
+//                    destination range -- a fixed partition, whatever the order of the list -- and rank 0 folds the CTAs' sums in
+//                    rank order through distributed shared memory.  An eighth with more than kHubSort entries is not sorted but
+//                    counted, over windows of kHubWindow destination rows (16-bit counts), which orders it as well.
+constexpr int kHubSplitMin = 512;
+constexpr int kHubSort = 2048;
+constexpr int kHubWindow = 4096;
+constexpr int kHubCluster = 8;
+constexpr int kHubEvery = 4;  // one of so many clusters of the launch takes hubs
+
+template <typename T>
+struct HubSmem {
+    uint32_t words[kHubSort];  // the list, or the counts of a window
+    T part[8][32];
+    T sum[32];
+    int sel[256];
+    int wcnt[8];
+    int count;
+};
+
+// This thread's column of sum over the sorted list[lo .. hi) of w * dy[d].
+template <int VEC, int MODE>
+__device__ __forceinline__ void hub_add_rows(const GatherParams& p, const int* list, int lo, int hi, const typename Vec<VEC>::T* dy,
+                                             typename Vec<VEC>::T& acc) {
+    using T = typename Vec<VEC>::T;
+    constexpr int UNR = 8;
+    for (int j0 = lo; j0 < hi; j0 += UNR) {
+        T v[UNR];
+        float w[UNR];
+#pragma unroll
+        for (int u = 0; u < UNR; ++u) {
+            const int dj = list[min(j0 + u, hi - 1)];
+            w[u] = gather_weight<MODE>(p, dj);
+            v[u] = __ldg(dy + (int64_t)dj * (p.ldy / VEC));
+        }
+#pragma unroll
+        for (int u = 0; u < UNR; ++u)
+            if (j0 + u < hi) Vec<VEC>::fma(acc, w[u], v[u]);
+    }
 }
 
-// Clusters of kHubCluster CTAs for the hubs of kHubSplitMin + 1 .. kHubSortMax entries.
-template <int VEC, int MODE, int NACC>
-__global__ void __launch_bounds__(256) agg_bwd_hub_cluster_kernel(const GatherParams p) {
-    gather_hubs_sorted<VEC, MODE, NACC, true>(p, (int)blockIdx.x, (int)gridDim.x);
-}
-
-// A CTA per hub with more than kHubSortMax entries.  The hub's destination rows are counted into a shared-memory array
-// over a window of the destination range (16-bit counts, two per word), which orders them without sorting; warp k then
-// adds the rows of the k-th eighth of the window in ascending order, and the eight partial sums are folded in a fixed
-// order.  The 64 KB counting pass costs microseconds per hub whatever its size, hence only for the very long lists.
-constexpr int kHubWindow = 32768;
-
-template <int VEC, int MODE, int NACC>
-__global__ void __launch_bounds__(256) agg_bwd_hub_kernel(const GatherParams p) {
+template <int VEC, int MODE, bool CLUSTER>
+__device__ __forceinline__ void gather_hubs(const GatherParams& p, int block, int n_blocks, HubSmem<typename Vec<VEC>::T>& sm) {
+    namespace cg = cooperative_groups;
     using V = Vec<VEC>;
     using T = typename V::T;
-    extern __shared__ __align__(16) unsigned char hub_smem[];
-    uint32_t* cnt32 = reinterpret_cast<uint32_t*>(hub_smem);                            // kHubWindow / 2 words
-    T* part = reinterpret_cast<T*>(hub_smem + kHubWindow * 2);                           // [8][NACC][32]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int chunks = p.dim / VEC;
+    const int chunks = p.dim / VEC, tiles = (chunks + 31) / 32;
     const int n_dst = p.n_dst_dev ? min(max(__ldg(p.n_dst_dev), 0), p.n_dst) : p.n_dst;
-    const int n_hubs = min(__ldg(p.hubs), p.n_src);
-    constexpr int UNR = 4;
-    for (int h = blockIdx.x; h < n_hubs; h += gridDim.x) {
-        const int s = __ldg(p.hubs + 1 + h);
-        const int a = __ldg(p.t_indptr + s), b = __ldg(p.t_indptr + s + 1);
-        if (b - a <= kHubSortMax) continue;  // sorted by a CTA or a cluster instead
-        const float ws = (MODE == FGL_AGG_SYMNORM) ? 1.0f / sqrtf((float)__ldg(p.src_deg + s)) : 1.0f;
-        const bool self = p.dy_self != nullptr && s < n_dst;
-        for (int c0 = 0; c0 < chunks; c0 += 32 * NACC) {
-            T total[NACC];  // warp 0 keeps the row's running sum over the windows
-#pragma unroll
-            for (int k = 0; k < NACC; ++k) total[k] = V::zero();
-            for (int w0 = 0; w0 < n_dst; w0 += kHubWindow) {
-                for (int i = threadIdx.x; i < kHubWindow / 2; i += 256) cnt32[i] = 0u;
-                __syncthreads();
-                for (int e = a + (int)threadIdx.x; e < b; e += 256) {
-                    const int off = __ldg(p.t_dst + e) - w0;
-                    if (off >= 0 && off < kHubWindow) atomicAdd(cnt32 + (off >> 1), 1u << (16 * (off & 1)));
-                }
-                __syncthreads();
-                T acc[NACC];
-#pragma unroll
-                for (int k = 0; k < NACC; ++k) acc[k] = V::zero();
-                const int lo = warp * (kHubWindow / 8), hi = min(lo + kHubWindow / 8, n_dst - w0);
-                for (int base = lo; base < hi; base += 32) {
-                    const uint32_t word = cnt32[(base + lane) >> 1];
-                    const int c = (int)((word >> (16 * ((base + lane) & 1))) & 0xffffu);
-                    unsigned m = __ballot_sync(0xffffffffu, c > 0);
-                    while (m) {  // warp-uniform
-                        int dd[UNR];
-                        float wd[UNR];
-                        T v[UNR][NACC];
-#pragma unroll
-                        for (int u = 0; u < UNR; ++u) {
-                            dd[u] = -1;
-                            wd[u] = 0.0f;
-                            if (m) {
-                                const int j = __ffs(m) - 1;
-                                m &= m - 1;
-                                dd[u] = w0 + base + j;
-                                wd[u] = (float)__shfl_sync(0xffffffffu, c, j);
-                            }
-                        }
-#pragma unroll
-                        for (int u = 0; u < UNR; ++u) {
-                            const int dj = dd[u] < 0 ? 0 : dd[u];
-                            if (dd[u] >= 0) wd[u] *= gather_weight<MODE>(p, dj);
-                            const T* row = reinterpret_cast<const T*>(p.dy + (int64_t)dj * p.ldy);
-#pragma unroll
-                            for (int k = 0; k < NACC; ++k) {
-                                const int cc = c0 + k * 32 + lane;
-                                v[u][k] = cc < chunks ? __ldg(row + cc) : V::zero();
-                            }
-                        }
-#pragma unroll
-                        for (int u = 0; u < UNR; ++u)
-                            if (dd[u] >= 0) {
-#pragma unroll
-                                for (int k = 0; k < NACC; ++k) V::fma(acc[k], wd[u], v[u][k]);
-                            }
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < NACC; ++k) part[(warp * NACC + k) * 32 + lane] = acc[k];
-                __syncthreads();
-                if (warp == 0) {
-                    for (int q = 0; q < 8; ++q)
-#pragma unroll
-                        for (int k = 0; k < NACC; ++k) V::fma(total[k], 1.0f, part[(q * NACC + k) * 32 + lane]);
-                }
-                __syncthreads();
-            }
-            if (warp == 0) {
-                T* out = reinterpret_cast<T*>(p.dx + (int64_t)s * p.ldx);
-#pragma unroll
-                for (int k = 0; k < NACC; ++k) {
-                    const int c = c0 + k * 32 + lane;
-                    if (c < chunks) {
-                        T r = (MODE == FGL_AGG_SYMNORM) ? V::scale(total[k], ws) : total[k];
-                        if (self) V::fma(r, 1.0f, __ldg(reinterpret_cast<const T*>(p.dy_self + (int64_t)s * p.ld_self) + c));
-                        out[c] = r;
-                    }
-                }
-            }
+    const int rank = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
+    const int unit = CLUSTER ? block / kHubCluster : block;
+    const int n_units = CLUSTER ? n_blocks / kHubCluster : n_blocks;
+    const int64_t n_work = (int64_t)min(__ldg(p.hubs), p.n_src) * tiles;  // (hub, tile) pairs; this unit has unit, unit + n_units, ...
+    int* list = reinterpret_cast<int*>(sm.words);
+    // Which of them are of this size class is found 256 at a time, a thread per pair, and compacted in order -- every CTA of a
+    // cluster arrives at the same selection -- instead of one dependent pair of loads per hub in turn.
+    for (int64_t base = 0; base * n_units + unit < n_work; base += 256) {
+        const int64_t mine = (base + threadIdx.x) * n_units + unit;
+        bool ok = false;
+        if (mine < n_work) {
+            const int s = __ldg(p.hubs + 1 + mine / tiles);
+            const int deg = __ldg(p.t_indptr + s + 1) - __ldg(p.t_indptr + s);
+            ok = CLUSTER ? deg > kHubSplitMin : deg <= kHubSplitMin;
         }
+        const unsigned bal = __ballot_sync(0xffffffffu, ok);
+        if (lane == 0) sm.wcnt[warp] = __popc(bal);
+        __syncthreads();
+        int before = 0, n_sel = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (q < warp) before += sm.wcnt[q];
+            n_sel += sm.wcnt[q];
+        }
+        if (ok) sm.sel[before + __popc(bal & ((1u << lane) - 1u))] = (int)threadIdx.x;
+        __syncthreads();
+        for (int i_sel = 0; i_sel < n_sel; ++i_sel) {
+            const int64_t work = (base + sm.sel[i_sel]) * n_units + unit;
+            const int s = __ldg(p.hubs + 1 + work / tiles), c = (int)(work % tiles) * 32 + lane;
+            const bool in = c < chunks;
+            const int a = __ldg(p.t_indptr + s), deg = __ldg(p.t_indptr + s + 1) - a;
+            const T* dy = reinterpret_cast<const T*>(p.dy) + (in ? c : 0);
+            const int seg = CLUSTER ? (n_dst + kHubCluster - 1) / kHubCluster : n_dst;
+            const int d_lo = rank * seg, d_hi = min(n_dst, d_lo + seg);
+            T acc = V::zero();
+            int m = deg;
+            if (CLUSTER) {
+                if (threadIdx.x == 0) sm.count = 0;
+                __syncthreads();
+                for (int i = threadIdx.x; i < deg; i += 256) {
+                    const int d = __ldg(p.t_dst + a + i);
+                    if (d >= d_lo && d < d_hi) {
+                        const int at = atomicAdd(&sm.count, 1);
+                        if (at < kHubSort) list[at] = d;
+                    }
+                }
+                __syncthreads();
+                m = sm.count;
+            } else {
+                for (int i = threadIdx.x; i < deg; i += 256) list[i] = __ldg(p.t_dst + a + i);
+            }
+            if (m <= kHubSort) {
+                int n2 = 64;
+                while (n2 < m) n2 <<= 1;
+                for (int i = m + (int)threadIdx.x; i < n2; i += 256) list[i] = 0x7fffffff;
+                __syncthreads();
+                for (int k = 2; k <= n2; k <<= 1) {
+                    for (int q = k >> 1; q > 0; q >>= 1) {
+                        for (int i = threadIdx.x; i < n2 / 2; i += 256) {
+                            const int x0 = 2 * i - (i & (q - 1)), x1 = x0 + q;  // the i-th pair of this step
+                            const int x = list[x0], y = list[x1];
+                            if ((x > y) == ((x0 & k) == 0)) {
+                                list[x0] = y;
+                                list[x1] = x;
+                            }
+                        }
+                        __syncthreads();
+                    }
+                }
+                const int per = (m + 7) / 8;
+                hub_add_rows<VEC, MODE>(p, list, warp * per, min(warp * per + per, m), dy, acc);
+            } else {
+                for (int w0 = d_lo; w0 < d_hi; w0 += kHubWindow) {
+                    __syncthreads();  // the previous window's counts have been read
+                    for (int i = threadIdx.x; i < kHubWindow / 2; i += 256) sm.words[i] = 0u;
+                    __syncthreads();
+                    for (int e = a + (int)threadIdx.x; e < a + deg; e += 256) {
+                        const int d = __ldg(p.t_dst + e), off = d - w0;
+                        if (d < d_hi && off >= 0 && off < kHubWindow) atomicAdd(sm.words + (off >> 1), 1u << (16 * (off & 1)));
+                    }
+                    __syncthreads();
+                    const int hi = min(kHubWindow, d_hi - w0);
+                    for (int off = warp * (kHubWindow / 8); off < min((warp + 1) * (kHubWindow / 8), hi); ++off) {
+                        const int n = (int)((sm.words[off >> 1] >> (16 * (off & 1))) & 0xffffu);
+                        if (n) V::fma(acc, (float)n * gather_weight<MODE>(p, w0 + off), __ldg(dy + (int64_t)(w0 + off) * (p.ldy / VEC)));
+                    }
+                }
+            }
+            sm.part[warp][lane] = acc;
+            __syncthreads();
+            T total = V::zero();
+            if (warp == 0) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) V::fma(total, 1.0f, sm.part[q][lane]);
+                if (CLUSTER) sm.sum[lane] = total;
+            }
+            if (CLUSTER) {
+                cg::this_cluster().sync();
+                if (rank == 0 && warp == 0)
+                    for (int q = 1; q < kHubCluster; ++q) V::fma(total, 1.0f, cg::this_cluster().map_shared_rank(sm.sum, q)[lane]);
+            }
+            if (rank == 0 && warp == 0 && in) {
+                if (MODE == FGL_AGG_SYMNORM) total = V::scale(total, 1.0f / sqrtf((float)__ldg(p.src_deg + s)));
+                if (p.dy_self != nullptr && s < n_dst)
+                    V::fma(total, 1.0f, __ldg(reinterpret_cast<const T*>(p.dy_self + (int64_t)s * p.ld_self) + c));
+                reinterpret_cast<T*>(p.dx + (int64_t)s * p.ldx)[c] = total;
+            }
+            if (CLUSTER) cg::this_cluster().sync();  // rank 0 has read the sums
+            __syncthreads();                         // list and partial sums are consumed
+        }
+        __syncthreads();
     }
 }
 
-// Clusters of kHubCluster CTAs, one cluster per hub at a time; about two clusters' worth of CTAs per SM-octet.
-static void launch_hub_clusters(void (*kernel)(const GatherParams), const GatherParams& p, int sms, size_t dyn, cudaStream_t st) {
-    cudaLaunchConfig_t cfg{};
-    const int n_clusters = std::max(1, 2 * sms / kHubCluster);
-    cfg.gridDim = dim3((unsigned)(n_clusters * kHubCluster));
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = dyn;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kHubCluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, p);
+// One launch of clusters: of every kHubEvery one takes hubs (while there are hub clusters), the others' CTAs the remaining sources.
+// What the launch needs is row data in flight: held to 64 registers (four CTAs per SM; six where a lane's load is 8 or 4 bytes)
+// it is faster than with the 110 the compiler would take, a few spills included (inner block of 26 k x 173 k rows, 374 k edges:
+// 256 floats 166 -> 108 us; reads of the rows, 410 MB, and writes, 177 MB, then go through the L2 at 5.4 TB/s).
+template <int VEC, int MODE, int NACC>
+__global__ void __cluster_dims__(kHubCluster, 1, 1) __launch_bounds__(256, VEC == 4 ? 4 : 6) agg_bwd_gather_kernel(const GatherParams p) {
+    __shared__ HubSmem<typename Vec<VEC>::T> sm;
+    const int cluster = (int)blockIdx.x / kHubCluster, r = (int)blockIdx.x % kHubCluster;
+    const int hub_clusters = p.hub_ctas / kHubCluster;
+    if (cluster < hub_clusters * kHubEvery && cluster % kHubEvery == 0) {
+        const int block = cluster / kHubEvery * kHubCluster + r;
+        gather_hubs<VEC, MODE, true>(p, block, p.hub_ctas, sm);
+        gather_hubs<VEC, MODE, false>(p, block, p.hub_ctas, sm);
+    } else {
+        const int others = cluster - min(cluster / kHubEvery + 1, hub_clusters);
+        gather_small_sources<VEC, MODE, NACC>(p, others * kHubCluster + r, (int)gridDim.x - p.hub_ctas);
+    }
 }
 
 template <int VEC, int MODE>
 static void launch_gather_nacc(const GatherParams& p, int sms, cudaStream_t st) {
     const int chunks = p.dim / VEC;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)p.n_src + 7) / 8, (int64_t)sms * 8));
-    const int hub_grid = 2 * sms;
-#define FGL_GATHER(NACC)                                                                                           \
-    {                                                                                                              \
-        const size_t dyn = (size_t)kHubWindow * 2 + sizeof(typename Vec<VEC>::T) * 8 * NACC * 32;                  \
-        const size_t dyn_sorted = (size_t)kHubSortMax * sizeof(int) + sizeof(typename Vec<VEC>::T) * 9 * NACC * 32; \
-        GatherParams q = p;                                                                                        \
-        q.hub_ctas = 6 * sms;                                                                                      \
-        agg_bwd_gather_kernel<VEC, MODE, NACC><<<grid + q.hub_ctas, 256, dyn_sorted, st>>>(q);                     \
-        launch_hub_clusters(agg_bwd_hub_cluster_kernel<VEC, MODE, NACC>, p, sms, dyn_sorted, st);                  \
-        cudaFuncSetAttribute(agg_bwd_hub_kernel<VEC, MODE, NACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn); \
-        agg_bwd_hub_kernel<VEC, MODE, NACC><<<hub_grid, 256, dyn, st>>>(p);                                        \
-    }
-    if (chunks <= 32) FGL_GATHER(1)
-    else if (chunks <= 64) FGL_GATHER(2)
-    else FGL_GATHER(4)
-#undef FGL_GATHER
+    GatherParams q = p;
+    const int64_t want = ((int64_t)p.n_src + 64 * kHubCluster - 1) / (64 * kHubCluster);  // clusters, eight sources per warp
+    const int small = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * 8 / kHubCluster));
+    const int hub_clusters = std::max(1, std::min(2 * sms / kHubCluster, small / (kHubEvery - 1)));
+    q.hub_ctas = hub_clusters * kHubCluster;
+    const int grid = std::max(small + hub_clusters, hub_clusters * kHubEvery - (kHubEvery - 2)) * kHubCluster;
+    if (chunks <= 32) agg_bwd_gather_kernel<VEC, MODE, 1><<<grid, 256, 0, st>>>(q);
+    else if (chunks <= 64) agg_bwd_gather_kernel<VEC, MODE, 2><<<grid, 256, 0, st>>>(q);
+    else agg_bwd_gather_kernel<VEC, MODE, 4><<<grid, 256, 0, st>>>(q);
 }
 
 template <int VEC>
@@ -1690,25 +1800,23 @@ int fgl_block_transpose(fgl_ws* ws, const int32_t* indptr, const int32_t* src, i
     if (!ws || n_dst < 0 || n_src < 0 || t_cap < 0) return FGL_ERR_INVALID;
     if (!t_indptr || !hubs || (n_src > 0 && !work) || (t_cap > 0 && !t_dst) || (n_dst > 0 && (!indptr || !src))) return FGL_ERR_INVALID;
     cudaStream_t st = (cudaStream_t)stream;
-    int sms = ws->sm_count > 0 ? ws->sm_count : 148;
-    if (cudaMemsetAsync(hubs, 0, sizeof(int32_t), st) != cudaSuccess) return FGL_ERR_CUDA;
-    if (n_src == 0) return cudaMemsetAsync(t_indptr, 0, sizeof(int32_t), st) == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
-    if (cudaMemsetAsync(work, 0, sizeof(int32_t) * 2 * (size_t)n_src, st) != cudaSuccess) return FGL_ERR_CUDA;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n_dst + 7) / 8, (int64_t)sms * 8));
-    {
-        DeviceGuard guard(ws->device);
-        if (n_dst > 0)
-            transpose_edges_kernel<<<grid, 256, 0, st>>>(indptr, src, n_dst, n_src, n_dst_dev, work, nullptr, nullptr, nullptr, 0,
-                                                         ws->status, 0);
-    }
-    int rc = fgl_exclusive_sum(ws, work, n_src, t_indptr, stream);
-    if (rc != FGL_OK) return rc;
+    std::lock_guard<std::mutex> lock(ws->mu);
     DeviceGuard guard(ws->device);
-    if (n_dst > 0)
-        transpose_edges_kernel<<<grid, 256, 0, st>>>(indptr, src, n_dst, n_src, n_dst_dev, nullptr, t_indptr, work + n_src, t_dst,
-                                                     t_cap, ws->status, 1);
-    list_hubs_kernel<<<std::max(1, std::min((n_src + 255) / 256, sms * 4)), 256, 0, st>>>(t_indptr, n_src, hubs);
-    return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
+    static std::atomic<int> cached{0};  // the same on every device of this architecture
+    int per_sm = cached.load(std::memory_order_relaxed);
+    if (per_sm == 0) {
+        FGL_CUDA_OK(ws, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, transpose_block_kernel, kTransposeThreads, 0));
+        cached.store(per_sm, std::memory_order_relaxed);
+    }
+    // two rows per group of lanes and four sources per thread: fewer CTAs make the phases longer, more the barriers
+    const int64_t items = std::max<int64_t>((int64_t)n_dst * 8, n_src / 4);
+    const int64_t most = std::min<int64_t>(kTransposeMaxCtas, (int64_t)std::min(per_sm, 2) * ws->sm_count);
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(most, (items + kTransposeThreads - 1) / kTransposeThreads));
+    TransposeParams p{indptr, src, n_dst, n_src, n_dst_dev, t_indptr, t_dst, t_cap, hubs, work,
+                      (unsigned long long*)(ws->status + kWsTeamWord), ws->status + kWsTeamWord + 32, ws->status};
+    void* args[] = {(void*)&p};
+    FGL_CUDA_OK(ws, cudaLaunchCooperativeKernel((const void*)transpose_block_kernel, dim3(grid), dim3(kTransposeThreads), args, 0, st));
+    return FGL_OK;
 }
 
 int fgl_agg_bwd_gather(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int32_t* t_indptr, const int32_t* t_dst,

@@ -32,6 +32,12 @@ struct Workspace {
     std::string last_error;
 };
 
+// The status allocation: status words, then (from kWsTeamWord on) for launches that take no scratch a barrier counter, the
+// number it was at when the last launch ended (two 64-bit words), and a word per CTA.
+constexpr int kWsTeamWord = 16;
+constexpr int kWsTeamMax = 640;
+constexpr int kWsStatusBytes = (kWsTeamWord + 32 + kWsTeamMax) * 4;
+
 int ws_ensure(Workspace* ws, int64_t table_slots, int64_t scratch_bytes);
 
 // The pair of events a caller asked to have recorded around the next window-level launch (fgl_ws_time_next_launch):
@@ -188,6 +194,7 @@ struct Team {
     unsigned epoch;
     unsigned long long* bar;
     int32_t* status;
+    unsigned long long base = 0;  // what the counter was at when the launch began
     long long spin_limit = kSpinLimit;
 };
 
@@ -197,36 +204,34 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
     return v;
 }
 
-// Returns false when the launch was aborted (another CTA timed out); the caller then returns.
-__device__ __forceinline__ bool team_barrier(Team& t, int* s_flag) {
+// Returns false when the launch was aborted (another CTA timed out); the caller then returns.  A poll is one load -- a second
+// one, of the abort flag, doubled the time until an arrival was seen; that flag is looked at every 32 polls.  (A flag per CTA
+// that every CTA's threads poll saves the additions, but 296 CTAs polling the same ten lines made a barrier 8 us longer.)
+__device__ __forceinline__ bool team_barrier(Team& t) {
     t.epoch += 1;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int aborted = 0;
-        __threadfence();
-        atomicAdd(t.bar, 1ULL);
-        const unsigned long long target = (unsigned long long)t.epoch * (unsigned long long)t.size;
+    int aborted = 0;
+    if (threadIdx.x == 0 && t.size > 1) {
+        // released behind the CTA's writes (ordered before it by __syncthreads)
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(t.bar), "l"(1ULL) : "memory");
+        const unsigned long long target = t.base + (unsigned long long)t.epoch * (unsigned long long)t.size;
         long long spins = 0;
         while (ld_acquire_u64(t.bar) < target) {
+            if ((++spins & 31) != 0) continue;
             if (*(volatile int32_t*)(t.status + 1) != 0) {
                 aborted = 1;
                 break;
             }
-            if (++spins > t.spin_limit) {
+            if (spins > t.spin_limit) {
                 set_status(t.status, FGL_ERR_TIMEOUT);
                 atomicExch(t.status + 1, 1);
                 aborted = 1;
                 break;
             }
-            __nanosleep(32);
+            if (spins > 1024) __nanosleep(64);
         }
-        __threadfence();
-        *s_flag = aborted;
     }
-    __syncthreads();
-    const bool ok = (*s_flag == 0);
-    __syncthreads();
-    return ok;
+    return __syncthreads_or(aborted) == 0;
 }
 
 

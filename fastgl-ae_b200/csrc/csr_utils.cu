@@ -105,7 +105,6 @@ __global__ void __launch_bounds__(kScanThreads) exclusive_sum_kernel(const int32
                                                                      unsigned long long* bar, int32_t* partial,
                                                                      int32_t* status) {
     __shared__ int s_scan[40];
-    __shared__ int s_flag;
     constexpr int kTile = kScanThreads * kScanItems;
     const int64_t n_tiles = (n + kTile - 1) / kTile;
     const int64_t tiles_per = (n_tiles + gridDim.x - 1) / gridDim.x;
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(kScanThreads) exclusive_sum_kernel(const int32
     t.epoch = 0;
     t.bar = bar;
     t.status = status;
-    if (!team_barrier(t, &s_flag)) return;
+    if (!team_barrier(t)) return;
 
     int a = 0, b = 0;
     for (int q = threadIdx.x; q < (int)gridDim.x; q += kScanThreads) {
@@ -277,7 +276,6 @@ __global__ void __launch_bounds__(256) window_overlap_kernel(const int32_t* __re
 // has, so the wait runs out after spin_limit polls, records FGL_ERR_TIMEOUT, raises the abort flag and returns.
 __global__ void __launch_bounds__(32) barrier_timeout_kernel(unsigned long long* bar, int32_t* status, long long spin_limit,
                                                              int32_t* passed) {
-    __shared__ int s_flag;
     Team t;
     t.rank = blockIdx.x;
     t.size = gridDim.x + 1;
@@ -285,7 +283,7 @@ __global__ void __launch_bounds__(32) barrier_timeout_kernel(unsigned long long*
     t.bar = bar;
     t.status = status;
     t.spin_limit = spin_limit;
-    if (team_barrier(t, &s_flag) && threadIdx.x == 0) atomicAdd(passed, 1);  // cannot happen: nobody sends the last arrival
+    if (team_barrier(t) && threadIdx.x == 0) atomicAdd(passed, 1);  // cannot happen: nobody sends the last arrival
 }
 
 }  // namespace fgl

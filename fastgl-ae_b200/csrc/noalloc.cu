@@ -35,7 +35,6 @@ static __device__ __align__(256) unsigned long long g_noalloc_scratch[(kNaWords 
 __global__ void __launch_bounds__(kNaThreads) exclusive_sum_noalloc_kernel(const int32_t* __restrict__ in, int64_t n,
                                                                            int32_t* __restrict__ out, int32_t* scratch) {
     __shared__ int s_scan[40];
-    __shared__ int s_flag;
     unsigned long long* bar = reinterpret_cast<unsigned long long*>(scratch);
     int32_t* status = scratch + 2;
     int32_t* partial = scratch + 32;
@@ -57,7 +56,7 @@ __global__ void __launch_bounds__(kNaThreads) exclusive_sum_noalloc_kernel(const
     t.epoch = 0;
     t.bar = bar;
     t.status = status;
-    if (!team_barrier(t, &s_flag)) return;
+    if (!team_barrier(t)) return;
 
     int a = 0, b = 0;
     for (int q = threadIdx.x; q < (int)gridDim.x; q += kNaThreads) {

@@ -284,7 +284,6 @@ constexpr int kMaxTeam = 512;    // CTAs per team (a cooperative grid of 512-thr
 
 struct Smem {
     int scan[40];
-    int flag;
     int v[kThreads];
     long long start[kThreads];
     int deg[kThreads];
@@ -753,7 +752,7 @@ __device__ __forceinline__ bool phase_sample(const KParams& p, const Hop& h, Tab
                 const int v = __ldcg(h.nodes + s);
                 if (v >= 0 && (int64_t)v < p.n_nodes) table_insert_seed(tab, (uint32_t)v, (uint32_t)s, p.status);
             }
-            if (!team_barrier(t, &sm.flag)) return false;
+            if (!team_barrier(t)) return false;
         }
     }
     if (t.rank == 0 && threadIdx.x == 0) {
@@ -1066,7 +1065,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
                 __stcg(h.node_deg + s, deg);
                 if (deg > 0) atomicAdd(sums + (s >> p.tile_shift[0]), min(deg, p.fanout[0]));
             }
-            if (given_up(p, team_barrier(t, &sm.flag))) return;
+            if (given_up(p, team_barrier(t))) return;
         } else {
             h.nodes = const_cast<int32_t*>(seeds);  // MODE_SAMPLE reads the seeds in place
         }
@@ -1097,20 +1096,20 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
                 turn = next;
             } else {
                 phase_count_seeds<PtrT>(p, h, t, sm, p.team_sums);
-                if (given_up(p, team_barrier(t, &sm.flag))) return;
+                if (given_up(p, team_barrier(t))) return;
             }
 
             if (MODE == MODE_FUSED && !h.last_hop) phase_count_old(h, t);
             int e0, e1;
             if (given_up(p, phase_sample<PtrT, MODE, ARRIVAL>(p, h, tab, log2, used, team_id, t, sm, picks, p.team_sums, cnt, e0, e1))) return;
             if (MODE == MODE_SAMPLE) break;
-            if (given_up(p, team_barrier(t, &sm.flag))) return;
+            if (given_up(p, team_barrier(t))) return;
 
             if (!ARRIVAL) {
                 n_cur = phase_rank_tracked<PtrT>(p, h, tab, h.blk_src, e0, e1, n_cur, t, sm, cnt);
                 n_cur = (int)min((int64_t)n_cur, h.nodes_cap);
                 if (t.rank == 0 && threadIdx.x == 0) h.counts[hop + 1] = n_cur;
-                if (given_up(p, team_barrier(t, &sm.flag))) return;
+                if (given_up(p, team_barrier(t))) return;
                 phase_relabel_tracked(tab, h.blk_src, e0, e1);
             } else {
                 n_cur = (int)min((int64_t)n_cur + __ldcg(cnt), h.nodes_cap);
@@ -1126,7 +1125,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
         }
         // Once every CTA has finished reading the tables, empty them for the next mini-batch: a coalesced sweep of the
         // team's (L2-resident) slots, a 16-byte store per two.
-        if (given_up(p, team_barrier(t, &sm.flag))) return;
+        if (given_up(p, team_barrier(t))) return;
         if (p.status_host && t.rank == 0 && threadIdx.x == 0) {
             const int32_t code = *(volatile int32_t*)p.status;
             if (code != FGL_OK) *(volatile int32_t*)p.status_host = code;
@@ -1138,7 +1137,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
             for (int i = t.rank * kThreads + (int)threadIdx.x; i < (1 << (k - 1)); i += t.size * kThreads) base[i] = ones;
         }
         if (b + p.n_teams < p.n_batches) {
-            if (given_up(p, team_barrier(t, &sm.flag))) return;
+            if (given_up(p, team_barrier(t))) return;
         }
     }
 }
@@ -1174,7 +1173,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) map_kernel(const __grid_co
             table_insert_seed(tab, (uint32_t)v, (uint32_t)s, p.status);
     }
     if (t.rank == 0 && threadIdx.x == 0) p.counts[1] = n_seeds;
-    if (!team_barrier(t, &sm.flag)) return;
+    if (!team_barrier(t)) return;
 
     int e0, e1;
     chunk_of(n_edges, t.rank, t.size, e0, e1);
@@ -1213,13 +1212,13 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) map_kernel(const __grid_co
             if (d < 0) set_status(p.status, FGL_ERR_BOUNDS);
         }
     }
-    if (!team_barrier(t, &sm.flag)) return;
+    if (!team_barrier(t)) return;
     if (!ARRIVAL) {
         phase_count_first(tab, p.map_src, e0, e1, t, sm, team_sums);
-        if (!team_barrier(t, &sm.flag)) return;
+        if (!team_barrier(t)) return;
         const int n_total = phase_rank(p, tab, p.map_src, e0, e1, unique, nodes_cap, n_seeds, t, sm, team_sums);
         if (t.rank == 0 && threadIdx.x == 0) p.counts[1] = (int)min((int64_t)n_total, nodes_cap);
-        if (!team_barrier(t, &sm.flag)) return;
+        if (!team_barrier(t)) return;
     }
     phase_relabel(tab, p.map_src, e0, e1);
 }

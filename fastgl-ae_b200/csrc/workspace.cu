@@ -79,8 +79,8 @@ int fgl_ws_create(int device, fgl_ws** out) {
     ws->device = device;
     fgl::DeviceGuard guard(device);
     cudaError_t e = cudaDeviceGetAttribute(&ws->sm_count, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaMalloc(&ws->status, 16 * sizeof(int32_t) + 512 * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMemset(ws->status, 0, 16 * sizeof(int32_t) + 512 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMalloc(&ws->status, fgl::kWsStatusBytes);
+    if (e == cudaSuccess) e = cudaMemset(ws->status, 0, fgl::kWsStatusBytes);
     if (e == cudaSuccess) e = cudaMallocHost(&ws->host_pinned, 64 * sizeof(int32_t));
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -124,6 +124,8 @@ int fgl_ws_check(fgl_ws* ws, void* stream) {
     FGL_CUDA_OK(ws, cudaStreamSynchronize(st));
     const int code = ws->host_pinned[0];
     if (code != FGL_OK) {
+        // a launch that gave up has left the barrier counter half-way
+        FGL_CUDA_OK(ws, cudaMemsetAsync(ws->status + fgl::kWsTeamWord, 0, 32 * sizeof(int32_t), st));
         ws->last_error = std::string("device status: ") + fgl_status_str(code);
         ws->table_dirty = true;  // a failed launch may have left keys behind
     }

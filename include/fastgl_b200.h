@@ -361,13 +361,13 @@ int fgl_agg_bwd_self(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int3
 
 /* Aggregation backward as a gather, deterministic: the same result as fgl_agg_bwd / fgl_agg_bwd_self (the scatters
  * K9 / K11 of the reference, aggregate_acc_kernel.cu:468-517, :555-596, which add with atomics in arbitrary order), but
- * every row dx[s] is produced by one warp -- or, for a source with more than 32 edges in the block, one CTA -- that
+ * every row dx[s] is produced by one warp -- or, for a source with more than 128 edges in the block, one CTA per tile -- that
  * adds the rows dy[d] of the edges (d, s) in ascending order of d.  Two runs give the same bits; dx needs no
  * initialisation (rows without edges become zero, or dy_self[s]); dy_self may be NULL.
  *
  * fgl_block_transpose builds the per-source lists once per block: t_indptr (n_src + 1 offsets), t_dst (the edges'
  * destination rows grouped by source, t_cap >= number of edges), hubs (n_src + 1 words: the number of sources with
- * more than 32 edges, then their ids).  work is scratch of 2 * n_src words.  A source id outside [0, n_src) records
+ * more than 128 edges, then their ids).  work is scratch of 2 * n_src words.  A source id outside [0, n_src) records
  * FGL_ERR_BOUNDS and is skipped.  n_dst_dev as in fgl_agg_fwd. */
 int fgl_block_transpose(fgl_ws* ws, const int32_t* indptr, const int32_t* src, int32_t n_dst, int32_t n_src,
                         int32_t* t_indptr, int32_t* t_dst, int64_t t_cap, int32_t* hubs, int32_t* work,
