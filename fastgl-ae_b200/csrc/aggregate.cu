@@ -780,9 +780,27 @@ static int pick_vec(int dim, const void* a, int64_t lda, const void* b, int64_t 
     return 1;
 }
 
+// Asked once: every call costs as much as a launch's arguments (the GPUs of a box are alike).
+static int sm_count() {
+    static std::atomic<int> cached{0};
+    int sms = cached.load(std::memory_order_relaxed);
+    if (sms == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+            return 148;
+        cached.store(sms, std::memory_order_relaxed);
+    }
+    return sms;
+}
+
+// dx[0 .. n_src) = 0
+static cudaError_t zero_rows(float* dx, int64_t ldx, int32_t dim, int32_t n_src, cudaStream_t st) {
+    if (ldx == dim) return cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)dim * (size_t)n_src, st);
+    return cudaMemset2DAsync(dx, sizeof(float) * (size_t)ldx, 0, sizeof(float) * (size_t)dim, (size_t)n_src, st);
+}
+
 static int agg_grid_x(int n_rows, int n_batches) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     const int64_t want = ((int64_t)n_rows + kAggWarps - 1) / kAggWarps;
     const int64_t cap = std::max<int64_t>(1, ((int64_t)sms * 8 + n_batches - 1) / n_batches);
     return (int)std::max<int64_t>(1, std::min<int64_t>(want, cap));
@@ -801,26 +819,34 @@ static bool staged_applies(const AggParams& p, int vec) {
     return vec == 4 && p.shards == nullptr && p.dim / 4 <= 32 && p.ldx * 4 <= 0xffffffffLL;
 }
 
+// The shared memory a kernel may ask for, set once per kernel and device instead of before every launch.
+template <auto kernel>
+static void allow_shared(int bytes) {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    const uint64_t bit = 1ULL << (dev & 63);
+    if (done.load(std::memory_order_relaxed) & bit) return;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+        done.fetch_or(bit, std::memory_order_relaxed);
+}
+
 template <int MODE>
 static void launch_fwd_staged(const AggParams& p, cudaStream_t st) {
-    static int sms = 0, smem_optin = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    }
-    // as many warps per SM as their row slots fit beside the kernel's static shared memory
+    const int sms = sm_count();
+    constexpr int64_t kRoom = (227 - 8) * 1024;  // beside the kernel's static shared memory
     const int64_t per_warp = (int64_t)kAggSlots * (p.dim / 4) * 16;
-    const int warps = (int)std::max<int64_t>(1, std::min<int64_t>(kAggStagedMaxWarps, ((int64_t)smem_optin - 8 * 1024) / per_warp));
-    const size_t dyn = (size_t)warps * per_warp;
+    // As many warps per SM as their row slots fit; a block of few rows is spread over the SMs instead of filling a few.
     const int64_t rows = p.n_batches > 0 ? 0x7fffffff : p.n_dst;  // window launches fill the GPU
+    const int64_t fit = std::min<int64_t>(kAggStagedMaxWarps, kRoom / per_warp);
+    const int warps = (int)std::max<int64_t>(1, std::min<int64_t>(fit, std::max<int64_t>(4, (rows + sms - 1) / sms)));
+    const size_t dyn = (size_t)warps * per_warp;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sms, (rows + warps - 1) / warps));
     if (p.row_map) {
-        cudaFuncSetAttribute(agg_fwd_staged_kernel<MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+        allow_shared<agg_fwd_staged_kernel<MODE, true>>((int)kRoom);
         agg_fwd_staged_kernel<MODE, true><<<grid, warps * 32, dyn, st>>>(p);
     } else {
-        cudaFuncSetAttribute(agg_fwd_staged_kernel<MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+        allow_shared<agg_fwd_staged_kernel<MODE, false>>((int)kRoom);
         agg_fwd_staged_kernel<MODE, false><<<grid, warps * 32, dyn, st>>>(p);
     }
 }
@@ -1047,8 +1073,7 @@ int fgl_agg_edge_bwd(fgl_ws* ws, const int32_t* indptr, const int32_t* src, cons
     if (n_src == 0) return FGL_OK;
     if (!dx) return FGL_ERR_INVALID;
     cudaStream_t st = (cudaStream_t)stream;
-    if (cudaMemset2DAsync(dx, sizeof(float) * (size_t)ldx, 0, sizeof(float) * (size_t)dim, (size_t)n_src, st) != cudaSuccess)
-        return FGL_ERR_CUDA;
+    if (zero_rows(dx, ldx, dim, n_src, st) != cudaSuccess) return FGL_ERR_CUDA;
     if (n_dst == 0) return FGL_OK;
     if (!indptr || !dy || !edge_w) return FGL_ERR_INVALID;
     AggParams p{};
@@ -1151,8 +1176,7 @@ static int agg_bwd_impl(fgl_ws* ws, int32_t mode, const int32_t* indptr, const i
         const int64_t items = (int64_t)n_src * ((dim + 3) / 4);
         const int grid = (int)std::min<int64_t>((items + 255) / 256, 148 * 16);
         init_self_rows_kernel<<<grid, 256, 0, st>>>(dx, ldx, dy_self, ld_self, dim, n_dst, n_src, n_dst_dev);
-    } else if (cudaMemset2DAsync(dx, sizeof(float) * (size_t)ldx, 0, sizeof(float) * (size_t)dim, (size_t)n_src, st) !=
-               cudaSuccess) {
+    } else if (zero_rows(dx, ldx, dim, n_src, st) != cudaSuccess) {
         return FGL_ERR_CUDA;
     }
     if (n_dst == 0) return FGL_OK;

@@ -92,6 +92,7 @@ struct KParams {
     int32_t* status;               // [0] first error, [1] abort flag
     int32_t* counts_host;          // pinned host copies (may be NULL)
     int32_t* status_host;
+    int32_t seq;                   // closes a counts row on the host
 };
 
 // ----------------------------------------------------------------------------------------------
@@ -560,7 +561,11 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
                 const uint32_t lo = (uint32_t)cur[q];
                 const bool pending = mine || (lo & kPending);
                 if (hit) r[q] = pending ? ~((int)(bucket[q] * kBucket) + at[q]) : (int)lo;
-                if (hit && mine) created |= 1u << q;
+                if (hit && mine) {
+                    created |= 1u << q;
+                    if (!ARRIVAL && !h.last_hop)  // the ranking phase reads this node's offsets
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"((const PtrT*)p.indptr + g[q]));
+                }
                 if (!ARRIVAL && hit && pending && !mine && lo > (kPending | (uint32_t)(off[q] + gl))) lower |= 1u << q;
                 if (hit) open &= ~(1u << q);
                 if (full) bucket[q] = (bucket[q] + 1) & tab.mask;
@@ -671,14 +676,20 @@ __device__ __forceinline__ void phase_count_old(const Hop& h, const Team& t) {
 
 // Sum of the team's partials before `rank` and over the whole team.
 __device__ __forceinline__ void team_prefix(const int32_t* team_sums, const Team& t, Smem& sm, int& before, int& total) {
+    // every warp for itself: a few loads more, but no barriers of the CTA
     int a = 0, b = 0;
-    for (int q = threadIdx.x; q < t.size; q += kThreads) {
+    for (int q = threadIdx.x & 31; q < t.size; q += 32) {
         const int x = __ldcg(team_sums + q);
         b += x;
         if (q < t.rank) a += x;
     }
-    before = block_sum(a, sm.scan);
-    total = block_sum(b, sm.scan);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    before = a;
+    total = b;
 }
 
 // The fused kernel's table of 2^log2 slots: it lies at slot 2^log2 of the team's region, so the tables of a mini-batch do
@@ -1004,6 +1015,23 @@ __device__ __forceinline__ bool given_up(const KParams& p, bool ok) {
     return !ok;
 }
 
+// The mini-batch's numbers are settled (behind the barrier after its last ranking): the team's first warp, which wrote them,
+// copies them to the host.  What is left -- relabelling the last hop, emptying the tables -- goes on while the host prepares
+// what comes next.
+__device__ __forceinline__ void tell_host(const KParams& p, const Hop& h, int b, int rank) {
+    if (p.counts_host == nullptr || rank != 0 || threadIdx.x >= 32) return;
+    __syncwarp();
+    volatile int32_t* row = p.counts_host + (size_t)b * FGL_COUNTS_STRIDE;
+    if (threadIdx.x < FGL_COUNTS_STRIDE - 1) row[threadIdx.x] = *(volatile int32_t*)(h.counts + threadIdx.x);
+    if (threadIdx.x == 31) {
+        const int32_t code = *(volatile int32_t*)p.status;
+        if (code != FGL_OK) *(volatile int32_t*)p.status_host = code;
+    }
+    __threadfence_system();
+    __syncwarp();
+    if (threadIdx.x == 0) row[FGL_COUNTS_STRIDE - 1] = p.seq;
+}
+
 template <typename PtrT, int MODE, bool ARRIVAL>
 __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __grid_constant__ KParams p) {
     __shared__ Smem sm;
@@ -1110,26 +1138,19 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
                 n_cur = (int)min((int64_t)n_cur, h.nodes_cap);
                 if (t.rank == 0 && threadIdx.x == 0) h.counts[hop + 1] = n_cur;
                 if (given_up(p, team_barrier(t))) return;
+                if (h.last_hop) tell_host(p, h, b, t.rank);
                 phase_relabel_tracked(tab, h.blk_src, e0, e1);
             } else {
                 n_cur = (int)min((int64_t)n_cur + __ldcg(cnt), h.nodes_cap);
                 if (t.rank == 0 && threadIdx.x == 0) h.counts[hop + 1] = n_cur;
+                if (h.last_hop) tell_host(p, h, b, t.rank);
                 phase_relabel(tab, h.blk_src, e0, e1);
             }
         }
         if (MODE == MODE_SAMPLE) break;
-        if (p.counts_host && t.rank == 0 && threadIdx.x < 32) {  // the counts row is this warp's own
-            __syncwarp();
-            if (threadIdx.x < FGL_COUNTS_STRIDE)
-                p.counts_host[(size_t)b * FGL_COUNTS_STRIDE + threadIdx.x] = *(volatile int32_t*)(h.counts + threadIdx.x);
-        }
         // Once every CTA has finished reading the tables, empty them for the next mini-batch: a coalesced sweep of the
         // team's (L2-resident) slots, a 16-byte store per two.
         if (given_up(p, team_barrier(t))) return;
-        if (p.status_host && t.rank == 0 && threadIdx.x == 0) {
-            const int32_t code = *(volatile int32_t*)p.status;
-            if (code != FGL_OK) *(volatile int32_t*)p.status_host = code;
-        }
         for (unsigned m = used; m; m &= m - 1) {
             const int k = __ffs(m) - 1;
             uint4* base = reinterpret_cast<uint4*>(hop_table(p, team_id, k).slots);
@@ -1567,6 +1588,7 @@ int fgl_sample_map_fused_extra(fgl_ws* ws, const fgl_fused_args* a, const fgl_fu
     if (extra) {
         kp.counts_host = extra->counts_host;
         kp.status_host = extra->status_host;
+        kp.seq = extra->seq;
         for (int h = 0; h < a->n_hops; ++h) kp.blk_dst[h] = extra->block_dst[h];
     }
     kp.table = ws->table;

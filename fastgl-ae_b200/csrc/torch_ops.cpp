@@ -14,6 +14,8 @@
 #include <torch/csrc/utils/pybind.h>
 
 #include <array>
+#include <atomic>
+#include <chrono>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -207,8 +209,37 @@ void fused_graph(fgl_fused_args& a, const at::Tensor& edge_ptr, const at::Tensor
     for (int h = 0; h < f.hops; ++h) a.fanout[h] = f.fanout[h];
 }
 
-// One launch for a window of mini-batches, into the buffers of a FusedBatch; counts_host / status_host: its pinned copies.
-void sample_map_fused(py::handle ptr_o, py::handle src_o, py::handle seeds_o, py::handle seed_counts_o, const std::vector<int64_t>& fanouts,
+std::atomic<uint32_t> g_seq{0};
+
+int32_t next_seq() {
+    return (g_seq.fetch_add(1, std::memory_order_relaxed) & 0x3fffffff) + 1;  // never zero
+}
+
+// Waits until the rows of a launch's counts are closed with `seq`; false if the launch gave up, or if it takes so long that the
+// caller had better sleep on an event.
+bool poll_counts(const volatile int32_t* rows, const volatile int32_t* status, int64_t n, int32_t seq) {
+    const auto until = std::chrono::steady_clock::now() + std::chrono::milliseconds(5);
+    for (int64_t b = 0; b < n; ++b) {
+        for (unsigned spins = 0; rows[b * FGL_COUNTS_STRIDE + FGL_COUNTS_STRIDE - 1] != seq; ++spins) {
+            if (*status != FGL_OK) return false;
+            if ((spins & 1023) == 1023 && std::chrono::steady_clock::now() > until) return false;
+        }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return true;
+}
+
+bool wait_counts(const at::Tensor& counts_host, const at::Tensor& status_host, int32_t seq) {
+    const auto* rows = static_cast<const int32_t*>(counts_host.data_ptr());
+    const auto* status = static_cast<const int32_t*>(status_host.data_ptr());
+    const int64_t n = counts_host.size(0);
+    py::gil_scoped_release nogil;
+    return poll_counts(rows, status, n, seq);
+}
+
+// One launch for a window of mini-batches, into the buffers of a FusedBatch; counts_host / status_host: its pinned copies, whose
+// rows the launch closes with the number returned.
+int32_t sample_map_fused(py::handle ptr_o, py::handle src_o, py::handle seeds_o, py::handle seed_counts_o, const std::vector<int64_t>& fanouts,
                       int flags, uint64_t rng_seed, uint64_t rng_ctr, int n_teams, int64_t table_slots, const at::Tensor& nodes,
                       const at::Tensor& counts, const std::vector<at::Tensor>& indptr, const std::vector<at::Tensor>& block_src,
                       py::handle counts_host, py::handle status_host) {
@@ -242,8 +273,10 @@ void sample_map_fused(py::handle ptr_o, py::handle src_o, py::handle seeds_o, py
         x.counts_host = static_cast<int32_t*>(tensor(counts_host, "counts_host").data_ptr());
         x.status_host = static_cast<int32_t*>(tensor(status_host, "status_host").data_ptr());
         *x.status_host = 0;
+        x.seq = next_seq();
     }
     check(api.fgl_sample_map_fused_extra(c.ws, &a, &x, c.st()), "sample_map_fused", c.ws);
+    return x.seq;
 }
 
 // Pinned words the blocking calls of a thread are answered in (one per thread: two threads may wait at once).
@@ -281,6 +314,7 @@ py::object sample_blocks(py::handle src_o, py::handle ptr_o, py::handle seeds_o,
     x.counts_host = words;
     x.status_host = words + FGL_COUNTS_STRIDE;
     *x.status_host = 0;
+    x.seq = next_seq();
     int64_t at_word = head, ptr_at[FGL_MAX_HOPS], src_at[FGL_MAX_HOPS], dst_at[FGL_MAX_HOPS];
     const int64_t nodes_at = at_word;
     at_word += up(f.cap[f.hops]);
@@ -310,8 +344,8 @@ py::object sample_blocks(py::handle src_o, py::handle ptr_o, py::handle seeds_o,
         py::gil_scoped_release nogil;
         rc = api.fgl_sample_map_fused_extra(c.ws, &a, &x, c.st());
         if (rc == FGL_OK) {
-            c.stream.synchronize();
-            if (*x.status_host != FGL_OK) rc = api.fgl_ws_check(c.ws, c.st());
+            if (!poll_counts(words, x.status_host, 1, x.seq)) c.stream.synchronize();
+            if (*(volatile int32_t*)x.status_host != FGL_OK) rc = api.fgl_ws_check(c.ws, c.st());
         }
     }
     check(rc, "sample_blocks", c.ws);
@@ -883,6 +917,7 @@ PYBIND11_MODULE(_ops, m) {
     m.def("sample_node_csr", &sample_node_csr);
     m.def("transfer_edge_id", &transfer_edge_id);
     m.def("sample_map_fused", &sample_map_fused);
+    m.def("wait_counts", &wait_counts);
     m.def("sample_blocks", &sample_blocks);
     m.def("cal_deg", &cal_deg);
     m.def("exclusive_sum", &exclusive_sum);

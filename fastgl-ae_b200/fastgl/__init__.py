@@ -814,6 +814,7 @@ class FusedBatch:
         self._status_pinned = None
         self._event = None
         self._written = False
+        self._seq = 0
         self._readback = None
         self.device_status = 0   # the workspace's status word as of the last asynchronous read-back (0 = no error)
 
@@ -842,10 +843,14 @@ class FusedBatch:
             self._event.synchronize()
 
     def counts_host(self) -> torch.Tensor:
+        """The counts on the host (waits for them).  They arrive before the launch that writes them ends: the buffers they
+        describe are complete for work on the launch's stream, and for other streams behind an event on it."""
         if self._counts_host is None:
             if self._readback is not None:
-                self._readback.synchronize()
+                if not (self._written and _ops.wait_counts(self._counts_pinned, self._status_pinned, self._seq)):
+                    self._readback.synchronize()
                 self._counts_host = self._counts_pinned.clone()
+                self._counts_host[:, COUNTS_STRIDE - 1] = 0     # the launch's number
                 self.device_status = int(self._status_pinned[0])
                 self._readback = None
             else:
@@ -913,10 +918,11 @@ def sample_map_fused(edge_ptr, src_edges, seeds, seed_counts, fanouts, replace=N
             _time_next_launch(dev, timing)
     # (a captured launch is replayed at times that the host does not see)
     out._written = out._counts_pinned is not None and not torch.cuda.is_current_stream_capturing()
-    _ops.sample_map_fused(edge_ptr, src_edges, seeds, seed_counts, [int(f) for f in fanouts], flags,
-                          _config["rng_seed"] if rng_seed is None else rng_seed, _next_ctr() if rng_ctr is None else rng_ctr,
-                          int(n_teams), int(table_slots), out.nodes, out.counts, out.block_indptr, out.block_src,
-                          *((out._counts_pinned, out._status_pinned) if out._written else (None, None)))
+    out._seq = _ops.sample_map_fused(edge_ptr, src_edges, seeds, seed_counts, [int(f) for f in fanouts], flags,
+                                     _config["rng_seed"] if rng_seed is None else rng_seed,
+                                     _next_ctr() if rng_ctr is None else rng_ctr, int(n_teams), int(table_slots), out.nodes,
+                                     out.counts, out.block_indptr, out.block_src,
+                                     *((out._counts_pinned, out._status_pinned) if out._written else (None, None)))
     if out._written:
         out._event.record(torch.cuda.current_stream(dev))
     return out

@@ -169,12 +169,14 @@ int fgl_sample_map_fused(fgl_ws* ws, const fgl_fused_args* args, void* stream);
  * seed_stride seeds).  block_dst[h] (n_batches == 1 only) receives the
  * block-local destination id of every edge of hop h (what fgl_map leaves in dst).  counts_host and status_host are
  * pinned host memory that the kernel itself writes: the counts rows, and the workspace's status word if it is not zero
- * (the caller zeroes it before the launch).  They hold their values once the launch has completed, so that waiting for
- * an event behind it is all a read-back takes. */
+ * (the caller zeroes it before the launch).  A row is written, behind any status, as soon as its mini-batch's numbers are
+ * settled and closed with `seq` in its last word, so that a host that polls that word can prepare the next launches while
+ * this one finishes; a launch that gives up leaves a status and no `seq`. */
 typedef struct fgl_fused_extra {
     int32_t* block_dst[FGL_MAX_HOPS];
     int32_t* counts_host;
     int32_t* status_host;
+    int32_t seq;
 } fgl_fused_extra;
 int fgl_sample_map_fused_extra(fgl_ws* ws, const fgl_fused_args* args, const fgl_fused_extra* extra, void* stream);
 
