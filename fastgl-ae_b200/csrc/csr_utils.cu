@@ -168,7 +168,9 @@ struct StageParams {
 };
 
 constexpr int kStageThreads = 256;
-constexpr int64_t kStageBytesPerBlock = kStageThreads * 16 * 8;  // 32 KB per CTA
+// 8 KB per CTA: two accesses per thread, both on their way at once (with 32 KB and one access after the other a mini-batch's
+// blocks took 5 to 6 us to stage, whatever their size)
+constexpr int64_t kStageBytesPerBlock = kStageThreads * 16 * 2;
 
 __global__ void __launch_bounds__(kStageThreads) stage_segments_kernel(const __grid_constant__ StageParams p) {
     if (blockIdx.x == 0 && threadIdx.x < p.n_words) p.words_dst[threadIdx.x] = p.words[threadIdx.x];
@@ -181,13 +183,29 @@ __global__ void __launch_bounds__(kStageThreads) stage_segments_kernel(const __g
     const char* src = static_cast<const char*>(p.seg[s].src);
     if ((((uintptr_t)dst | (uintptr_t)src) & 15) == 0) {
         const int64_t v_hi = lo + ((hi - lo) / 16) * 16;
-        for (int64_t o = lo + (int64_t)threadIdx.x * 16; o < v_hi; o += kStageThreads * 16)
-            *reinterpret_cast<uint4*>(dst + o) = *reinterpret_cast<const uint4*>(src + o);
+        const int64_t o0 = lo + (int64_t)threadIdx.x * 16, o1 = o0 + kStageThreads * 16;
+        uint4 v0{}, v1{};
+        if (o0 < v_hi) v0 = *reinterpret_cast<const uint4*>(src + o0);
+        if (o1 < v_hi) v1 = *reinterpret_cast<const uint4*>(src + o1);
+        if (o0 < v_hi) *reinterpret_cast<uint4*>(dst + o0) = v0;
+        if (o1 < v_hi) *reinterpret_cast<uint4*>(dst + o1) = v1;
         for (int64_t o = v_hi + (int64_t)threadIdx.x * 4; o < hi; o += kStageThreads * 4)
             *reinterpret_cast<uint32_t*>(dst + o) = *reinterpret_cast<const uint32_t*>(src + o);
     } else {
-        for (int64_t o = lo + (int64_t)threadIdx.x * 4; o < hi; o += kStageThreads * 4)
-            *reinterpret_cast<uint32_t*>(dst + o) = *reinterpret_cast<const uint32_t*>(src + o);
+#pragma unroll
+        for (int q0 = 0; q0 < 8; q0 += 4) {
+            uint32_t v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int64_t o = lo + ((int64_t)(q0 + q) * kStageThreads + threadIdx.x) * 4;
+                v[q] = o < hi ? *reinterpret_cast<const uint32_t*>(src + o) : 0u;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int64_t o = lo + ((int64_t)(q0 + q) * kStageThreads + threadIdx.x) * 4;
+                if (o < hi) *reinterpret_cast<uint32_t*>(dst + o) = v[q];
+            }
+        }
     }
 }
 

@@ -279,7 +279,7 @@ struct Hop {
     uint64_t ctr;
 };
 
-constexpr int kMaxTiles = 4096;  // node tiles per hop; a thread of a 512-thread CTA scans eight of their counts
+constexpr int kMaxTiles = 8 * kThreads;  // node tiles per hop; a thread scans eight of their counts
 constexpr int kMinTileShift = 3;
 constexpr int kMaxTeam = 512;    // CTAs per team (a cooperative grid of 512-thread CTAs has at most a few hundred)
 
@@ -346,16 +346,11 @@ __device__ __forceinline__ int edge_owner(const Smem& sm, int size, int e) {
 }
 
 // A node that joins the list with local id `local`: what the next hop needs of it.
-template <typename PtrT>
-__device__ __forceinline__ void note_node(const KParams& p, const Hop& h, int local, int g) {
-    if (!h.last_hop && (int64_t)local < h.deg_cap) {
-        long long start;
-        int deg;
-        load_adj<PtrT>(p, g, start, deg);
-        __stcg(h.node_start + local, start);
-        __stcg(h.node_deg + local, deg);
-        atomicAdd(h.next_sums + (local >> h.next_shift), min(deg, h.next_fanout));
-    }
+__device__ __forceinline__ void note_node(const Hop& h, int local, long long start, int deg) {
+    if ((int64_t)local >= h.deg_cap) return;
+    __stcg(h.node_start + local, start);
+    __stcg(h.node_deg + local, deg);
+    if (deg > 0) atomicAdd(h.next_sums + (local >> h.next_shift), min(deg, h.next_fanout));
 }
 
 // Second half of an insert in arrival-order mode: the claiming thread takes the next local id and publishes it.
@@ -369,7 +364,12 @@ __device__ __forceinline__ int arrival_assign(const KParams& p, const Hop& h, co
     const uint32_t pos = (uint32_t)~r;
     if ((int64_t)local < h.nodes_cap) {
         h.nodes[local] = g;
-        note_node<PtrT>(p, h, local, g);
+        if (!h.last_hop) {
+            long long start;
+            int deg;
+            load_adj<PtrT>(p, g, start, deg);
+            note_node(h, local, start, deg);
+        }
         atomicExch(tab.slots + pos, ((unsigned long long)(uint32_t)g << 32) | (uint32_t)local);
         return local;
     }
@@ -416,7 +416,8 @@ __device__ __forceinline__ void emit_edge(const KParams& p, const Hop& h, const 
 // phase's instructions.)
 // The dependent loads of the group's seeds -- picked sources, buckets, claims -- are issued seed by seed before the
 // first is used, so that kSeedsPerIter round trips are in flight per lane; a key whose bucket is full goes round again
-// together with the others' retries.
+// together with the others' retries.  (Requesting the next round's sources before this round's inserts, CTAs of 256 or 384
+// threads with more registers, and three or four seeds per round were all measured: none is faster.)
 // Element (i, j) of the 4 x 4 words of a quad of lanes (lane i holds row i) goes to (j, i).
 __device__ __forceinline__ void quad_transpose(uint4& w) {
     const bool odd = threadIdx.x & 1, high = threadIdx.x & 2;
@@ -445,27 +446,22 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
     constexpr int KS = kSeedsPerIter;
     const int gid = threadIdx.x / G, gl = threadIdx.x % G;
     const int gbase = (threadIdx.x & 31) & ~(G - 1);  // first lane of the group within its warp
-    for (int it = 0; it * kGroups * KS < tile_n; ++it) {
-        int v[KS], off[KS], g[KS], deg[KS];
+    // Stage 1 of a round of seeds: the picks, and the requests for the picked sources.
+    auto picks = [&](int it, int (&g)[KS]) {
+        int deg[KS];
         long long start[KS];
-        bool has[KS];
         uint32_t pk[KS];
         bool any_hub = false;
 #pragma unroll
         for (int q = 0; q < KS; ++q) {
             const int j = (it * KS + q) * kGroups + gid;
-            v[q] = 0;
-            off[q] = 0;
             g[q] = 0;
             deg[q] = 0;
             start[q] = 0;
             if (j < tile_n) {
                 deg[q] = sm.deg[j];
-                v[q] = sm.v[j];
-                off[q] = sm.off[j];
                 start[q] = sm.start[j];
             }
-            has[q] = gl < min(deg[q], fanout);
             pk[q] = (uint32_t)gl;
             any_hub |= deg[q] > fanout;
         }
@@ -499,10 +495,28 @@ __device__ __forceinline__ void sample_tile_groups(const KParams& p, const Hop& 
                 }
             }
         }
-        // stage 1: the picked sources
 #pragma unroll
         for (int q = 0; q < KS; ++q)
-            if (has[q]) g[q] = ld_adjacency(p.indices + start[q] + (long long)pk[q]);
+            if (gl < min(deg[q], fanout)) g[q] = ld_adjacency(p.indices + start[q] + (long long)pk[q]);
+    };
+    const int rounds = (tile_n + kGroups * KS - 1) / (kGroups * KS);
+    int g[KS];
+    for (int it = 0; it < rounds; ++it) {
+        picks(it, g);
+        int v[KS], off[KS];
+        bool has[KS];
+#pragma unroll
+        for (int q = 0; q < KS; ++q) {
+            const int j = (it * KS + q) * kGroups + gid;
+            v[q] = 0;
+            off[q] = 0;
+            has[q] = false;
+            if (j < tile_n) {
+                has[q] = gl < min(sm.deg[j], fanout);
+                v[q] = sm.v[j];
+                off[q] = sm.off[j];
+            }
+        }
         if (h.out_dst) {
 #pragma unroll
             for (int q = 0; q < KS; ++q)
@@ -827,20 +841,20 @@ __device__ __forceinline__ bool phase_sample(const KParams& p, const Hop& h, Tab
 // ---- fused kernel, first-occurrence order ------------------------------------------------------------------------------
 // Phase D: the possibly-first edges that still hold their slot are the first occurrences.  Local ids in edge order;
 // the node, its adjacency offset and degree (unless this is the last hop) join the list; the edge entry becomes the id.
-// Eight consecutive edges per thread: two 128-bit loads of entries, then up to eight slot loads in flight.
-template <typename PtrT>
+// kPer (4 or 8) consecutive edges per thread: 128-bit loads of entries, then up to kPer slot loads in flight, then as many of
+// the new nodes' offsets.
+template <typename PtrT, int kPer>
 __device__ __forceinline__ int phase_rank_tracked(const KParams& p, const Hop& h, const Table& tab, int32_t* edges, int e0, int e1,
                                                   int n_before, const Team& t, Smem& sm, const int32_t* team_cnt) {
     int before, total;
     team_prefix(team_cnt, t, sm, before, total);
     int running = n_before + before;
-    constexpr int kPer = 8;
     for (int tile0 = e0 & ~3; tile0 < e1; tile0 += kPer * kThreads) {
         const int eb = tile0 + kPer * (int)threadIdx.x;
         int m[kPer];
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int at = eb + 4 * half;
+        for (int part = 0; part < kPer / 4; ++part) {
+            const int at = eb + 4 * part;
             int4 x = make_int4(0, 0, 0, 0);
             if (at + 3 >= e0 && at + 3 < e1) {
                 x = __ldcg(reinterpret_cast<const int4*>(edges + at));  // the row is 16-byte aligned
@@ -849,10 +863,10 @@ __device__ __forceinline__ int phase_rank_tracked(const KParams& p, const Hop& h
                 if (at + 1 < e1) x.y = __ldcg(edges + at + 1);
                 if (at + 2 < e1) x.z = __ldcg(edges + at + 2);
             }
-            m[4 * half + 0] = x.x;
-            m[4 * half + 1] = x.y;
-            m[4 * half + 2] = x.z;
-            m[4 * half + 3] = x.w;
+            m[4 * part + 0] = x.x;
+            m[4 * part + 1] = x.y;
+            m[4 * part + 2] = x.z;
+            m[4 * part + 3] = x.w;
         }
         unsigned long long cur[kPer];
 #pragma unroll
@@ -867,6 +881,17 @@ __device__ __forceinline__ int phase_rank_tracked(const KParams& p, const Hop& h
             if (!(m[q] < 0 && (uint32_t)cur[q] == (kPending | (uint32_t)(eb + q)))) m[q] = 0;  // keep first occurrences
             firsts += m[q] < 0 ? 1 : 0;
         }
+        // the new nodes' adjacency offsets and degrees, all on their way before the first is stored
+        long long start[kPer];
+        int deg[kPer];
+        if (!h.last_hop) {
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) {
+                start[q] = 0;
+                deg[q] = 0;
+                if (m[q] < 0) load_adj<PtrT>(p, (int)(cur[q] >> 32), start[q], deg[q]);
+            }
+        }
         int tile_total;
         int local = running + block_excl_scan(firsts, sm.scan, tile_total);
 #pragma unroll
@@ -878,7 +903,7 @@ __device__ __forceinline__ int phase_rank_tracked(const KParams& p, const Hop& h
                     h.nodes[local] = (int)key;
                     tab.slots[pos] = ((unsigned long long)key << 32) | (uint32_t)local;
                     edges[eb + q] = local;
-                    note_node<PtrT>(p, h, local, (int)key);
+                    if (!h.last_hop) note_node(h, local, start[q], deg[q]);
                 } else {
                     set_status(p.status, FGL_ERR_CAPACITY);
                     tab.slots[pos] = ((unsigned long long)key << 32);
@@ -1134,7 +1159,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sample_map_kernel(const __
             if (given_up(p, team_barrier(t))) return;
 
             if (!ARRIVAL) {
-                n_cur = phase_rank_tracked<PtrT>(p, h, tab, h.blk_src, e0, e1, n_cur, t, sm, cnt);
+                n_cur = h.last_hop ? phase_rank_tracked<PtrT, 8>(p, h, tab, h.blk_src, e0, e1, n_cur, t, sm, cnt)
+                                   : phase_rank_tracked<PtrT, 4>(p, h, tab, h.blk_src, e0, e1, n_cur, t, sm, cnt);
                 n_cur = (int)min((int64_t)n_cur, h.nodes_cap);
                 if (t.rank == 0 && threadIdx.x == 0) h.counts[hop + 1] = n_cur;
                 if (given_up(p, team_barrier(t))) return;

@@ -459,25 +459,32 @@ at::Tensor aggregate(int mode, py::handle ptr_o, py::handle src_o, py::handle x_
 
 // dw = x^T dy, into `out` if given.  A caller who lets torch multiply in TF32 gets torch's product; so does a contraction that is
 // shorter than the output is wide (nothing to split).
-at::Tensor weight_grad(const Call& c, const at::Tensor& x, const at::Tensor& dy, const at::Tensor& out_given = at::Tensor()) {
+at::Tensor weight_grad(const Call& c, const at::Tensor& x, const at::Tensor& dy, const at::Tensor& out_given = at::Tensor(),
+                       const at::Tensor& scratch_given = at::Tensor()) {
     const int64_t k = x.size(0), m = x.size(1), n = dy.size(1);
     TORCH_CHECK(dy.size(0) == k, "x and dy must have the same number of rows");
     at::Tensor out = out_given.defined() ? out_given : at::empty({m, n}, x.options());
     auto rows = [](const at::Tensor& t) { return t.stride(1) == 1 && t.stride(0) >= t.size(1); };
     if (!rows(x) || !rows(dy) || !rows(out) || k < std::max(m, n) || k > 0x7fffffffLL || at::globalContext().allowTF32CuBLAS())
         return at::mm_out(out, x.t(), dy);
-    at::Tensor scratch;
+    at::Tensor scratch = scratch_given;
     const int64_t floats = api.fgl_weight_grad_scratch(c.ws, (int32_t)m, (int32_t)n, (int32_t)k);
-    if (floats > 0) scratch = at::empty({floats}, x.options());
+    TORCH_CHECK(!scratch.defined() || scratch.numel() >= floats, "scratch must hold weight_grad_scratch(...) floats");
+    if (!scratch.defined() && floats > 0) scratch = at::empty({floats}, x.options());
     check(api.fgl_weight_grad(c.ws, (int32_t)m, (int32_t)n, (int32_t)k, ptr<float>(x), x.stride(0), ptr<float>(dy), dy.stride(0),
                               ptr<float>(out), out.stride(0), ptr<float>(scratch), c.st()), "weight_grad", c.ws);
     return out;
 }
 
-at::Tensor weight_grad_op(py::handle x_o, py::handle dy_o, py::handle out_o) {
+at::Tensor weight_grad_op(py::handle x_o, py::handle dy_o, py::handle out_o, py::handle scratch_o) {
     const at::Tensor &x = rows_f32(x_o, "x"), &dy = rows_f32(dy_o, "dy");
     Call c(x);
-    return weight_grad(c, x, dy, out_o.is_none() ? at::Tensor() : rows_f32(out_o, "out"));
+    return weight_grad(c, x, dy, out_o.is_none() ? at::Tensor() : rows_f32(out_o, "out"),
+                       scratch_o.is_none() ? at::Tensor() : f32(scratch_o, "scratch"));
+}
+
+int64_t weight_grad_scratch(int device, int64_t m, int64_t n, int64_t k) {
+    return api.fgl_weight_grad_scratch(workspace(device), (int32_t)m, (int32_t)n, (int32_t)k);
 }
 
 struct Transposed {
@@ -936,6 +943,7 @@ PYBIND11_MODULE(_ops, m) {
     m.def("edge_weight_grad", &edge_weight_grad);
     m.def("softmax_xent", &softmax_xent);
     m.def("weight_grad", &weight_grad_op);
+    m.def("weight_grad_scratch", &weight_grad_scratch);
     m.def("gcn_step", &gcn_step);
     m.def("gin_step", &gin_step);
     m.def("gat_step", &gat_step);

@@ -4,8 +4,10 @@
 // (GraphConv.py:86-99, train_fastgl.py:366-372); here each is one launch, so that a captured training step
 // is a few dozen kernels instead of a few hundred.  All are HBM/L2-bound streaming kernels: 128-bit accesses,
 // grid sized from the element count, no shared-memory staging needed.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "fastgl_b200.h"
@@ -108,7 +110,7 @@ relu_dropout_bwd_kernel(float* __restrict__ dy, int64_t ldy, const float* __rest
                         float* d3 = split3 + (r + k) * ld3 + c;
                         d3[0] = h;
                         d3[block_stride] = l;
-                        d3[2 * block_stride] = h;
+                        if (!(flags & FGL_EW_TWO_BLOCKS)) d3[2 * block_stride] = h;
                     }
                 } else if (mask) {
                     if (r + k < r1) dy[(r + k) * ldy + c] = g[k];
@@ -170,7 +172,7 @@ relu_dropout_bwd_vec_kernel(float* __restrict__ dy, int64_t ldy, const float* __
                         float* d3 = split3 + rr * ld3 + 4 * cg;
                         *reinterpret_cast<float4*>(d3) = h;
                         *reinterpret_cast<float4*>(d3 + block_stride) = l;
-                        *reinterpret_cast<float4*>(d3 + 2 * block_stride) = h;
+                        if (!(flags & FGL_EW_TWO_BLOCKS)) *reinterpret_cast<float4*>(d3 + 2 * block_stride) = h;
                     } else if (mask) {
                         *reinterpret_cast<float4*>(dy + rr * ldy + 4 * cg) = g[k];
                     }
@@ -200,6 +202,32 @@ relu_dropout_bwd_vec_kernel(float* __restrict__ dy, int64_t ldy, const float* __
     }
 }
 
+// loss[0] = (sum of row_loss in a fixed order) / n_valid, by the last CTA of the launch that wrote row_loss: thread t adds rows
+// t, t + 256, ... in order, then the 256 partial sums are folded by a fixed tree, so the loss is reproducible from run to run.
+// ticket: zero between launches.
+__device__ __forceinline__ void mean_by_last_cta(const float* row_loss, int n_rows, int n_valid, float* loss, unsigned int* ticket) {
+    __shared__ float part[kEwThreads];
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (last) *ticket = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    float t = 0.f;
+    for (int r = threadIdx.x; r < n_rows; r += kEwThreads) t += __ldcg(row_loss + r);
+    part[threadIdx.x] = t;
+    __syncthreads();
+    for (int w = kEwThreads / 2; w; w >>= 1) {
+        if ((int)threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) loss[0] = n_valid > 0 ? part[0] / (float)n_valid : 0.f;
+}
+
 // Mean softmax cross-entropy over the first n_valid rows, and its gradient; a warp per row.
 // row_loss[r] = logsumexp(z_r) - z_r[label_r] (0 for rows that do not count);
 // dlogits[r, c] = (softmax(z_r)[c] - [c == label_r]) / n_valid for r < n_valid and 0 below.
@@ -209,40 +237,43 @@ __global__ void __launch_bounds__(kXentWarps * 32)
 softmax_xent_rows_kernel(const float* __restrict__ logits, int64_t ld, const int64_t* __restrict__ labels,
                          const int32_t* __restrict__ label_ids, int64_t n_labels, int n_rows, int n_classes,
                          const int32_t* __restrict__ n_valid_dev, int n_valid_host, float* __restrict__ row_loss,
-                         float* __restrict__ dlogits, int64_t ldd, int32_t* __restrict__ status) {
+                         float* __restrict__ dlogits, int64_t ldd, int32_t* __restrict__ status, float* __restrict__ loss,
+                         unsigned int* __restrict__ ticket) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r = blockIdx.x * kXentWarps + warp;
-    if (r >= n_rows) return;
     int n_valid = n_valid_dev ? n_valid_dev[0] : n_valid_host;
     n_valid = n_valid < 0 ? 0 : (n_valid > n_rows ? n_rows : n_valid);
-    const float inv = n_valid > 0 ? 1.f / (float)n_valid : 0.f;
-    const float* z = logits + (int64_t)r * ld;
-    float* d = dlogits + (int64_t)r * ldd;
-    float mine = 0.f;
-    bool counted = false;
-    if (r < n_valid) {
-        const int64_t at = label_ids ? (int64_t)label_ids[r] : (int64_t)r;
-        const int64_t label = at >= 0 && at < n_labels ? labels[at] : -1;
-        if (label < 0 || label >= n_classes) {
-            if (lane == 0) atomicCAS(status, FGL_OK, FGL_ERR_BOUNDS);
-        } else {
-            counted = true;
-            float m = -INFINITY;
-            for (int c = lane; c < n_classes; c += 32) m = fmaxf(m, z[c]);
+    if (r < n_rows) {
+        const float inv = n_valid > 0 ? 1.f / (float)n_valid : 0.f;
+        const float* z = logits + (int64_t)r * ld;
+        float* d = dlogits + (int64_t)r * ldd;
+        float mine = 0.f;
+        bool counted = false;
+        if (r < n_valid) {
+            const int64_t at = label_ids ? (int64_t)label_ids[r] : (int64_t)r;
+            const int64_t label = at >= 0 && at < n_labels ? labels[at] : -1;
+            if (label < 0 || label >= n_classes) {
+                if (lane == 0) atomicCAS(status, FGL_OK, FGL_ERR_BOUNDS);
+            } else {
+                counted = true;
+                float m = -INFINITY;
+                for (int c = lane; c < n_classes; c += 32) m = fmaxf(m, z[c]);
 #pragma unroll
-            for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            float s = 0.f;
-            for (int c = lane; c < n_classes; c += 32) s += expf(z[c] - m);
+                for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+                float s = 0.f;
+                for (int c = lane; c < n_classes; c += 32) s += expf(z[c] - m);
 #pragma unroll
-            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            mine = m + logf(s) - z[label];
-            const float rs = inv / s;
-            for (int c = lane; c < n_classes; c += 32) d[c] = expf(z[c] - m) * rs - (c == (int)label ? inv : 0.f);
+                for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                mine = m + logf(s) - z[label];
+                const float rs = inv / s;
+                for (int c = lane; c < n_classes; c += 32) d[c] = expf(z[c] - m) * rs - (c == (int)label ? inv : 0.f);
+            }
         }
+        if (!counted)
+            for (int c = lane; c < n_classes; c += 32) d[c] = 0.f;
+        if (lane == 0) row_loss[r] = mine;
     }
-    if (!counted)
-        for (int c = lane; c < n_classes; c += 32) d[c] = 0.f;
-    if (lane == 0) row_loss[r] = mine;
+    mean_by_last_cta(row_loss, n_rows, n_valid, loss, ticket);
 }
 
 // The output layer and its loss in one pass: logits = x W + b for a narrow W (n_classes <= 32 * CPL), then the
@@ -262,7 +293,8 @@ linear_xent_kernel(const float* __restrict__ x, int64_t ldx, int k, const float*
                    const float* __restrict__ bias, const int64_t* __restrict__ labels, const int32_t* __restrict__ label_ids,
                    int64_t n_labels, int n_rows, int n_classes, const int32_t* __restrict__ n_valid_dev, int n_valid_host,
                    float* __restrict__ row_loss, float* __restrict__ dlogits, int64_t ldd, float* __restrict__ dbias,
-                   float* __restrict__ logits_out, int64_t ldl, int32_t* __restrict__ status) {
+                   float* __restrict__ logits_out, int64_t ldl, int32_t* __restrict__ status, float* __restrict__ loss,
+                   unsigned int* __restrict__ ticket) {
     __shared__ float part[kLinXentWarps][kLinXentRows][32 * CPL];
     __shared__ float db[32 * CPL];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -288,17 +320,26 @@ linear_xent_kernel(const float* __restrict__ x, int64_t ldx, int k, const float*
             for (int r = 0; r < kLinXentRows; ++r)
                 xr[r] = (r < rows_here && kb + lane < k_hi) ? x[(int64_t)(row0 + r) * ldx + kb + lane] : 0.f;
             const int cols = min(32, k_hi - kb);
-#pragma unroll 8
-            for (int t = 0; t < cols; ++t) {
-                const float* wr = w + (int64_t)(kb + t) * ldw;
-                float wv[CPL];
+            // the rows of W arrive kAhead at a time: what this loop waits for is the L2
+            constexpr int kAhead = CPL == 4 ? 8 : 16;
 #pragma unroll
-                for (int q = 0; q < CPL; ++q) wv[q] = (lane + 32 * q < n_classes) ? __ldg(wr + lane + 32 * q) : 0.f;
+            for (int t0 = 0; t0 < 32; t0 += kAhead) {
+                float wv[kAhead][CPL];
 #pragma unroll
-                for (int r = 0; r < kLinXentRows; ++r) {
-                    const float xv = __shfl_sync(0xffffffffu, xr[r], t);
+                for (int u = 0; u < kAhead; ++u) {
+                    const float* wr = w + (int64_t)(kb + t0 + u) * ldw;
 #pragma unroll
-                    for (int q = 0; q < CPL; ++q) acc[r][q] = fmaf(xv, wv[q], acc[r][q]);
+                    for (int q = 0; q < CPL; ++q) wv[u][q] = (t0 + u < cols && lane + 32 * q < n_classes) ? __ldg(wr + lane + 32 * q) : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) {
+                    if (t0 + u >= cols) break;
+#pragma unroll
+                    for (int r = 0; r < kLinXentRows; ++r) {
+                        const float xv = __shfl_sync(0xffffffffu, xr[r], t0 + u);
+#pragma unroll
+                        for (int q = 0; q < CPL; ++q) acc[r][q] = fmaf(xv, wv[u][q], acc[r][q]);
+                    }
                 }
             }
         }
@@ -376,27 +417,7 @@ linear_xent_kernel(const float* __restrict__ x, int64_t ldx, int k, const float*
     if (dbias)
         for (int c = threadIdx.x; c < n_classes; c += blockDim.x)
             if (db[c] != 0.f) atomicAdd(dbias + c, db[c]);
-}
-
-// loss[0] = (sum of row_loss in a fixed order) / n_valid: thread t adds rows t, t + 256, ... in order, then the
-// 256 partial sums are folded by a fixed tree, so the loss is reproducible from run to run.
-__global__ void __launch_bounds__(kEwThreads)
-softmax_xent_mean_kernel(const float* __restrict__ row_loss, int n_rows, const int32_t* __restrict__ n_valid_dev,
-                         int n_valid_host, float* __restrict__ loss) {
-    __shared__ float part[kEwThreads];
-    float t = 0.f;
-    for (int r = threadIdx.x; r < n_rows; r += kEwThreads) t += row_loss[r];
-    part[threadIdx.x] = t;
-    __syncthreads();
-    for (int w = kEwThreads / 2; w; w >>= 1) {
-        if ((int)threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        int n_valid = n_valid_dev ? n_valid_dev[0] : n_valid_host;
-        n_valid = n_valid < 0 ? 0 : (n_valid > n_rows ? n_rows : n_valid);
-        loss[0] = n_valid > 0 ? part[0] / (float)n_valid : 0.f;
-    }
+    mean_by_last_cta(row_loss, n_rows, n_valid, loss, ticket);
 }
 
 // Adam with L2 weight decay over flat buffers, torch.optim.Adam's arithmetic:
@@ -406,12 +427,23 @@ softmax_xent_mean_kernel(const float* __restrict__ row_loss, int n_rows, const i
 __global__ void __launch_bounds__(kEwThreads)
 adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, int64_t n,
             float lr, float b1, float b2, float eps, float wd, int32_t* __restrict__ step, unsigned int* __restrict__ ticket) {
-    const int t = *(volatile int32_t*)step + 1;
-    const AdamCoef c = adam_coef(lr, b1, b2, eps, wd, t);
-    for (int64_t i = ((int64_t)blockIdx.x * kEwThreads + threadIdx.x) * 4; i < n; i += (int64_t)gridDim.x * kEwThreads * 4) {
+    // the first elements are on their way while the coefficients (two powers) are computed
+    const int64_t first = ((int64_t)blockIdx.x * kEwThreads + threadIdx.x) * 4;
+    float4 pp{}, gg{}, mm{}, vv{};
+    auto fetch = [&](int64_t i) {
         if (i + 4 <= n) {
-            float4 pp = *reinterpret_cast<float4*>(p + i), gg = *reinterpret_cast<const float4*>(g + i);
-            float4 mm = *reinterpret_cast<float4*>(m + i), vv = *reinterpret_cast<float4*>(v + i);
+            pp = *reinterpret_cast<float4*>(p + i);
+            gg = *reinterpret_cast<const float4*>(g + i);
+            mm = *reinterpret_cast<float4*>(m + i);
+            vv = *reinterpret_cast<float4*>(v + i);
+        }
+    };
+    const int t = *(volatile int32_t*)step + 1;
+    fetch(first);
+    const AdamCoef c = adam_coef(lr, b1, b2, eps, wd, t);
+    for (int64_t i = first; i < n; i += (int64_t)gridDim.x * kEwThreads * 4) {
+        if (i != first) fetch(i);
+        if (i + 4 <= n) {
             adam_update(c, pp.x, gg.x, mm.x, vv.x);
             adam_update(c, pp.y, gg.y, mm.y, vv.y);
             adam_update(c, pp.z, gg.z, mm.z, vv.z);
@@ -453,11 +485,11 @@ struct SplitDst {
 };
 
 template <bool VEC4>
-__global__ void __launch_bounds__(kEwThreads)
-split_tf32_kernel(const float* __restrict__ x, int64_t rows, int cols, int64_t ldx, const SplitDst d) {
+__device__ __forceinline__ void split_elements(const float* __restrict__ x, int64_t rows, int cols, int64_t ldx, const SplitDst& d, int64_t first,
+                                               int64_t stride) {
     const int per_row = VEC4 ? cols / 4 : cols;
     const int64_t total = rows * per_row;
-    for (int64_t g = (int64_t)blockIdx.x * kEwThreads + threadIdx.x; g < total; g += (int64_t)gridDim.x * kEwThreads) {
+    for (int64_t g = first; g < total; g += stride) {
         const int64_t r = g / per_row;
         const int c = (int)(g - r * per_row) * (VEC4 ? 4 : 1);
         if (VEC4) {
@@ -476,45 +508,81 @@ split_tf32_kernel(const float* __restrict__ x, int64_t rows, int cols, int64_t l
     }
 }
 
+template <bool VEC4>
+__global__ void __launch_bounds__(kEwThreads)
+split_tf32_kernel(const float* __restrict__ x, int64_t rows, int cols, int64_t ldx, const SplitDst d) {
+    split_elements<VEC4>(x, rows, cols, ldx, d, (int64_t)blockIdx.x * kEwThreads + threadIdx.x, (int64_t)gridDim.x * kEwThreads);
+}
+
+// Several matrices in one launch; blockIdx.y is the matrix.
+constexpr int kSplitMaxJobs = 8;
+struct SplitMany {
+    const float* x[kSplitMaxJobs];
+    int64_t rows[kSplitMaxJobs], ldx[kSplitMaxJobs];
+    int cols[kSplitMaxJobs];
+    bool vec[kSplitMaxJobs];
+    SplitDst dst[kSplitMaxJobs];
+};
+
+__global__ void __launch_bounds__(kEwThreads) split_tf32_many_kernel(const __grid_constant__ SplitMany m) {
+    const int j = blockIdx.y;
+    const int64_t first = (int64_t)blockIdx.x * kEwThreads + threadIdx.x, stride = (int64_t)gridDim.x * kEwThreads;
+    if (m.vec[j]) split_elements<true>(m.x[j], m.rows[j], m.cols[j], m.ldx[j], m.dst[j], first, stride);
+    else split_elements<false>(m.x[j], m.rows[j], m.cols[j], m.ldx[j], m.dst[j], first, stride);
+}
+
 // out[r, c] = sum over slabs s and blocks (a, b) of part[s][a * rows + r][b * block_stride + c]: folds the 2 x 2 block
-// product [X_hi | X_lo]^T [dZ_hi | dZ_lo] (and its split-K slabs) into the weight gradient.  A warp per group of 32
-// consecutive outputs of one row; the slabs are spread over the warps of a CTA (every lane keeps the n_a * n_b loads of
+// product [X_hi | X_lo]^T [dZ_hi | dZ_lo] (and its split-K slabs) into the weight gradient.  A CTA per group of 32 vectors (four
+// floats where the widths allow it) of one row; the slabs are spread over the warps of a CTA (every lane keeps the n_a * n_b loads of
 // its slab in flight together) and meet in shared memory, where they are added in slab order.
 constexpr int kFoldWarps = 8;
 
+template <int VEC>
 __global__ void __launch_bounds__(kFoldWarps * 32)
 fold_blocks_kernel(const float* __restrict__ part, int n_slabs, int n_a, int n_b, int rows, int cols, int block_stride,
                    int64_t ld_part, int64_t slab_stride, float* __restrict__ out, int64_t ldo) {
-    __shared__ float partial[kFoldWarps][32];
+    using T = typename std::conditional<VEC == 4, float4, float>::type;
+    __shared__ __align__(16) float partial[kFoldWarps][32 * VEC];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int groups_per_row = (cols + 31) / 32;
+    const int groups_per_row = (cols + 32 * VEC - 1) / (32 * VEC);
     const int64_t n_groups = (int64_t)rows * groups_per_row;
     for (int64_t g = blockIdx.x; g < n_groups; g += gridDim.x) {
-        const int r = (int)(g / groups_per_row), c = (int)(g - (int64_t)r * groups_per_row) * 32 + lane;
-        float acc = 0.f;
+        const int r = (int)(g / groups_per_row), c0 = (int)(g - (int64_t)r * groups_per_row) * 32 * VEC, c = c0 + lane * VEC;
+        float acc[VEC] = {};
         if (c < cols) {
             for (int s = warp; s < n_slabs; s += kFoldWarps) {
                 const float* base = part + s * slab_stride + (int64_t)r * ld_part + c;
-                float v[4] = {0.f, 0.f, 0.f, 0.f};
+                float v[4][VEC] = {};
+                auto get = [&](int q, const float* at) { *reinterpret_cast<T*>(v[q]) = *reinterpret_cast<const T*>(at); };
                 if (n_a == 2 && n_b == 2) {   // the 2 x 2 block product: four independent loads
-                    v[0] = base[0];
-                    v[1] = base[block_stride];
-                    v[2] = base[(int64_t)rows * ld_part];
-                    v[3] = base[(int64_t)rows * ld_part + block_stride];
+                    get(0, base);
+                    get(1, base + block_stride);
+                    get(2, base + (int64_t)rows * ld_part);
+                    get(3, base + (int64_t)rows * ld_part + block_stride);
                 } else {
                     for (int a = 0; a < n_a; ++a)
-                        for (int b = 0; b < n_b; ++b) v[0] += base[(int64_t)a * rows * ld_part + (int64_t)b * block_stride];
+                        for (int b = 0; b < n_b; ++b) {
+                            get(1, base + (int64_t)a * rows * ld_part + (int64_t)b * block_stride);
+#pragma unroll
+                            for (int q = 0; q < VEC; ++q) {
+                                v[0][q] += v[1][q];
+                                v[1][q] = 0.f;
+                            }
+                        }
                 }
-                acc += (v[0] + v[1]) + (v[2] + v[3]);
+#pragma unroll
+                for (int q = 0; q < VEC; ++q) acc[q] += (v[0][q] + v[1][q]) + (v[2][q] + v[3][q]);
             }
         }
-        partial[warp][lane] = acc;
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) partial[warp][lane * VEC + q] = acc[q];
         __syncthreads();
-        if (warp == 0 && c < cols) {
+        for (int i = threadIdx.x; i < 32 * VEC; i += kFoldWarps * 32) {
+            if (c0 + i >= cols) break;
             float t = 0.f;
 #pragma unroll
-            for (int w = 0; w < kFoldWarps; ++w) t += partial[w][lane];
-            out[(int64_t)r * ldo + c] = t;
+            for (int w = 0; w < kFoldWarps; ++w) t += partial[w][i];
+            out[(int64_t)r * ldo + c0 + i] = t;
         }
         __syncthreads();
     }
@@ -524,6 +592,9 @@ static int ew_grid(int64_t work_items) {
     const int64_t blocks = (work_items + kEwThreads - 1) / kEwThreads;
     return (int)(blocks < 1 ? 1 : (blocks > 148 * 16 ? 148 * 16 : blocks));
 }
+
+// The word the loss kernels count their CTAs in.
+static unsigned int* loss_ticket(fgl_ws* ws) { return reinterpret_cast<unsigned int*>(ws->status + kWsTeamWord + 8); }
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
@@ -624,8 +695,8 @@ int fgl_softmax_xent(fgl_ws* ws, const float* logits, int64_t ld, const int64_t*
     }
     cudaStream_t st = (cudaStream_t)stream;
     softmax_xent_rows_kernel<<<(n_rows + kXentWarps - 1) / kXentWarps, kXentWarps * 32, 0, st>>>(
-        logits, ld, labels, label_ids, n_labels, n_rows, n_classes, n_valid_dev, n_valid, row_loss, dlogits, ldd, ws->status);
-    softmax_xent_mean_kernel<<<1, kEwThreads, 0, st>>>(row_loss, n_rows, n_valid_dev, n_valid, loss);
+        logits, ld, labels, label_ids, n_labels, n_rows, n_classes, n_valid_dev, n_valid, row_loss, dlogits, ldd, ws->status,
+        loss, loss_ticket(ws));
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
@@ -642,12 +713,11 @@ int fgl_linear_softmax_xent(fgl_ws* ws, const float* x, int64_t ldx, int32_t k, 
 #define FGL_LINXENT(CPL)                                                                                              \
     linear_xent_kernel<CPL><<<grid, kLinXentWarps * 32, 0, st>>>(x, ldx, k, w, ldw, bias, labels, label_ids, n_labels, \
                                                                  n_rows, n_classes, n_valid_dev, n_valid, row_loss,   \
-                                                                 dlogits, ldd, dbias, logits_out, ldl, ws->status)
+                                                                 dlogits, ldd, dbias, logits_out, ldl, ws->status, loss, loss_ticket(ws))
     if (n_classes <= 32) FGL_LINXENT(1);
     else if (n_classes <= 64) FGL_LINXENT(2);
     else FGL_LINXENT(4);
 #undef FGL_LINXENT
-    softmax_xent_mean_kernel<<<1, kEwThreads, 0, st>>>(row_loss, n_rows, n_valid_dev, n_valid, loss);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
@@ -662,27 +732,51 @@ int fgl_adam_step(float* param, const float* grad, float* exp_avg, float* exp_av
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
-int fgl_split_tf32(const float* x, int64_t rows, int64_t cols, int64_t ldx, int n_dst, float* const* dst, const int64_t* ld_dst,
-                   const int32_t* lo_part, void* stream) {
-    if (rows < 0 || cols < 0 || cols > 0x7fffffffLL || ldx < cols || n_dst < 1 || n_dst > kSplitMaxDst || !dst || !ld_dst || !lo_part)
-        return FGL_ERR_INVALID;
-    if (rows == 0 || cols == 0) return FGL_OK;
-    if (!x) return FGL_ERR_INVALID;
-    SplitDst d{};
+// The destinations of one matrix and whether all its accesses can be 16 bytes wide; false: an argument is wrong.
+static bool split_dst(const float* x, int64_t rows, int64_t cols, int64_t ldx, int n_dst, float* const* dst, const int64_t* ld_dst,
+                      const int32_t* lo_part, SplitDst& d, bool& vec) {
+    if (rows < 0 || cols < 0 || cols > 0x7fffffffLL || ldx < cols || n_dst < 1 || n_dst > kSplitMaxDst || (!x && rows > 0 && cols > 0)) return false;
     d.n = n_dst;
-    bool vec = cols % 4 == 0 && ldx % 4 == 0 && aligned16(x);
+    vec = cols % 4 == 0 && ldx % 4 == 0 && aligned16(x);
     for (int q = 0; q < n_dst; ++q) {
-        if (!dst[q] || ld_dst[q] < cols) return FGL_ERR_INVALID;
+        if (rows > 0 && cols > 0 && (!dst[q] || ld_dst[q] < cols)) return false;
         d.ptr[q] = dst[q];
         d.ld[q] = ld_dst[q];
         d.lo_part[q] = lo_part[q] ? 1 : 0;
         vec = vec && ld_dst[q] % 4 == 0 && aligned16(dst[q]);
     }
+    return true;
+}
+
+int fgl_split_tf32(const float* x, int64_t rows, int64_t cols, int64_t ldx, int n_dst, float* const* dst, const int64_t* ld_dst,
+                   const int32_t* lo_part, void* stream) {
+    SplitDst d{};
+    bool vec = false;
+    if (!dst || !ld_dst || !lo_part || !split_dst(x, rows, cols, ldx, n_dst, dst, ld_dst, lo_part, d, vec)) return FGL_ERR_INVALID;
+    if (rows == 0 || cols == 0) return FGL_OK;
     const int64_t items = rows * (vec ? cols / 4 : cols);
     if (vec)
         split_tf32_kernel<true><<<ew_grid(items), kEwThreads, 0, (cudaStream_t)stream>>>(x, rows, (int)cols, ldx, d);
     else
         split_tf32_kernel<false><<<ew_grid(items), kEwThreads, 0, (cudaStream_t)stream>>>(x, rows, (int)cols, ldx, d);
+    return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
+}
+
+int fgl_split_tf32_many(const fgl_split_job* jobs, int32_t n_jobs, void* stream) {
+    if (n_jobs < 0 || n_jobs > kSplitMaxJobs || (n_jobs > 0 && !jobs)) return FGL_ERR_INVALID;
+    SplitMany m{};
+    int64_t most = 0;
+    for (int j = 0; j < n_jobs; ++j) {
+        const fgl_split_job& w = jobs[j];
+        if (!split_dst(w.x, w.rows, w.cols, w.ldx, w.n_dst, w.dst, w.ld_dst, w.lo_part, m.dst[j], m.vec[j])) return FGL_ERR_INVALID;
+        m.x[j] = w.x;
+        m.rows[j] = w.rows;
+        m.cols[j] = (int)w.cols;
+        m.ldx[j] = w.ldx;
+        most = std::max(most, m.rows[j] * (m.vec[j] ? w.cols / 4 : w.cols));
+    }
+    if (most == 0) return FGL_OK;
+    split_tf32_many_kernel<<<dim3(ew_grid(most), n_jobs), kEwThreads, 0, (cudaStream_t)stream>>>(m);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
@@ -693,9 +787,15 @@ int fgl_fold_blocks(const float* part, int32_t n_slabs, int32_t n_a, int32_t n_b
         return FGL_ERR_INVALID;
     if (rows == 0 || cols == 0) return FGL_OK;
     if (!part || !out) return FGL_ERR_INVALID;
-    const int64_t groups = (int64_t)rows * ((cols + 31) / 32);
-    fold_blocks_kernel<<<(unsigned)std::min<int64_t>(groups, 148 * 16), kFoldWarps * 32, 0, (cudaStream_t)stream>>>(
-        part, n_slabs, n_a, n_b, rows, cols, block_stride, ld_part, slab_stride, out, ldo);
+    const bool vec = cols % 4 == 0 && block_stride % 4 == 0 && ld_part % 4 == 0 && slab_stride % 4 == 0 && aligned16(part);
+    const int64_t groups = (int64_t)rows * (vec ? (cols + 127) / 128 : (cols + 31) / 32);
+    const unsigned grid = (unsigned)std::min<int64_t>(groups, 148 * 16);
+    if (vec)
+        fold_blocks_kernel<4><<<grid, kFoldWarps * 32, 0, (cudaStream_t)stream>>>(part, n_slabs, n_a, n_b, rows, cols, block_stride, ld_part,
+                                                                                 slab_stride, out, ldo);
+    else
+        fold_blocks_kernel<1><<<grid, kFoldWarps * 32, 0, (cudaStream_t)stream>>>(part, n_slabs, n_a, n_b, rows, cols, block_stride, ld_part,
+                                                                                 slab_stride, out, ldo);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 

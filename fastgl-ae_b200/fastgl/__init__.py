@@ -32,9 +32,9 @@ from ._capi import (AGG_MEAN, AGG_SUM, AGG_SYMNORM, COUNTS_STRIDE, FLAG_MAP_ARRI
 
 __all__ = [
     "sample_node", "transfer_edge_id", "cal_deg", "exclusive_sum", "forward_gcn", "backward_gcn",
-    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "weight_grad", "gat_attention", "gat_attention_backward", "sample_node_csr", "sample_blocks", "aggregate", "aggregate_backward", "aggregate_window",
+    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "weight_grad", "weight_grad_scratch", "gat_attention", "gat_attention_backward", "sample_node_csr", "sample_blocks", "aggregate", "aggregate_backward", "aggregate_window",
     "sample_map_fused", "fused_capacity", "stage_segments", "stage_segments_raw", "gather_rows", "ShardedTable", "set_sampling", "seed", "FusedBatch",
-    "exclusive_sum_noalloc", "exclusive_sum_noalloc_status", "check_status", "status_str", "PeerSync", "allreduce_adam_", "window_overlap", "TransposedBlock", "transpose_block", "split_tf32", "split_tf32_raw", "fold_blocks", "probe_access_pattern",
+    "exclusive_sum_noalloc", "exclusive_sum_noalloc_status", "check_status", "status_str", "PeerSync", "allreduce_adam_", "window_overlap", "TransposedBlock", "transpose_block", "split_tf32", "split_tf32_many", "split_tf32_raw", "fold_blocks", "probe_access_pattern",
     "AGG_SUM", "AGG_MEAN", "AGG_SYMNORM",
 ]
 
@@ -467,11 +467,11 @@ def bias_relu_dropout_(y, bias=None, p_drop=0.0, relu=True, rng_seed=None, rng_c
     return y
 
 
-def relu_dropout_backward_(dy, out=None, p_drop=0.0, dbias=None, masked=True, split3=None, block_stride=None):
+def relu_dropout_backward_(dy, out=None, p_drop=0.0, dbias=None, masked=True, split3=None, block_stride=None, blocks=3):
     """In place over ``dy``: the gradient through dropout(relu(.)) given the forward output ``out`` (``masked``), and
     ``dbias += column sums`` of the result.  Returns ``dy``.  With ``split3`` (a float32 matrix of ``dy``'s rows) the
     result is written there instead, as ``[hi | lo | hi]`` TF32 parts ``block_stride`` (default: ``dy``'s width) columns
-    apart, and ``dy`` is left as it was; returns ``split3``."""
+    apart (the first ``blocks`` of the three: 2 or 3), and ``dy`` is left as it was; returns ``split3``."""
     _check_rows_f32(dy, "dy")
     if masked:
         _check_rows_f32(out, "out")
@@ -487,11 +487,14 @@ def relu_dropout_backward_(dy, out=None, p_drop=0.0, dbias=None, masked=True, sp
         bs = dy.size(1) if block_stride is None else int(block_stride)
         if split3.size(0) != dy.size(0) or bs < dy.size(1) or split3.size(1) < 2 * bs + dy.size(1):
             raise RuntimeError("split3 must have dy's rows and room for three blocks block_stride columns apart")
+        if blocks not in (2, 3):
+            raise RuntimeError("blocks must be 2 or 3")
         with _on_device(dev):
             rc = lib().fgl_relu_dropout_bwd_split(_ptr(dy), ctypes.c_int64(dy.stride(0)), _ptr(out if masked else None),
                                                   ctypes.c_int64(out.stride(0) if masked else dy.size(1)), ctypes.c_int64(dy.size(0)),
                                                   ctypes.c_int32(dy.size(1)), ctypes.c_float(p_drop), _ptr(dbias),
-                                                  ctypes.c_int32(1 if masked else 0), _ptr(split3), ctypes.c_int64(split3.stride(0)),
+                                                  ctypes.c_int32((1 if masked else 0) | (_capi.EW_TWO_BLOCKS if blocks == 2 else 0)),
+                                                  _ptr(split3), ctypes.c_int64(split3.stride(0)),
                                                   ctypes.c_int64(bs), _stream(dev))
         _raise(rc, "relu_dropout_backward_")
         return split3
@@ -594,6 +597,33 @@ def split_tf32(x, dst=None):
                                   ctypes.c_int(len(dst)), ptrs, lds, parts, _stream(dev))
     _raise(rc, "split_tf32")
     return ret
+
+
+def split_tf32_many(jobs):
+    """``split_tf32`` of several matrices in one launch: a list of up to 8 ``(x, dst)`` as ``split_tf32`` takes them."""
+    if not jobs:
+        return
+    if len(jobs) > 8:
+        raise RuntimeError("split_tf32_many takes up to 8 matrices")
+    items = (_capi.SplitJob * len(jobs))()
+    for it, (x, dst) in zip(items, jobs):
+        _check_rows_f32(x, "x")
+        if not 1 <= len(dst) <= 8:
+            raise RuntimeError("split_tf32 takes 1 to 8 destinations")
+        it.x, it.rows, it.cols, it.n_dst = x.data_ptr(), x.size(0), x.size(1), len(dst)
+        it.ldx = x.stride(0) if x.size(0) > 1 else max(x.stride(0), x.size(1))
+        for q, (t, part) in enumerate(dst):
+            _check_rows_f32(t, f"dst[{q}]")
+            if tuple(t.shape) != tuple(x.shape) or t.device != x.device:
+                raise RuntimeError("every destination must have x's shape and device")
+            if part not in ("hi", "lo"):
+                raise RuntimeError("a destination takes the part 'hi' or 'lo'")
+            it.dst[q], it.lo_part[q] = t.data_ptr(), int(part == "lo")
+            it.ld_dst[q] = t.stride(0) if t.size(0) > 1 else max(t.stride(0), t.size(1))
+    dev = jobs[0][0].device
+    with _on_device(dev):
+        rc = lib().fgl_split_tf32_many(items, ctypes.c_int32(len(jobs)), _stream(dev))
+    _raise(rc, "split_tf32_many")
 
 
 def fold_blocks(part, n_a, n_b, rows, cols, block_stride, out):
@@ -726,10 +756,17 @@ def edge_weight_grad(edge_ptr, src_edges, input_feat, d_out, num_heads):
     return _ops.edge_weight_grad(edge_ptr, src_edges, input_feat, d_out, int(num_heads))
 
 
-def weight_grad(x, dy, out=None):
+def weight_grad(x, dy, out=None, scratch=None):
     """``x^T dy`` for float32 matrices of many rows (the weight gradient of a dense layer), the contraction split over the
-    GPU in a fixed order.  Rows may be column slices of wider buffers; ``out`` receives the result when given."""
-    return _ops.weight_grad(x, dy, out)
+    GPU in a fixed order.  Rows may be column slices of wider buffers; ``out`` receives the result when given, ``scratch``
+    (float32, ``weight_grad_scratch`` entries) is allocated when not."""
+    return _ops.weight_grad(x, dy, out, scratch)
+
+
+def weight_grad_scratch(m, n, rows, device) -> int:
+    """Floats of scratch that ``weight_grad`` takes for an m x n result over ``rows`` rows."""
+    dev = torch.device(device)
+    return _ops.weight_grad_scratch(torch.cuda.current_device() if dev.index is None else dev.index, int(m), int(n), int(rows))
 
 
 def gat_attention(edge_ptr, src_edges, feat, attn_l, attn_r, dst_nodes, num_heads, negative_slope=0.2):

@@ -21,7 +21,8 @@ def _plain(module) -> bool:
 
 
 def plan(trainer):
-    """A function (fb, b, counts row) -> loss that leaves the gradients in ``trainer.grads``, or None."""
+    """A function (trainer, fb, b, counts row) -> loss that leaves the gradients in ``trainer.grads``, or None.  (It does not
+    hold the trainer: a trainer that is dropped gives its memory back at once.)"""
     model, feat, labels = trainer.model, trainer.feat, trainer.labels
     if (type(model) not in (layers.GCN, layers.GIN, layers.GAT) or not torch.is_tensor(feat) or not feat.is_cuda
             or feat.dtype != torch.float32 or feat.dim() != 2 or feat.stride(1) != 1 or not trainer._plain_labels
@@ -40,7 +41,7 @@ def plan(trainer):
     if model.layers[0].weights.size(0) != feat.size(1):
         return None
 
-    def step(fb, b, counts):
+    def step(trainer, fb, b, counts):
         weights, grads = _step_tensors(trainer, [layer.weights for layer in model.layers])
         p_drop = float(model.dropout.p) if model.training else 0.0
         if weights is None or p_drop >= 1.0 or not _plain(model):
@@ -65,7 +66,7 @@ def _plan_gat(trainer):
     if model.layers[0].fc.weight.size(1) != feat.size(1):
         return None
 
-    def step(fb, b, counts):
+    def step(trainer, fb, b, counts):
         params = [p for layer in model.layers for p in (layer.fc.weight, layer.attn_l, layer.attn_r)]
         params, grads = _step_tensors(trainer, params)
         if params is None or not _plain(model) or any(layer.training and layer.attn_drop.p > 0 for layer in model.layers):

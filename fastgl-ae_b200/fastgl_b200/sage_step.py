@@ -55,6 +55,8 @@ class SageStepProgram:
         self.dlogits = torch.zeros((self.pad_dst[L - 1], outs[L - 1]), **f32)
         self.loss = torch.zeros(1, **f32)
         self.row_loss = torch.zeros(self.pad_dst[L - 1], **f32)
+        self.part = [torch.empty(max(1, fastgl.weight_grad_scratch(2 * ins[i], outs[i], self.pad_dst[i], dev)), **f32)
+                     for i in range(L)] if matmul == "fp32" else None
         if matmul not in ("fp32", "3xtf32"):
             raise ValueError("matmul must be 'fp32' or '3xtf32'")
         # The weight-gradient products feed nothing but the optimizer, so they run on a second stream beside the chain
@@ -89,13 +91,22 @@ class SageStepProgram:
         w = c if width is None else width
         fastgl.split_tf32(x, [(x3[:, :c], "hi"), (x3[:, w: w + c], "lo"), (x3[:, 2 * w: 2 * w + c], "hi")])
 
-    def _split_weight(self, i):
-        w = self.layers[i].weight.data
-        k, m = w.shape
-        mp = self.mp[i]
-        v, c = self.wv3[i], self.wc3[i]
-        fastgl.split_tf32(w, [(v[:k], "hi"), (v[k: 2 * k], "hi"), (v[2 * k:], "lo"),
-                              (c[:, :m], "hi"), (c[:, mp: mp + m], "hi"), (c[:, 2 * mp: 2 * mp + m], "lo")])
+    def _split_weights(self):
+        """Both operand forms of every layer's weight that a product reads: forward [W_hi ; W_hi ; W_lo] (not the fused
+        output layer's), input gradient [W_hi | W_hi | W_lo] (not the first layer's)."""
+        jobs = []
+        for i, layer in enumerate(self.layers):
+            w = layer.weight.data
+            k, m = w.shape
+            mp, v, c = self.mp[i], self.wv3[i], self.wc3[i]
+            dst = []
+            if i < self.L - 1 or m > 128:
+                dst += [(v[:k], "hi"), (v[k: 2 * k], "hi"), (v[2 * k:], "lo")]
+            if i > 0:
+                dst += [(c[:, :m], "hi"), (c[:, mp: mp + m], "hi"), (c[:, 2 * mp: 2 * mp + m], "lo")]
+            if dst:
+                jobs.append((w, dst))
+        fastgl.split_tf32_many(jobs)
 
     def forward_backward(self) -> torch.Tensor:
         """Forward, loss and backward; the parameter gradients land in the flat gradient buffer.  Returns the loss
@@ -116,8 +127,7 @@ class SageStepProgram:
         split = self.split
         x_split = set()
         if split:
-            for i in range(L):
-                self._split_weight(i)
+            self._split_weights()
         last = self.layers[L - 1]
         fused_head = last.weight.size(1) <= 128        # output layer and loss in one launch
         for i, layer in enumerate(self.layers):
@@ -176,7 +186,8 @@ class SageStepProgram:
                 if split:       # straight into the operand form of layer i - 1's two gradient products
                     fastgl.relu_dropout_backward_(self.dh[i], out=self.z[i - 1], p_drop=p if training else 0.0,
                                                   dbias=self.layers[i - 1].bias.grad, split3=self.g3[i - 1],
-                                                  block_stride=self.mp[i - 1])
+                                                  block_stride=self.mp[i - 1],
+                                                  blocks=3 if i > 1 else 2)      # the third block is for the input gradient
                     dz = None
                 else:
                     dz = fastgl.relu_dropout_backward_(self.dh[i], out=self.z[i - 1], p_drop=p if training else 0.0,
@@ -201,4 +212,4 @@ class SageStepProgram:
                 torch.mm(x2.t(), g2, out=part)
             fastgl.fold_blocks(part, 2, 2, k, m, mp, gw)
             return
-        fastgl.weight_grad(x, dz, out=gw)
+        fastgl.weight_grad(x, dz, out=gw, scratch=self.part[i])

@@ -462,7 +462,7 @@ class Trainer:
                 return loss
         if self._model_step is not None and labels_of is None and layer0 is None:
             c = fb.counts_list()[b]
-            loss = self._model_step(fb, b, c)
+            loss = self._model_step(self, fb, b, c)
             if loss is not None:
                 self._sync_and_step()
                 self.sampled_edges += sum(c[8: 8 + len(self.fanouts)])

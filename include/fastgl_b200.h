@@ -50,6 +50,7 @@ extern "C" {
 
 /* flags of fgl_bias_relu_dropout / fgl_relu_dropout_bwd */
 #define FGL_EW_RELU 1     /* apply ReLU (forward) / the ReLU-and-dropout mask (backward) */
+#define FGL_EW_TWO_BLOCKS 2  /* fgl_relu_dropout_bwd_split: [hi | lo] alone, for a gradient that no further product reads */
 
 #define FGL_MAX_HOPS 7
 #define FGL_COUNTS_STRIDE 16 /* per mini-batch: [0..7] node counts n_0..n_L, [8..15] edge counts per hop */
@@ -449,6 +450,17 @@ int fgl_adam_step(float* param, const float* grad, float* exp_avg, float* exp_av
  * may overlap x. */
 int fgl_split_tf32(const float* x, int64_t rows, int64_t cols, int64_t ldx, int n_dst, float* const* dst, const int64_t* ld_dst,
                    const int32_t* lo_part, void* stream);
+
+/* The same for up to 8 matrices in one launch (the weights of a model). */
+typedef struct fgl_split_job {
+    const float* x;
+    int64_t rows, cols, ldx;
+    int32_t n_dst;
+    int32_t lo_part[8];
+    float* dst[8];
+    int64_t ld_dst[8];
+} fgl_split_job;
+int fgl_split_tf32_many(const fgl_split_job* jobs, int32_t n_jobs, void* stream);
 
 /* out[r, c] = sum over s < n_slabs, a < n_a, b < n_b of part[s][a * rows + r][b * block_stride + c], part being
  * n_slabs matrices of n_a * rows rows with leading dimension ld_part, slab_stride floats apart.  Folds the 2 x 2
