@@ -345,12 +345,12 @@ __device__ __forceinline__ int edge_owner(const Smem& sm, int size, int e) {
     return r;
 }
 
-// A node that joins the list with local id `local`: what the next hop needs of it.
-__device__ __forceinline__ void note_node(const Hop& h, int local, long long start, int deg) {
-    if ((int64_t)local >= h.deg_cap) return;
+// A node that joins the list with local id `local`: what the next hop needs of it.  Returns its edges there.
+__device__ __forceinline__ int note_node(const Hop& h, int local, long long start, int deg) {
+    if ((int64_t)local >= h.deg_cap) return 0;
     __stcg(h.node_start + local, start);
     __stcg(h.node_deg + local, deg);
-    if (deg > 0) atomicAdd(h.next_sums + (local >> h.next_shift), min(deg, h.next_fanout));
+    return min(deg, h.next_fanout);
 }
 
 // Second half of an insert in arrival-order mode: the claiming thread takes the next local id and publishes it.
@@ -368,7 +368,8 @@ __device__ __forceinline__ int arrival_assign(const KParams& p, const Hop& h, co
             long long start;
             int deg;
             load_adj<PtrT>(p, g, start, deg);
-            note_node(h, local, start, deg);
+            const int k = note_node(h, local, start, deg);
+            if (k > 0) atomicAdd(h.next_sums + (local >> h.next_shift), k);
         }
         atomicExch(tab.slots + pos, ((unsigned long long)(uint32_t)g << 32) | (uint32_t)local);
         return local;
@@ -676,15 +677,15 @@ __device__ __forceinline__ void phase_count_seeds(const KParams& p, const Hop& h
     if (threadIdx.x == 0) __stcg(team_sums + t.rank, total);
 }
 
-// The nodes that are in the list already are destinations of the next hop too: their edges, by tile (eight nodes or
-// more, so eight lanes meet in one addition).
+// The nodes that are in the list already are destinations of the next hop too: their edges, by tile (of eight nodes or
+// more: eight lanes, or all of a warp, meet in one addition).
 __device__ __forceinline__ void phase_count_old(const Hop& h, const Team& t) {
     for (int s0 = t.rank * kThreads; s0 < h.n_seeds; s0 += t.size * kThreads) {
         const int s = s0 + (int)threadIdx.x;
         int k = s < h.n_seeds ? min(__ldcg(h.node_deg + s), h.next_fanout) : 0;
-#pragma unroll
-        for (int o = 1; o < (1 << kMinTileShift); o <<= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-        if ((s & ((1 << kMinTileShift) - 1)) == 0 && k > 0) atomicAdd(h.next_sums + (s >> h.next_shift), k);
+        const int lanes = h.next_shift >= 5 ? 32 : 1 << kMinTileShift;
+        for (int o = 1; o < lanes; o <<= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+        if ((s & (lanes - 1)) == 0 && k > 0) atomicAdd(h.next_sums + (s >> h.next_shift), k);
     }
 }
 
@@ -894,6 +895,7 @@ __device__ __forceinline__ int phase_rank_tracked(const KParams& p, const Hop& h
         }
         int tile_total;
         int local = running + block_excl_scan(firsts, sm.scan, tile_total);
+        int node_tile = -1, node_sum = 0;  // this thread's new nodes have consecutive ids: mostly one tile
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
             if (m[q] < 0) {
@@ -903,13 +905,36 @@ __device__ __forceinline__ int phase_rank_tracked(const KParams& p, const Hop& h
                     h.nodes[local] = (int)key;
                     tab.slots[pos] = ((unsigned long long)key << 32) | (uint32_t)local;
                     edges[eb + q] = local;
-                    if (!h.last_hop) note_node(h, local, start[q], deg[q]);
+                    if (!h.last_hop) {
+                        const int k = note_node(h, local, start[q], deg[q]);
+                        if ((local >> h.next_shift) != node_tile) {
+                            if (node_sum > 0) atomicAdd(h.next_sums + node_tile, node_sum);
+                            node_tile = local >> h.next_shift;
+                            node_sum = 0;
+                        }
+                        node_sum += k;
+                    }
                 } else {
                     set_status(p.status, FGL_ERR_CAPACITY);
                     tab.slots[pos] = ((unsigned long long)key << 32);
                     edges[eb + q] = 0;
                 }
                 ++local;
+            }
+        }
+        if (!h.last_hop) {
+            // A warp's nodes are consecutive too: one addition where they lie in one tile.  (Tiles of 512 nodes, which large
+            // mini-batches have, took 512 additions at one address.)
+            const unsigned act = __ballot_sync(0xffffffffu, node_sum > 0);
+            if (act != 0) {
+                const int leader = __ffs(act) - 1;
+                const int lead_tile = __shfl_sync(0xffffffffu, node_tile, leader);
+                if (__all_sync(0xffffffffu, node_sum == 0 || node_tile == lead_tile)) {
+                    const int sum = __reduce_add_sync(0xffffffffu, node_sum);
+                    if ((int)(threadIdx.x & 31) == leader) atomicAdd(h.next_sums + lead_tile, sum);
+                } else if (node_sum > 0) {
+                    atomicAdd(h.next_sums + node_tile, node_sum);
+                }
             }
         }
         running += tile_total;
