@@ -102,6 +102,13 @@ struct AggParams {
     int64_t n_rows;
     int64_t n_map;
     int32_t* status;
+    // forward, optional: the result (also) as TF32 parts, [hi | lo] or [hi | lo | hi] split_stride columns apart
+    float* split;
+    int64_t ld_split, split_stride;
+    int32_t split_blocks;
+    // backward, optional: a self gradient that is added to dx[d] as one more edge of row d
+    const float* dy_self;
+    int64_t ld_dy_self;
 };
 
 __device__ __forceinline__ void agg_bad_id(const AggParams& p) {
@@ -167,7 +174,29 @@ __device__ __forceinline__ void window_offsets(const AggParams& p, long long* s_
 // entries of row i+1, the source ids of row i+2 and the offsets of row i+3 are in flight, and every loaded value is
 // first touched one iteration after it was requested.  The row's own input row (the "self" copy) is requested
 // together with the first batch of neighbour rows, not before it.
-template <int VEC, int MODE, bool HAS_MAP, int NACC, int UNR>
+//
+// SPLIT: the result leaves as the TF32 parts that an error-compensated product reads ([hi | lo | hi], see split_tf32_kernel),
+// beside or instead of the plain rows, so that no pass of its own reads the rows again to split them.
+template <int VEC, bool SPLIT>
+__device__ __forceinline__ void put_out(const AggParams& p, int64_t row, int c, const typename Vec<VEC>::T& v) {
+    using T = typename Vec<VEC>::T;
+    if (!SPLIT || p.out) reinterpret_cast<T*>(p.out + row * p.ldo)[c] = v;
+    if (SPLIT) {
+        T h, l;
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) {
+            const float x = reinterpret_cast<const float*>(&v)[q], xh = to_tf32(x);
+            reinterpret_cast<float*>(&h)[q] = xh;
+            reinterpret_cast<float*>(&l)[q] = to_tf32(x - xh);
+        }
+        float* s = p.split + row * p.ld_split;
+        reinterpret_cast<T*>(s)[c] = h;
+        reinterpret_cast<T*>(s + p.split_stride)[c] = l;
+        if (p.split_blocks > 2) reinterpret_cast<T*>(s + 2 * p.split_stride)[c] = h;
+    }
+}
+
+template <int VEC, int MODE, bool HAS_MAP, int NACC, int UNR, bool SPLIT = false>
 __global__ void __launch_bounds__(kAggThreads, FGL_AGG_MIN_CTAS) agg_fwd_kernel(const AggParams p) {
     using V = Vec<VEC>;
     using T = typename V::T;
@@ -182,8 +211,7 @@ __global__ void __launch_bounds__(kAggThreads, FGL_AGG_MIN_CTAS) agg_fwd_kernel(
     const int64_t total = p.n_dst_dev ? min((int64_t)max(__ldg(p.n_dst_dev), 0), padded) : padded;
     // padding rows of a launch sized for more rows than the block has: zero them
     for (int64_t g = total + warp_global; g < padded; g += n_warps) {
-        T* orow = reinterpret_cast<T*>(p.out + g * p.ldo);
-        for (int c = lane; c < chunks; c += 32) orow[c] = V::zero();
+        for (int c = lane; c < chunks; c += 32) put_out<VEC, SPLIT>(p, g, c, V::zero());
     }
     const bool want_self = p.self_out != nullptr || p.passthrough != 0;
 
@@ -276,7 +304,6 @@ __global__ void __launch_bounds__(kAggThreads, FGL_AGG_MIN_CTAS) agg_fwd_kernel(
         }
         const int32_t* src = p.src + (int64_t)b * p.src_stride;
         const int32_t* row_map = HAS_MAP ? p.row_map + (int64_t)b * p.row_map_stride : nullptr;
-        T* orow = reinterpret_cast<T*>(p.out + g * p.ldo);
 
         // ---- requests of this iteration, all issued before anything is consumed ------------------------------------
         // (1) the row's own input row (narrow rows: one vector per lane, kept in a register until it is stored)
@@ -315,10 +342,11 @@ __global__ void __launch_bounds__(kAggThreads, FGL_AGG_MIN_CTAS) agg_fwd_kernel(
         }
         if (a >= e_end) {  // aggregate_acc_kernel.cu:307-308, :405-406
             if (NACC == 1) {
-                if (lane < chunks) orow[lane] = p.passthrough ? self_v : V::zero();
+                if (lane < chunks) put_out<VEC, SPLIT>(p, g, lane, p.passthrough ? self_v : V::zero());
             } else {
                 const T* xr = reinterpret_cast<const T*>(x_row(p, self_row < 0 ? 0 : self_row));
-                for (int c = lane; c < chunks; c += 32) orow[c] = (p.passthrough && self_row >= 0) ? __ldg(xr + c) : V::zero();
+                for (int c = lane; c < chunks; c += 32)
+                    put_out<VEC, SPLIT>(p, g, c, (p.passthrough && self_row >= 0) ? __ldg(xr + c) : V::zero());
             }
             continue;
         }
@@ -399,7 +427,8 @@ __global__ void __launch_bounds__(kAggThreads, FGL_AGG_MIN_CTAS) agg_fwd_kernel(
 #pragma unroll
             for (int k = 0; k < NACC; ++k) {
                 const int c = c0 + k * 32 + lane;
-                if (c < chunks) orow[c] = (MODE == FGL_AGG_SUM || MODE == FGL_AGG_EDGE) ? acc[k] : V::scale(acc[k], scale);
+                if (c < chunks)
+                    put_out<VEC, SPLIT>(p, g, c, (MODE == FGL_AGG_SUM || MODE == FGL_AGG_EDGE) ? acc[k] : V::scale(acc[k], scale));
             }
         }
     }
@@ -674,6 +703,11 @@ __global__ void __launch_bounds__(kAggThreads) agg_bwd_kernel(const AggParams p)
     const int n_dst = p.n_dst_dev ? min(max(__ldg(p.n_dst_dev), 0), p.n_dst) : p.n_dst;
     for (int d = warp_global; d < n_dst; d += n_warps) {
         const int a = __ldg(p.indptr + d), b = __ldg(p.indptr + d + 1);
+        if (p.dy_self) {
+            const T* srow = reinterpret_cast<const T*>(p.dy_self + (int64_t)d * p.ld_dy_self);
+            T* xr = reinterpret_cast<T*>(p.out + (int64_t)d * p.ldo);
+            for (int c = lane; c < chunks; c += 32) red_add(xr + c, __ldg(srow + c));
+        }
         if (a >= b) continue;  // aggregate_acc_kernel.cu:498-500, :580-582
         float scale = 1.0f;
         if (MODE == FGL_AGG_MEAN) scale = 1.0f / (float)(b - a);
@@ -1165,14 +1199,16 @@ int fgl_gather_rows(fgl_ws* ws, const float* table, const float* const* shards, 
 static int agg_bwd_impl(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int32_t* src, const int32_t* src_deg,
                         const int32_t* dst_deg, const float* dy, int64_t ldy, const float* dy_self, int64_t ld_self,
                         int32_t dim, int32_t n_dst, int32_t n_src, float* dx, int64_t ldx, const int32_t* n_dst_dev,
-                        void* stream) {
+                        bool accumulate, void* stream) {
     if (mode < FGL_AGG_SUM || mode > FGL_AGG_SYMNORM || n_dst < 0 || n_src < 0 || dim < 1 || ldy < dim || ldx < dim)
         return FGL_ERR_INVALID;
     if (dy_self && (ld_self < dim || n_dst > n_src)) return FGL_ERR_INVALID;
     if (n_src == 0) return FGL_OK;
     if (!dx) return FGL_ERR_INVALID;
     cudaStream_t st = (cudaStream_t)stream;
-    if (dy_self && n_dst > 0) {
+    if (accumulate) {
+        // dx holds what the scatter adds to
+    } else if (dy_self && n_dst > 0) {
         const int64_t items = (int64_t)n_src * ((dim + 3) / 4);
         const int grid = (int)std::min<int64_t>((items + 255) / 256, 148 * 16);
         init_self_rows_kernel<<<grid, 256, 0, st>>>(dx, ldx, dy_self, ld_self, dim, n_dst, n_src, n_dst_dev);
@@ -1197,7 +1233,13 @@ static int agg_bwd_impl(fgl_ws* ws, int32_t mode, const int32_t* indptr, const i
     p.n_dst_dev = n_dst_dev;
     p.status = status_of(ws);
     const int grid = agg_grid_x(n_dst, 1);
-    switch (pick_vec(dim, dy, ldy, dx, ldx)) {
+    int vec = pick_vec(dim, dy, ldy, dx, ldx);
+    if (accumulate && dy_self) {
+        p.dy_self = dy_self;
+        p.ld_dy_self = ld_self;
+        vec = std::min(vec, pick_vec(dim, dy_self, ld_self, dx, ldx));
+    }
+    switch (vec) {
         case 4: launch_bwd_mode<4>(mode, p, grid, st); break;
         case 2: launch_bwd_mode<2>(mode, p, grid, st); break;
         default: launch_bwd_mode<1>(mode, p, grid, st); break;
@@ -1209,7 +1251,51 @@ int fgl_agg_bwd(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int32_t* 
                 const int32_t* dst_deg, const float* dy, int64_t ldy, int32_t dim, int32_t n_dst, int32_t n_src, float* dx,
                 int64_t ldx, const int32_t* n_dst_dev, void* stream) {
     return agg_bwd_impl(ws, mode, indptr, src, src_deg, dst_deg, dy, ldy, nullptr, 0, dim, n_dst, n_src, dx, ldx, n_dst_dev,
-                        stream);
+                        false, stream);
+}
+
+int fgl_agg_bwd_add(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int32_t* src, const int32_t* src_deg,
+                    const int32_t* dst_deg, const float* dy, int64_t ldy, const float* dy_self, int64_t ld_self,
+                    int32_t dim, int32_t n_dst, int32_t n_src, float* dx, int64_t ldx, const int32_t* n_dst_dev,
+                    void* stream) {
+    return agg_bwd_impl(ws, mode, indptr, src, src_deg, dst_deg, dy, ldy, dy_self, ld_self, dim, n_dst, n_src, dx, ldx, n_dst_dev,
+                        true, stream);
+}
+
+int fgl_agg_fwd_split(fgl_ws* ws, const int32_t* indptr, const int32_t* src, const float* x, int64_t n_rows, int64_t ldx,
+                      int32_t dim, int32_t n_dst, float* out, int64_t ldo, float* split, int64_t ld_split,
+                      int64_t split_stride, int32_t blocks, const int32_t* n_dst_dev, void* stream) {
+    if (n_dst < 0 || dim < 1 || ldx < dim || (out && ldo < dim) || n_rows < 0 || blocks < 2 || blocks > 3 || split_stride < dim ||
+        ld_split < (blocks - 1) * split_stride + dim)
+        return FGL_ERR_INVALID;
+    if (n_dst == 0) return FGL_OK;
+    if (!indptr || !x || !split || n_rows < 1) return FGL_ERR_INVALID;
+    // 128-bit rows alone: a caller with other rows splits them in a pass of its own
+    if (dim % 4 != 0 || split_stride % 4 != 0 || pick_vec(dim, x, ldx, split, ld_split) != 4 ||
+        (out && pick_vec(dim, x, ldx, out, ldo) != 4))
+        return FGL_ERR_INVALID;
+    AggParams p{};
+    p.indptr = indptr;
+    p.src = src;
+    p.x = x;
+    p.out = out;
+    p.ldx = ldx;
+    p.ldo = ldo;
+    p.dim = dim;
+    p.n_dst = n_dst;
+    p.n_dst_dev = n_dst_dev;
+    p.n_rows = n_rows;
+    p.status = status_of(ws);
+    p.split = split;
+    p.ld_split = ld_split;
+    p.split_stride = split_stride;
+    p.split_blocks = blocks;
+    const int grid = agg_grid_x(n_dst, 1);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (dim <= 128) agg_fwd_kernel<4, FGL_AGG_MEAN, false, 1, FGL_AGG_UNR1, true><<<grid, kAggThreads, 0, st>>>(p);
+    else if (dim <= 256) agg_fwd_kernel<4, FGL_AGG_MEAN, false, 2, 4, true><<<grid, kAggThreads, 0, st>>>(p);
+    else agg_fwd_kernel<4, FGL_AGG_MEAN, false, 4, 2, true><<<grid, kAggThreads, 0, st>>>(p);
+    return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
 int fgl_agg_bwd_self(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int32_t* src, const int32_t* src_deg,
@@ -1218,7 +1304,7 @@ int fgl_agg_bwd_self(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int3
                      void* stream) {
     if (!dy_self && n_dst > 0) return FGL_ERR_INVALID;
     return agg_bwd_impl(ws, mode, indptr, src, src_deg, dst_deg, dy, ldy, dy_self, ld_self, dim, n_dst, n_src, dx, ldx,
-                        n_dst_dev, stream);
+                        n_dst_dev, false, stream);
 }
 
 }  // extern "C"

@@ -237,6 +237,13 @@ __device__ __forceinline__ bool team_barrier(Team& t) {
 
 #endif  // __CUDACC__
 
+// x rounded to TF32 (10-bit mantissa, round to nearest), as an fp32 value
+__device__ __forceinline__ float to_tf32(float x) {
+    uint32_t u;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
+    return __uint_as_float(u);
+}
+
 }  // namespace fgl
 
 struct fgl_ws : public fgl::Workspace {};

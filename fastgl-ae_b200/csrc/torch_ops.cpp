@@ -35,7 +35,7 @@ void* g_lib = nullptr;
     X(fgl_status_str) X(fgl_last_error) X(fgl_ws_create) X(fgl_ws_check) X(fgl_sample) X(fgl_map) X(fgl_fused_capacity) \
     X(fgl_sample_map_fused_extra) X(fgl_cal_deg) X(fgl_exclusive_sum) X(fgl_stage_segments) X(fgl_agg_fwd)              \
     X(fgl_agg_fwd_window_counts) X(fgl_agg_edge_fwd) X(fgl_agg_edge_bwd) X(fgl_agg_edge_wgrad) X(fgl_agg_bwd)            \
-    X(fgl_agg_bwd_self) X(fgl_block_transpose) X(fgl_agg_bwd_gather) X(fgl_gather_rows) X(fgl_ws_time_next_launch)           \
+    X(fgl_agg_bwd_self) X(fgl_agg_bwd_add) X(fgl_block_transpose) X(fgl_agg_bwd_gather) X(fgl_gather_rows) X(fgl_ws_time_next_launch)           \
     X(fgl_gat_fwd) X(fgl_gat_bwd) X(fgl_gat_bwd_partials) X(fgl_softmax_xent) X(fgl_adam_step) \
     X(fgl_block_degrees) X(fgl_mask_rows) X(fgl_weight_grad) X(fgl_weight_grad_scratch)
 
@@ -493,7 +493,7 @@ struct Transposed {
 
 at::Tensor agg_bwd(int mode, const at::Tensor& edge_ptr, const at::Tensor& src, const at::Tensor& dy, int64_t n_src, const at::Tensor& src_deg,
                    const at::Tensor& dst_deg, const at::Tensor& n_dst_dev, const at::Tensor& d_self, const at::Tensor& out_given,
-                   const Transposed* tb) {
+                   const Transposed* tb, bool accumulate = false) {
     const int64_t n_dst = dy.size(0), dim = dy.size(1);
     TORCH_CHECK(mode != FGL_AGG_SYMNORM || (src_deg.defined() && dst_deg.defined() && src_deg.numel() >= n_src && dst_deg.numel() >= n_dst),
                 "sym-norm needs src_norm_degs[src_nodes] and dst_norm_degs[n_dst]");
@@ -508,6 +508,11 @@ at::Tensor agg_bwd(int mode, const at::Tensor& edge_ptr, const at::Tensor& src, 
                                     ptr<int32_t>(tb->hubs), ptr<int32_t>(src_deg), ptr<int32_t>(dst_deg), ptr<float>(dy), dy.stride(0),
                                     ptr<float>(d_self), d_self.defined() ? d_self.stride(0) : dim, (int32_t)dim, (int32_t)n_dst,
                                     (int32_t)n_src, ptr<float>(dx), dx.stride(0), ptr<int32_t>(n_dst_dev), c.st());
+    else if (accumulate)
+        rc = api.fgl_agg_bwd_add(c.ws, mode, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), ptr<int32_t>(src_deg), ptr<int32_t>(dst_deg),
+                                 ptr<float>(dy), dy.stride(0), ptr<float>(d_self), d_self.defined() ? d_self.stride(0) : dim,
+                                 (int32_t)dim, (int32_t)n_dst, (int32_t)n_src, ptr<float>(dx), dx.stride(0), ptr<int32_t>(n_dst_dev),
+                                 c.st());
     else if (d_self.defined())
         rc = api.fgl_agg_bwd_self(c.ws, mode, ptr<int32_t>(edge_ptr), ptr<int32_t>(src), ptr<int32_t>(src_deg), ptr<int32_t>(dst_deg),
                                   ptr<float>(dy), dy.stride(0), ptr<float>(d_self), d_self.stride(0), (int32_t)dim, (int32_t)n_dst,
@@ -522,7 +527,7 @@ at::Tensor agg_bwd(int mode, const at::Tensor& edge_ptr, const at::Tensor& src, 
 
 at::Tensor aggregate_backward(int mode, py::handle ptr_o, py::handle src_o, py::handle dy_o, int64_t n_src, py::handle src_deg,
                               py::handle dst_deg, py::handle n_dst_dev, py::handle d_self, py::handle out, py::handle t_indptr,
-                              py::handle t_dst, py::handle hubs) {
+                              py::handle t_dst, py::handle hubs, bool accumulate) {
     Transposed tb;
     const bool gather = !t_indptr.is_none();
     if (gather) tb = {tensor(t_indptr, "t_indptr"), tensor(t_dst, "t_dst"), tensor(hubs, "hubs")};
@@ -530,7 +535,7 @@ at::Tensor aggregate_backward(int mode, py::handle ptr_o, py::handle src_o, py::
                    optional_i32(src_deg, "src_norm_degs"), optional_i32(dst_deg, "dst_norm_degs"),
                    n_dst_dev.is_none() ? at::Tensor() : tensor(n_dst_dev, "n_dst_dev"),
                    d_self.is_none() ? at::Tensor() : rows_f32(d_self, "d_self"), out.is_none() ? at::Tensor() : rows_f32(out, "out"),
-                   gather ? &tb : nullptr);
+                   gather ? &tb : nullptr, accumulate);
 }
 
 void transpose_block(py::handle ptr_o, py::handle src_o, int64_t n_dst, int64_t n_src, py::handle n_dst_dev, const at::Tensor& t_indptr,

@@ -29,7 +29,8 @@ __global__ void __launch_bounds__(kEwThreads)
 bias_relu_dropout_kernel(float* __restrict__ y, int64_t ld, int64_t n_rows, int dim, const float* __restrict__ bias,
                          uint32_t drop_below, float keep_scale, uint64_t rng_seed, uint64_t rng_ctr,
                          const int32_t* __restrict__ rng_ctr_dev, int flags, float* __restrict__ copy_out,
-                         int64_t ld_copy, int64_t n_copy_rows) {
+                         int64_t ld_copy, int64_t n_copy_rows, float* __restrict__ split, int64_t ld_split,
+                         int64_t split_stride) {
     const int64_t groups_per_row = dim / VEC;
     const int64_t total = n_rows * groups_per_row;
     const uint64_t ctr = rng_ctr + (rng_ctr_dev ? (uint64_t)(uint32_t)rng_ctr_dev[0] : 0ull);
@@ -52,7 +53,20 @@ bias_relu_dropout_kernel(float* __restrict__ y, int64_t ld, int64_t n_rows, int 
                 v.w = w.w < drop_below ? 0.f : v.w * keep_scale;
             }
             *reinterpret_cast<float4*>(p) = v;
-            if (r < n_copy_rows) *reinterpret_cast<float4*>(copy_out + r * ld_copy + c) = v;
+            if (r < n_copy_rows) {
+                if (copy_out) *reinterpret_cast<float4*>(copy_out + r * ld_copy + c) = v;
+                if (split) {  // the TF32 parts of the copy, as the error-compensated product of the next layer reads them
+                    float4 h, l;
+                    h.x = to_tf32(v.x); l.x = to_tf32(v.x - h.x);
+                    h.y = to_tf32(v.y); l.y = to_tf32(v.y - h.y);
+                    h.z = to_tf32(v.z); l.z = to_tf32(v.z - h.z);
+                    h.w = to_tf32(v.w); l.w = to_tf32(v.w - h.w);
+                    float* s = split + r * ld_split + c;
+                    *reinterpret_cast<float4*>(s) = h;
+                    *reinterpret_cast<float4*>(s + split_stride) = l;
+                    if (!(flags & FGL_EW_TWO_BLOCKS)) *reinterpret_cast<float4*>(s + 2 * split_stride) = h;
+                }
+            }
         } else {
             float v = *p + (bias ? bias[c] : 0.f);
             if (relu) v = fmaxf(v, 0.f);
@@ -76,13 +90,6 @@ constexpr int kBwdRowBatch = 8;
 
 // SPLIT: dz is not written back over dy but as [hi | lo | hi] TF32 parts (see split_tf32_kernel) into split3, the three
 // blocks block_stride columns apart: the form in which the error-compensated products read it.
-// x rounded to TF32 (10-bit mantissa, round to nearest), as an fp32 value
-__device__ __forceinline__ float to_tf32(float x) {
-    uint32_t u;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
-    return __uint_as_float(u);
-}
-
 template <bool SPLIT>
 __global__ void __launch_bounds__(kEwThreads)
 relu_dropout_bwd_kernel(float* __restrict__ dy, int64_t ldy, const float* __restrict__ out, int64_t ldo, int64_t n_rows,
@@ -294,7 +301,7 @@ linear_xent_kernel(const float* __restrict__ x, int64_t ldx, int k, const float*
                    int64_t n_labels, int n_rows, int n_classes, const int32_t* __restrict__ n_valid_dev, int n_valid_host,
                    float* __restrict__ row_loss, float* __restrict__ dlogits, int64_t ldd, float* __restrict__ dbias,
                    float* __restrict__ logits_out, int64_t ldl, int32_t* __restrict__ status, float* __restrict__ loss,
-                   unsigned int* __restrict__ ticket) {
+                   unsigned int* __restrict__ ticket, float* __restrict__ split, int64_t ld_split, int64_t split_stride) {
     __shared__ float part[kLinXentWarps][kLinXentRows][32 * CPL];
     __shared__ float db[32 * CPL];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -305,6 +312,12 @@ linear_xent_kernel(const float* __restrict__ x, int64_t ldx, int k, const float*
     const float inv = n_valid > 0 ? 1.f / (float)n_valid : 0.f;
     // rows that need their logits: the valid ones, or all of them when the caller wants the logits
     const int rows_here = min(kLinXentRows, (logits_out ? n_rows : n_valid) - row0);
+    // the label of the row that this warp finishes: two dependent reads, on their way under the product
+    int64_t label = -1;
+    if (warp < kLinXentRows && row0 + warp < n_valid) {
+        const int64_t at = label_ids ? (int64_t)__ldg(label_ids + row0 + warp) : (int64_t)(row0 + warp);
+        if (at >= 0 && at < n_labels) label = __ldg(labels + at);
+    }
 
     float acc[kLinXentRows][CPL];
 #pragma unroll
@@ -370,9 +383,8 @@ linear_xent_kernel(const float* __restrict__ x, int64_t ldx, int k, const float*
         }
         float mine = 0.f;
         bool counted = false;
+        float* s = split ? split + (int64_t)r * ld_split : nullptr;
         if (r < n_valid) {
-            const int64_t at = label_ids ? (int64_t)label_ids[r] : (int64_t)r;
-            const int64_t label = at >= 0 && at < n_labels ? labels[at] : -1;
             if (label < 0 || label >= n_classes) {
                 if (lane == 0) atomicCAS(status, FGL_OK, FGL_ERR_BOUNDS);
             } else {
@@ -404,13 +416,22 @@ linear_xent_kernel(const float* __restrict__ x, int64_t ldx, int k, const float*
                     if (c < n_classes) {
                         const float g = e[q] * rs - (c == (int)label ? inv : 0.f);
                         d[c] = g;
+                        if (s) {
+                            const float h = to_tf32(g);
+                            s[c] = h;
+                            s[split_stride + c] = to_tf32(g - h);
+                            s[2 * split_stride + c] = h;
+                        }
                         if (dbias) atomicAdd(&db[c], g);
                     }
                 }
             }
         }
         if (!counted)
-            for (int c = lane; c < n_classes; c += 32) d[c] = 0.f;
+            for (int c = lane; c < n_classes; c += 32) {
+                d[c] = 0.f;
+                if (s) s[c] = s[split_stride + c] = s[2 * split_stride + c] = 0.f;
+            }
         if (lane == 0) row_loss[r] = mine;
     }
     __syncthreads();
@@ -604,12 +625,15 @@ using namespace fgl;
 
 extern "C" {
 
-int fgl_bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, const float* bias, float p_drop,
-                          uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
-                          int64_t ld_copy, int64_t n_copy_rows, void* stream) {
+static int bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, const float* bias, float p_drop,
+                             uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
+                             int64_t ld_copy, int64_t n_copy_rows, float* split, int64_t ld_split, int64_t split_stride,
+                             void* stream) {
     if (n_rows < 0 || dim <= 0 || ld < dim || (n_rows > 0 && !y) || !(p_drop >= 0.f && p_drop < 1.f)) return FGL_ERR_INVALID;
-    if (!copy_out) n_copy_rows = 0;
-    if (n_copy_rows < 0 || n_copy_rows > n_rows || (n_copy_rows > 0 && ld_copy < dim)) return FGL_ERR_INVALID;
+    if (!copy_out && !split) n_copy_rows = 0;
+    if (n_copy_rows < 0 || n_copy_rows > n_rows || (copy_out && n_copy_rows > 0 && ld_copy < dim)) return FGL_ERR_INVALID;
+    const int blocks = flags & FGL_EW_TWO_BLOCKS ? 2 : 3;
+    if (split && (split_stride < dim || ld_split < (blocks - 1) * split_stride + dim)) return FGL_ERR_INVALID;
     if (n_rows == 0) return FGL_OK;
     // an element is dropped when its 32-bit word is below p * 2^32
     const double thresh = (double)p_drop * 4294967296.0;
@@ -617,16 +641,34 @@ int fgl_bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, con
     const float keep_scale = p_drop > 0.f ? 1.f / (1.f - p_drop) : 1.f;
     cudaStream_t st = (cudaStream_t)stream;
     const bool vec = dim % 4 == 0 && ld % 4 == 0 && aligned16(y) && (!bias || aligned16(bias)) &&
-                     (n_copy_rows == 0 || (ld_copy % 4 == 0 && aligned16(copy_out)));
+                     (n_copy_rows == 0 || !copy_out || (ld_copy % 4 == 0 && aligned16(copy_out)));
+    // whole 16-byte vectors alone: a caller with other rows splits them in a pass of its own
+    if (split && !(vec && ld_split % 4 == 0 && split_stride % 4 == 0 && aligned16(split))) return FGL_ERR_INVALID;
     if (vec)
         bias_relu_dropout_kernel<4><<<ew_grid(n_rows * (dim / 4)), kEwThreads, 0, st>>>(
             y, ld, n_rows, dim, bias, drop_below, keep_scale, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
-            n_copy_rows);
+            n_copy_rows, split, ld_split, split_stride);
     else
         bias_relu_dropout_kernel<1><<<ew_grid(n_rows * dim), kEwThreads, 0, st>>>(
             y, ld, n_rows, dim, bias, drop_below, keep_scale, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
-            n_copy_rows);
+            n_copy_rows, nullptr, 0, 0);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
+}
+
+int fgl_bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, const float* bias, float p_drop,
+                          uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
+                          int64_t ld_copy, int64_t n_copy_rows, void* stream) {
+    return bias_relu_dropout(y, ld, n_rows, dim, bias, p_drop, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
+                             n_copy_rows, nullptr, 0, 0, stream);
+}
+
+int fgl_bias_relu_dropout_split(float* y, int64_t ld, int64_t n_rows, int32_t dim, const float* bias, float p_drop,
+                                uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
+                                int64_t ld_copy, int64_t n_copy_rows, float* split, int64_t ld_split, int64_t split_stride,
+                                void* stream) {
+    if (!split) return FGL_ERR_INVALID;
+    return bias_relu_dropout(y, ld, n_rows, dim, bias, p_drop, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
+                             n_copy_rows, split, ld_split, split_stride, stream);
 }
 
 static int relu_dropout_bwd_launch(float* dy, int64_t ldy, const float* out, int64_t ldo, int64_t n_rows, int32_t dim, float p_drop,
@@ -700,10 +742,12 @@ int fgl_softmax_xent(fgl_ws* ws, const float* logits, int64_t ld, const int64_t*
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
-int fgl_linear_softmax_xent(fgl_ws* ws, const float* x, int64_t ldx, int32_t k, const float* w, int64_t ldw, const float* bias,
-                            const int64_t* labels, const int32_t* label_ids, int64_t n_labels, int32_t n_rows,
-                            int32_t n_classes, const int32_t* n_valid_dev, int32_t n_valid, float* loss, float* dlogits,
-                            int64_t ldd, float* dbias, float* logits_out, int64_t ldl, float* row_loss, void* stream) {
+static int linear_xent(fgl_ws* ws, const float* x, int64_t ldx, int32_t k, const float* w, int64_t ldw, const float* bias,
+                       const int64_t* labels, const int32_t* label_ids, int64_t n_labels, int32_t n_rows,
+                       int32_t n_classes, const int32_t* n_valid_dev, int32_t n_valid, float* loss, float* dlogits,
+                       int64_t ldd, float* dbias, float* logits_out, int64_t ldl, float* row_loss, float* split,
+                       int64_t ld_split, int64_t split_stride, void* stream) {
+    if (split && (split_stride < n_classes || ld_split < 2 * split_stride + n_classes)) return FGL_ERR_INVALID;
     if (!ws || n_rows < 0 || k <= 0 || n_classes <= 0 || n_classes > 128 || ldx < k || ldw < n_classes || ldd < n_classes ||
         !loss || (logits_out && ldl < n_classes) || (n_rows > 0 && (!x || !w || !labels || !dlogits || !row_loss)))
         return FGL_ERR_INVALID;
@@ -713,12 +757,31 @@ int fgl_linear_softmax_xent(fgl_ws* ws, const float* x, int64_t ldx, int32_t k, 
 #define FGL_LINXENT(CPL)                                                                                              \
     linear_xent_kernel<CPL><<<grid, kLinXentWarps * 32, 0, st>>>(x, ldx, k, w, ldw, bias, labels, label_ids, n_labels, \
                                                                  n_rows, n_classes, n_valid_dev, n_valid, row_loss,   \
-                                                                 dlogits, ldd, dbias, logits_out, ldl, ws->status, loss, loss_ticket(ws))
+                                                                 dlogits, ldd, dbias, logits_out, ldl, ws->status, loss, loss_ticket(ws), \
+                                                                 split, ld_split, split_stride)
     if (n_classes <= 32) FGL_LINXENT(1);
     else if (n_classes <= 64) FGL_LINXENT(2);
     else FGL_LINXENT(4);
 #undef FGL_LINXENT
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
+}
+
+int fgl_linear_softmax_xent(fgl_ws* ws, const float* x, int64_t ldx, int32_t k, const float* w, int64_t ldw, const float* bias,
+                            const int64_t* labels, const int32_t* label_ids, int64_t n_labels, int32_t n_rows,
+                            int32_t n_classes, const int32_t* n_valid_dev, int32_t n_valid, float* loss, float* dlogits,
+                            int64_t ldd, float* dbias, float* logits_out, int64_t ldl, float* row_loss, void* stream) {
+    return linear_xent(ws, x, ldx, k, w, ldw, bias, labels, label_ids, n_labels, n_rows, n_classes, n_valid_dev, n_valid, loss, dlogits,
+                       ldd, dbias, logits_out, ldl, row_loss, nullptr, 0, 0, stream);
+}
+
+int fgl_linear_softmax_xent_split(fgl_ws* ws, const float* x, int64_t ldx, int32_t k, const float* w, int64_t ldw, const float* bias,
+                                  const int64_t* labels, const int32_t* label_ids, int64_t n_labels, int32_t n_rows,
+                                  int32_t n_classes, const int32_t* n_valid_dev, int32_t n_valid, float* loss, float* dlogits,
+                                  int64_t ldd, float* dbias, float* row_loss, float* split, int64_t ld_split,
+                                  int64_t split_stride, void* stream) {
+    if (!split) return FGL_ERR_INVALID;
+    return linear_xent(ws, x, ldx, k, w, ldw, bias, labels, label_ids, n_labels, n_rows, n_classes, n_valid_dev, n_valid, loss, dlogits,
+                       ldd, dbias, nullptr, 0, row_loss, split, ld_split, split_stride, stream);
 }
 
 int fgl_adam_step(float* param, const float* grad, float* exp_avg, float* exp_avg_sq, int64_t n, float lr, float beta1,

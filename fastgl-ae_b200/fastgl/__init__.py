@@ -32,7 +32,7 @@ from ._capi import (AGG_MEAN, AGG_SUM, AGG_SYMNORM, COUNTS_STRIDE, FLAG_MAP_ARRI
 
 __all__ = [
     "sample_node", "transfer_edge_id", "cal_deg", "exclusive_sum", "forward_gcn", "backward_gcn",
-    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "weight_grad", "weight_grad_scratch", "gat_attention", "gat_attention_backward", "sample_node_csr", "sample_blocks", "aggregate", "aggregate_backward", "aggregate_window",
+    "forwaed_gin", "backward_gin", "forward_gat", "backward_gat", "edge_weight_grad", "weight_grad", "weight_grad_scratch", "gat_attention", "gat_attention_backward", "sample_node_csr", "sample_blocks", "aggregate", "aggregate_split", "aggregate_backward", "aggregate_window",
     "sample_map_fused", "fused_capacity", "stage_segments", "stage_segments_raw", "gather_rows", "ShardedTable", "set_sampling", "seed", "FusedBatch",
     "exclusive_sum_noalloc", "exclusive_sum_noalloc_status", "check_status", "status_str", "PeerSync", "allreduce_adam_", "window_overlap", "TransposedBlock", "transpose_block", "split_tf32", "split_tf32_many", "split_tf32_raw", "fold_blocks", "probe_access_pattern",
     "AGG_SUM", "AGG_MEAN", "AGG_SYMNORM",
@@ -428,24 +428,55 @@ def transpose_block(edge_ptr, src_edges, dst_nodes, src_nodes, n_dst_dev=None, o
 
 
 def aggregate_backward(mode, edge_ptr, src_edges, d_out, src_nodes, src_norm_degs=None, dst_norm_degs=None,
-                       n_dst_dev=None, d_self=None, out=None, transposed: TransposedBlock | None = None):
+                       n_dst_dev=None, d_self=None, out=None, transposed: TransposedBlock | None = None, accumulate=False):
     """d_x[src] += w * d_out[d] over every edge; returns d_x float32[src_nodes, dim].  ``n_dst_dev`` as in
     ``aggregate``.  ``d_self`` (float32[n_dst, dim], rows may be a column slice) is the gradient of a self term:
     d_x starts from it in its first n_dst rows instead of from zero.  ``d_out`` may be a column slice too;
     ``out`` receives the result when given.  With ``transposed`` (``transpose_block`` of the same block) the result is
-    gathered row by row in a fixed order -- bit-reproducible -- instead of scattered with atomic reductions."""
+    gathered row by row in a fixed order -- bit-reproducible -- instead of scattered with atomic reductions.  With
+    ``accumulate`` the result is added to what ``out`` holds (a scatter alone, without its initialisation)."""
     tb = transposed
+    if accumulate and (tb is not None or out is None):
+        raise RuntimeError("accumulate needs out, and adds with the scatter alone")
     return _ops.aggregate_backward(int(mode), edge_ptr, src_edges, d_out, int(src_nodes), src_norm_degs, dst_norm_degs, n_dst_dev,
-                                   d_self, out, *((None, None, None) if tb is None else (tb.t_indptr, tb.t_dst, tb.hubs)))
+                                   d_self, out, *((None, None, None) if tb is None else (tb.t_indptr, tb.t_dst, tb.hubs)),
+                                   bool(accumulate))
+
+
+def aggregate_split(edge_ptr, src_edges, input_feat, dst_nodes, split, split_stride, blocks=3, out=None, n_dst_dev=None):
+    """``aggregate(AGG_MEAN, ..)`` whose result is written as ``[hi | lo | hi]`` TF32 parts (the first ``blocks`` of the
+    three) into ``split``, ``split_stride`` columns apart, and to ``out`` as it is when that is given.  Rows of whole
+    16-byte vectors only."""
+    _check_i32(edge_ptr, "edge_ptr")
+    _check_i32(src_edges, "src_edges")
+    _check_rows_f32(input_feat, "input_feat")
+    _check_rows_f32(split, "split")
+    n_dst, dim = int(dst_nodes), input_feat.size(1)
+    if edge_ptr.numel() < n_dst + 1 or split.size(0) < n_dst or split.size(1) < (blocks - 1) * split_stride + dim:
+        raise RuntimeError("edge_ptr or split is too small for dst_nodes rows")
+    if out is not None:
+        _check_rows_f32(out, "out")
+        if out.size(0) < n_dst or out.size(1) != dim:
+            raise RuntimeError("out must be float32[dst_nodes, dim]")
+    dev = input_feat.device
+    with _on_device(dev):
+        rc = lib().fgl_agg_fwd_split(_ws(dev), _ptr(edge_ptr), _ptr(src_edges), _ptr(input_feat), ctypes.c_int64(input_feat.size(0)),
+                                     ctypes.c_int64(input_feat.stride(0)), ctypes.c_int32(dim), ctypes.c_int32(n_dst), _ptr(out),
+                                     ctypes.c_int64(0 if out is None else out.stride(0)), _ptr(split),
+                                     ctypes.c_int64(split.stride(0)), ctypes.c_int64(split_stride), ctypes.c_int32(blocks),
+                                     _ptr(n_dst_dev), _stream(dev))
+    _raise(rc, "aggregate_split")
 
 
 # ------------------------------------------------------------------------------------------------
 # element-wise kernels of the training step (no counterpart among the reference's operators)
 # ------------------------------------------------------------------------------------------------
-def bias_relu_dropout_(y, bias=None, p_drop=0.0, relu=True, rng_seed=None, rng_ctr=0, rng_ctr_dev=None, copy_out=None):
+def bias_relu_dropout_(y, bias=None, p_drop=0.0, relu=True, rng_seed=None, rng_ctr=0, rng_ctr_dev=None, copy_out=None,
+                       split=None, split_stride=None, blocks=3):
     """In place: y = dropout(relu(y + bias)).  ``rng_ctr_dev`` (int32 CUDA tensor) is added to ``rng_ctr`` on the
     device, so a captured launch draws a new mask per replay.  ``copy_out`` (float32[k, dim], k <= rows, may be a
-    column slice) also receives the first k result rows.  Returns ``y``."""
+    column slice) also receives the first k result rows; so does ``split`` (k rows) as ``[hi | lo | hi]`` TF32 parts (the
+    first ``blocks`` of the three) ``split_stride`` columns apart, for rows of whole 16-byte vectors.  Returns ``y``."""
     _check_rows_f32(y, "y")
     if copy_out is not None:
         _check_rows_f32(copy_out, "copy_out")
@@ -456,6 +487,20 @@ def bias_relu_dropout_(y, bias=None, p_drop=0.0, relu=True, rng_seed=None, rng_c
         if bias.numel() != y.size(1):
             raise RuntimeError("bias must have one entry per column")
     dev = y.device
+    if split is not None:
+        _check_rows_f32(split, "split")
+        rows = split.size(0) if copy_out is None else copy_out.size(0)
+        if rows > y.size(0) or split.size(0) != rows or split.size(1) < (blocks - 1) * split_stride + y.size(1) or blocks not in (2, 3):
+            raise RuntimeError("split must have copy_out's rows and room for its blocks split_stride columns apart")
+        with _on_device(dev):
+            rc = lib().fgl_bias_relu_dropout_split(
+                _ptr(y), ctypes.c_int64(y.stride(0)), ctypes.c_int64(y.size(0)), ctypes.c_int32(y.size(1)), _ptr(bias),
+                ctypes.c_float(p_drop), ctypes.c_uint64(_config["rng_seed"] if rng_seed is None else rng_seed), ctypes.c_uint64(rng_ctr),
+                _ptr(rng_ctr_dev), ctypes.c_int32((1 if relu else 0) | (_capi.EW_TWO_BLOCKS if blocks == 2 else 0)), _ptr(copy_out),
+                ctypes.c_int64(copy_out.stride(0) if copy_out is not None else 0), ctypes.c_int64(rows), _ptr(split),
+                ctypes.c_int64(split.stride(0)), ctypes.c_int64(split_stride), _stream(dev))
+        _raise(rc, "bias_relu_dropout_")
+        return y
     with _on_device(dev):
         rc = lib().fgl_bias_relu_dropout(_ptr(y), ctypes.c_int64(y.stride(0)), ctypes.c_int64(y.size(0)), ctypes.c_int32(y.size(1)),
                                          _ptr(bias), ctypes.c_float(p_drop),
@@ -515,9 +560,10 @@ def softmax_xent(logits, labels, label_ids=None, n_valid=None, loss=None, dlogit
 
 
 def linear_softmax_xent(x, weight, bias, labels, label_ids=None, n_valid=None, loss=None, dlogits=None, row_loss=None,
-                        dbias=None, logits=None):
+                        dbias=None, logits=None, split3=None, block_stride=None):
     """``softmax_xent(x @ weight + bias, ...)`` in one pass for at most 128 classes: returns (loss, dlogits); ``dbias``
-    (float32[n_classes], zeroed by the caller) also receives the bias gradient and ``logits`` the logits."""
+    (float32[n_classes], zeroed by the caller) also receives the bias gradient and ``logits`` the logits.  ``split3``
+    (not together with ``logits``) also receives dlogits as ``[hi | lo | hi]`` TF32 parts ``block_stride`` columns apart."""
     _check_rows_f32(x, "x")
     _check_rows_f32(weight, "weight")
     if weight.size(0) != x.size(1) or weight.size(1) > 128:
@@ -547,6 +593,20 @@ def linear_softmax_xent(x, weight, bias, labels, label_ids=None, n_valid=None, l
     if n_valid_dev is not None:
         _check_i32(n_valid_dev, "n_valid")
     ws = _ws(dev)
+    if split3 is not None:
+        _check_rows_f32(split3, "split3")
+        if logits is not None or split3.size(0) < n_rows or split3.size(1) < 2 * block_stride + n_classes:
+            raise RuntimeError("split3 must hold x's rows and three blocks block_stride columns apart, and excludes logits")
+        with _on_device(dev):
+            rc = lib().fgl_linear_softmax_xent_split(
+                ws, _ptr(x), ctypes.c_int64(x.stride(0)), ctypes.c_int32(k), _ptr(weight), ctypes.c_int64(weight.stride(0)),
+                _ptr(bias), _ptr(labels), _ptr(label_ids), ctypes.c_int64(labels.numel()), ctypes.c_int32(n_rows),
+                ctypes.c_int32(n_classes), _ptr(n_valid_dev),
+                ctypes.c_int32(n_rows if n_valid is None or n_valid_dev is not None else int(n_valid)), _ptr(loss), _ptr(dlogits),
+                ctypes.c_int64(dlogits.stride(0)), _ptr(dbias), _ptr(row_loss), _ptr(split3), ctypes.c_int64(split3.stride(0)),
+                ctypes.c_int64(block_stride), _stream(dev))
+        _raise(rc, "linear_softmax_xent", ws)
+        return loss, dlogits
     with _on_device(dev):
         rc = lib().fgl_linear_softmax_xent(
             ws, _ptr(x), ctypes.c_int64(x.stride(0)), ctypes.c_int32(k), _ptr(weight), ctypes.c_int64(weight.stride(0)),

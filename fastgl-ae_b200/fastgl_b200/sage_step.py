@@ -123,9 +123,19 @@ class SageStepProgram:
     def _forward_backward(self) -> torch.Tensor:
         L, p = self.L, self.p_drop
         training = self.model.training
-        self.grads.zero()
         split = self.split
         x_split = set()
+        # What the backward adds to -- the bias gradients and every layer's input gradient -- is emptied beside the forward, on
+        # the second stream (the scatter then needs no launch that initialises its rows: 10 us at 42 k x 256).
+        main = torch.cuda.current_stream()
+        zeroed = main
+        if self.overlap:
+            zeroed = self.side
+            zeroed.wait_stream(main)
+        with torch.cuda.stream(zeroed):
+            self.grads.zero()
+            for t in self.dh[1:]:
+                t.zero_()
         if split:
             self._split_weights()
         last = self.layers[L - 1]
@@ -134,7 +144,7 @@ class SageStepProgram:
             if i == L - 1 and fused_head:
                 break
             if split:
-                if not (i == 0 and self.x0_presplit):
+                if i not in x_split and not (i == 0 and self.x0_presplit):
                     self._split3(self.cat[i], self.x3[i])
                 x_split.add(i)
                 torch.mm(self.x3[i], self.wv3[i], out=self.z[i])
@@ -144,31 +154,44 @@ class SageStepProgram:
                 blk = self.blocks[i + 1]
                 d = self.layers[i + 1].input_dim
                 nxt = self.cat[i + 1]
-                fastgl.bias_relu_dropout_(self.z[i], layer.bias, p if training else 0.0, relu=True, rng_seed=self.rng_seed,
-                                          rng_ctr=(i + 1) << 40, rng_ctr_dev=self.step_word, copy_out=nxt[:, :d])
-                fastgl.aggregate(fastgl.AGG_MEAN, blk.indptr, blk.src, self.z[i], self.pad_dst[i + 1],
-                                 zero_deg_passthrough=False, out=nxt[:, d:], n_dst_dev=blk.n_dst_dev)
+                drop = dict(relu=True, rng_seed=self.rng_seed, rng_ctr=(i + 1) << 40, rng_ctr_dev=self.step_word)
+                if split and d % 4 == 0:
+                    # straight into the operand form of the next layer's products; the plain rows only for the fused output
+                    # layer, which reads them (and whose weight gradient reads two of the three blocks)
+                    head = i + 1 == L - 1 and fused_head
+                    x3, blocks = self.x3[i + 1], 2 if head else 3
+                    fastgl.bias_relu_dropout_(self.z[i], layer.bias, p if training else 0.0, **drop, copy_out=nxt[:, :d] if head else None,
+                                              split=x3, split_stride=2 * d, blocks=blocks)
+                    fastgl.aggregate_split(blk.indptr, blk.src, self.z[i], self.pad_dst[i + 1], x3[:, d:], 2 * d, blocks,
+                                           out=nxt[:, d:] if head else None, n_dst_dev=blk.n_dst_dev)
+                    x_split.add(i + 1)
+                else:
+                    fastgl.bias_relu_dropout_(self.z[i], layer.bias, p if training else 0.0, **drop, copy_out=nxt[:, :d])
+                    fastgl.aggregate(fastgl.AGG_MEAN, blk.indptr, blk.src, self.z[i], self.pad_dst[i + 1],
+                                     zero_deg_passthrough=False, out=nxt[:, d:], n_dst_dev=blk.n_dst_dev)
             else:
                 fastgl.bias_relu_dropout_(self.z[i], layer.bias, 0.0, relu=False)
+        if self.overlap:
+            main.wait_stream(zeroed)
         if fused_head:
             fastgl.linear_softmax_xent(self.cat[L - 1], last.weight, last.bias, self.labels, label_ids=self.seeds,
                                        n_valid=self.sizes[L - 1: L], loss=self.loss, dlogits=self.dlogits,
-                                       row_loss=self.row_loss, dbias=last.bias.grad)
+                                       row_loss=self.row_loss, dbias=last.bias.grad,
+                                       **(dict(split3=self.g3[L - 1], block_stride=self.mp[L - 1]) if split else {}))
         else:
             fastgl.softmax_xent(self.z[L - 1], self.labels, label_ids=self.seeds, n_valid=self.sizes[L - 1: L], loss=self.loss,
                                 dlogits=self.dlogits, row_loss=self.row_loss)
-        dz = self.dlogits
+        dz = None if split and fused_head else self.dlogits     # None: it was written in the operand form
         for i in reversed(range(L)):
             layer = self.layers[i]
             if i == L - 1 and not fused_head:
                 fastgl.relu_dropout_backward_(dz, masked=False, dbias=layer.bias.grad)
             if split:
-                if dz is not None:          # the output layer's gradient; the inner ones were written split already
+                if dz is not None:
                     self._split3(dz, self.g3[i], self.mp[i])
                 if i not in x_split:
                     self._split3(self.cat[i], self.x3[i])
             if self.overlap:
-                main = torch.cuda.current_stream()
                 self.side.wait_stream(main)            # the operands of this layer's weight gradient are ready
                 with torch.cuda.stream(self.side):
                     self._weight_grad(i, dz)
@@ -182,7 +205,7 @@ class SageStepProgram:
                 else:
                     torch.mm(dz, layer.weight.t(), out=self.dcat[i])
                 fastgl.aggregate_backward(fastgl.AGG_MEAN, blk.indptr, blk.src, self.dcat[i][:, d:], self.pad_dst[i - 1],
-                                          n_dst_dev=blk.n_dst_dev, d_self=self.dcat[i][:, :d], out=self.dh[i])
+                                          n_dst_dev=blk.n_dst_dev, d_self=self.dcat[i][:, :d], out=self.dh[i], accumulate=True)
                 if split:       # straight into the operand form of layer i - 1's two gradient products
                     fastgl.relu_dropout_backward_(self.dh[i], out=self.z[i - 1], p_drop=p if training else 0.0,
                                                   dbias=self.layers[i - 1].bias.grad, split3=self.g3[i - 1],

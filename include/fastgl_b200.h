@@ -50,7 +50,7 @@ extern "C" {
 
 /* flags of fgl_bias_relu_dropout / fgl_relu_dropout_bwd */
 #define FGL_EW_RELU 1     /* apply ReLU (forward) / the ReLU-and-dropout mask (backward) */
-#define FGL_EW_TWO_BLOCKS 2  /* fgl_relu_dropout_bwd_split: [hi | lo] alone, for a gradient that no further product reads */
+#define FGL_EW_TWO_BLOCKS 2  /* fgl_relu_dropout_bwd_split, fgl_bias_relu_dropout_split: [hi | lo] alone, where no product reads the third */
 
 #define FGL_MAX_HOPS 7
 #define FGL_COUNTS_STRIDE 16 /* per mini-batch: [0..7] node counts n_0..n_L, [8..15] edge counts per hop */
@@ -263,6 +263,13 @@ int fgl_agg_fwd(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int32_t* 
                 int64_t ldx, int32_t dim, int32_t n_dst, int32_t flags, float* out, int64_t ldo,
                 const int32_t* n_dst_dev, void* stream);
 
+/* fgl_agg_fwd with FGL_AGG_MEAN whose result is (also) written as error-compensated TF32 operands (see fgl_split_tf32):
+ * split[d, c] = hi, split[d, split_stride + c] = lo and, with blocks = 3, split[d, 2 * split_stride + c] = hi.  out may be
+ * NULL.  Rows of whole 16-byte vectors only (FGL_ERR_INVALID otherwise).  A row without in-edges is zero. */
+int fgl_agg_fwd_split(fgl_ws* ws, const int32_t* indptr, const int32_t* src, const float* x, int64_t n_rows, int64_t ldx,
+                      int32_t dim, int32_t n_dst, float* out, int64_t ldo, float* split, int64_t ld_split,
+                      int64_t split_stride, int32_t blocks, const int32_t* n_dst_dev, void* stream);
+
 /* fgl_agg_fwd over a feature table that is row-sharded across GPUs: shards (device array of n pointers, each a
  * table of the same leading dimension, mapped into this GPU's address space -- its own HBM or a peer's over
  * NVLink) replaces x (x may then be NULL); global row r is shards[r / rows_per_shard][r % rows_per_shard].
@@ -362,6 +369,13 @@ int fgl_agg_bwd_self(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int3
                      int32_t dim, int32_t n_dst, int32_t n_src, float* dx, int64_t ldx, const int32_t* n_dst_dev,
                      void* stream);
 
+/* fgl_agg_bwd, and with dy_self != NULL fgl_agg_bwd_self, into a dx that holds what is added to: nothing is initialised, and
+ * dy_self[d] is added to dx[d] like one more edge.  For a caller that can zero dx off the critical path. */
+int fgl_agg_bwd_add(fgl_ws* ws, int32_t mode, const int32_t* indptr, const int32_t* src, const int32_t* src_deg,
+                    const int32_t* dst_deg, const float* dy, int64_t ldy, const float* dy_self, int64_t ld_self,
+                    int32_t dim, int32_t n_dst, int32_t n_src, float* dx, int64_t ldx, const int32_t* n_dst_dev,
+                    void* stream);
+
 /* Aggregation backward as a gather, deterministic: the same result as fgl_agg_bwd / fgl_agg_bwd_self (the scatters
  * K9 / K11 of the reference, aggregate_acc_kernel.cu:468-517, :555-596, which add with atomics in arbitrary order), but
  * every row dx[s] is produced by one warp -- or, for a source with more than 128 edges in the block, one CTA per tile -- that
@@ -396,6 +410,14 @@ int fgl_bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, con
                           uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
                           int64_t ld_copy, int64_t n_copy_rows, void* stream);
 
+/* fgl_bias_relu_dropout that also writes the first n_copy_rows result rows as error-compensated TF32 operands (see
+ * fgl_split_tf32), [hi | lo | hi] split_stride columns apart (with FGL_EW_TWO_BLOCKS [hi | lo]).  copy_out may be NULL.
+ * Rows of whole 16-byte vectors only (FGL_ERR_INVALID otherwise). */
+int fgl_bias_relu_dropout_split(float* y, int64_t ld, int64_t n_rows, int32_t dim, const float* bias, float p_drop,
+                                uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
+                                int64_t ld_copy, int64_t n_copy_rows, float* split, int64_t ld_split, int64_t split_stride,
+                                void* stream);
+
 /* Backward of fgl_bias_relu_dropout: with FGL_EW_RELU, dy[r, c] becomes dy[r, c] / (1 - p_drop) where the
  * forward output out[r, c] is positive and 0 elsewhere (an element is positive exactly when it passed both the
  * ReLU and the dropout); without the flag dy is left as it is.  dbias (may be NULL; dim <= 2048) is incremented
@@ -429,6 +451,14 @@ int fgl_linear_softmax_xent(fgl_ws* ws, const float* x, int64_t ldx, int32_t k, 
                             const int64_t* labels, const int32_t* label_ids, int64_t n_labels, int32_t n_rows,
                             int32_t n_classes, const int32_t* n_valid_dev, int32_t n_valid, float* loss, float* dlogits,
                             int64_t ldd, float* dbias, float* logits_out, int64_t ldl, float* row_loss, void* stream);
+
+/* fgl_linear_softmax_xent that also writes dlogits as error-compensated TF32 operands (see fgl_split_tf32), [hi | lo | hi]
+ * split_stride columns apart. */
+int fgl_linear_softmax_xent_split(fgl_ws* ws, const float* x, int64_t ldx, int32_t k, const float* w, int64_t ldw, const float* bias,
+                                  const int64_t* labels, const int32_t* label_ids, int64_t n_labels, int32_t n_rows,
+                                  int32_t n_classes, const int32_t* n_valid_dev, int32_t n_valid, float* loss, float* dlogits,
+                                  int64_t ldd, float* dbias, float* row_loss, float* split, int64_t ld_split,
+                                  int64_t split_stride, void* stream);
 
 /* One Adam step with L2 weight decay over flat fp32 buffers of n elements (16-byte aligned), with the arithmetic
  * of torch.optim.Adam: g += wd * p; m = b1 m + (1 - b1) g; v = b2 v + (1 - b2) g^2;
