@@ -198,6 +198,7 @@ __device__ __forceinline__ void put_out(const AggParams& p, int64_t row, int c, 
 
 template <int VEC, int MODE, bool HAS_MAP, int NACC, int UNR, bool SPLIT = false>
 __global__ void __launch_bounds__(kAggThreads, FGL_AGG_MIN_CTAS) agg_fwd_kernel(const AggParams p) {
+    if (!after_the_kernels_before()) return;
     using V = Vec<VEC>;
     using T = typename V::T;
     __shared__ long long s_off[kAggMaxWindow + 1];
@@ -467,6 +468,7 @@ __device__ __forceinline__ float4 lds128(unsigned smem_src) {
 
 template <int MODE, bool HAS_MAP>
 __global__ void __launch_bounds__(kAggStagedMaxWarps * 32, 1) agg_fwd_staged_kernel(const AggParams p) {
+    if (!after_the_kernels_before()) return;
     using V = Vec<4>;
     using T = float4;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -658,6 +660,7 @@ __global__ void __launch_bounds__(kAggStagedMaxWarps * 32, 1) agg_fwd_staged_ker
 // Replaces the CPU index_select + host-to-device copy of load_subtensors (train_fastgl.py:161-184).
 template <int VEC>
 __global__ void __launch_bounds__(kAggThreads) gather_rows_kernel(const AggParams p, const int32_t* __restrict__ ids, int64_t n_ids) {
+    if (!after_the_kernels_before()) return;
     using T = typename Vec<VEC>::T;
     const int lane = threadIdx.x & 31;
     const int64_t warp_global = (int64_t)blockIdx.x * kAggWarps + (threadIdx.x >> 5);
@@ -693,6 +696,7 @@ __device__ __forceinline__ void red_add(float* addr, const float& v) { atomicAdd
 // Backward: dx[src[e],:] += w_e * scale_d * dy[d,:]; vector reductions (red.global.add.v4.f32 on sm_100a)
 template <int VEC, int MODE, int NACC>
 __global__ void __launch_bounds__(kAggThreads) agg_bwd_kernel(const AggParams p) {
+    if (!after_the_kernels_before()) return;
     using V = Vec<VEC>;
     using T = typename V::T;
     const int lane = threadIdx.x & 31;
@@ -760,6 +764,7 @@ __global__ void __launch_bounds__(kAggThreads) agg_bwd_kernel(const AggParams p)
 // multiply their vectors, reduce within runs of lanes that share a head, and the first lane of each run adds.
 template <int VEC>
 __global__ void __launch_bounds__(kAggThreads) agg_edge_wgrad_kernel(const AggParams p, float* __restrict__ dw) {
+    if (!after_the_kernels_before()) return;
     using T = typename Vec<VEC>::T;
     const int lane = threadIdx.x & 31;
     const int warp_global = blockIdx.x * kAggWarps + (threadIdx.x >> 5);
@@ -843,9 +848,9 @@ static int agg_grid_x(int n_rows, int n_batches) {
 template <int VEC, int MODE, int NACC, int UNR>
 static void launch_fwd(const AggParams& p, dim3 grid, cudaStream_t st) {
     if (p.row_map)
-        agg_fwd_kernel<VEC, MODE, true, NACC, UNR><<<grid, kAggThreads, 0, st>>>(p);
+        launch(agg_fwd_kernel<VEC, MODE, true, NACC, UNR>, grid, kAggThreads, 0, st, p);
     else
-        agg_fwd_kernel<VEC, MODE, false, NACC, UNR><<<grid, kAggThreads, 0, st>>>(p);
+        launch(agg_fwd_kernel<VEC, MODE, false, NACC, UNR>, grid, kAggThreads, 0, st, p);
 }
 
 // Whether agg_fwd_staged_kernel applies: 128-bit rows of at most 32 vectors in a single dense table.
@@ -878,10 +883,10 @@ static void launch_fwd_staged(const AggParams& p, cudaStream_t st) {
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sms, (rows + warps - 1) / warps));
     if (p.row_map) {
         allow_shared<agg_fwd_staged_kernel<MODE, true>>((int)kRoom);
-        agg_fwd_staged_kernel<MODE, true><<<grid, warps * 32, dyn, st>>>(p);
+        launch(agg_fwd_staged_kernel<MODE, true>, grid, warps * 32, dyn, st, p);
     } else {
         allow_shared<agg_fwd_staged_kernel<MODE, false>>((int)kRoom);
-        agg_fwd_staged_kernel<MODE, false><<<grid, warps * 32, dyn, st>>>(p);
+        launch(agg_fwd_staged_kernel<MODE, false>, grid, warps * 32, dyn, st, p);
     }
 }
 
@@ -931,11 +936,11 @@ template <int VEC, int MODE>
 static void launch_bwd_nacc(const AggParams& p, int grid, cudaStream_t st) {
     const int chunks = p.dim / VEC;
     if (chunks <= 32)
-        agg_bwd_kernel<VEC, MODE, 1><<<grid, kAggThreads, 0, st>>>(p);
+        launch(agg_bwd_kernel<VEC, MODE, 1>, grid, kAggThreads, 0, st, p);
     else if (chunks <= 64)
-        agg_bwd_kernel<VEC, MODE, 2><<<grid, kAggThreads, 0, st>>>(p);
+        launch(agg_bwd_kernel<VEC, MODE, 2>, grid, kAggThreads, 0, st, p);
     else
-        agg_bwd_kernel<VEC, MODE, 4><<<grid, kAggThreads, 0, st>>>(p);
+        launch(agg_bwd_kernel<VEC, MODE, 4>, grid, kAggThreads, 0, st, p);
 }
 
 template <int VEC>
@@ -952,6 +957,7 @@ static void launch_bwd_mode(int mode, const AggParams& p, int grid, cudaStream_t
 __global__ void __launch_bounds__(256)
 init_self_rows_kernel(float* __restrict__ dx, int64_t ldx, const float* __restrict__ dy_self, int64_t ld_self, int dim,
                       int n_dst, int n_src, const int32_t* __restrict__ n_dst_dev) {
+    if (!after_the_kernels_before()) return;
     if (n_dst_dev) n_dst = min(max(__ldg(n_dst_dev), 0), n_dst);  // padded launch: rows at or beyond the real count are zero
     const int groups = (dim + 3) / 4;
     const int64_t total = (int64_t)n_src * groups;
@@ -1161,9 +1167,9 @@ int fgl_agg_edge_wgrad(fgl_ws* ws, const int32_t* indptr, const int32_t* src, in
     while (vec > 1 && (dim / n_heads) % vec != 0) vec /= 2;
     const int grid = agg_grid_x(n_dst, 1);
     switch (vec) {
-        case 4: agg_edge_wgrad_kernel<4><<<grid, kAggThreads, 0, st>>>(p, dw); break;
-        case 2: agg_edge_wgrad_kernel<2><<<grid, kAggThreads, 0, st>>>(p, dw); break;
-        default: agg_edge_wgrad_kernel<1><<<grid, kAggThreads, 0, st>>>(p, dw); break;
+        case 4: launch(agg_edge_wgrad_kernel<4>, grid, kAggThreads, 0, st, p, dw); break;
+        case 2: launch(agg_edge_wgrad_kernel<2>, grid, kAggThreads, 0, st, p, dw); break;
+        default: launch(agg_edge_wgrad_kernel<1>, grid, kAggThreads, 0, st, p, dw); break;
     }
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
@@ -1189,9 +1195,9 @@ int fgl_gather_rows(fgl_ws* ws, const float* table, const float* const* shards, 
     const int grid = agg_grid_x((int)std::min<int64_t>((n_ids + 3) / 4, 0x7fffffff), 1);
     cudaStream_t st = (cudaStream_t)stream;
     switch (vec) {
-        case 4: gather_rows_kernel<4><<<grid, kAggThreads, 0, st>>>(p, ids, n_ids); break;
-        case 2: gather_rows_kernel<2><<<grid, kAggThreads, 0, st>>>(p, ids, n_ids); break;
-        default: gather_rows_kernel<1><<<grid, kAggThreads, 0, st>>>(p, ids, n_ids); break;
+        case 4: launch(gather_rows_kernel<4>, grid, kAggThreads, 0, st, p, ids, n_ids); break;
+        case 2: launch(gather_rows_kernel<2>, grid, kAggThreads, 0, st, p, ids, n_ids); break;
+        default: launch(gather_rows_kernel<1>, grid, kAggThreads, 0, st, p, ids, n_ids); break;
     }
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
@@ -1211,7 +1217,7 @@ static int agg_bwd_impl(fgl_ws* ws, int32_t mode, const int32_t* indptr, const i
     } else if (dy_self && n_dst > 0) {
         const int64_t items = (int64_t)n_src * ((dim + 3) / 4);
         const int grid = (int)std::min<int64_t>((items + 255) / 256, 148 * 16);
-        init_self_rows_kernel<<<grid, 256, 0, st>>>(dx, ldx, dy_self, ld_self, dim, n_dst, n_src, n_dst_dev);
+        launch(init_self_rows_kernel, grid, 256, 0, st, dx, ldx, dy_self, ld_self, dim, n_dst, n_src, n_dst_dev);
     } else if (zero_rows(dx, ldx, dim, n_src, st) != cudaSuccess) {
         return FGL_ERR_CUDA;
     }
@@ -1292,9 +1298,9 @@ int fgl_agg_fwd_split(fgl_ws* ws, const int32_t* indptr, const int32_t* src, con
     p.split_blocks = blocks;
     const int grid = agg_grid_x(n_dst, 1);
     cudaStream_t st = (cudaStream_t)stream;
-    if (dim <= 128) agg_fwd_kernel<4, FGL_AGG_MEAN, false, 1, FGL_AGG_UNR1, true><<<grid, kAggThreads, 0, st>>>(p);
-    else if (dim <= 256) agg_fwd_kernel<4, FGL_AGG_MEAN, false, 2, 4, true><<<grid, kAggThreads, 0, st>>>(p);
-    else agg_fwd_kernel<4, FGL_AGG_MEAN, false, 4, 2, true><<<grid, kAggThreads, 0, st>>>(p);
+    if (dim <= 128) launch(agg_fwd_kernel<4, FGL_AGG_MEAN, false, 1, FGL_AGG_UNR1, true>, grid, kAggThreads, 0, st, p);
+    else if (dim <= 256) launch(agg_fwd_kernel<4, FGL_AGG_MEAN, false, 2, 4, true>, grid, kAggThreads, 0, st, p);
+    else launch(agg_fwd_kernel<4, FGL_AGG_MEAN, false, 4, 2, true>, grid, kAggThreads, 0, st, p);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 

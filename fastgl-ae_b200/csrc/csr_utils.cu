@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(1024) cal_deg_small_kernel(const int32_t* __re
 __global__ void __launch_bounds__(256) block_degrees_kernel(const int32_t* __restrict__ indptr, const int32_t* __restrict__ src,
                                                             int n_dst, int n_src, int64_t n_edges, int32_t* __restrict__ dst_deg,
                                                             int32_t* __restrict__ src_deg) {
+    if (!after_the_kernels_before()) return;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (int64_t i = first; i < n_dst; i += stride) dst_deg[i] = __ldg(indptr + i + 1) - __ldg(indptr + i);
     for (int64_t e = first; e < n_edges; e += stride) {
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(256) block_degrees_kernel(const int32_t* __res
 template <typename T>
 __global__ void __launch_bounds__(256) mask_rows_kernel(const int32_t* __restrict__ indptr, int n_dst, int dim, const float* __restrict__ x,
                                                         int64_t ldx, float* __restrict__ y, int64_t ldy) {
+    if (!after_the_kernels_before()) return;
     constexpr int VEC = sizeof(T) / 4;
     const int lane = threadIdx.x & 31;
     for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < n_dst; r += gridDim.x * 8) {
@@ -173,6 +175,7 @@ constexpr int kStageThreads = 256;
 constexpr int64_t kStageBytesPerBlock = kStageThreads * 16 * 2;
 
 __global__ void __launch_bounds__(kStageThreads) stage_segments_kernel(const __grid_constant__ StageParams p) {
+    if (!after_the_kernels_before()) return;
     if (blockIdx.x == 0 && threadIdx.x < p.n_words) p.words_dst[threadIdx.x] = p.words[threadIdx.x];
     int s = 0;
     while (s + 1 < p.n_segs && (int64_t)blockIdx.x >= p.first_block[s + 1]) ++s;
@@ -332,7 +335,7 @@ int fgl_block_degrees(const int32_t* indptr, const int32_t* src, int32_t n_dst, 
     if (n_src > 0 && cudaMemsetAsync(src_deg, 0, sizeof(int32_t) * (size_t)n_src, st) != cudaSuccess) return FGL_ERR_CUDA;
     const int64_t items = std::max<int64_t>(n_dst, n_edges);
     if (items == 0) return FGL_OK;
-    block_degrees_kernel<<<(int)std::min<int64_t>((items + 255) / 256, 148 * 8), 256, 0, st>>>(indptr, src, n_dst, n_src, n_edges, dst_deg, src_deg);
+    launch(block_degrees_kernel, (int)std::min<int64_t>((items + 255) / 256, 148 * 8), 256, 0, st, indptr, src, n_dst, n_src, n_edges, dst_deg, src_deg);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
@@ -341,8 +344,8 @@ int fgl_mask_rows(const int32_t* indptr, int32_t n_dst, int32_t dim, const float
     if (n_dst == 0) return FGL_OK;
     const int grid = (int)std::min<int64_t>(((int64_t)n_dst + 7) / 8, 148 * 8);
     const bool vec = dim % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
-    if (vec) mask_rows_kernel<float4><<<grid, 256, 0, (cudaStream_t)stream>>>(indptr, n_dst, dim, x, ldx, y, ldy);
-    else mask_rows_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>(indptr, n_dst, dim, x, ldx, y, ldy);
+    if (vec) launch(mask_rows_kernel<float4>, grid, 256, 0, (cudaStream_t)stream, indptr, n_dst, dim, x, ldx, y, ldy);
+    else launch(mask_rows_kernel<float>, grid, 256, 0, (cudaStream_t)stream, indptr, n_dst, dim, x, ldx, y, ldy);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
@@ -369,7 +372,7 @@ int fgl_stage_segments(const fgl_segment* segs, int32_t n_segs, int32_t* words_d
     p.n_words = n_words;
     if (blocks == 0) blocks = 1;
     if (blocks > 0x7fffffffLL) return FGL_ERR_INVALID;
-    stage_segments_kernel<<<(unsigned)blocks, kStageThreads, 0, (cudaStream_t)stream>>>(p);
+    launch(stage_segments_kernel, (unsigned)blocks, kStageThreads, 0, (cudaStream_t)stream, p);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 

@@ -49,6 +49,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // el[n, h] = <feat[n, h], attn_l[h]> for every source, er likewise for the destinations (the first n_dst sources): a warp
 // per node and head.
 __global__ void __launch_bounds__(kGatThreads) gat_scores_kernel(const GatParams p) {
+    if (!after_the_kernels_before()) return;
     const int lane = threadIdx.x & 31;
     const int64_t n_warps = (int64_t)gridDim.x * kGatWarps;
     for (int64_t u = (int64_t)blockIdx.x * kGatWarps + (threadIdx.x >> 5); u < (int64_t)p.n_src * p.heads; u += n_warps) {
@@ -114,6 +115,7 @@ __device__ __forceinline__ void vfma(typename GVec<VEC>::T& a, float w, const ty
 // A warp per destination row.  An edge whose source is out of range gets the coefficient zero and is reported.
 template <int VEC>
 __global__ void __launch_bounds__(kGatThreads) gat_fwd_kernel(const GatParams p) {
+    if (!after_the_kernels_before()) return;
     using T = typename GVec<VEC>::T;
     const int lane = threadIdx.x & 31;
     const int n_warps = gridDim.x * kGatWarps;
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(kGatThreads) gat_fwd_kernel(const GatParams p)
 // up in shared memory and leaves one row of `partial`.
 template <int VEC>
 __global__ void __launch_bounds__(kGatThreads) gat_bwd_kernel(const GatParams p) {
+    if (!after_the_kernels_before()) return;
     using T = typename GVec<VEC>::T;
     extern __shared__ float cols[];  // [2 * dim]: attn_l's columns, then attn_r's
     const int lane = threadIdx.x & 31;
@@ -312,6 +315,7 @@ __global__ void __launch_bounds__(kGatThreads) gat_bwd_kernel(const GatParams p)
 
 // Column sums of [n_rows][n_cols]: a CTA per 32 columns, its warps take every eighth row each.
 __global__ void __launch_bounds__(kGatThreads) column_sums_kernel(const float* __restrict__ x, int n_rows, int n_cols, float* __restrict__ out) {
+    if (!after_the_kernels_before()) return;
     __shared__ float part[kGatWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + lane;
@@ -372,12 +376,12 @@ int fgl_gat_fwd(fgl_ws* ws, const int32_t* indptr, const int32_t* src, const flo
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t cap = (int64_t)ws->sm_count * 8;
     const int score_grid = (int)std::min<int64_t>(((int64_t)n_src * heads + kGatWarps - 1) / kGatWarps, cap);
-    gat_scores_kernel<<<score_grid, kGatThreads, 0, st>>>(p);
+    launch(gat_scores_kernel, score_grid, kGatThreads, 0, st, p);
     const int grid = (int)std::min<int64_t>(((int64_t)n_dst + kGatWarps - 1) / kGatWarps, cap);
     if (vec4_rows(p.dim, width, feat, ldf, out, ldo, nullptr, nullptr))
-        gat_fwd_kernel<4><<<grid, kGatThreads, 0, st>>>(p);
+        launch(gat_fwd_kernel<4>, grid, kGatThreads, 0, st, p);
     else
-        gat_fwd_kernel<1><<<grid, kGatThreads, 0, st>>>(p);
+        launch(gat_fwd_kernel<1>, grid, kGatThreads, 0, st, p);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
@@ -425,8 +429,8 @@ int fgl_gat_bwd(fgl_ws* ws, const int32_t* indptr, const int32_t* src, const flo
     const bool vec = vec4_rows(p.dim, width, feat, ldf, dy, ldy, attn_l, attn_r) && ((uintptr_t)dfeat & 15) == 0;
     void (*kernel)(const GatParams) = vec ? gat_bwd_kernel<4> : gat_bwd_kernel<1>;
     if (dyn > 48 * 1024) FGL_CUDA_OK(ws, cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    kernel<<<grid, kGatThreads, dyn, st>>>(p);
-    column_sums_kernel<<<(2 * p.dim + 31) / 32, kGatThreads, 0, st>>>(p.partial, grid, 2 * p.dim, dattn);
+    launch(kernel, grid, kGatThreads, dyn, st, p);
+    launch(column_sums_kernel, (2 * p.dim + 31) / 32, kGatThreads, 0, st, p.partial, grid, 2 * p.dim, dattn);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 

@@ -80,6 +80,7 @@ struct Slab {
 
 template <int BM, int BN, int TN, bool VA, bool VB>
 __global__ void __launch_bounds__(BM / 8 * (BN / TN)) gemm_kernel(const GemmParams p) {
+    if (!after_the_kernels_before()) return;
     constexpr int kThreads = BM / 8 * (BN / TN);
     constexpr int kCols = BN / TN;  // threads side by side
     __shared__ __align__(16) float sa[2][kBK][BM + 4];
@@ -155,6 +156,7 @@ constexpr int kFoldThreads = 256;
 template <int VEC>
 __global__ void __launch_bounds__(kFoldThreads) gemm_fold_kernel(const float* __restrict__ part, int slices, int64_t slice_stride, int m, int n,
                                                                  float* __restrict__ c, int64_t ldc) {
+    if (!after_the_kernels_before()) return;
     __shared__ float s[kFoldThreads / 32][32 * VEC];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t at = ((int64_t)blockIdx.x * 32 + lane) * VEC, total = (int64_t)m * n;
@@ -218,10 +220,10 @@ static GemmPlan plan_gemm(int sms, int m, int n, int k) {
 template <int BM, int BN, int TN>
 static void launch_gemm(const GemmParams& p, dim3 grid, bool va, bool vb, cudaStream_t st) {
     constexpr int threads = BM / 8 * (BN / TN);
-    if (va && vb) gemm_kernel<BM, BN, TN, true, true><<<grid, threads, 0, st>>>(p);
-    else if (va) gemm_kernel<BM, BN, TN, true, false><<<grid, threads, 0, st>>>(p);
-    else if (vb) gemm_kernel<BM, BN, TN, false, true><<<grid, threads, 0, st>>>(p);
-    else gemm_kernel<BM, BN, TN, false, false><<<grid, threads, 0, st>>>(p);
+    if (va && vb) launch(gemm_kernel<BM, BN, TN, true, true>, grid, threads, 0, st, p);
+    else if (va) launch(gemm_kernel<BM, BN, TN, true, false>, grid, threads, 0, st, p);
+    else if (vb) launch(gemm_kernel<BM, BN, TN, false, true>, grid, threads, 0, st, p);
+    else launch(gemm_kernel<BM, BN, TN, false, false>, grid, threads, 0, st, p);
 }
 
 static void launch_gemm_tile(const GemmPlan& g, const GemmParams& p, dim3 grid, bool va, bool vb, cudaStream_t st) {
@@ -250,9 +252,9 @@ static void gemm_with(const GemmPlan& g, const float* a, int64_t lda, const floa
     if (split) {
         const int64_t mn = (int64_t)m * n;
         if (mn % 4 == 0 && ((uintptr_t)scratch & 15) == 0)
-            gemm_fold_kernel<4><<<(unsigned)((mn / 4 + 31) / 32), kFoldThreads, 0, st>>>(scratch, g.slices, p.slice_stride, m, n, c, ldc);
+            launch(gemm_fold_kernel<4>, (unsigned)((mn / 4 + 31) / 32), kFoldThreads, 0, st, scratch, g.slices, p.slice_stride, m, n, c, ldc);
         else
-            gemm_fold_kernel<1><<<(unsigned)((mn + 31) / 32), kFoldThreads, 0, st>>>(scratch, g.slices, p.slice_stride, m, n, c, ldc);
+            launch(gemm_fold_kernel<1>, (unsigned)((mn + 31) / 32), kFoldThreads, 0, st, scratch, g.slices, p.slice_stride, m, n, c, ldc);
     }
 }
 

@@ -31,6 +31,7 @@ bias_relu_dropout_kernel(float* __restrict__ y, int64_t ld, int64_t n_rows, int 
                          const int32_t* __restrict__ rng_ctr_dev, int flags, float* __restrict__ copy_out,
                          int64_t ld_copy, int64_t n_copy_rows, float* __restrict__ split, int64_t ld_split,
                          int64_t split_stride) {
+    if (!after_the_kernels_before()) return;
     const int64_t groups_per_row = dim / VEC;
     const int64_t total = n_rows * groups_per_row;
     const uint64_t ctr = rng_ctr + (rng_ctr_dev ? (uint64_t)(uint32_t)rng_ctr_dev[0] : 0ull);
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(kEwThreads)
 relu_dropout_bwd_kernel(float* __restrict__ dy, int64_t ldy, const float* __restrict__ out, int64_t ldo, int64_t n_rows,
                         int rows_per_cta, int dim, float keep_scale, float* __restrict__ dbias, int flags,
                         float* __restrict__ split3, int64_t ld3, int block_stride) {
+    if (!after_the_kernels_before()) return;
     const int64_t r0 = (int64_t)blockIdx.x * rows_per_cta;
     const int64_t r1 = r0 + rows_per_cta < n_rows ? r0 + rows_per_cta : n_rows;
     const bool mask = flags & FGL_EW_RELU;
@@ -141,6 +143,7 @@ __global__ void __launch_bounds__(kEwThreads)
 relu_dropout_bwd_vec_kernel(float* __restrict__ dy, int64_t ldy, const float* __restrict__ out, int64_t ldo, int64_t n_rows,
                             int rows_per_cta, int dim, float keep_scale, float* __restrict__ dbias, int flags,
                             float* __restrict__ split3, int64_t ld3, int block_stride) {
+    if (!after_the_kernels_before()) return;
     __shared__ float4 sums[kEwThreads];
     const int groups = dim >> 2;                       // column groups of four floats; <= 256
     const int lanes = kEwThreads / groups;             // rows covered per pass
@@ -246,6 +249,7 @@ softmax_xent_rows_kernel(const float* __restrict__ logits, int64_t ld, const int
                          const int32_t* __restrict__ n_valid_dev, int n_valid_host, float* __restrict__ row_loss,
                          float* __restrict__ dlogits, int64_t ldd, int32_t* __restrict__ status, float* __restrict__ loss,
                          unsigned int* __restrict__ ticket) {
+    if (!after_the_kernels_before()) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r = blockIdx.x * kXentWarps + warp;
     int n_valid = n_valid_dev ? n_valid_dev[0] : n_valid_host;
@@ -302,6 +306,7 @@ linear_xent_kernel(const float* __restrict__ x, int64_t ldx, int k, const float*
                    float* __restrict__ row_loss, float* __restrict__ dlogits, int64_t ldd, float* __restrict__ dbias,
                    float* __restrict__ logits_out, int64_t ldl, int32_t* __restrict__ status, float* __restrict__ loss,
                    unsigned int* __restrict__ ticket, float* __restrict__ split, int64_t ld_split, int64_t split_stride) {
+    if (!after_the_kernels_before()) return;
     __shared__ float part[kLinXentWarps][kLinXentRows][32 * CPL];
     __shared__ float db[32 * CPL];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -448,6 +453,7 @@ linear_xent_kernel(const float* __restrict__ x, int64_t ldx, int k, const float*
 __global__ void __launch_bounds__(kEwThreads)
 adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, int64_t n,
             float lr, float b1, float b2, float eps, float wd, int32_t* __restrict__ step, unsigned int* __restrict__ ticket) {
+    if (!after_the_kernels_before()) return;
     // the first elements are on their way while the coefficients (two powers) are computed
     const int64_t first = ((int64_t)blockIdx.x * kEwThreads + threadIdx.x) * 4;
     float4 pp{}, gg{}, mm{}, vv{};
@@ -532,6 +538,7 @@ __device__ __forceinline__ void split_elements(const float* __restrict__ x, int6
 template <bool VEC4>
 __global__ void __launch_bounds__(kEwThreads)
 split_tf32_kernel(const float* __restrict__ x, int64_t rows, int cols, int64_t ldx, const SplitDst d) {
+    if (!after_the_kernels_before()) return;
     split_elements<VEC4>(x, rows, cols, ldx, d, (int64_t)blockIdx.x * kEwThreads + threadIdx.x, (int64_t)gridDim.x * kEwThreads);
 }
 
@@ -546,6 +553,7 @@ struct SplitMany {
 };
 
 __global__ void __launch_bounds__(kEwThreads) split_tf32_many_kernel(const __grid_constant__ SplitMany m) {
+    if (!after_the_kernels_before()) return;
     const int j = blockIdx.y;
     const int64_t first = (int64_t)blockIdx.x * kEwThreads + threadIdx.x, stride = (int64_t)gridDim.x * kEwThreads;
     if (m.vec[j]) split_elements<true>(m.x[j], m.rows[j], m.cols[j], m.ldx[j], m.dst[j], first, stride);
@@ -562,6 +570,7 @@ template <int VEC>
 __global__ void __launch_bounds__(kFoldWarps * 32)
 fold_blocks_kernel(const float* __restrict__ part, int n_slabs, int n_a, int n_b, int rows, int cols, int block_stride,
                    int64_t ld_part, int64_t slab_stride, float* __restrict__ out, int64_t ldo) {
+    if (!after_the_kernels_before()) return;
     using T = typename std::conditional<VEC == 4, float4, float>::type;
     __shared__ __align__(16) float partial[kFoldWarps][32 * VEC];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -645,11 +654,11 @@ static int bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, 
     // whole 16-byte vectors alone: a caller with other rows splits them in a pass of its own
     if (split && !(vec && ld_split % 4 == 0 && split_stride % 4 == 0 && aligned16(split))) return FGL_ERR_INVALID;
     if (vec)
-        bias_relu_dropout_kernel<4><<<ew_grid(n_rows * (dim / 4)), kEwThreads, 0, st>>>(
+        launch(bias_relu_dropout_kernel<4>, ew_grid(n_rows * (dim / 4)), kEwThreads, 0, st, 
             y, ld, n_rows, dim, bias, drop_below, keep_scale, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
             n_copy_rows, split, ld_split, split_stride);
     else
-        bias_relu_dropout_kernel<1><<<ew_grid(n_rows * dim), kEwThreads, 0, st>>>(
+        launch(bias_relu_dropout_kernel<1>, ew_grid(n_rows * dim), kEwThreads, 0, st, 
             y, ld, n_rows, dim, bias, drop_below, keep_scale, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
             n_copy_rows, nullptr, 0, 0);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
@@ -697,18 +706,18 @@ static int relu_dropout_bwd_launch(float* dy, int64_t ldy, const float* out, int
         int64_t nb = (n_rows + band - 1) / band;
         nb = nb < 4 * 148 ? nb : 4 * 148;   // four CTAs per SM, each walking its share of the bands
         if (split3)
-            relu_dropout_bwd_vec_kernel<true><<<(unsigned)nb, kEwThreads, 0, (cudaStream_t)stream>>>(
+            launch(relu_dropout_bwd_vec_kernel<true>, (unsigned)nb, kEwThreads, 0, (cudaStream_t)stream, 
                 dy, ldy, out, ldo, n_rows, (int)band, dim, keep, dbias, flags, split3, ld3, (int)block_stride);
         else
-            relu_dropout_bwd_vec_kernel<false><<<(unsigned)nb, kEwThreads, 0, (cudaStream_t)stream>>>(
+            launch(relu_dropout_bwd_vec_kernel<false>, (unsigned)nb, kEwThreads, 0, (cudaStream_t)stream, 
                 dy, ldy, out, ldo, n_rows, (int)band, dim, keep, dbias, flags, nullptr, 0, 0);
         return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
     }
     if (split3)
-        relu_dropout_bwd_kernel<true><<<(unsigned)blocks, kEwThreads, 0, (cudaStream_t)stream>>>(
+        launch(relu_dropout_bwd_kernel<true>, (unsigned)blocks, kEwThreads, 0, (cudaStream_t)stream, 
             dy, ldy, out, ldo, n_rows, (int)rows_per_cta, dim, keep, dbias, flags, split3, ld3, (int)block_stride);
     else
-        relu_dropout_bwd_kernel<false><<<(unsigned)blocks, kEwThreads, 0, (cudaStream_t)stream>>>(
+        launch(relu_dropout_bwd_kernel<false>, (unsigned)blocks, kEwThreads, 0, (cudaStream_t)stream, 
             dy, ldy, out, ldo, n_rows, (int)rows_per_cta, dim, keep, dbias, flags, nullptr, 0, 0);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
@@ -736,7 +745,7 @@ int fgl_softmax_xent(fgl_ws* ws, const float* logits, int64_t ld, const int64_t*
         return cudaMemsetAsync(loss, 0, sizeof(float), (cudaStream_t)stream) == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    softmax_xent_rows_kernel<<<(n_rows + kXentWarps - 1) / kXentWarps, kXentWarps * 32, 0, st>>>(
+    launch(softmax_xent_rows_kernel, (n_rows + kXentWarps - 1) / kXentWarps, kXentWarps * 32, 0, st, 
         logits, ld, labels, label_ids, n_labels, n_rows, n_classes, n_valid_dev, n_valid, row_loss, dlogits, ldd, ws->status,
         loss, loss_ticket(ws));
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
@@ -755,7 +764,7 @@ static int linear_xent(fgl_ws* ws, const float* x, int64_t ldx, int32_t k, const
     if (n_rows == 0) return cudaMemsetAsync(loss, 0, sizeof(float), st) == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
     const int grid = (n_rows + kLinXentRows - 1) / kLinXentRows;
 #define FGL_LINXENT(CPL)                                                                                              \
-    linear_xent_kernel<CPL><<<grid, kLinXentWarps * 32, 0, st>>>(x, ldx, k, w, ldw, bias, labels, label_ids, n_labels, \
+    launch(linear_xent_kernel<CPL>, grid, kLinXentWarps * 32, 0, st, x, ldx, k, w, ldw, bias, labels, label_ids, n_labels, \
                                                                  n_rows, n_classes, n_valid_dev, n_valid, row_loss,   \
                                                                  dlogits, ldd, dbias, logits_out, ldl, ws->status, loss, loss_ticket(ws), \
                                                                  split, ld_split, split_stride)
@@ -790,7 +799,7 @@ int fgl_adam_step(float* param, const float* grad, float* exp_avg, float* exp_av
     if (n == 0) return FGL_OK;
     if (!aligned16(param) || !aligned16(grad) || !aligned16(exp_avg) || !aligned16(exp_avg_sq)) return FGL_ERR_INVALID;
     // step_dev[0] = completed steps, step_dev[1] = the kernel's arrival ticket (zero between launches)
-    adam_kernel<<<ew_grid((n + 3) / 4), kEwThreads, 0, (cudaStream_t)stream>>>(
+    launch(adam_kernel, ew_grid((n + 3) / 4), kEwThreads, 0, (cudaStream_t)stream, 
         param, grad, exp_avg, exp_avg_sq, n, lr, beta1, beta2, eps, weight_decay, step_dev, (unsigned int*)(step_dev + 1));
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
@@ -819,9 +828,9 @@ int fgl_split_tf32(const float* x, int64_t rows, int64_t cols, int64_t ldx, int 
     if (rows == 0 || cols == 0) return FGL_OK;
     const int64_t items = rows * (vec ? cols / 4 : cols);
     if (vec)
-        split_tf32_kernel<true><<<ew_grid(items), kEwThreads, 0, (cudaStream_t)stream>>>(x, rows, (int)cols, ldx, d);
+        launch(split_tf32_kernel<true>, ew_grid(items), kEwThreads, 0, (cudaStream_t)stream, x, rows, (int)cols, ldx, d);
     else
-        split_tf32_kernel<false><<<ew_grid(items), kEwThreads, 0, (cudaStream_t)stream>>>(x, rows, (int)cols, ldx, d);
+        launch(split_tf32_kernel<false>, ew_grid(items), kEwThreads, 0, (cudaStream_t)stream, x, rows, (int)cols, ldx, d);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
@@ -839,7 +848,7 @@ int fgl_split_tf32_many(const fgl_split_job* jobs, int32_t n_jobs, void* stream)
         most = std::max(most, m.rows[j] * (m.vec[j] ? w.cols / 4 : w.cols));
     }
     if (most == 0) return FGL_OK;
-    split_tf32_many_kernel<<<dim3(ew_grid(most), n_jobs), kEwThreads, 0, (cudaStream_t)stream>>>(m);
+    launch(split_tf32_many_kernel, dim3(ew_grid(most), n_jobs), kEwThreads, 0, (cudaStream_t)stream, m);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
@@ -854,10 +863,10 @@ int fgl_fold_blocks(const float* part, int32_t n_slabs, int32_t n_a, int32_t n_b
     const int64_t groups = (int64_t)rows * (vec ? (cols + 127) / 128 : (cols + 31) / 32);
     const unsigned grid = (unsigned)std::min<int64_t>(groups, 148 * 16);
     if (vec)
-        fold_blocks_kernel<4><<<grid, kFoldWarps * 32, 0, (cudaStream_t)stream>>>(part, n_slabs, n_a, n_b, rows, cols, block_stride, ld_part,
+        launch(fold_blocks_kernel<4>, grid, kFoldWarps * 32, 0, (cudaStream_t)stream, part, n_slabs, n_a, n_b, rows, cols, block_stride, ld_part,
                                                                                  slab_stride, out, ldo);
     else
-        fold_blocks_kernel<1><<<grid, kFoldWarps * 32, 0, (cudaStream_t)stream>>>(part, n_slabs, n_a, n_b, rows, cols, block_stride, ld_part,
+        launch(fold_blocks_kernel<1>, grid, kFoldWarps * 32, 0, (cudaStream_t)stream, part, n_slabs, n_a, n_b, rows, cols, block_stride, ld_part,
                                                                                  slab_stride, out, ldo);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
