@@ -679,16 +679,17 @@ def main():
         steps_per_epoch = tr.steps_per_epoch()
         # kernels of this library: per window one fused sampling launch and one first-layer aggregation launch; per
         # step one staging launch and, inside the replayed step program, per inner layer one forward aggregation, one
-        # self-gradient initialisation and one backward scatter, per hidden layer one bias/ReLU/dropout epilogue and
-        # one backward of it, two launches for the output layer with its loss, and one Adam launch (5 L - 1).  The
-        # op-by-op path (--no-graph) launches one forward and one backward aggregation per inner layer.
+        # bias/ReLU/dropout epilogue, one backward scatter and one ReLU/dropout backward, one launch for the output layer
+        # with its loss and one Adam launch (4 L - 1).  The op-by-op path (--no-graph) launches one forward and one
+        # backward aggregation per inner layer.
         n_windows = (args.steps + args.window - 1) // args.window
         n_layers = len(cfg["fanouts"])
-        per_step = (5 * n_layers - 1) if tr.graphed is not None else 2 * (n_layers - 1)
+        per_step = (4 * n_layers - 1) if tr.graphed is not None else 2 * (n_layers - 1)
         if tr.graphed is not None and args.matmul == "3xtf32":
-            # operand splits (n_layers weights, n_layers layer inputs -- the first one while staging --, the output
-            # layer's gradient) and n_layers folds of the weight-gradient blocks
-            per_step += 3 * n_layers + 1
+            # one split of the input layer's rows, one of all weights, n_layers folds of the weight-gradient blocks
+            per_step += 2 + n_layers
+        if tr.graphed is not None and args.matmul == "fp32":
+            per_step += 2 * n_layers      # weight gradients: the products and their folds
         launches = args.steps * per_step + 2 * n_windows
         epoch_s = steps_per_epoch * ms / args.steps * 1e-3
         line = {"metric": "sampled_edges_per_s", "value": value, "unit": "edges/s", "n_gpus": world, "steps": args.steps,

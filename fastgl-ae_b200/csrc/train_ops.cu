@@ -30,8 +30,9 @@ bias_relu_dropout_kernel(float* __restrict__ y, int64_t ld, int64_t n_rows, int 
                          uint32_t drop_below, float keep_scale, uint64_t rng_seed, uint64_t rng_ctr,
                          const int32_t* __restrict__ rng_ctr_dev, int flags, float* __restrict__ copy_out,
                          int64_t ld_copy, int64_t n_copy_rows, float* __restrict__ split, int64_t ld_split,
-                         int64_t split_stride) {
+                         int64_t split_stride, const int32_t* __restrict__ n_rows_dev) {
     if (!after_the_kernels_before()) return;
+    if (n_rows_dev) n_rows = min((int64_t)max(__ldg(n_rows_dev), 0), n_rows);   // the padding rows are left alone
     const int64_t groups_per_row = dim / VEC;
     const int64_t total = n_rows * groups_per_row;
     const uint64_t ctr = rng_ctr + (rng_ctr_dev ? (uint64_t)(uint32_t)rng_ctr_dev[0] : 0ull);
@@ -95,18 +96,19 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(kEwThreads)
 relu_dropout_bwd_kernel(float* __restrict__ dy, int64_t ldy, const float* __restrict__ out, int64_t ldo, int64_t n_rows,
                         int rows_per_cta, int dim, float keep_scale, float* __restrict__ dbias, int flags,
-                        float* __restrict__ split3, int64_t ld3, int block_stride) {
+                        float* __restrict__ split3, int64_t ld3, int block_stride, const int32_t* __restrict__ n_rows_dev) {
     if (!after_the_kernels_before()) return;
     const int64_t r0 = (int64_t)blockIdx.x * rows_per_cta;
     const int64_t r1 = r0 + rows_per_cta < n_rows ? r0 + rows_per_cta : n_rows;
     const bool mask = flags & FGL_EW_RELU;
+    const int64_t real = n_rows_dev ? (int64_t)__ldg(n_rows_dev) : n_rows;   // the rows from there on become zero, unread
     for (int c = threadIdx.x; c < dim; c += kEwThreads) {
         float acc = 0.f;
         for (int64_t r = r0; r < r1; r += kBwdRowBatch) {
             float g[kBwdRowBatch], o[kBwdRowBatch];
 #pragma unroll
             for (int k = 0; k < kBwdRowBatch; ++k) {
-                const bool in = r + k < r1;
+                const bool in = r + k < r1 && r + k < real;
                 g[k] = in ? dy[(r + k) * ldy + c] : 0.f;
                 o[k] = (in && mask) ? out[(r + k) * ldo + c] : 1.f;
             }
@@ -121,7 +123,7 @@ relu_dropout_bwd_kernel(float* __restrict__ dy, int64_t ldy, const float* __rest
                         d3[block_stride] = l;
                         if (!(flags & FGL_EW_TWO_BLOCKS)) d3[2 * block_stride] = h;
                     }
-                } else if (mask) {
+                } else if (mask || n_rows_dev) {
                     if (r + k < r1) dy[(r + k) * ldy + c] = g[k];
                 }
                 acc += g[k];
@@ -142,7 +144,7 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(kEwThreads)
 relu_dropout_bwd_vec_kernel(float* __restrict__ dy, int64_t ldy, const float* __restrict__ out, int64_t ldo, int64_t n_rows,
                             int rows_per_cta, int dim, float keep_scale, float* __restrict__ dbias, int flags,
-                            float* __restrict__ split3, int64_t ld3, int block_stride) {
+                            float* __restrict__ split3, int64_t ld3, int block_stride, const int32_t* __restrict__ n_rows_dev) {
     if (!after_the_kernels_before()) return;
     __shared__ float4 sums[kEwThreads];
     const int groups = dim >> 2;                       // column groups of four floats; <= 256
@@ -150,6 +152,7 @@ relu_dropout_bwd_vec_kernel(float* __restrict__ dy, int64_t ldy, const float* __
     const int cg = threadIdx.x % groups, rl = threadIdx.x / groups;
     const bool active = rl < lanes;
     const bool mask = flags & FGL_EW_RELU;
+    const int64_t real = n_rows_dev ? (int64_t)__ldg(n_rows_dev) : n_rows;   // the rows from there on become zero, unread
     constexpr int kPasses = 4;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int64_t r0 = (int64_t)blockIdx.x * rows_per_cta; active && r0 < n_rows; r0 += (int64_t)gridDim.x * rows_per_cta) {
@@ -159,7 +162,7 @@ relu_dropout_bwd_vec_kernel(float* __restrict__ dy, int64_t ldy, const float* __
 #pragma unroll
             for (int k = 0; k < kPasses; ++k) {
                 const int64_t rr = r + (int64_t)k * lanes;
-                const bool in = rr < r1;
+                const bool in = rr < r1 && rr < real;
                 g[k] = in ? *reinterpret_cast<const float4*>(dy + rr * ldy + 4 * cg) : make_float4(0.f, 0.f, 0.f, 0.f);
                 o[k] = (in && mask) ? *reinterpret_cast<const float4*>(out + rr * ldo + 4 * cg) : make_float4(1.f, 1.f, 1.f, 1.f);
             }
@@ -183,7 +186,7 @@ relu_dropout_bwd_vec_kernel(float* __restrict__ dy, int64_t ldy, const float* __
                         *reinterpret_cast<float4*>(d3) = h;
                         *reinterpret_cast<float4*>(d3 + block_stride) = l;
                         if (!(flags & FGL_EW_TWO_BLOCKS)) *reinterpret_cast<float4*>(d3 + 2 * block_stride) = h;
-                    } else if (mask) {
+                    } else if (mask || n_rows_dev) {
                         *reinterpret_cast<float4*>(dy + rr * ldy + 4 * cg) = g[k];
                     }
                 }
@@ -637,7 +640,7 @@ extern "C" {
 static int bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, const float* bias, float p_drop,
                              uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
                              int64_t ld_copy, int64_t n_copy_rows, float* split, int64_t ld_split, int64_t split_stride,
-                             void* stream) {
+                             const int32_t* n_rows_dev, void* stream) {
     if (n_rows < 0 || dim <= 0 || ld < dim || (n_rows > 0 && !y) || !(p_drop >= 0.f && p_drop < 1.f)) return FGL_ERR_INVALID;
     if (!copy_out && !split) n_copy_rows = 0;
     if (n_copy_rows < 0 || n_copy_rows > n_rows || (copy_out && n_copy_rows > 0 && ld_copy < dim)) return FGL_ERR_INVALID;
@@ -654,13 +657,13 @@ static int bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, 
     // whole 16-byte vectors alone: a caller with other rows splits them in a pass of its own
     if (split && !(vec && ld_split % 4 == 0 && split_stride % 4 == 0 && aligned16(split))) return FGL_ERR_INVALID;
     if (vec)
-        launch(bias_relu_dropout_kernel<4>, ew_grid(n_rows * (dim / 4)), kEwThreads, 0, st, 
+        launch(bias_relu_dropout_kernel<4>, ew_grid(n_rows * (dim / 4)), kEwThreads, 0, st,
             y, ld, n_rows, dim, bias, drop_below, keep_scale, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
-            n_copy_rows, split, ld_split, split_stride);
+            n_copy_rows, split, ld_split, split_stride, n_rows_dev);
     else
-        launch(bias_relu_dropout_kernel<1>, ew_grid(n_rows * dim), kEwThreads, 0, st, 
+        launch(bias_relu_dropout_kernel<1>, ew_grid(n_rows * dim), kEwThreads, 0, st,
             y, ld, n_rows, dim, bias, drop_below, keep_scale, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
-            n_copy_rows, nullptr, 0, 0);
+            n_copy_rows, nullptr, 0, 0, n_rows_dev);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
@@ -668,20 +671,20 @@ int fgl_bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, con
                           uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
                           int64_t ld_copy, int64_t n_copy_rows, void* stream) {
     return bias_relu_dropout(y, ld, n_rows, dim, bias, p_drop, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
-                             n_copy_rows, nullptr, 0, 0, stream);
+                             n_copy_rows, nullptr, 0, 0, nullptr, stream);
 }
 
 int fgl_bias_relu_dropout_split(float* y, int64_t ld, int64_t n_rows, int32_t dim, const float* bias, float p_drop,
                                 uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
                                 int64_t ld_copy, int64_t n_copy_rows, float* split, int64_t ld_split, int64_t split_stride,
-                                void* stream) {
-    if (!split) return FGL_ERR_INVALID;
+                                const int32_t* n_rows_dev, void* stream) {
     return bias_relu_dropout(y, ld, n_rows, dim, bias, p_drop, rng_seed, rng_ctr, rng_ctr_dev, flags, copy_out, ld_copy,
-                             n_copy_rows, split, ld_split, split_stride, stream);
+                             n_copy_rows, split, ld_split, split_stride, n_rows_dev, stream);
 }
 
 static int relu_dropout_bwd_launch(float* dy, int64_t ldy, const float* out, int64_t ldo, int64_t n_rows, int32_t dim, float p_drop,
-                                   float* dbias, int32_t flags, float* split3, int64_t ld3, int64_t block_stride, void* stream) {
+                                   float* dbias, int32_t flags, float* split3, int64_t ld3, int64_t block_stride,
+                                   const int32_t* n_rows_dev, void* stream) {
     if (n_rows < 0 || dim <= 0 || dim > kBwdMaxColsPerThread * kEwThreads || ldy < dim || (n_rows > 0 && !dy) ||
         !(p_drop >= 0.f && p_drop < 1.f))
         return FGL_ERR_INVALID;
@@ -706,25 +709,25 @@ static int relu_dropout_bwd_launch(float* dy, int64_t ldy, const float* out, int
         int64_t nb = (n_rows + band - 1) / band;
         nb = nb < 4 * 148 ? nb : 4 * 148;   // four CTAs per SM, each walking its share of the bands
         if (split3)
-            launch(relu_dropout_bwd_vec_kernel<true>, (unsigned)nb, kEwThreads, 0, (cudaStream_t)stream, 
-                dy, ldy, out, ldo, n_rows, (int)band, dim, keep, dbias, flags, split3, ld3, (int)block_stride);
+            launch(relu_dropout_bwd_vec_kernel<true>, (unsigned)nb, kEwThreads, 0, (cudaStream_t)stream,
+                dy, ldy, out, ldo, n_rows, (int)band, dim, keep, dbias, flags, split3, ld3, (int)block_stride, n_rows_dev);
         else
-            launch(relu_dropout_bwd_vec_kernel<false>, (unsigned)nb, kEwThreads, 0, (cudaStream_t)stream, 
-                dy, ldy, out, ldo, n_rows, (int)band, dim, keep, dbias, flags, nullptr, 0, 0);
+            launch(relu_dropout_bwd_vec_kernel<false>, (unsigned)nb, kEwThreads, 0, (cudaStream_t)stream,
+                dy, ldy, out, ldo, n_rows, (int)band, dim, keep, dbias, flags, nullptr, 0, 0, n_rows_dev);
         return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
     }
     if (split3)
-        launch(relu_dropout_bwd_kernel<true>, (unsigned)blocks, kEwThreads, 0, (cudaStream_t)stream, 
-            dy, ldy, out, ldo, n_rows, (int)rows_per_cta, dim, keep, dbias, flags, split3, ld3, (int)block_stride);
+        launch(relu_dropout_bwd_kernel<true>, (unsigned)blocks, kEwThreads, 0, (cudaStream_t)stream,
+            dy, ldy, out, ldo, n_rows, (int)rows_per_cta, dim, keep, dbias, flags, split3, ld3, (int)block_stride, n_rows_dev);
     else
-        launch(relu_dropout_bwd_kernel<false>, (unsigned)blocks, kEwThreads, 0, (cudaStream_t)stream, 
-            dy, ldy, out, ldo, n_rows, (int)rows_per_cta, dim, keep, dbias, flags, nullptr, 0, 0);
+        launch(relu_dropout_bwd_kernel<false>, (unsigned)blocks, kEwThreads, 0, (cudaStream_t)stream,
+            dy, ldy, out, ldo, n_rows, (int)rows_per_cta, dim, keep, dbias, flags, nullptr, 0, 0, n_rows_dev);
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }
 
 int fgl_relu_dropout_bwd(float* dy, int64_t ldy, const float* out, int64_t ldo, int64_t n_rows, int32_t dim, float p_drop,
                          float* dbias, int32_t flags, void* stream) {
-    return relu_dropout_bwd_launch(dy, ldy, out, ldo, n_rows, dim, p_drop, dbias, flags, nullptr, 0, 0, stream);
+    return relu_dropout_bwd_launch(dy, ldy, out, ldo, n_rows, dim, p_drop, dbias, flags, nullptr, 0, 0, nullptr, stream);
 }
 
 int fgl_relu_dropout_bwd_split(const float* dy, int64_t ldy, const float* out, int64_t ldo, int64_t n_rows, int32_t dim,
@@ -732,7 +735,13 @@ int fgl_relu_dropout_bwd_split(const float* dy, int64_t ldy, const float* out, i
                                void* stream) {
     if (!split3) return FGL_ERR_INVALID;
     return relu_dropout_bwd_launch(const_cast<float*>(dy), ldy, out, ldo, n_rows, dim, p_drop, dbias, flags, split3, ld3,
-                                   block_stride, stream);
+                                   block_stride, nullptr, stream);
+}
+
+int fgl_relu_dropout_bwd_rows(float* dy, int64_t ldy, const float* out, int64_t ldo, int64_t n_rows, const int32_t* n_rows_dev,
+                              int32_t dim, float p_drop, float* dbias, int32_t flags, float* split3, int64_t ld3,
+                              int64_t block_stride, void* stream) {
+    return relu_dropout_bwd_launch(dy, ldy, out, ldo, n_rows, dim, p_drop, dbias, flags, split3, ld3, block_stride, n_rows_dev, stream);
 }
 
 int fgl_softmax_xent(fgl_ws* ws, const float* logits, int64_t ld, const int64_t* labels, const int32_t* label_ids,
@@ -745,7 +754,7 @@ int fgl_softmax_xent(fgl_ws* ws, const float* logits, int64_t ld, const int64_t*
         return cudaMemsetAsync(loss, 0, sizeof(float), (cudaStream_t)stream) == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    launch(softmax_xent_rows_kernel, (n_rows + kXentWarps - 1) / kXentWarps, kXentWarps * 32, 0, st, 
+    launch(softmax_xent_rows_kernel, (n_rows + kXentWarps - 1) / kXentWarps, kXentWarps * 32, 0, st,
         logits, ld, labels, label_ids, n_labels, n_rows, n_classes, n_valid_dev, n_valid, row_loss, dlogits, ldd, ws->status,
         loss, loss_ticket(ws));
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
@@ -799,7 +808,7 @@ int fgl_adam_step(float* param, const float* grad, float* exp_avg, float* exp_av
     if (n == 0) return FGL_OK;
     if (!aligned16(param) || !aligned16(grad) || !aligned16(exp_avg) || !aligned16(exp_avg_sq)) return FGL_ERR_INVALID;
     // step_dev[0] = completed steps, step_dev[1] = the kernel's arrival ticket (zero between launches)
-    launch(adam_kernel, ew_grid((n + 3) / 4), kEwThreads, 0, (cudaStream_t)stream, 
+    launch(adam_kernel, ew_grid((n + 3) / 4), kEwThreads, 0, (cudaStream_t)stream,
         param, grad, exp_avg, exp_avg_sq, n, lr, beta1, beta2, eps, weight_decay, step_dev, (unsigned int*)(step_dev + 1));
     return cudaGetLastError() == cudaSuccess ? FGL_OK : FGL_ERR_CUDA;
 }

@@ -472,11 +472,12 @@ def aggregate_split(edge_ptr, src_edges, input_feat, dst_nodes, split, split_str
 # element-wise kernels of the training step (no counterpart among the reference's operators)
 # ------------------------------------------------------------------------------------------------
 def bias_relu_dropout_(y, bias=None, p_drop=0.0, relu=True, rng_seed=None, rng_ctr=0, rng_ctr_dev=None, copy_out=None,
-                       split=None, split_stride=None, blocks=3):
+                       split=None, split_stride=None, blocks=3, n_rows_dev=None):
     """In place: y = dropout(relu(y + bias)).  ``rng_ctr_dev`` (int32 CUDA tensor) is added to ``rng_ctr`` on the
     device, so a captured launch draws a new mask per replay.  ``copy_out`` (float32[k, dim], k <= rows, may be a
     column slice) also receives the first k result rows; so does ``split`` (k rows) as ``[hi | lo | hi]`` TF32 parts (the
-    first ``blocks`` of the three) ``split_stride`` columns apart, for rows of whole 16-byte vectors.  Returns ``y``."""
+    first ``blocks`` of the three) ``split_stride`` columns apart, for rows of whole 16-byte vectors.  ``n_rows_dev`` (int32 CUDA tensor): the number of
+    rows that count; the others are left alone.  Returns ``y``."""
     _check_rows_f32(y, "y")
     if copy_out is not None:
         _check_rows_f32(copy_out, "copy_out")
@@ -487,18 +488,21 @@ def bias_relu_dropout_(y, bias=None, p_drop=0.0, relu=True, rng_seed=None, rng_c
         if bias.numel() != y.size(1):
             raise RuntimeError("bias must have one entry per column")
     dev = y.device
+    if split is not None or n_rows_dev is not None:
+        rows = 0 if copy_out is None else copy_out.size(0)
     if split is not None:
         _check_rows_f32(split, "split")
-        rows = split.size(0) if copy_out is None else copy_out.size(0)
+        rows = split.size(0) if copy_out is None else rows
         if rows > y.size(0) or split.size(0) != rows or split.size(1) < (blocks - 1) * split_stride + y.size(1) or blocks not in (2, 3):
             raise RuntimeError("split must have copy_out's rows and room for its blocks split_stride columns apart")
+    if split is not None or n_rows_dev is not None:
         with _on_device(dev):
             rc = lib().fgl_bias_relu_dropout_split(
                 _ptr(y), ctypes.c_int64(y.stride(0)), ctypes.c_int64(y.size(0)), ctypes.c_int32(y.size(1)), _ptr(bias),
                 ctypes.c_float(p_drop), ctypes.c_uint64(_config["rng_seed"] if rng_seed is None else rng_seed), ctypes.c_uint64(rng_ctr),
                 _ptr(rng_ctr_dev), ctypes.c_int32((1 if relu else 0) | (_capi.EW_TWO_BLOCKS if blocks == 2 else 0)), _ptr(copy_out),
                 ctypes.c_int64(copy_out.stride(0) if copy_out is not None else 0), ctypes.c_int64(rows), _ptr(split),
-                ctypes.c_int64(split.stride(0)), ctypes.c_int64(split_stride), _stream(dev))
+                ctypes.c_int64(0 if split is None else split.stride(0)), ctypes.c_int64(split_stride or 0), _ptr(n_rows_dev), _stream(dev))
         _raise(rc, "bias_relu_dropout_")
         return y
     with _on_device(dev):
@@ -512,11 +516,13 @@ def bias_relu_dropout_(y, bias=None, p_drop=0.0, relu=True, rng_seed=None, rng_c
     return y
 
 
-def relu_dropout_backward_(dy, out=None, p_drop=0.0, dbias=None, masked=True, split3=None, block_stride=None, blocks=3):
+def relu_dropout_backward_(dy, out=None, p_drop=0.0, dbias=None, masked=True, split3=None, block_stride=None, blocks=3,
+                           n_rows_dev=None):
     """In place over ``dy``: the gradient through dropout(relu(.)) given the forward output ``out`` (``masked``), and
     ``dbias += column sums`` of the result.  Returns ``dy``.  With ``split3`` (a float32 matrix of ``dy``'s rows) the
     result is written there instead, as ``[hi | lo | hi]`` TF32 parts ``block_stride`` (default: ``dy``'s width) columns
-    apart (the first ``blocks`` of the three: 2 or 3), and ``dy`` is left as it was; returns ``split3``."""
+    apart (the first ``blocks`` of the three: 2 or 3), and ``dy`` is left as it was; returns ``split3``.
+    ``n_rows_dev`` (int32 CUDA tensor): the number of rows that count; the others are not read and become zero."""
     _check_rows_f32(dy, "dy")
     if masked:
         _check_rows_f32(out, "out")
@@ -534,6 +540,17 @@ def relu_dropout_backward_(dy, out=None, p_drop=0.0, dbias=None, masked=True, sp
             raise RuntimeError("split3 must have dy's rows and room for three blocks block_stride columns apart")
         if blocks not in (2, 3):
             raise RuntimeError("blocks must be 2 or 3")
+    if n_rows_dev is not None:
+        with _on_device(dev):
+            rc = lib().fgl_relu_dropout_bwd_rows(_ptr(dy), ctypes.c_int64(dy.stride(0)), _ptr(out if masked else None),
+                                                 ctypes.c_int64(out.stride(0) if masked else dy.size(1)), ctypes.c_int64(dy.size(0)),
+                                                 _ptr(n_rows_dev), ctypes.c_int32(dy.size(1)), ctypes.c_float(p_drop), _ptr(dbias),
+                                                 ctypes.c_int32((1 if masked else 0) | (_capi.EW_TWO_BLOCKS if blocks == 2 else 0)),
+                                                 _ptr(split3), ctypes.c_int64(0 if split3 is None else split3.stride(0)),
+                                                 ctypes.c_int64(0 if split3 is None else bs), _stream(dev))
+        _raise(rc, "relu_dropout_backward_")
+        return dy if split3 is None else split3
+    if split3 is not None:
         with _on_device(dev):
             rc = lib().fgl_relu_dropout_bwd_split(_ptr(dy), ctypes.c_int64(dy.stride(0)), _ptr(out if masked else None),
                                                   ctypes.c_int64(out.stride(0) if masked else dy.size(1)), ctypes.c_int64(dy.size(0)),

@@ -154,7 +154,8 @@ class SageStepProgram:
                 blk = self.blocks[i + 1]
                 d = self.layers[i + 1].input_dim
                 nxt = self.cat[i + 1]
-                drop = dict(relu=True, rng_seed=self.rng_seed, rng_ctr=(i + 1) << 40, rng_ctr_dev=self.step_word)
+                drop = dict(relu=True, rng_seed=self.rng_seed, rng_ctr=(i + 1) << 40, rng_ctr_dev=self.step_word,
+                            n_rows_dev=self.sizes[i: i + 1])
                 if split and d % 4 == 0:
                     # straight into the operand form of the next layer's products; the plain rows only for the fused output
                     # layer, which reads them (and whose weight gradient reads two of the three blocks)
@@ -210,11 +211,12 @@ class SageStepProgram:
                     fastgl.relu_dropout_backward_(self.dh[i], out=self.z[i - 1], p_drop=p if training else 0.0,
                                                   dbias=self.layers[i - 1].bias.grad, split3=self.g3[i - 1],
                                                   block_stride=self.mp[i - 1],
+                                                  n_rows_dev=self.sizes[i - 1: i],
                                                   blocks=3 if i > 1 else 2)      # the third block is for the input gradient
                     dz = None
                 else:
                     dz = fastgl.relu_dropout_backward_(self.dh[i], out=self.z[i - 1], p_drop=p if training else 0.0,
-                                                       dbias=self.layers[i - 1].bias.grad)
+                                                       dbias=self.layers[i - 1].bias.grad, n_rows_dev=self.sizes[i - 1: i])
         if self.overlap:
             torch.cuda.current_stream().wait_stream(self.side)      # the optimizer step that follows needs every gradient
         return self.loss

@@ -411,12 +411,13 @@ int fgl_bias_relu_dropout(float* y, int64_t ld, int64_t n_rows, int32_t dim, con
                           int64_t ld_copy, int64_t n_copy_rows, void* stream);
 
 /* fgl_bias_relu_dropout that also writes the first n_copy_rows result rows as error-compensated TF32 operands (see
- * fgl_split_tf32), [hi | lo | hi] split_stride columns apart (with FGL_EW_TWO_BLOCKS [hi | lo]).  copy_out may be NULL.
- * Rows of whole 16-byte vectors only (FGL_ERR_INVALID otherwise). */
+ * fgl_split_tf32), [hi | lo | hi] split_stride columns apart (with FGL_EW_TWO_BLOCKS [hi | lo]).  copy_out and split may be
+ * NULL; with split, rows of whole 16-byte vectors only (FGL_ERR_INVALID otherwise).  n_rows_dev (may be NULL): the real row count
+ * of a padded launch; the rows from there on are neither changed nor copied. */
 int fgl_bias_relu_dropout_split(float* y, int64_t ld, int64_t n_rows, int32_t dim, const float* bias, float p_drop,
                                 uint64_t rng_seed, uint64_t rng_ctr, const int32_t* rng_ctr_dev, int32_t flags, float* copy_out,
                                 int64_t ld_copy, int64_t n_copy_rows, float* split, int64_t ld_split, int64_t split_stride,
-                                void* stream);
+                                const int32_t* n_rows_dev, void* stream);
 
 /* Backward of fgl_bias_relu_dropout: with FGL_EW_RELU, dy[r, c] becomes dy[r, c] / (1 - p_drop) where the
  * forward output out[r, c] is positive and 0 elsewhere (an element is positive exactly when it passed both the
@@ -431,6 +432,12 @@ int fgl_relu_dropout_bwd(float* dy, int64_t ldy, const float* out, int64_t ldo, 
 int fgl_relu_dropout_bwd_split(const float* dy, int64_t ldy, const float* out, int64_t ldo, int64_t n_rows, int32_t dim,
                                float p_drop, float* dbias, int32_t flags, float* split3, int64_t ld3, int64_t block_stride,
                                void* stream);
+
+/* fgl_relu_dropout_bwd (split3 NULL) or fgl_relu_dropout_bwd_split of a padded launch: the rows from n_rows_dev[0] on are not
+ * read, and their result is zero. */
+int fgl_relu_dropout_bwd_rows(float* dy, int64_t ldy, const float* out, int64_t ldo, int64_t n_rows, const int32_t* n_rows_dev,
+                              int32_t dim, float p_drop, float* dbias, int32_t flags, float* split3, int64_t ld3,
+                              int64_t block_stride, void* stream);
 
 /* Mean softmax cross-entropy over the first n_valid rows and its gradient.  The label of row r is
  * labels[label_ids ? label_ids[r] : r] (labels: int64[n_labels], values in [0, n_classes); an index or a label

@@ -103,3 +103,25 @@ def test_scatter_that_adds(fastgl, mode, dim, offset):
         # t additions in any order, and the rounding of the weighted row: (t + 2) half-ulps of the sum of magnitudes
         bound = (terms[:, None] + 2) * 2.0 ** -24 * size
         assert bool(((got.double().cpu() - want).abs() <= bound).all())
+
+
+# a padded launch: the rows from the real count on are left alone (forward) or become zero unread (backward)
+@pytest.mark.parametrize("dim", [47, 256])       # scalar and vector kernels
+@pytest.mark.parametrize("real", [0, 1, 37, 50])
+def test_padding_rows_of_the_relu(fastgl, dim, real):
+    rows = 50
+    n = torch.tensor([real], dtype=torch.int32, device="cuda")
+    y, dy = torch.randn(rows, dim, device="cuda"), torch.randn(rows, dim, device="cuda")
+    want = fastgl.bias_relu_dropout_(y.clone(), None, 0.5, rng_ctr=5)
+    copy = torch.full_like(y, 7.0)
+    got = fastgl.bias_relu_dropout_(y.clone(), None, 0.5, rng_ctr=5, n_rows_dev=n, copy_out=copy)
+    assert torch.equal(got[:real], want[:real]) and torch.equal(got[real:], y[real:])
+    assert torch.equal(copy[:real], want[:real]) and bool((copy[real:] == 7.0).all())
+    bias, bias0 = torch.zeros(dim, device="cuda"), torch.zeros(dim, device="cuda")
+    ref = fastgl.relu_dropout_backward_(dy[:real].clone(), out=want[:real], p_drop=0.5, dbias=bias0) if real else dy[:0]
+    poisoned, out = dy.clone(), want.clone()
+    poisoned[real:] = out[real:] = float("nan")
+    back = fastgl.relu_dropout_backward_(poisoned, out=out, p_drop=0.5, dbias=bias, n_rows_dev=n)
+    assert torch.equal(back[:real], ref) and not bool(back[real:].any())
+    # at most 50 terms, added in another order: 51 half-ulps of the sum of magnitudes
+    assert bool(((bias - bias0).abs() <= 51 * 2.0 ** -24 * 2 * ref.abs().sum(0)).all())
