@@ -796,6 +796,7 @@ std::pair<at::Tensor, at::Tensor> step_loss(const Call& c, const at::Tensor& log
 at::Tensor gcn_step(const at::Tensor& table, const at::Tensor& nodes, const std::vector<at::Tensor>& indptr, const std::vector<at::Tensor>& src,
                     int64_t batch, const std::vector<int64_t>& counts, const std::vector<at::Tensor>& weights,
                     const std::vector<at::Tensor>& grads, const std::vector<bool>& aggregate_first, double p_drop, const at::Tensor& labels) {
+    at::AutoDispatchBelowADInplaceOrView no_autograd;
     Call c(table);
     const StepBatch s = step_batch(nodes, indptr, src, batch, counts);
     const int L = (int)s.blocks.size();
@@ -845,6 +846,7 @@ at::Tensor gcn_step(const at::Tensor& table, const at::Tensor& nodes, const std:
 at::Tensor gin_step(const at::Tensor& table, const at::Tensor& nodes, const std::vector<at::Tensor>& indptr, const std::vector<at::Tensor>& src,
                     int64_t batch, const std::vector<int64_t>& counts, const std::vector<at::Tensor>& weights,
                     const std::vector<at::Tensor>& grads, double p_drop, const at::Tensor& labels) {
+    at::AutoDispatchBelowADInplaceOrView no_autograd;
     Call c(table);
     const StepBatch s = step_batch(nodes, indptr, src, batch, counts);
     const int L = (int)s.blocks.size();
@@ -871,11 +873,12 @@ at::Tensor gat_step(const at::Tensor& table, const at::Tensor& nodes, const std:
                     int64_t batch, const std::vector<int64_t>& counts, const std::vector<at::Tensor>& params,
                     const std::vector<at::Tensor>& grads, const std::vector<int64_t>& heads, const std::vector<double>& slope,
                     const std::vector<bool>& attention_grad, const at::Tensor& labels) {
+    at::AutoDispatchBelowADInplaceOrView no_autograd;
     Call c(table);
     const StepBatch s = step_batch(nodes, indptr, src, batch, counts);
     const int L = (int)s.blocks.size();
     const auto opt = table.options();
-    std::vector<at::Tensor> x(L), feat(L), alpha(L), el(L), er(L);
+    std::vector<at::Tensor> x(L), feat(L), scores(L);   // scores: alpha [edges][heads], el [n_src][heads], er [n_dst][heads]
     at::Tensor h = at::empty({s.blocks[0].n_src, table.size(1)}, opt);
     check(api.fgl_gather_rows(c.ws, ptr<float>(table), nullptr, 0, table.size(0), table.stride(0), (int32_t)table.size(1), s.nodes,
                               s.blocks[0].n_src, ptr<float>(h), h.stride(0), c.st()), "gather_rows");
@@ -886,12 +889,11 @@ at::Tensor gat_step(const at::Tensor& table, const at::Tensor& nodes, const std:
         x[i] = h;
         feat[i] = at::mm(h, w.t());
         h = at::empty({b.n_dst, dim}, opt);
-        alpha[i] = at::empty({b.n_edges, heads[i]}, opt);
-        el[i] = at::empty({b.n_src, heads[i]}, opt);
-        er[i] = at::empty({b.n_dst, heads[i]}, opt);
+        scores[i] = at::empty({(b.n_edges + b.n_src + b.n_dst) * heads[i]}, opt);
+        float* alpha = ptr<float>(scores[i]);
         check(api.fgl_gat_fwd(c.ws, b.indptr, b.src, ptr<float>(feat[i]), dim, ptr<float>(l), ptr<float>(r), (int32_t)heads[i],
-                              (int32_t)(dim / heads[i]), b.n_dst, b.n_src, (float)slope[i], ptr<float>(el[i]), ptr<float>(er[i]),
-                              ptr<float>(alpha[i]), ptr<float>(h), dim, c.st()), "gat_attention");
+                              (int32_t)(dim / heads[i]), b.n_dst, b.n_src, (float)slope[i], alpha + b.n_edges * heads[i],
+                              alpha + (b.n_edges + b.n_src) * heads[i], alpha, ptr<float>(h), dim, c.st()), "gat_attention");
     }
     auto [loss, d] = step_loss(c, h, labels, s);
     for (int i = L - 1; i >= 0; --i) {
@@ -899,19 +901,25 @@ at::Tensor gat_step(const at::Tensor& table, const at::Tensor& nodes, const std:
         const at::Tensor &w = params[3 * i], &l = params[3 * i + 1], &r = params[3 * i + 2];
         const int64_t dim = w.size(0);
         at::Tensor dfeat = at::empty({b.n_src, dim}, opt);
+        float* alpha = ptr<float>(scores[i]);
         if (attention_grad[i]) {
             const int rows = api.fgl_gat_bwd_partials(c.ws, (int32_t)heads[i], (int32_t)(dim / heads[i]), b.n_dst);
             at::Tensor scratch = at::empty({(int64_t)rows * 2 * dim + (b.n_edges + b.n_dst) * heads[i]}, opt);
-            at::Tensor dattn = at::empty({2, dim}, opt);
-            check(api.fgl_gat_bwd(c.ws, b.indptr, b.src, ptr<float>(feat[i]), dim, ptr<float>(l), ptr<float>(r), ptr<float>(el[i]),
-                                  ptr<float>(er[i]), ptr<float>(alpha[i]), ptr<float>(d), d.stride(0), (int32_t)heads[i],
+            // both vectors' gradients in one piece, if the flat gradient holds them so
+            const bool in_place = ptr<float>(grads[3 * i + 2]) == ptr<float>(grads[3 * i + 1]) + dim;
+            at::Tensor dattn = in_place ? grads[3 * i + 1] : at::empty({2, dim}, opt);
+            check(api.fgl_gat_bwd(c.ws, b.indptr, b.src, ptr<float>(feat[i]), dim, ptr<float>(l), ptr<float>(r),
+                                  alpha + b.n_edges * heads[i], alpha + (b.n_edges + b.n_src) * heads[i], alpha, ptr<float>(d),
+                                  d.stride(0), (int32_t)heads[i],
                                   (int32_t)(dim / heads[i]), b.n_dst, b.n_src, b.n_edges, (float)slope[i], ptr<float>(scratch),
                                   ptr<float>(dfeat), ptr<float>(dattn), c.st()), "gat_attention_backward");
-            fgl_segment seg[2] = {{ptr<float>(grads[3 * i + 1]), ptr<float>(dattn), dim * 4},
-                                  {ptr<float>(grads[3 * i + 2]), ptr<float>(dattn) + dim, dim * 4}};
-            check(api.fgl_stage_segments(seg, 2, nullptr, nullptr, 0, c.st()), "gat_attention_backward");
+            if (!in_place) {
+                fgl_segment seg[2] = {{ptr<float>(grads[3 * i + 1]), ptr<float>(dattn), dim * 4},
+                                      {ptr<float>(grads[3 * i + 2]), ptr<float>(dattn) + dim, dim * 4}};
+                check(api.fgl_stage_segments(seg, 2, nullptr, nullptr, 0, c.st()), "gat_attention_backward");
+            }
         } else {
-            check(api.fgl_agg_edge_bwd(c.ws, b.indptr, b.src, ptr<float>(alpha[i]), (int32_t)heads[i], ptr<float>(d), d.stride(0),
+            check(api.fgl_agg_edge_bwd(c.ws, b.indptr, b.src, alpha, (int32_t)heads[i], ptr<float>(d), d.stride(0),
                                        (int32_t)dim, b.n_dst, b.n_src, ptr<float>(dfeat), dim, c.st()), "backward_gat");
         }
         at::Tensor g = grads[3 * i];

@@ -17,7 +17,16 @@ def _plain(module) -> bool:
     """No hooks anywhere that an explicit sequence of launches would pass by."""
     if torch.nn.modules.module._global_forward_hooks or torch.nn.modules.module._global_forward_pre_hooks:
         return False
-    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in module.modules())
+    return _no_hooks(module)
+
+
+def _no_hooks(m) -> bool:
+    if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks:
+        return False
+    for child in m._modules.values():
+        if child is not None and not _no_hooks(child):
+            return False
+    return True
 
 
 def plan(trainer):
